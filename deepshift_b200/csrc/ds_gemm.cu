@@ -565,6 +565,8 @@ int launch_conv(const GemmParams& p, bool fp, cudaStream_t st)
     return rc;
 }
 
+}  // namespace
+
 int setup_common(GemmParams& p, int bits, int base, const ds_fuse_t* fuse, bool& use_fp)
 {
     if (bits < 1 || bits > 7) return DS_ERR_UNSUPPORTED;  // the reference's range, shift.cu:194-385
@@ -650,6 +652,8 @@ int setup_common(GemmParams& p, int bits, int base, const ds_fuse_t* fuse, bool&
     }
     return DS_OK;
 }
+
+namespace {
 
 // Sets *flag to 1 if any |x| exceeds `limit` (the flag was zeroed before).  One pass, 16-byte loads
 // for the aligned bulk.
@@ -842,6 +846,45 @@ int conv2d_run(const void* x, const int32_t* packed, const int32_t* bias, void* 
 }
 
 }  // namespace
+
+long long check_shrink_x() { return g_check_shrink_x; }
+
+// The integer path behind a tensor-core launch: runs only if *gate == want.  A linear layer arrives as a
+// 1x1 convolution on 1x1 images; its arguments have passed the checks of the caller.
+int launch_gated_int(const void* x, const int32_t* packed, const int32_t* bias, void* out, int B, int C, int H, int W,
+                     int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits, int base, const ds_fuse_t* fuse,
+                     const int* gate, int want, cudaStream_t st)
+{
+    const int OH = (H + 2 * ph - KH) / sh + 1, OW = (W + 2 * pw - KW) / sw + 1;
+    GemmParams p = {};
+    p.x = x; p.packed = packed; p.bias = bias; p.out = out;
+    p.M = B * OH * OW; p.K = C * KH * KW; p.N = OC;
+    p.C = C; p.H = H; p.W = W; p.OC = OC; p.KH = KH; p.KW = KW;
+    p.sh = sh; p.sw = sw; p.ph = ph; p.pw = pw; p.OH = OH; p.OW = OW; p.P = OH * OW;
+    ds_fuse_t f = *fuse;
+    f.act_bits = 0;
+    f.prepared = nullptr;
+    f.prepared_bytes = 0;
+    bool fp = false;
+    const int rc = setup_common(p, bits, base, &f, fp);
+    if (rc) return rc;
+    p.gate = gate;
+    p.gate_want = want;
+    set_check_extents(p, (long long)B * C * H * W);
+    if (H == 1 && W == 1 && KH == 1 && KW == 1 && ph == 0 && pw == 0) {
+        const long long tiles128 = ((long long)(p.M + 127) / 128) * ((p.N + 127) / 128);
+        if (p.M <= 64 || tiles128 * 2 < 148) {
+            const int r64 = launch_cfg<256, 8, 32, 4, 16, MODE_INT, AM_LINEAR>(p, st);
+            if (r64 != DS_ERR_UNSUPPORTED) return r64;
+        }
+        return launch_am<AM_LINEAR>(p, false, st);
+    }
+    p.magic_khw = magic_of(KH * KW);
+    p.magic_kw = magic_of(KW);
+    p.magic_kh = magic_of(KH);
+    return launch_conv(p, false, st);
+}
+
 }  // namespace ds
 
 extern "C" int ds_conv2d_ex(const void* x, const int32_t* packed, const int32_t* bias, void* out, int B,

@@ -1,0 +1,876 @@
+// Tensor-core shift GEMM / convolution (tcgen05, kind::i8).  The arithmetic is described in ds_tc.cuh.
+//
+// Three kernels per call:
+//   tc_pack_*     x (int32 or fp32, quantised here) -> two byte planes l and h, pixel-major with a physical
+//                 zero border.  One pass over x; from here on a filter tap is an address offset.
+//   tc_expand     packed weights -> s8 operand tiles in the order the MMA reads them, and const[n].  Once per
+//                 layer for callers that keep it.
+//   tc_run        the product.  Persistent, one CTA per SM, warp-specialised:
+//                   warps 0-     two or three producer warpgroups, thread = output row = TMEM lane.  A thread loads 16
+//                                values (16 bytes of l, 16 of h) and turns them into the sixteen planes with
+//                                byte-parallel shifts and masks: 132 instructions per 16 values, then two
+//                                32-column tcgen05.st.  The operand A never exists in shared memory.
+//                   next four    epilogue: tcgen05.ld, constants, residual / ReLU / rounding, store.
+//                   next         one thread issues the MMAs: 128 x BN x 32 bytes, A from TMEM, B from shared memory.
+//                   last         one thread fetches weight tiles with cp.async.bulk into a ring.
+//                 TMEM: a ring of BN-column accumulator slots, so that the epilogue of a tile overlaps the next tile's
+//                 MMAs, and one A slot per producer warpgroup (sixteen planes x 16 bytes x 128 rows).
+//
+// What bounds it: the s8 MMA rate, 16 byte-products per shift-accumulate (8192 per SM and clock: 144 T
+// shift-op/s at 1.9 GHz).  A from TMEM because shared memory could not carry both operands: at BN = 64 an
+// MMA of 32 cycles would read 4 KiB of A and 2 KiB of B, 192 bytes per cycle where 128 are available.
+#include "ds_tc.cuh"
+
+namespace ds {
+
+int* kernel_error_flag();
+
+namespace {
+
+constexpr int TC_TMEM_COLS = 512;
+
+// Per column width: WG producer warpgroups, each with an operand slot of its own (64 columns: sixteen planes x 16
+// bytes; a slot shared between warpgroups could not be guarded by a phase parity, since a warpgroup may be two
+// phases away from it), and as many accumulator slots as the remaining columns hold.  Two warpgroups keep up with the MMAs
+// of 128 columns (512 cycles per 128 rows x 16 values), three are needed for 64 (256 cycles).
+template <int BN>
+struct TcTile {
+    static constexpr int WG = BN == 128 ? 2 : 3;
+    static constexpr int THREADS = (4 * WG + 6) * 32;  // + 4 epilogue warps + MMA warp + loader warp
+    static constexpr int ACC_COLS = TC_TMEM_COLS - 64 * WG;
+    static constexpr int NACC = ACC_COLS / BN < 6 ? ACC_COLS / BN : 6;
+    static constexpr int STAGE = BN * TC_PLANES * TC_KG;
+    static constexpr int STAGES = BN == 128 ? 6 : 8;
+};
+
+template <int BN>
+struct TcSmem {
+    alignas(1024) unsigned char b[TcTile<BN>::STAGES][TcTile<BN>::STAGE];
+    alignas(8) unsigned long long bfull[TcTile<BN>::STAGES];
+    unsigned long long bempty[TcTile<BN>::STAGES];
+    unsigned long long afull[TcTile<BN>::WG];
+    unsigned long long aempty[TcTile<BN>::WG];
+    unsigned long long accfull[6];
+    unsigned long long accempty[6];
+    unsigned long long done;
+    unsigned tmem;
+    int err;
+    int last_flag;
+    alignas(16) int colc[2][128];
+};
+
+constexpr int TC_WAIT_LIMIT = 1 << 17;     // rounds of one wait before giving up (about half a second)
+constexpr unsigned TC_WAIT_NS = 1000000;   // suspend hint of one round
+
+__device__ __forceinline__ unsigned s32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void bar_init(unsigned long long* b, int count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(s32(b)), "r"(count) : "memory");
+}
+
+__device__ __forceinline__ void bar_arrive(unsigned long long* b)
+{
+    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(s32(b)) : "memory");
+}
+
+__device__ __forceinline__ bool bar_try(unsigned long long* b, unsigned parity)
+{
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(s32(b)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
+__device__ __forceinline__ bool bar_try_long(unsigned long long* b, unsigned parity)
+{
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(s32(b)), "r"(parity), "r"(TC_WAIT_NS)
+        : "memory");
+    return ok != 0;
+}
+
+// Bounded wait; whoever gives up sets the CTA's error word, and every wait that finds it set gives up too.
+// The first rounds carry no suspend hint: with one, a wait between warps of the main loop wakes up later
+// (7 % of the whole kernel).
+__device__ __forceinline__ bool bar_wait(unsigned long long* b, unsigned parity, volatile int* err)
+{
+    for (int i = 0; i < 32; ++i)
+        if (bar_try(b, parity)) return true;
+    for (int i = 0; i < TC_WAIT_LIMIT; ++i) {
+        if (bar_try_long(b, parity)) return true;
+        if (*err) return false;
+    }
+    *err = 1;
+    return false;
+}
+
+__device__ __forceinline__ void tc_commit(unsigned long long* b)
+{
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(b)) : "memory");
+}
+
+__device__ __forceinline__ void tc_mma_i8(unsigned d, unsigned a, unsigned long long bdesc, unsigned idesc, unsigned acc)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
+        "r"(a), "l"(bdesc), "r"(idesc), "r"(acc)
+        : "memory");
+}
+
+// True in one lane of the (converged) warp, always the same one.
+__device__ __forceinline__ bool elect_one()
+{
+    unsigned e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e)::"memory");
+    return e != 0;
+}
+
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+#define TC_R4(v, i) "r"(v[i]), "r"(v[i + 1]), "r"(v[i + 2]), "r"(v[i + 3])
+#define TC_W4(v, i) "=r"(v[i]), "=r"(v[i + 1]), "=r"(v[i + 2]), "=r"(v[i + 3])
+
+__device__ __forceinline__ void tmem_st32(unsigned addr, const unsigned (&v)[32])
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
+        "%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(addr),
+        TC_R4(v, 0), TC_R4(v, 4), TC_R4(v, 8), TC_R4(v, 12), TC_R4(v, 16), TC_R4(v, 20), TC_R4(v, 24), TC_R4(v, 28)
+        : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld32(unsigned addr, int (&v)[32])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
+        "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n\ttcgen05.wait::ld.sync.aligned;"
+        : TC_W4(v, 0), TC_W4(v, 4), TC_W4(v, 8), TC_W4(v, 12), TC_W4(v, 16), TC_W4(v, 20), TC_W4(v, 24), TC_W4(v, 28)
+        : "r"(addr)
+        : "memory");
+}
+
+// 16 bytes from an address aligned to `align` (16, 8 or 4).
+__device__ __forceinline__ uint4 ld16(const unsigned char* a, int align)
+{
+    if (align == 16) return __ldg(reinterpret_cast<const uint4*>(a));
+    uint4 v;
+    if (align == 8) {
+        const uint2 x = __ldg(reinterpret_cast<const uint2*>(a)), y = __ldg(reinterpret_cast<const uint2*>(a) + 1);
+        v = make_uint4(x.x, x.y, y.x, y.y);
+    } else {
+        const unsigned* w = reinterpret_cast<const unsigned*>(a);
+        v = make_uint4(__ldg(w), __ldg(w + 1), __ldg(w + 2), __ldg(w + 3));
+    }
+    return v;
+}
+
+// Planes 0-7 of four values (one byte each of l and h): word q of each plane.
+__device__ __forceinline__ void planes_low(unsigned l, unsigned h, unsigned (&v)[32], int q)
+{
+    const unsigned b7 = (l >> 7) & 0x01010101u, b15 = (h >> 7) & 0x01010101u;
+    v[q] = (l & 0x7F7F7F7Fu) + b7 + 2u * (h & 0x01010101u);  // <= 130: no carry between bytes
+    v[4 + q] = (l >> 1) & 0x3F3F3F3Fu;
+    v[8 + q] = (l >> 2) & 0x3F3F3F3Fu;
+    v[12 + q] = (l >> 3) & 0x1F1F1F1Fu;
+    v[16 + q] = (l >> 4) & 0x0F0F0F0Fu;
+    v[20 + q] = (l >> 5) & 0x07070707u;
+    v[24 + q] = (l >> 6) & 0x03030303u;
+    v[28 + q] = (h - b15) + b7;                               // 0..255: b15 set means h >= 128
+}
+
+__device__ __forceinline__ void planes_high(unsigned h, unsigned (&v)[32], int q)
+{
+    v[q] = h;
+    v[4 + q] = (h >> 1) & 0x7F7F7F7Fu;
+    v[8 + q] = (h >> 2) & 0x3F3F3F3Fu;
+    v[12 + q] = (h >> 3) & 0x1F1F1F1Fu;
+    v[16 + q] = (h >> 4) & 0x0F0F0F0Fu;
+    v[20 + q] = (h >> 5) & 0x07070707u;
+    v[24 + q] = (h >> 6) & 0x03030303u;
+    v[28 + q] = (h >> 7) & 0x01010101u;
+}
+
+struct Unit {
+    int tile, sp, m0, n0, nt, g0, g1;
+};
+
+template <int BN, int S>
+__device__ __forceinline__ Unit unit_of(const TcRun& p, int u)
+{
+    Unit r;
+    r.tile = u / p.splits;
+    r.sp = u - r.tile * p.splits;
+    int mt;
+    if (p.m_fast) {
+        r.nt = r.tile / p.grid_m;
+        mt = r.tile - r.nt * p.grid_m;
+    } else {
+        mt = r.tile / p.grid_n;
+        r.nt = r.tile - mt * p.grid_n;
+    }
+    r.m0 = mt * (S * TC_ROWS);
+    r.n0 = r.nt * BN;
+    r.g0 = r.sp * p.gps;
+    r.g1 = min(p.G, r.g0 + p.gps);
+    return r;
+}
+
+__device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+
+// Epilogue of 32 columns of one row: v (the int32 sums) at row m, columns n..n+31.
+__device__ __forceinline__ void tc_store(const TcRun& p, int (&v)[32], const int* colc, int m, int n, long long rowoff)
+{
+    if (m >= p.M) return;
+    int* oi = static_cast<int*>(p.out);
+    float* of = static_cast<float*>(p.out);
+    const bool f32 = p.out_kind == DS_OUT_F32;
+    auto finish = [&](int a, int r) -> int {
+        if (p.residual) a = __float2int_rn(__int2float_rn(a) + __int2float_rn(r));
+        if (p.relu) a = max(a, 0);
+        if (p.requant) a = min(max(a, p.rq_lo), p.rq_hi) * p.rq_mul + p.rq_add;
+        if (p.round_f32) a = __float2int_rn(__int2float_rn(a));
+        return a;
+    };
+    const int live = min(32, p.N - n);
+    if (p.P == 1 && (p.N & 3) == 0) {
+        const long long o0 = rowoff + n;
+#pragma unroll
+        for (int c = 0; c < 32; c += 4) {
+            if (c >= live) break;
+            const int4 cc = *reinterpret_cast<const int4*>(colc + c);
+            int4 r = make_int4(0, 0, 0, 0);
+            if (p.residual && DS_O_OK(p, p.residual, p.residual + o0 + c, 16))
+                r = make_int4(p.residual[o0 + c], p.residual[o0 + c + 1], p.residual[o0 + c + 2], p.residual[o0 + c + 3]);
+            const int a = finish(v[c] + cc.x, r.x), b = finish(v[c + 1] + cc.y, r.y), d = finish(v[c + 2] + cc.z, r.z),
+                      e = finish(v[c + 3] + cc.w, r.w);
+            if (!f32) {
+                if (DS_O_OK(p, oi, oi + o0 + c, 16)) *reinterpret_cast<int4*>(oi + o0 + c) = make_int4(a, b, d, e);
+            } else if (DS_O_OK(p, of, of + o0 + c, 16)) {
+                *reinterpret_cast<float4*>(of + o0 + c) =
+                    make_float4(__int2float_rn(a) * p.inv_scale, __int2float_rn(b) * p.inv_scale,
+                                __int2float_rn(d) * p.inv_scale, __int2float_rn(e) * p.inv_scale);
+            }
+        }
+        return;
+    }
+    long long o = rowoff + (long long)n * p.P;
+#pragma unroll
+    for (int c0 = 0; c0 < 32; c0 += 8) {
+        if (c0 >= live) break;
+        int r[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            r[c] = 0;
+            const int* ra = p.residual + o + (long long)c * p.P;
+            if (p.residual && c0 + c < live && DS_O_OK(p, p.residual, ra, 4)) r[c] = *ra;
+        }
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            if (c0 + c < live) {
+                const int a = finish(v[c0 + c] + colc[c0 + c], r[c]);
+                if (!f32) {
+                    if (DS_O_OK(p, oi, oi + o, 4)) oi[o] = a;
+                } else if (DS_O_OK(p, of, of + o, 4)) {
+                    of[o] = __int2float_rn(a) * p.inv_scale;
+                }
+            }
+            o += p.P;
+        }
+    }
+}
+
+template <int BN, int S>
+__global__ void __launch_bounds__(TcTile<BN>::THREADS, 1) tc_run_kernel(const TcRun p)
+{
+    using T = TcTile<BN>;
+    extern __shared__ unsigned char smem_raw[];
+    TcSmem<BN>& s = *reinterpret_cast<TcSmem<BN>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    if (p.gate && *p.gate != p.gate_want) return;  // the other arithmetic path serves this input
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    volatile int* err = &s.err;
+
+    if (threadIdx.x == 0) {
+        s.err = 0;
+        for (int i = 0; i < T::STAGES; ++i) {
+            bar_init(&s.bfull[i], 1);
+            bar_init(&s.bempty[i], 1);
+        }
+        for (int i = 0; i < T::WG; ++i) {
+            bar_init(&s.afull[i], 4);
+            bar_init(&s.aempty[i], 1);
+        }
+        for (int i = 0; i < T::NACC; ++i) {
+            bar_init(&s.accfull[i], 1);
+            bar_init(&s.accempty[i], 4);
+        }
+        bar_init(&s.done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 4 * T::WG + 4) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(&s.tmem)), "n"(TC_TMEM_COLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const unsigned tmem = *reinterpret_cast<volatile unsigned*>(&s.tmem);
+    const unsigned tmem_a = tmem + T::ACC_COLS;
+
+    if (warp < 4 * T::WG) {
+        // ---- producers: expand activations into TMEM -------------------------------------------------
+        const int wg = warp >> 2;
+        const int row = threadIdx.x & 127;
+        const unsigned lane_base = unsigned(warp & 3) << 21;  // TMEM lane (warp % 4) * 32 in bits 16-31
+        unsigned roff[S];
+        int u = blockIdx.x, sub = 0, g = 0, g1 = 0, j = 0, kh = 0;
+        auto enter = [&]() {
+            if (u >= p.units) return;
+            const Unit un = unit_of<BN, S>(p, u);
+            g = un.g0;
+            g1 = un.g1;
+            kh = g / p.J;
+            j = g - kh * p.J;
+            sub = 0;
+#pragma unroll
+            for (int i = 0; i < S; ++i) {
+                const int m = min(un.m0 + i * TC_ROWS + row, p.M - 1);
+                const int b = m / p.P, pp = m - b * p.P;
+                const int oh = pp / p.OW, ow = pp - oh * p.OW;
+                roff[i] = unsigned(b) * p.img_bytes + unsigned(oh) * p.row_step + unsigned(ow) * p.col_step;
+            }
+        };
+        auto step = [&]() {
+            if (++sub < S) return;
+            sub = 0;
+            if (++g == g1) {
+                u += gridDim.x;
+                enter();
+            } else if (++j == p.J) {
+                j = 0;
+                ++kh;
+            }
+        };
+        uint4 nl = make_uint4(0, 0, 0, 0), nh = nl;
+        auto fetch = [&]() {
+            unsigned off = roff[0];
+#pragma unroll
+            for (int i = 1; i < S; ++i)
+                if (sub == i) off = roff[i];
+            const unsigned char* a = p.act + (off + unsigned(kh) * p.kh_step + unsigned(j) * 16u);
+            nl = ld16(a, p.align);
+            nh = ld16(a + p.plane, p.align);
+        };
+        enter();
+        for (int i = 0; i < wg && u < p.units; ++i) step();
+        if (u < p.units) fetch();
+        for (unsigned round = 0; u < p.units;) {
+            const uint4 l = nl, h = nh;
+#pragma unroll
+            for (int i = 0; i < T::WG; ++i)
+                if (u < p.units) step();
+            if (u < p.units) fetch();
+            unsigned v[32];
+            planes_low(l.x, h.x, v, 0);
+            planes_low(l.y, h.y, v, 1);
+            planes_low(l.z, h.z, v, 2);
+            planes_low(l.w, h.w, v, 3);
+            // one hand-shake per 16 values: two (a slot per eight planes) cost a third of the rate at 128 columns
+            if (round > 0 && !bar_wait(&s.aempty[wg], (round - 1) & 1u, err)) u = p.units;
+            ++round;
+            __syncwarp();
+            tc_fence_after();
+            tmem_st32(tmem_a + lane_base + wg * 64, v);
+            planes_high(h.x, v, 0);
+            planes_high(h.y, v, 1);
+            planes_high(h.z, v, 2);
+            planes_high(h.w, v, 3);
+            tmem_st32(tmem_a + lane_base + wg * 64 + 32, v);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) bar_arrive(&s.afull[wg]);
+        }
+    } else if (warp < 4 * T::WG + 4) {
+        // ---- epilogue ----------------------------------------------------------------------------------
+        const int row = threadIdx.x & 127;
+        const unsigned lane_base = unsigned(warp & 3) << 21;
+        unsigned acc = 0;
+        int par = 0;
+        bool bad = false;
+        for (int u = blockIdx.x; u < p.units && !bad; u += gridDim.x, acc += S, par ^= 1) {
+            const Unit un = unit_of<BN, S>(p, u);
+            // column constants of this tile; two copies, so a slow warp still reads the previous tile's
+            if (row < BN) {
+                const int n = un.n0 + row;
+                s.colc[par][row] = n < p.N ? __ldg(p.colc + n) + (p.bias ? __ldg(p.bias + n) : 0) : 0;
+            }
+            epi_bar();
+#pragma unroll 1
+            for (int i = 0; i < S; ++i) {
+                const unsigned a = acc + i, slot = a % T::NACC;
+                if (!bar_wait(&s.accfull[slot], (a / T::NACC) & 1u, err)) {
+                    bad = true;
+                    break;
+                }
+                __syncwarp();
+                tc_fence_after();
+                const int m = un.m0 + i * TC_ROWS + row;
+                const int b = m / p.P, pp = m - b * p.P;
+                const long long rowoff = (long long)b * p.OC * p.P + pp;
+#pragma unroll 1
+                for (int c = 0; c < BN; c += 32) {
+                    int v[32];
+                    tmem_ld32(tmem + lane_base + slot * BN + c, v);
+                    if (c + 32 >= BN) {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) bar_arrive(&s.accempty[slot]);
+                    }
+                    if (p.splits == 1) {
+                        tc_store(p, v, &s.colc[par][c], m, un.n0 + c, rowoff);
+                    } else {
+                        int* dst = p.partials + ((long long)(un.tile * p.splits + un.sp) * S + i) * (BN * TC_ROWS) +
+                                   c * TC_ROWS + row;
+#pragma unroll
+                        for (int q = 0; q < 32; ++q) __stcg(dst + q * TC_ROWS, v[q]);
+                    }
+                }
+            }
+            if (p.splits > 1 && !bad) {
+                // the split that arrives last adds all partial sums in order and applies the epilogue
+                __threadfence();
+                epi_bar();
+                if (row == 0) s.last_flag = atomicAdd(p.counters + un.tile, 1) == p.splits - 1;
+                epi_bar();
+                if (s.last_flag) {
+                    __threadfence();
+#pragma unroll 1
+                    for (int i = 0; i < S; ++i) {
+                        const int m = un.m0 + i * TC_ROWS + row;
+                        const int b = m / p.P, pp = m - b * p.P;
+                        const long long rowoff = (long long)b * p.OC * p.P + pp;
+#pragma unroll 1
+                        for (int c = 0; c < BN; c += 32) {
+                            int v[32];
+#pragma unroll
+                            for (int q = 0; q < 32; ++q) v[q] = 0;
+#pragma unroll 1
+                            for (int k = 0; k < p.splits; ++k) {
+                                const int* src = p.partials + ((long long)(un.tile * p.splits + k) * S + i) * (BN * TC_ROWS) +
+                                                 c * TC_ROWS + row;
+#pragma unroll
+                                for (int q = 0; q < 32; ++q) v[q] += __ldcg(src + q * TC_ROWS);
+                            }
+                            tc_store(p, v, &s.colc[par][c], m, un.n0 + c, rowoff);
+                        }
+                    }
+                }
+                epi_bar();  // last_flag is read by all before the next unit writes it
+            }
+        }
+    } else if (warp == 4 * T::WG + 4) {
+        // ---- MMA issue ---------------------------------------------------------------------------------
+        // The whole warp walks the loop and an elected lane issues: control flow and addresses stay
+        // warp-uniform, and every ring index is a counter that wraps.  (One divergent lane with indices by
+        // division took 1100 cycles per four MMAs, whatever their width: 42 T shift-op/s at M = 8192.)
+        // A wait that gives up does not leave the loop: the error word makes all later ones return at once,
+        // and every access stays inside shared and tensor memory.
+        // D s32, A u8, B s8, both K-major, N = BN, M = 128
+        constexpr unsigned idesc = (2u << 4) | (0u << 7) | (1u << 10) | (unsigned(BN / 8) << 17) | (8u << 24);
+        // B: no swizzle, core matrices of 8 columns x 16 bytes; 128 bytes from one to the next along N, one
+        // plane (BN * 16 bytes) along K
+        const unsigned long long desc0 =
+            (1ull << 46) | (8ull << 32) | ((unsigned long long)BN << 16) | (s32(&s.b[0][0]) >> 4);
+        unsigned slot = 0, aph = 0, st = 0, bph = 0, aslot = 0, accph = 1;
+        for (int u = blockIdx.x; u < p.units; u += gridDim.x) {
+            const Unit un = unit_of<BN, S>(p, u);
+            unsigned d[S], accs[S];
+#pragma unroll
+            for (int i = 0; i < S; ++i) {
+                accs[i] = aslot;
+                d[i] = tmem + aslot * BN;
+                bar_wait(&s.accempty[aslot], accph, err);  // the first round finds the slots free
+                if (++aslot == unsigned(T::NACC)) {
+                    aslot = 0;
+                    accph ^= 1u;
+                }
+            }
+            unsigned more = 0;  // the first MMA of a unit overwrites the accumulator
+            for (int g = un.g0; g < un.g1; ++g) {
+                bar_wait(&s.bfull[st], bph, err);
+                const unsigned long long bdesc = desc0 + st * unsigned(T::STAGE >> 4);
+#pragma unroll
+                for (int i = 0; i < S; ++i) {
+                    bar_wait(&s.afull[slot], aph, err);
+                    tc_fence_after();
+                    if (elect_one()) {
+#pragma unroll
+                        for (int q = 0; q < 8; ++q)
+                            tc_mma_i8(d[i], tmem_a + slot * 64 + q * 8, bdesc + q * (2 * BN), idesc, q == 0 ? more : 1u);
+                        tc_commit(&s.aempty[slot]);
+                        if (i == S - 1) tc_commit(&s.bempty[st]);
+                    }
+                    __syncwarp();
+                    if (++slot == unsigned(T::WG)) {
+                        slot = 0;
+                        aph ^= 1u;
+                    }
+                }
+                more = 1;
+                if (++st == unsigned(T::STAGES)) {
+                    st = 0;
+                    bph ^= 1u;
+                }
+            }
+            if (elect_one()) {
+#pragma unroll
+                for (int i = 0; i < S; ++i) tc_commit(&s.accfull[accs[i]]);
+            }
+            __syncwarp();
+        }
+        if (elect_one()) tc_commit(&s.done);  // nothing of this CTA is in flight when the columns go back
+        for (int i = 0; i < TC_WAIT_LIMIT; ++i)
+            if (bar_try(&s.done, 0)) break;
+        __syncwarp();
+    } else {
+        // ---- weight tiles: one thread ------------------------------------------------------------------
+        if (lane == 0) {
+            unsigned bs = 0;
+            bool ok = true;
+            for (int u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
+                const Unit un = unit_of<BN, S>(p, u);
+                const unsigned char* src = p.wexp + ((long long)un.nt * p.G + un.g0) * T::STAGE;
+                for (int g = un.g0; g < un.g1; ++g, ++bs, src += T::STAGE) {
+                    const unsigned st = bs % T::STAGES;
+                    if (bs >= unsigned(T::STAGES)) {
+                        ok = bar_wait(&s.bempty[st], (bs / T::STAGES - 1) & 1u, err);
+                        if (!ok) break;
+                    }
+                    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(
+                                     s32(&s.bfull[st])),
+                                 "r"(unsigned(T::STAGE))
+                                 : "memory");
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                     s32(&s.b[st][0])),
+                                 "l"(src), "r"(unsigned(T::STAGE)), "r"(s32(&s.bfull[st]))
+                                 : "memory");
+                }
+            }
+            // Let every copy land before the CTA ends (the MMA thread has waited for all of them unless a
+            // wait gave up).
+            for (unsigned k = bs > unsigned(T::STAGES) ? bs - T::STAGES : 0; k < bs; ++k)
+                for (int i = 0; i < 64; ++i)
+                    if (bar_try(&s.bfull[k % T::STAGES], (k / T::STAGES) & 1u)) break;
+        }
+        __syncwarp();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 4 * T::WG + 4)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(TC_TMEM_COLS));
+    if (threadIdx.x == 0 && s.err) *p.err_flag = 1;
+}
+
+// ---- activations -> byte planes -----------------------------------------------------------------------
+// Code of the raw word `v` of x, as operand_of defines it for the integer path.
+template <int INK>
+__device__ __forceinline__ int pack_code(const TcPack& p, int v)
+{
+    if (INK == INK_I32) return v;
+    if (INK == INK_I32_CLAMP) return min(max(v, p.rq_lo), p.rq_hi) * p.rq_mul + p.rq_add;
+    if (p.in_kind == DS_IN_F32_CONV) return __float2int_rz(quant_conv_f(__int_as_float(v), p.q));
+    return __float2int_rz(truncf(__int_as_float(v) * p.q.scale));
+}
+
+// Bytes l and h of four codes; notes a code that does not fit 16 bits.
+__device__ __forceinline__ void pack4(const int (&c)[4], unsigned& l, unsigned& h, bool& over)
+{
+    unsigned y[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        y[e] = unsigned(c[e]) + 32768u;
+        over |= y[e] > 65535u;
+    }
+    const unsigned a = __byte_perm(y[0], y[1], 0x5140), b = __byte_perm(y[2], y[3], 0x5140);  // l0 l1 h0 h1
+    l = __byte_perm(a, b, 0x5410);
+    h = __byte_perm(a, b, 0x7632);
+}
+
+// NCHW -> pixel-major planes.  A block takes 1024 / CW padded pixels x 4 CW channels: lanes run over pixels
+// when reading (coalesced in x), over channels when writing (coalesced in the planes).  HBM-bound: 4 bytes
+// read and 2 written per value.
+template <int INK>
+__global__ void __launch_bounds__(256) tc_pack_nchw_kernel(const TcPack p, int cw_log)
+{
+    __shared__ unsigned sl[2048], sh[2048];
+    const int CW = 1 << cw_log, PIX = 1024 >> cw_log;
+    const long long q0 = (long long)blockIdx.x * PIX;
+    const int cw0 = blockIdx.y << cw_log;
+    if (p.counters && blockIdx.y == 0)
+        for (long long i = blockIdx.x * 256ll + threadIdx.x; i < p.ncounters; i += gridDim.x * 256ll) p.counters[i] = 0;
+    const long long hw = (long long)p.H * p.W;
+    const int* x = static_cast<const int*>(p.x);
+    bool over = false;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int i = threadIdx.x + 256 * k;
+        const int pix = i & (PIX - 1), cw = i >> (10 - cw_log);
+        const long long q = q0 + pix;
+        int c4[4] = {0, 0, 0, 0};
+        if (q < p.Q) {
+            const unsigned qi = unsigned(q);
+            const unsigned rowi = qi / unsigned(p.Wp);
+            const int w = int(qi - rowi * unsigned(p.Wp)) - p.pw;
+            const unsigned b = rowi / unsigned(p.Hp);
+            const int h = int(rowi - b * unsigned(p.Hp)) - p.ph;
+            if (unsigned(h) < unsigned(p.H) && unsigned(w) < unsigned(p.W)) {
+                const int c = 4 * (cw0 + cw);
+                const int* src = x + ((long long)b * p.C + c) * hw + (long long)h * p.W + w;
+                int raw[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) raw[e] = (c + e < p.C && DS_X_OK(p, src + e * hw, 4)) ? __ldg(src + e * hw) : 0;
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (c + e < p.C) c4[e] = pack_code<INK>(p, raw[e]);
+            }
+        }
+        unsigned l, h;
+        pack4(c4, l, h, over);
+        sl[pix * (CW + 1) + cw] = l;
+        sh[pix * (CW + 1) + cw] = h;
+    }
+    if (over && p.flag) *p.flag = 1;
+    __syncthreads();
+    const int cwords = p.Cp >> 2;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int i = threadIdx.x + 256 * k;
+        const int cw = i & (CW - 1), pix = i >> cw_log;
+        const long long q = q0 + pix;
+        if (q < p.Q && cw0 + cw < cwords) {
+            unsigned* dst = reinterpret_cast<unsigned*>(p.act + q * p.Cp) + cw0 + cw;
+            *dst = sl[pix * (CW + 1) + cw];
+            *reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(dst) + p.plane) = sh[pix * (CW + 1) + cw];
+        }
+    }
+}
+
+// Rows of a matrix [Q, C]: 4 values of a row per thread.
+template <int INK>
+__global__ void __launch_bounds__(256) tc_pack_rows_kernel(const TcPack p)
+{
+    const unsigned words = unsigned(p.Cp) >> 2;
+    const unsigned total = unsigned(p.Q) * words;  // plane bytes < 2^31, so this fits
+    const bool vec = p.C % 4 == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15u) == 0;
+    const unsigned i0 = blockIdx.x * 256u + threadIdx.x;
+    if (p.counters)
+        for (unsigned i = i0; i < unsigned(p.ncounters); i += gridDim.x * 256u) p.counters[i] = 0;
+    bool over = false;
+    for (unsigned i = i0; i < total; i += gridDim.x * 256u) {
+        const unsigned m = i / words, w = i - m * words;
+        const int k = int(4 * w);
+        const int* src = static_cast<const int*>(p.x) + (long long)m * p.C + k;
+        int raw[4] = {0, 0, 0, 0}, c4[4];
+        if (vec && k + 4 <= p.C) {
+            if (DS_X_OK(p, src, 16)) {
+                const int4 v = __ldg(reinterpret_cast<const int4*>(src));
+                raw[0] = v.x; raw[1] = v.y; raw[2] = v.z; raw[3] = v.w;
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (k + e < p.C && DS_X_OK(p, src + e, 4)) raw[e] = __ldg(src + e);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) c4[e] = k + e < p.C ? pack_code<INK>(p, raw[e]) : 0;
+        unsigned l, h;
+        pack4(c4, l, h, over);
+        unsigned* dst = reinterpret_cast<unsigned*>(p.act) + i;
+        *dst = l;
+        *reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(dst) + p.plane) = h;
+    }
+    if (over && p.flag) *p.flag = 1;
+}
+
+// ---- weights -> operand tiles -------------------------------------------------------------------------
+// Coefficient of plane f for a right shift r in 0..15 (ds_tc.cuh).
+__device__ __forceinline__ int tc_coef(int r, int f)
+{
+    if (r == 0) return f == 0 ? 1 : (f == 7 || f == 8 || f == 15) ? 127 : f == 9 ? 4 : 0;
+    if (r == 1) return f == 1 ? 1 : (f == 7 || f == 8 || f == 15) ? 64 : 0;
+    if (r <= 6) return f == r ? 1 : f == 8 ? 1 << (8 - r) : 0;
+    if (r == 7) return (f == 7 || f == 8 || f == 15) ? 1 : 0;
+    return f == r ? 1 : 0;
+}
+
+// Packed field of weight (n, k): r in 0..15 with bit 4 for a negative weight, or 32 for a zero weight.
+__device__ __forceinline__ int tc_code(const TcExpand& p, unsigned field)
+{
+    const int r = int(field & ((1u << p.dec.bits) - 1u));
+    if (r >= 32) return 32;
+    return min(r, 15) | (((field >> p.dec.bits) & 1u) ? 0 : 16);
+}
+
+constexpr int TC_COLC_BLOCKS = 16;  // blocks per column tile that compute const[n]
+
+// Block (g, nt): the operand tile of group g, columns nt * BN.. -- [16 planes][BN][16 bytes].  A thread makes
+// four planes of one column: 16 table words (four planes each, sign applied), transposed 4 x 4 bytes.
+// Blocks g = G.. compute the column constants -sum s 2^(15-r).
+__global__ void __launch_bounds__(256) tc_expand_kernel(const TcExpand p)
+{
+    const int n0 = blockIdx.y * p.BN;
+    const unsigned fmask = (1u << p.dec.fw) - 1u;
+    if (int(blockIdx.x) >= p.G) {
+        const int per = p.BN / TC_COLC_BLOCKS;  // 2, 4 or 8 columns: one per warp
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int n = n0 + (int(blockIdx.x) - p.G) * per + warp;
+        if (warp >= per || n >= p.N) return;
+        const int* src = p.packed + (long long)n * p.dec.row_len;
+        unsigned sum = 0;
+        for (int w = lane; w < p.dec.row_len; w += 32) {
+            unsigned word = DS_W_OK(p, src + w, 4) ? unsigned(__ldg(src + w)) : 0u;
+            const int k = w * p.dec.num;
+            for (int i = 0; i < p.dec.num && k + i < p.K; ++i, word >>= p.dec.fw) {
+                const int c = tc_code(p, word & fmask);
+                if (c < 32) {
+                    const unsigned v = 1u << (15 - (c & 15));
+                    sum += (c & 16) ? v : 0u - v;
+                }
+            }
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+        if (lane == 0) p.colc[n] = int(sum);
+        return;
+    }
+    __shared__ unsigned lut[4][33];                // [four planes][code]
+    __shared__ __align__(16) unsigned char codes[128 * 16];
+    const int g = blockIdx.x;
+    for (int i = threadIdx.x; i < 4 * 33; i += 256) {
+        const int q = i / 33, c = i - q * 33;
+        unsigned w = 0;
+        if (c < 32)
+            for (int e = 0; e < 4; ++e) {
+                int v = tc_coef(c & 15, 4 * q + e);
+                if (c & 16) v = -v;
+                w |= (unsigned(v) & 255u) << (8 * e);
+            }
+        lut[q][c] = w;
+    }
+    const int kh = g / p.J, j = g - kh * p.J;
+    for (int i = threadIdx.x; i < p.BN * 16; i += 256) {
+        const int e = i & 15, n = n0 + (i >> 4);
+        const int t = 16 * j + e;  // byte of the window row: (kw, c)
+        const int kw = t / p.Cp, c = t - kw * p.Cp;
+        int code = 32;
+        if (n < p.N && kw < p.KW && c < p.C) {
+            const int k = (c * p.KH + kh) * p.KW + kw;
+            const int w = k / p.dec.num;
+            const int* src = p.packed + (long long)n * p.dec.row_len + w;
+            if (DS_W_OK(p, src, 4)) code = tc_code(p, (unsigned(__ldg(src)) >> ((k - w * p.dec.num) * p.dec.fw)) & fmask);
+        }
+        codes[i] = (unsigned char)code;
+    }
+    __syncthreads();
+    uint4* out = reinterpret_cast<uint4*>(p.wexp + ((long long)blockIdx.y * p.G + g) * (p.BN * TC_PLANES * TC_KG));
+    for (int i = threadIdx.x; i < p.BN * 4; i += 256) {
+        const int n = i & (p.BN - 1), q = i / p.BN;
+        const uint4 cw = *reinterpret_cast<const uint4*>(codes + n * 16);
+        const unsigned cws[4] = {cw.x, cw.y, cw.z, cw.w};
+        unsigned o[4][4];  // [plane][word]
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            unsigned a[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) a[e] = lut[q][(cws[w] >> (8 * e)) & 255u];
+            const unsigned x01 = __byte_perm(a[0], a[1], 0x5140), y01 = __byte_perm(a[0], a[1], 0x7362);
+            const unsigned x23 = __byte_perm(a[2], a[3], 0x5140), y23 = __byte_perm(a[2], a[3], 0x7362);
+            o[0][w] = __byte_perm(x01, x23, 0x5410);
+            o[1][w] = __byte_perm(x01, x23, 0x7632);
+            o[2][w] = __byte_perm(y01, y23, 0x5410);
+            o[3][w] = __byte_perm(y01, y23, 0x7632);
+        }
+#pragma unroll
+        for (int f = 0; f < 4; ++f) out[(4 * q + f) * p.BN + n] = make_uint4(o[f][0], o[f][1], o[f][2], o[f][3]);
+    }
+}
+
+template <int BN, int S>
+int run_cfg(const TcRun& p0, cudaStream_t st)
+{
+    TcRun p = p0;
+    p.err_flag = kernel_error_flag();
+    const int dev = device_slot();
+    if (!p.err_flag || dev < 0) return DS_ERR_CUDA;
+    auto kern = tc_run_kernel<BN, S>;
+    const size_t smem = sizeof(TcSmem<BN>) + 1024;
+    static bool done[kMaxDevices];  // per instantiation and device
+    static int sms[kMaxDevices];
+    if (!done[dev]) {
+        int n = 0;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess ||
+            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            return DS_ERR_CUDA;
+        }
+        sms[dev] = n;
+        done[dev] = true;
+    }
+    const int grid = p.units < sms[dev] ? p.units : sms[dev];
+    kern<<<grid, TcTile<BN>::THREADS, smem, st>>>(p);
+    note_launch();
+    return cudaGetLastError() == cudaSuccess ? DS_OK : DS_ERR_CUDA;
+}
+
+}  // namespace
+
+int tc_launch_pack(const TcPack& p, cudaStream_t st)
+{
+    auto rows = [&](auto ink) {
+        const long long want = (p.Q * (p.Cp / 4) + 255) / 256;
+        tc_pack_rows_kernel<decltype(ink)::value><<<unsigned(want > 148 * 64 ? 148 * 64 : want), 256, 0, st>>>(p);
+    };
+    auto nchw = [&](auto ink) {
+        int lg = 0;
+        while (lg < 4 && (4 << lg) < p.Cp) ++lg;
+        const int pix = 1024 >> lg;
+        const dim3 grid(unsigned((p.Q + pix - 1) / pix), unsigned((p.Cp / 4 + (1 << lg) - 1) >> lg));
+        tc_pack_nchw_kernel<decltype(ink)::value><<<grid, 256, 0, st>>>(p, lg);
+    };
+    auto go = [&](auto ink) {
+        if (p.Hp == 1 && p.Wp == 1) rows(ink);
+        else nchw(ink);
+    };
+    if (p.in_kind == DS_IN_I32) go(std::integral_constant<int, INK_I32>());
+    else if (p.in_kind == DS_IN_I32_CLAMP) go(std::integral_constant<int, INK_I32_CLAMP>());
+    else go(std::integral_constant<int, INK_F32>());
+    note_launch();
+    return cudaGetLastError() == cudaSuccess ? DS_OK : DS_ERR_CUDA;
+}
+
+int tc_launch_expand(const TcExpand& p, int grid_n, cudaStream_t st)
+{
+    tc_expand_kernel<<<dim3(unsigned(p.G + TC_COLC_BLOCKS), unsigned(grid_n)), 256, 0, st>>>(p);
+    note_launch();
+    return cudaGetLastError() == cudaSuccess ? DS_OK : DS_ERR_CUDA;
+}
+
+int tc_launch_run(const TcRun& p, int BN, int S, cudaStream_t st)
+{
+    if (BN == 128) return S == 2 ? run_cfg<128, 2>(p, st) : run_cfg<128, 1>(p, st);
+    if (BN == 64) return S == 2 ? run_cfg<64, 2>(p, st) : run_cfg<64, 1>(p, st);
+    return S == 3 ? run_cfg<32, 3>(p, st) : run_cfg<32, 1>(p, st);
+}
+
+}  // namespace ds

@@ -1,0 +1,110 @@
+// Tensor-core path: declarations shared by ds_tc.cu (kernels, launches) and ds_tc_host.cu (entry points).
+//
+// The arithmetic.  out[m,n] = sum_k s[n,k] * (x[m,k] >> r[n,k]) is not a matrix product, because the
+// shift rounds every term.  For 16-bit codes and r in 0..15 it becomes one after widening K sixteenfold:
+// x >> r, as a function of x, lies in the span of sixteen byte-valued functions f_0..f_15 of x with
+// integer coefficients of at most 127, so
+//
+//     sum_k s * (x >> r)  =  sum_k sum_p f_p(x[m,k]) * (s[n,k] * c_p(r[n,k]))  +  const[n]
+//
+// is a u8 x s8 product with int32 accumulation, exact modulo 2^32 like the reference's sum.  With
+// y = x + 2^15 = 256 h + l (unsigned, so that x >> r = (y >> r) - 2^(15-r); the second part is const[n]):
+//
+//     f_0 = (l & 127) + (l >> 7) + 2 (h & 1)     y >> 0 = f_0 + 127 (f_7 + f_8 + f_15) + 4 f_9
+//     f_1 = (l >> 1) & 63                        y >> 1 = f_1 + 64 (f_7 + f_8 + f_15)
+//     f_r = l >> r           (r = 2..6)          y >> r = f_r + 2^(8-r) f_8
+//     f_7 = h + (l >> 7) - (h >> 7)              y >> 7 = f_7 + f_8 + f_15
+//     f_r = h >> (r - 8)     (r = 8..15)         y >> r = f_r
+//
+// Sixteen is the least possible: the sixteen functions x >> r are linearly independent.  The coefficient
+// 256 of the high byte (r = 0) does not fit an s8 operand; f_0, f_7 and f_9 are chosen so that two nearly
+// equal high-byte functions carry 127 each.  r in 16..31 equals r = 15 for 16-bit x, r >= 32 is a zero
+// weight.
+#pragma once
+#include "ds_gemm_common.cuh"
+
+namespace ds {
+
+constexpr int TC_ROWS = 128;    // rows (TMEM lanes) of one MMA
+constexpr int TC_PLANES = 16;   // functions f_p per value
+constexpr int TC_KG = 16;       // values of k per group: one 16-byte run of each plane
+
+// Geometry and tiling of one call; a pure function of its arguments (weights expanded for a geometry
+// fit every later call of the same geometry).
+struct TcGeom {
+    int B, C, H, W, OC, KH, KW, sh, sw, ph, pw, OH, OW;
+    int M, N, K, P;
+    int Hp, Wp, Cp;      // padded image and bytes per pixel of one byte plane (l or h) of the activations
+    int J, G;            // groups per window row: ceil(KW * Cp / 16); groups in all: KH * J
+    int align;           // every load starts at a multiple of this: 16, 8 or 4
+    long long plane;     // bytes of one byte plane
+    int BN, S;           // tile: S x 128 rows, BN columns
+    int grid_m, grid_n, splits, gps;  // gps: groups per split
+    long long act_bytes;      // both planes, then counters, then partial sums
+    long long counters_off, partials_off;
+    long long weight_bytes;   // expanded weights, then the column constants
+    long long colc_off;
+};
+
+struct TcRun {
+    const unsigned char* act;
+    long long plane;
+    const unsigned char* wexp;
+    const int* colc;
+    const int* bias;
+    const int* residual;
+    void* out;
+    int M, N, P, OC, OW, G, J, align;
+    unsigned img_bytes, row_step, col_step, kh_step;  // byte offsets inside a plane
+    int grid_m, grid_n, splits, gps, units, m_fast;
+    int* counters;
+    int* partials;
+    int out_kind, relu, requant, round_f32;
+    int rq_lo, rq_hi, rq_mul, rq_add;
+    float inv_scale;
+    const int* gate;
+    int gate_want;
+    int* err_flag;
+    long long chk_o_bytes;
+    int* chk_status;
+};
+
+struct TcPack {
+    const void* x;
+    unsigned char* act;
+    long long plane;
+    int B, C, H, W, ph, pw, Hp, Wp, Cp;
+    long long Q;         // padded pixels
+    int in_kind;
+    Quant q;
+    int rq_lo, rq_hi, rq_mul, rq_add;
+    int* flag;           // set to 1 when a code does not fit 16 bits; null = no check
+    int* counters;       // zeroed here for the launch behind
+    int ncounters;
+    long long chk_x_bytes;
+    int* chk_status;
+};
+
+struct TcExpand {
+    const int* packed;
+    unsigned char* wexp;
+    int* colc;
+    Decode dec;
+    int C, KH, KW, Cp, J, G, N, K, BN;
+    long long chk_w_bytes;
+    int* chk_status;
+};
+
+// ds_gemm.cu: the checks and constants every path shares; the integer path gated on *gate == want; bytes
+// taken off the declared extent of x (checked build).
+int setup_common(GemmParams& p, int bits, int base, const ds_fuse_t* fuse, bool& use_fp);
+int launch_gated_int(const void* x, const int32_t* packed, const int32_t* bias, void* out, int B, int C, int H, int W,
+                     int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits, int base, const ds_fuse_t* fuse,
+                     const int* gate, int want, cudaStream_t st);
+long long check_shrink_x();
+
+int tc_launch_pack(const TcPack& p, cudaStream_t st);
+int tc_launch_expand(const TcExpand& p, int grid_n, cudaStream_t st);
+int tc_launch_run(const TcRun& p, int BN, int S, cudaStream_t st);
+
+}  // namespace ds

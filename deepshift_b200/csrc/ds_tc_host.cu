@@ -1,0 +1,257 @@
+// Tensor-core path: geometry, tile choice and the ds_tc_* entry points.  Kernels: ds_tc.cu.
+#include "ds_tc.cuh"
+
+namespace ds {
+
+int* bounds_status_ptr();
+
+namespace {
+
+constexpr int kSms = 148;
+
+long long round16(long long v) { return (v + 15) & ~15ll; }
+
+// Bytes per pixel and plane, and the groups per window row that follow.  The (kw, c) run of one window row
+// is contiguous (KW * Cp bytes), so only its end is padded to 16; Cp a multiple of 4, 8 or 16 decides how
+// wide the loads are.  Fewest groups first, then the widest loads.
+void choose_pixel(TcGeom& g)
+{
+    int best_j = 1 << 30;
+    for (int a = 16; a >= 4; a >>= 1) {
+        const int cp = (g.C + a - 1) / a * a;
+        const int j = (g.KW * cp + 15) / 16;
+        if (j < best_j) {
+            best_j = j;
+            g.Cp = cp;
+        }
+    }
+    g.J = best_j;
+    g.G = g.KH * g.J;
+    g.align = 16;
+    // offsets are sums of multiples of Cp * sw, of the row pitch Wp * Cp and of 16
+    while (g.align > 4 && ((g.Cp * g.sw) % g.align || ((long long)g.Wp * g.Cp) % g.align)) g.align >>= 1;
+}
+
+// Clock cycles of one (group, 128 rows) item: eight MMAs of BN / 2 cycles, or what the producers need for
+// one item when that is longer.
+double item_cycles(int bn, int s)
+{
+    if (bn == 128) return s == 1 ? 640 : 530;  // one row block: the weight tile comes from L2 for 128 rows only
+    return bn == 64 ? 290 : 240;
+}
+
+// Tile and split with the smallest estimated time: waves of units over the SMs, a unit being the longer of
+// its MMAs and its epilogue (HBM share of an SM: 23 bytes per cycle), plus one epilogue that nothing hides.
+void choose_tile(TcGeom& g)
+{
+    double best = 1e30;
+    const int bns[3] = {128, 64, 32};
+    for (int bn : bns) {
+        if (bn > 32 && g.N <= bn / 2) continue;
+        const int smax = bn == 32 ? 3 : 2;  // row blocks that share a weight tile, and that TMEM holds twice
+        for (int s = 1; s <= smax; s += smax - 1) {
+            const long long gm = (g.M + s * TC_ROWS - 1ll) / (s * TC_ROWS), gn = (g.N + bn - 1) / bn;
+            const double epi = s * TC_ROWS * (double)bn * 4 / 23;
+            for (int sp = 1; sp <= 16; ++sp) {
+                const int gps = (g.G + sp - 1) / sp;
+                if (sp > 1 && (gps < 4 || (g.G + gps - 1) / gps != sp)) continue;
+                if (sp > 1 && gm * gn >= 2 * kSms) break;
+                const long long units = gm * gn * sp;
+                const double waves = double((units + kSms - 1) / kSms);
+                const double main = gps * s * item_cycles(bn, s) + 400;
+                double cost = waves * (main > epi ? main : epi) + (main > epi ? epi : main) + 3000;
+                if (sp > 1) cost += 2500 + sp * epi * 0.5;
+                if (cost < best) {
+                    best = cost;
+                    g.BN = bn;
+                    g.S = s;
+                    g.grid_m = int(gm);
+                    g.grid_n = int(gn);
+                    g.splits = sp;
+                    g.gps = gps;
+                }
+            }
+        }
+    }
+}
+
+// Fills the geometry; DS_ERR_UNSUPPORTED when 32-bit offsets do not reach.
+int tc_geometry(TcGeom& g, int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw, int ph, int pw)
+{
+    if (B < 0 || C <= 0 || H <= 0 || W <= 0 || OC <= 0 || KH <= 0 || KW <= 0 || sh <= 0 || sw <= 0 || ph < 0 || pw < 0)
+        return DS_ERR_BAD_ARG;
+    if (KH > 31 || KW > 31) return DS_ERR_UNSUPPORTED;
+    if ((long long)H + 2ll * ph < KH || (long long)W + 2ll * pw < KW) return DS_ERR_BAD_ARG;
+    if (B == 0) return DS_ERR_UNSUPPORTED;
+    g = TcGeom{};
+    g.B = B; g.C = C; g.H = H; g.W = W; g.OC = OC; g.KH = KH; g.KW = KW; g.sh = sh; g.sw = sw; g.ph = ph; g.pw = pw;
+    const long long hp = (long long)H + 2ll * ph, wp = (long long)W + 2ll * pw;
+    const long long oh = (hp - KH) / sh + 1, ow = (wp - KW) / sw + 1;
+    if (hp > (1 << 20) || wp > (1 << 20) || (long long)C * KH * KW > (1ll << 30)) return DS_ERR_UNSUPPORTED;
+    const long long M = B * oh * ow, K = (long long)C * KH * KW;
+    // what ds_conv2d_ex refuses with DS_ERR_RANGE stays with it
+    if ((long long)C * H * W >= (1ll << 29) || K * KH * KW >= (1ll << 32)) return DS_ERR_UNSUPPORTED;
+    const long long limit = 0x7FFFFFFFll - (1 << 20);
+    const long long pixels = B * hp * wp;
+    if (pixels > limit || M > limit) return DS_ERR_UNSUPPORTED;
+    g.Hp = int(hp); g.Wp = int(wp); g.OH = int(oh); g.OW = int(ow);
+    g.M = int(M); g.K = int(K); g.N = OC; g.P = int(oh * ow);
+    choose_pixel(g);
+    if (pixels * g.Cp > limit) return DS_ERR_UNSUPPORTED;
+    g.plane = round16(pixels * g.Cp + 16);  // the last group of a window row may read up to 15 bytes beyond it
+    choose_tile(g);
+    const long long tiles = (long long)g.grid_m * g.grid_n;
+    if (tiles * g.splits > limit || g.grid_n > 65535) return DS_ERR_UNSUPPORTED;
+    const long long counters = g.splits > 1 ? tiles : 0;
+    g.counters_off = 2 * g.plane;
+    g.partials_off = round16(g.counters_off + 16 + counters * 4);  // 16: the range flag comes first
+    g.act_bytes = g.partials_off + (g.splits > 1 ? tiles * g.splits * (long long)g.S * TC_ROWS * g.BN * 4 : 0);
+    g.colc_off = (long long)g.grid_n * g.G * g.BN * TC_PLANES * TC_KG;
+    g.weight_bytes = g.colc_off + round16(4ll * g.N);
+    return DS_OK;
+}
+
+enum { TC_NO = 0, TC_DIRECT, TC_GATED };
+
+// Whether the activations of this call are known to fit 16 bits (TC_DIRECT), may fit (TC_GATED: measured on
+// the device while packing, the integer path stands behind) or cannot be served.
+int tc_mode(const ds_fuse_t& f, int bits, int base)
+{
+    if (base != 0 || bits < 1 || bits > 7) return TC_NO;
+    const int I = f.act_integer_bits, F = f.act_fraction_bits;
+    const int code_bits = I == 1 ? F + 2 : I + F;
+    switch (f.in_kind) {
+        case DS_IN_I32:
+            if (f.act_bits == DS_ACT_BITS_AUTO) return TC_GATED;
+            return f.act_bits >= 1 && f.act_bits <= 15 ? TC_DIRECT : TC_NO;  // 16 promises |x| <= 2^15, one too many
+        case DS_IN_F32_CONV:
+        case DS_IN_I32_CLAMP: return I >= 1 && F >= 0 && code_bits <= 16 ? TC_DIRECT : TC_NO;
+        case DS_IN_F32_LINEAR: return I >= 1 && F >= 0 && I + F <= 16 ? TC_GATED : TC_NO;
+        default: return TC_NO;
+    }
+}
+
+}  // namespace
+}  // namespace ds
+
+using namespace ds;
+
+extern "C" int ds_tc_bytes(int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits,
+                           int base, const ds_fuse_t* fuse, int any_size, long long* act_bytes, long long* weight_bytes)
+{
+    if (!fuse || !act_bytes || !weight_bytes) return DS_ERR_BAD_ARG;
+    *act_bytes = *weight_bytes = 0;
+    if (tc_mode(*fuse, bits, base) == TC_NO) return DS_OK;
+    TcGeom g;
+    const int rc = tc_geometry(g, B, C, H, W, OC, KH, KW, sh, sw, ph, pw);
+    if (rc == DS_ERR_UNSUPPORTED) return DS_OK;
+    if (rc) return rc;
+    if (!any_size && ((double)g.M * g.N * g.K < double(1 << 26) || g.M <= 64)) return DS_OK;
+    *act_bytes = g.act_bytes;
+    *weight_bytes = g.weight_bytes;
+    return DS_OK;
+}
+
+extern "C" int ds_tc_expand(const int32_t* packed, int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw,
+                            int ph, int pw, int bits, int base, void* weights, long long weight_bytes, void* stream)
+{
+    if (!packed || !weights) return DS_ERR_BAD_ARG;
+    if (base != 0 || bits < 1 || bits > 7) return DS_ERR_UNSUPPORTED;
+    if (reinterpret_cast<uintptr_t>(weights) & 15u) return DS_ERR_ALIGN;
+    TcGeom g;
+    const int rc = tc_geometry(g, B, C, H, W, OC, KH, KW, sh, sw, ph, pw);
+    if (rc) return rc;
+    if (weight_bytes < g.weight_bytes) return DS_ERR_SCRATCH;
+    TcExpand p = {};
+    p.packed = packed;
+    p.wexp = static_cast<unsigned char*>(weights);
+    p.colc = reinterpret_cast<int*>(p.wexp + g.colc_off);
+    p.dec.bits = bits;
+    p.dec.fw = bits + 1;
+    p.dec.num = 32 / (bits + 1);
+    p.dec.base = 0;
+    p.dec.row_len = (g.K + p.dec.num - 1) / p.dec.num;
+    p.C = g.C; p.KH = g.KH; p.KW = g.KW; p.Cp = g.Cp; p.J = g.J; p.G = g.G; p.N = g.N; p.K = g.K; p.BN = g.BN;
+    p.chk_w_bytes = (long long)g.N * p.dec.row_len * 4;
+    p.chk_status = bounds_status_ptr();
+    return tc_launch_expand(p, g.grid_n, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int ds_tc_conv2d(const void* x, const int32_t* packed, const int32_t* bias, void* out, int B, int C, int H,
+                            int W, int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits, int base,
+                            const ds_fuse_t* fuse, void* act, long long act_bytes, const void* weights,
+                            long long weight_bytes, void* stream)
+{
+    if (!x || !packed || !out || !fuse || !act || !weights) return DS_ERR_BAD_ARG;
+    if ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(act) | reinterpret_cast<uintptr_t>(weights)) & 15u)
+        return DS_ERR_ALIGN;
+    const int mode = tc_mode(*fuse, bits, base);
+    if (mode == TC_NO) return DS_ERR_UNSUPPORTED;
+    TcGeom g;
+    int rc = tc_geometry(g, B, C, H, W, OC, KH, KW, sh, sw, ph, pw);
+    if (rc) return rc;
+    if (act_bytes < g.act_bytes || weight_bytes < g.weight_bytes) return DS_ERR_SCRATCH;
+    // the quantiser and clamp constants, checked as for every other path
+    GemmParams q = {};
+    bool fp = false;
+    q.K = g.K;
+    rc = setup_common(q, bits, base, fuse, fp);
+    if (rc) return rc;
+    if (fuse->residual && (reinterpret_cast<uintptr_t>(fuse->residual) & 3u)) return DS_ERR_ALIGN;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    unsigned char* a = static_cast<unsigned char*>(act);
+    int* flag = reinterpret_cast<int*>(a + g.counters_off);
+    int* counters = flag + 4;
+    const int ncounters = g.splits > 1 ? g.grid_m * g.grid_n : 0;
+
+    TcPack pk = {};
+    pk.x = x;
+    pk.act = a;
+    pk.plane = g.plane;
+    pk.B = g.B; pk.C = g.C; pk.H = g.H; pk.W = g.W; pk.ph = g.ph; pk.pw = g.pw; pk.Hp = g.Hp; pk.Wp = g.Wp; pk.Cp = g.Cp;
+    pk.Q = (long long)g.B * g.Hp * g.Wp;
+    pk.in_kind = q.in_kind;
+    pk.q = q.q;
+    pk.rq_lo = q.rq_lo; pk.rq_hi = q.rq_hi; pk.rq_mul = q.rq_mul; pk.rq_add = q.rq_add;
+    pk.counters = ncounters ? counters : nullptr;
+    pk.ncounters = ncounters;
+    pk.chk_x_bytes = (long long)g.B * g.C * g.H * g.W * 4 - check_shrink_x();
+    pk.chk_status = bounds_status_ptr();
+    if (mode == TC_GATED) {
+        if (cudaMemsetAsync(flag, 0, sizeof(int), st) != cudaSuccess) return DS_ERR_CUDA;
+        pk.flag = flag;
+    }
+    rc = tc_launch_pack(pk, st);
+    if (rc) return rc;
+
+    TcRun p = {};
+    p.act = a;
+    p.plane = g.plane;
+    p.wexp = static_cast<const unsigned char*>(weights);
+    p.colc = reinterpret_cast<const int*>(p.wexp + g.colc_off);
+    p.bias = bias;
+    p.residual = fuse->residual;
+    p.out = out;
+    p.M = g.M; p.N = g.N; p.P = g.P; p.OC = g.OC; p.OW = g.OW; p.G = g.G; p.J = g.J; p.align = g.align;
+    p.kh_step = unsigned(g.Wp) * unsigned(g.Cp);
+    p.img_bytes = unsigned(g.Hp) * p.kh_step;
+    p.row_step = unsigned(g.sh) * p.kh_step;
+    p.col_step = unsigned(g.sw) * unsigned(g.Cp);
+    p.grid_m = g.grid_m; p.grid_n = g.grid_n; p.splits = g.splits; p.gps = g.gps;
+    p.units = g.grid_m * g.grid_n * g.splits;
+    // neighbouring CTAs share the smaller operand's tiles through L2: rows fastest when the weights are the
+    // larger one
+    p.m_fast = g.weight_bytes > 2 * g.plane;
+    p.counters = counters;
+    p.partials = reinterpret_cast<int*>(a + g.partials_off);
+    p.out_kind = q.out_kind; p.relu = q.relu; p.requant = q.requant; p.round_f32 = q.round_f32;
+    p.rq_lo = q.rq_lo; p.rq_hi = q.rq_hi; p.rq_mul = q.rq_mul; p.rq_add = q.rq_add;
+    p.inv_scale = q.inv_scale;
+    p.gate = pk.flag;
+    p.gate_want = 0;
+    p.chk_o_bytes = (long long)g.M * g.N * 4;
+    p.chk_status = bounds_status_ptr();
+    rc = tc_launch_run(p, g.BN, g.S, st);
+    if (rc || mode != TC_GATED) return rc;
+    return launch_gated_int(x, packed, bias, out, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, bits, base, fuse, flag, 1, st);
+}

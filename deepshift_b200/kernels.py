@@ -103,6 +103,83 @@ def _fuse(in_kind=0, out_kind=0, act_integer_bits=0, act_fraction_bits=0, relu=F
     return f
 
 
+# ------------------------------------------------------------------------------------------------
+# Tensor-core path (ds_tc_*): 16-bit activations, right shifts.  A geometry is (B, C, H, W, OC, KH, KW, sh,
+# sw, ph, pw); a linear layer [M,K] x [N,K] is the 1x1 convolution (M, K, 1, 1, N, 1, 1, 1, 1, 0, 0).
+
+def tc_bytes(geometry, conc_weight, fuse, any_size=False):
+    """(scratch bytes, expanded-weight bytes) of a call on the tensor cores; (0, 0) when the call is served
+    by the other paths (left shifts, activations wider than 16 bits, too little work to pay the packing)."""
+    act, wt = ctypes.c_longlong(0), ctypes.c_longlong(0)
+    _ffi.check(_ffi.lib().ds_tc_bytes(*geometry, conc_weight.bits, conc_weight.base, fuse, int(any_size),
+                                      ctypes.byref(act), ctypes.byref(wt)), "tc_bytes")
+    return act.value, wt.value
+
+
+def tc_expand(geometry, conc_weight, nbytes, device):
+    """The layer's weights as the operand tiles of this geometry, in a new buffer."""
+    buf = torch.empty(nbytes, dtype=torch.uint8, device=device)
+    _ffi.check(_ffi.lib().ds_tc_expand(conc_weight.data.data_ptr(), *geometry, conc_weight.bits, conc_weight.base,
+                                       buf.data_ptr(), nbytes, _stream_ptr(device)), "tc_expand")
+    return buf
+
+
+def _tc_weights(geometry, conc_weight, nbytes, device):
+    """Expanded weights kept on the ``ConcWeight`` they were made from, as ``_prepared_weights`` keeps its
+    own.  The buffer is filled on the stream of the first call; calls on other streams wait for that.  While
+    a stream is being captured nothing is kept, and a buffer not known to be complete is not used (an event
+    from outside a capture cannot be waited for inside): the expansion becomes part of the graph."""
+    cache = conc_weight.__dict__.setdefault("_tc", {})
+    key = geometry + (conc_weight.bits, conc_weight.base, conc_weight.data.data_ptr(), str(device))
+    entry = cache.get(key)
+    stream = torch.cuda.current_stream(device)
+    capturing = torch.cuda.is_current_stream_capturing()
+    if entry is None:
+        buf = tc_expand(geometry, conc_weight, nbytes, device)
+        if not capturing:
+            event = torch.cuda.Event()
+            event.record(stream)
+            cache[key] = dict(buf=buf, event=event, ready=False)
+        return buf
+    if not entry["ready"]:
+        if capturing:
+            return tc_expand(geometry, conc_weight, nbytes, device)
+        if entry["event"].query():
+            entry["ready"] = True
+        else:
+            stream.wait_event(entry["event"])
+    return entry["buf"]
+
+
+def _tc_run(x, conc_weight, bias, out, geometry, fuse, keep_weights):
+    """Runs the call on the tensor cores if it is one for them; False otherwise.  Scratch comes from torch's
+    allocator, whose blocks are reused in stream order."""
+    act_bytes, weight_bytes = tc_bytes(geometry, conc_weight, fuse)
+    if act_bytes == 0:
+        return False
+    device = x.device
+    if keep_weights:
+        wt = _tc_weights(geometry, conc_weight, weight_bytes, device)
+    else:
+        wt = tc_expand(geometry, conc_weight, weight_bytes, device)
+    act = torch.empty(act_bytes, dtype=torch.uint8, device=device)
+    rc = _ffi.lib().ds_tc_conv2d(x.data_ptr(), conc_weight.data.data_ptr(),
+                                 bias.data_ptr() if bias is not None else None, out.data_ptr(), *geometry,
+                                 conc_weight.bits, conc_weight.base, fuse, act.data_ptr(), act_bytes, wt.data_ptr(),
+                                 weight_bytes, _stream_ptr(device))
+    _ffi.check(rc, "tc_conv2d")
+    return True
+
+
+def tc_serves_fp32_conv(input_shape, weight_shape, stride, padding, conc_weight, act_integer_bits, act_fraction_bits):
+    """Whether a shift convolution with fp32 input of these sizes runs on the tensor cores, which quantise
+    every value once: no quantising pass is needed in front."""
+    B, C, H, W = input_shape
+    geometry = (B, C, H, W, weight_shape[0], weight_shape[2], weight_shape[3]) + _pair(stride) + _pair(padding)
+    f = _fuse(_ffi.IN_F32_CONV, _ffi.OUT_F32, act_integer_bits, act_fraction_bits)
+    return tc_bytes(geometry, conc_weight, f)[0] > 0
+
+
 ACT_BITS_AUTO = -1   # DS_ACT_BITS_AUTO: the library measures the range of the activations on the device
 
 
@@ -126,6 +203,8 @@ def linear(input, shift, sign, bias=None, conc_weight=None, use_cuda=True, act_b
     f = _fuse(act_bits=ACT_BITS_AUTO if act_bits is None else act_bits,
               workspace=workspace(input.device) if M > 64 else None)
     with torch.cuda.device(input.device):
+        if M > 64 and _tc_run(input, conc_weight, bias, out, (M, K, 1, 1, N, 1, 1, 1, 1, 0, 0), f, False):
+            return out
         rc = _ffi.lib().ds_linear_ex(input.data_ptr(), conc_weight.data.data_ptr(),
                                      bias.data_ptr() if bias is not None else None, out.data_ptr(),
                                      M, K, N, conc_weight.bits, conc_weight.base, f,
@@ -160,6 +239,8 @@ def conv2d(input, shift, sign, bias=None, conc_weight=None, stride=1, padding=0,
     # ds_conv2d_i32 plus the split-K counter workspace (layers with few output tiles)
     f = _fuse(act_bits=ACT_BITS_AUTO if act_bits is None else act_bits, workspace=workspace(input.device))
     with torch.cuda.device(input.device):
+        if _tc_run(input, conc_weight, bias, out, (B, C, H, W, OC, KH, KW, sh, sw, ph, pw), f, False):
+            return out
         rc = _ffi.lib().ds_conv2d_ex(input.data_ptr(), conc_weight.data.data_ptr(),
                                      bias.data_ptr() if bias is not None else None, out.data_ptr(),
                                      B, C, H, W, OC, KH, KW, sh, sw, ph, pw, conc_weight.bits,
@@ -199,6 +280,8 @@ def linear_fused(input, out_features, bias_i32, conc_weight, *, in_kind=_ffi.IN_
     f = _fuse(in_kind, out_kind, act_integer_bits, act_fraction_bits, relu, requant, residual, act_bits, round_f32,
               workspace(input.device) if M > 64 else None)
     with torch.cuda.device(input.device):
+        if M > 16 and _tc_run(input, conc_weight, bias_i32, out, (M, K, 1, 1, out_features, 1, 1, 1, 1, 0, 0), f, True):
+            return out
         rc = _ffi.lib().ds_linear_ex(input.data_ptr(), conc_weight.data.data_ptr(),
                                      bias_i32.data_ptr() if bias_i32 is not None else None, out.data_ptr(),
                                      M, K, out_features, conc_weight.bits, conc_weight.base, f,
@@ -253,6 +336,8 @@ def conv2d_fused(input, weight_shape, bias_i32, conc_weight, stride=1, padding=0
               workspace(input.device))
     geometry = (B, C, H, W, OC, KH, KW, sh, sw, ph, pw)
     with torch.cuda.device(input.device):
+        if _tc_run(input, conc_weight, bias_i32, out, geometry, f, True):
+            return out
         prepared = _prepared_weights(conc_weight, geometry, f, input.device)
         if prepared is not None:
             f.prepared = prepared.data_ptr()

@@ -69,6 +69,7 @@ class _ShiftBase(nn.Module):
         elif cw.data.device != device:
             cw.data = cw.data.to(device)
             cw.__dict__.pop("_prepared", None)   # expanded copies live on the old device
+            cw.__dict__.pop("_tc", None)
         self.__dict__["_weight_key"] = key
         return cw
 
@@ -235,7 +236,9 @@ class Conv2dShift(_ConvNdShift):
                 raise RuntimeError("the shift convolution kernel supports neither dilation nor groups")
             x = input.float().contiguous()
             in_kind, act_bits = _ffi.IN_F32_CONV, 0
-            if utils.quantise_in_own_pass(self.kernel_size, self.out_channels):
+            cw = self._packed(x.device)
+            if utils.quantise_in_own_pass(self.kernel_size, self.out_channels) and not kernels.tc_serves_fp32_conv(
+                    x.shape, tuple(self.shift.shape), self.stride, padding, cw, self.act_integer_bits, self.act_fraction_bits):
                 # the kernel stages every input value once per filter tap and per tile of 128 output
                 # channels: from 9 such uses on, quantising once in a pass of its own is cheaper than
                 # quantising at every use; the codes are final (round_to_fixed is not idempotent for
@@ -243,7 +246,7 @@ class Conv2dShift(_ConvNdShift):
                 x = kernels.quantize(x, self.act_integer_bits, self.act_fraction_bits, like_conv=True)
                 in_kind, act_bits = _ffi.IN_I32, utils.code_bits(self.act_integer_bits, self.act_fraction_bits)
             out = kernels.conv2d_fused(x, tuple(self.shift.shape), self._bias_fixed(like_conv=True),
-                                       self._packed(x.device), self.stride, padding,
+                                       cw, self.stride, padding,
                                        in_kind=in_kind, out_kind=_ffi.OUT_F32,
                                        act_integer_bits=self.act_integer_bits,
                                        act_fraction_bits=self.act_fraction_bits, act_bits=act_bits,

@@ -223,12 +223,14 @@ class Conv2dShiftQ(_ConvNdShiftQ):
                 raise RuntimeError("the shift convolution kernel supports neither dilation nor groups")
             x = input.float().contiguous()
             in_kind, act_bits = _ffi.IN_F32_CONV, 0
-            if utils.quantise_in_own_pass(self.kernel_size, self.out_channels):
+            cw = self._packed(x.device)
+            if utils.quantise_in_own_pass(self.kernel_size, self.out_channels) and not kernels.tc_serves_fp32_conv(
+                    x.shape, tuple(self.weight.shape), self.stride, padding, cw, self.act_integer_bits, self.act_fraction_bits):
                 # every input value is staged once per filter tap and tile of 128 output channels:
                 # from 9 uses on, quantise once, in a pass of its own
                 x = self._input_codes(x)
                 in_kind, act_bits = _ffi.IN_I32, self._act_bits()
-            out = kernels.conv2d_fused(x, tuple(self.weight.shape), self._bias_fixed(), self._packed(x.device),
+            out = kernels.conv2d_fused(x, tuple(self.weight.shape), self._bias_fixed(), cw,
                                        self.stride, padding, in_kind=in_kind, out_kind=_ffi.OUT_F32,
                                        act_integer_bits=self.act_integer_bits,
                                        act_fraction_bits=self.act_fraction_bits, act_bits=act_bits,

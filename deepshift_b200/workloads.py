@@ -344,6 +344,7 @@ class IntPipeline(_Pipeline):
         t = {'x': self.x_in}
         fp32 = {'x': True}
         self.calls = []
+        self.tc = {}   # index of a call -> (geometry, scratch bytes, expanded weights)
         n_shift = sum(1 for s in net.steps if s[0] in ('conv', 'linear'))
         seen = 0
         for st in net.steps:
@@ -357,7 +358,8 @@ class IntPipeline(_Pipeline):
                 xin = t[src]
                 in_fp32 = fp32[src]
                 if op == 'conv':
-                    if in_fp32 and utils.quantise_in_own_pass((L.k, L.k), L.cout):
+                    if in_fp32 and utils.quantise_in_own_pass((L.k, L.k), L.cout) and not kernels.tc_serves_fp32_conv(
+                            tuple(xin.shape), L.weight_shape, L.stride, L.pad, self.packed[li], self.I, self.F):
                         # every input value would be converted many times: quantise it once in a
                         # pass of its own instead of inside the convolution's staging code
                         xq = torch.empty(xin.shape, dtype=torch.int32, device=dev)
@@ -378,6 +380,14 @@ class IntPipeline(_Pipeline):
                                      relu=bool(o.get('relu')), requant=False, residual=res,
                                      round_f32=not lastlayer, workspace=self.workspace)
                 self.calls.append((op, xin, li, L, out, fuse, res))
+                geometry = tuple(xin.shape) + (L.cout, L.k, L.k, L.stride, L.stride, L.pad, L.pad)
+                if op == 'linear':
+                    geometry = (xin.shape[0], xin.shape[1], 1, 1, L.cout, 1, 1, 1, 1, 0, 0)
+                act_bytes, weight_bytes = kernels.tc_bytes(geometry, self.packed[li], fuse)
+                if act_bytes:
+                    # tensor cores: weights expanded once, one scratch buffer for all layers of the pass
+                    self.tc[len(self.calls) - 1] = (geometry, act_bytes, kernels.tc_expand(
+                        geometry, self.packed[li], weight_bytes, dev))
                 dst = o.get('dst', 'x')
                 t[dst], fp32[dst] = out, lastlayer
             elif op == 'maxpool':
@@ -406,13 +416,22 @@ class IntPipeline(_Pipeline):
                 self.calls.append(('shortcutA', xin, out, pad))
                 t[st[2]], fp32[st[2]] = out, False
         self.out = t['x']
+        self.tc_act = torch.empty(max([v[1] for v in self.tc.values()], default=0), dtype=torch.uint8, device=dev)
 
     def _launch_all(self):
         lib = _ffi.lib()
         stream = torch.cuda.current_stream(self.device).cuda_stream
-        for c in self.calls:
+        for i, c in enumerate(self.calls):
             op = c[0]
-            if op == 'conv':
+            if i in self.tc:
+                _, xin, li, L, out, fuse, _res = c
+                cw = self.packed[li]
+                geometry, act_bytes, wt = self.tc[i]
+                rc = lib.ds_tc_conv2d(xin.data_ptr(), cw.data.data_ptr(), self.bias[li].data_ptr(), out.data_ptr(),
+                                      *geometry, cw.bits, cw.base, fuse, self.tc_act.data_ptr(), act_bytes,
+                                      wt.data_ptr(), wt.numel(), stream)
+                _ffi.check(rc, "tc_conv2d")
+            elif op == 'conv':
                 _, xin, li, L, out, fuse, _res = c
                 B, C, H, W = xin.shape
                 cw = self.packed[li]

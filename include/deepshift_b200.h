@@ -251,6 +251,37 @@ int ds_conv2d_prepare(const int32_t *packed, int B, int C, int H, int W, int OC,
                       long long *bytes_needed, void *stream);
 
 /*
+ * ---- Tensor-core path -----------------------------------------------------------------------------
+ *
+ * The same convolution (and linear layer: B = M, C = K, H = W = KH = KW = 1, strides 1, no padding) on the
+ * tensor cores, for 16-bit activations and right shifts (base == 0): results are bit-identical to
+ * ds_conv2d_ex / ds_linear_ex.  x + 2^15 is split into a low and a high byte plane (`act`), the weights are
+ * expanded to 16 bytes each (`weights`, about 16 * KH * ceil16(KW * C) * ceil(OC / tile) * tile bytes), and
+ * sixteen byte products per shift-accumulate replace the shift (see csrc/ds_tc.cuh).
+ *
+ * Activations must be known or found to fit 16 bits:
+ *   DS_IN_F32_CONV, DS_IN_I32_CLAMP   with I + F <= 16 (F + 2 <= 16 when I == 1);
+ *   DS_IN_I32                         with act_bits 1..15, or DS_ACT_BITS_AUTO;
+ *   DS_IN_F32_LINEAR                  with I + F <= 16.
+ * For the last two the packing pass looks at every code; when one does not fit, the tensor-core launch
+ * returns at once and the integer-path launch enqueued behind it does the work.  fuse->workspace and
+ * fuse->prepared are not used.
+ *
+ * ds_tc_bytes     sizes of `act` (scratch of one call, any contents, reusable in stream order) and `weights`;
+ *                 both 0 when the call is not served, or, unless any_size, has too little work to be worth it.
+ * ds_tc_expand    fills `weights` for one geometry; may be kept as long as the packed weights do not change.
+ * ds_tc_conv2d    the call.  Both buffers 16-byte aligned and at least as long as ds_tc_bytes said.  Enqueues
+ *                 two kernels (four with the measured range); works under stream capture.
+ */
+int ds_tc_bytes(int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits, int base,
+                const ds_fuse_t *fuse, int any_size, long long *act_bytes, long long *weight_bytes);
+int ds_tc_expand(const int32_t *packed, int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw, int ph,
+                 int pw, int bits, int base, void *weights, long long weight_bytes, void *stream);
+int ds_tc_conv2d(const void *x, const int32_t *packed, const int32_t *bias, void *out, int B, int C, int H, int W,
+                 int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits, int base, const ds_fuse_t *fuse,
+                 void *act, long long act_bytes, const void *weights, long long weight_bytes, void *stream);
+
+/*
  * ---- Staged activations: the TMA-fed convolution path (no counterpart in the reference) ----------
  *
  * For a chain of shift layers (a whole network) the activations can stay in the form the FP32-pipe

@@ -1,0 +1,155 @@
+"""The tensor-core path (ds_tc_*) against the CPU oracle: all results are integers, all comparisons exact."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from helpers import acts_q16, acts_wide, weights
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(dev, x, shift, sign, bias, s, p, *, in_kind=0, act_bits=15, out_f32=False, relu=False, residual=None, I=4, F=12,
+         round_f32=False):
+    """One call of any size through the C ABI, scratch and weights in buffers of exactly the asked size."""
+    from deepshift_b200 import _ffi, kernels, utils
+    B, C, H, W = x.shape
+    OC, _, KH, KW = shift.shape
+    cw = utils.compress_bits(torch.from_numpy(shift).float(), torch.from_numpy(sign).float(), device=dev)
+    geo = (B, C, H, W, OC, KH, KW, s[0], s[1], p[0], p[1])
+    OH, OW = (H + 2 * p[0] - KH) // s[0] + 1, (W + 2 * p[1] - KW) // s[1] + 1
+    xt = torch.from_numpy(x).to(dev)
+    bt = torch.from_numpy(bias).to(dev) if bias is not None else None
+    rt = torch.from_numpy(residual).to(dev) if residual is not None else None
+    f = kernels._fuse(in_kind, 1 if out_f32 else 0, I, F, relu=relu, act_bits=act_bits, residual=rt, round_f32=round_f32)
+    act, wt = kernels.tc_bytes(geo, cw, f, any_size=True)
+    assert act > 0 and wt > 0
+    weights_ = kernels.tc_expand(geo, cw, wt, dev)
+    scratch = torch.full((act + 64,), 0xA5, dtype=torch.uint8, device=dev)
+    out = torch.full((B * OC * OH * OW + 16,), 0x5EADBEE, dtype=torch.int32, device=dev)
+    rc = _ffi.lib().ds_tc_conv2d(xt.data_ptr(), cw.data.data_ptr(), bt.data_ptr() if bt is not None else None,
+                                 out.data_ptr(), *geo, cw.bits, cw.base, f, scratch.data_ptr(), act, weights_.data_ptr(),
+                                 wt, torch.cuda.current_stream(dev).cuda_stream)
+    assert rc == 0
+    torch.cuda.synchronize(dev)
+    assert kernels.last_kernel_error() == 0
+    assert bool((scratch[act:] == 0xA5).all()) and bool((out[-16:] == 0x5EADBEE).all())
+    y = out[:-16].reshape(B, OC, OH, OW)
+    return (y.view(torch.float32) if out_f32 else y).cpu().numpy()
+
+
+# (B, C, H, W, OC, KH, KW, stride, pad): edges of the 128-row blocks and of the 32 / 64 / 128-column tiles,
+# pixel widths of 4, 8 and 16 bytes, windows whose rows are no multiple of 16 bytes, K split over CTAs
+SHAPES = [(1, 16, 4, 4, 16, 1, 1, (1, 1), (0, 0)), (2, 3, 9, 11, 5, 3, 3, (1, 1), (1, 1)), (1, 1, 28, 28, 20, 5, 5, (1, 1), (0, 0)),
+          (3, 20, 12, 12, 50, 5, 5, (1, 1), (0, 0)), (2, 45, 31, 29, 70, 3, 3, (2, 2), (1, 1)),
+          (2, 3, 32, 32, 64, 7, 7, (2, 2), (3, 3)), (1, 64, 16, 8, 128, 3, 3, (1, 1), (1, 1)),
+          (1, 64, 16, 8, 129, 3, 3, (1, 1), (1, 1)), (5, 33, 13, 10, 257, 1, 1, (2, 2), (0, 0)),
+          (2, 512, 7, 7, 512, 3, 3, (1, 1), (1, 1)), (3, 17, 6, 9, 33, 2, 3, (1, 2), (1, 0)),
+          (40, 32, 28, 28, 64, 3, 3, (1, 1), (1, 1)), (33, 16, 32, 32, 16, 3, 3, (1, 1), (1, 1))]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_conv(oracle, cuda_device, shape):
+    B, C, H, W, OC, KH, KW, s, p = shape
+    rng = np.random.default_rng(sum(shape[:7]))
+    x = rng.integers(-16384, 16385, (B, C, H, W)).astype(np.int32)
+    shift, sign = weights(rng, (OC, C, KH, KW))
+    bias = rng.integers(-2000, 2000, OC).astype(np.int32)
+    got = _run(cuda_device, x, shift, sign, bias, s, p)
+    assert np.array_equal(got, oracle.conv2d(x, shift, sign, bias, s, p))
+
+
+@pytest.mark.parametrize("mkn", [(1, 64, 10), (127, 100, 31), (128, 2047, 1001), (129, 16, 64), (300, 4096, 130),
+                                 (1000, 33, 65), (640, 800, 500)])
+def test_linear_full_16_bit_range(oracle, cuda_device, mkn):
+    """Codes over the whole 16-bit range, its ends among them, found to fit while packing."""
+    M, K, N = mkn
+    rng = np.random.default_rng(M + K + N)
+    x = rng.integers(-32768, 32768, (M, K, 1, 1)).astype(np.int32)
+    x.flat[::7] = -32768
+    x.flat[3::11] = 32767
+    shift, sign = weights(rng, (N, K, 1, 1))
+    got = _run(cuda_device, x, shift, sign, None, (1, 1), (0, 0), act_bits=-1)
+    want = oracle.linear(x.reshape(M, K), shift.reshape(N, K), sign.reshape(N, K), None)
+    assert np.array_equal(got.reshape(M, N), want)
+
+
+@pytest.mark.parametrize("value", [32768, -32769, 1 << 30])
+def test_one_wide_code_sends_the_call_to_the_integer_path(oracle, cuda_device, value):
+    rng = np.random.default_rng(5)
+    x = acts_q16(rng, (3, 20, 9, 10))
+    x[2, 19, 8, 9] = value
+    shift, sign = weights(rng, (40, 20, 3, 3))
+    got = _run(cuda_device, x, shift, sign, None, (1, 1), (1, 1), act_bits=-1)
+    assert np.array_equal(got, oracle.conv2d(x, shift, sign, None, (1, 1), (1, 1)))
+    xl = acts_q16(rng, (90, 70, 1, 1))
+    xl[89, 69] = value
+    sl, gl = weights(rng, (33, 70, 1, 1))
+    got = _run(cuda_device, xl, sl, gl, None, (1, 1), (0, 0), act_bits=-1)
+    assert np.array_equal(got.reshape(90, 33), oracle.linear(xl.reshape(90, 70), sl.reshape(33, 70), gl.reshape(33, 70), None))
+
+
+@pytest.mark.parametrize("out_f32", [False, True])
+@pytest.mark.parametrize("geo", [(4, 24, 10, 10, 70, 3), (200, 96, 1, 1, 40, 1), (3, 256, 5, 5, 130, 3)])
+def test_clamped_input_residual_relu_rounding(oracle, cuda_device, geo, out_f32):
+    B, C, H, W, OC, k = geo
+    rng = np.random.default_rng(sum(geo))
+    x = acts_wide(rng, (B, C, H, W), 20)
+    shift, sign = weights(rng, (OC, C, k, k))
+    bias = rng.integers(-2000, 2000, OC).astype(np.int32)
+    res = rng.integers(-50000, 50000, (B, OC, H, W)).astype(np.int32)
+    got = _run(cuda_device, x, shift, sign, bias, (1, 1), (k // 2, k // 2), in_kind=3, act_bits=0, relu=True, residual=res,
+               out_f32=out_f32, round_f32=True)
+    acc = oracle.conv2d(np.clip(x, -32768, 28672), shift, sign, bias, (1, 1), (k // 2, k // 2))
+    v = np.maximum((acc.astype(np.float32) + res.astype(np.float32)).astype(np.int32), 0)
+    want = v.astype(np.float32) / np.float32(4096) if out_f32 else v
+    assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("IF", [(4, 12), (1, 14), (3, 8)])
+def test_fp32_input_is_quantised_while_packing(oracle, cuda_device, IF):
+    I, F = IF
+    rng = np.random.default_rng(I * 100 + F)
+    x = (rng.normal(0, 3, (3, 18, 11, 7))).astype(np.float32)
+    x[0, 0, 0, :4] = [0.0, -0.0, np.inf, -np.inf]
+    shift, sign = weights(rng, (35, 18, 3, 3))
+    codes = (np.sign(x) - 1) * 2 ** F if I == 1 else np.clip(np.floor(x * 2.0 ** F), -2 ** (I - 1 + F), (2 ** (I - 1) - 1) * 2 ** F)
+    got = _run(cuda_device, x, shift, sign, None, (1, 1), (1, 1), in_kind=1, act_bits=0, I=I, F=F)
+    assert np.array_equal(got, oracle.conv2d(codes.astype(np.int32), shift, sign, None, (1, 1), (1, 1)))
+
+
+@pytest.mark.parametrize("bits", [2, 3, 4, 5])
+def test_every_packing(oracle, cuda_device, bits):
+    """All field widths, without zero weights, and every right shift of the width."""
+    rng = np.random.default_rng(bits)
+    x = rng.integers(-32768, 32768, (70, 96, 1, 1)).astype(np.int32)
+    shift = -rng.integers(0, 2 ** bits, (48, 96, 1, 1)).astype(np.int32)
+    sign = rng.choice([-1, 1], (48, 96, 1, 1)).astype(np.int32)
+    shift[0, 0] = -(2 ** bits - 1)
+    got = _run(cuda_device, x, shift, sign, None, (1, 1), (0, 0), act_bits=-1)
+    assert np.array_equal(got.reshape(70, 48), oracle.linear(x.reshape(70, 96), shift.reshape(48, 96), sign.reshape(48, 96), None))
+
+
+def test_sizes_and_refusals(cuda_device):
+    from deepshift_b200 import _ffi, kernels, utils
+    rng = np.random.default_rng(1)
+    shift, sign = weights(rng, (64, 64, 3, 3))
+    cw = utils.compress_bits(torch.from_numpy(shift).float(), torch.from_numpy(sign).float(), device=cuda_device)
+    geo = (8, 64, 28, 28, 64, 3, 3, 1, 1, 1, 1)
+    assert kernels.tc_bytes(geo, cw, kernels._fuse(0, 0, act_bits=-1))[0] > 0
+    assert kernels.tc_bytes((1,) + geo[1:], cw, kernels._fuse(0, 0, act_bits=-1))[0] == 0      # too little work
+    for f in (kernels._fuse(0, 0, act_bits=16), kernels._fuse(0, 0, act_bits=0), kernels._fuse(3, 0, 5, 12),
+              kernels._fuse(2, 0, 16, 16)):
+        assert kernels.tc_bytes(geo, cw, f, any_size=True) == (0, 0)
+    left = utils.ConcWeight(cw.data, -1, cw.bits)
+    assert kernels.tc_bytes(geo, left, kernels._fuse(0, 0, act_bits=-1), any_size=True) == (0, 0)
+    f = kernels._fuse(0, 0, act_bits=-1)
+    act, wt = kernels.tc_bytes(geo, cw, f)
+    buf = torch.empty(max(act, wt), dtype=torch.uint8, device=cuda_device)
+    st = torch.cuda.current_stream(cuda_device).cuda_stream
+    assert _ffi.lib().ds_tc_expand(cw.data.data_ptr(), *geo, cw.bits, 0, buf.data_ptr(), wt - 1, st) == 6
+    assert _ffi.lib().ds_tc_expand(cw.data.data_ptr(), *geo, cw.bits, -1, buf.data_ptr(), wt, st) == 2
+    x = torch.zeros(geo[:4], dtype=torch.int32, device=cuda_device)
+    assert _ffi.lib().ds_tc_conv2d(x.data_ptr(), cw.data.data_ptr(), None, x.data_ptr(), *geo, cw.bits, 0, f, buf.data_ptr(),
+                                   act - 1, buf.data_ptr(), wt, st) == 6
