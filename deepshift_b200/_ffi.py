@@ -57,6 +57,8 @@ _SIGNATURES = {
     "ds_tc_expand": [_VP] + [_I] * 13 + [_VP, _LL, _VP],
     "ds_tc_conv2d": [_VP, _VP, _VP, _VP] + [_I] * 13 + [ctypes.POINTER(Fuse), _VP, _LL, _VP, _LL, _VP],
     "ds_compress": [_VP, _VP, _VP, _I, _I, _I, _I, _VP],
+    "ds_pack_range_f32": [_VP, _VP, _LL, _VP, _VP],
+    "ds_pack_f32": [_VP, _VP, _VP, _I, _I, _I, _I, _VP],
     "ds_quantize_f32": [_VP, _VP, _LL, _I, _I, _I, _VP],
     "ds_maxpool2d_i32": [_VP, _VP, _I, _I, _I, _I, _I, _I, _I, _VP],
     "ds_add_relu_f32": [_VP, _VP, _LL, _I, _VP],

@@ -1,5 +1,6 @@
 // Weight packing, the standalone quantiser, the issue-rate probe and the status strings.
 #include <climits>
+#include <type_traits>
 
 #include "ds_common.cuh"
 
@@ -33,6 +34,96 @@ __global__ void compress_kernel(const int32_t* __restrict__ shiftp, const int32_
         }
         packed[i] = int32_t(value);
     }
+}
+
+// ---- packing straight from a layer's fp32 parameters ----
+// Right shift of one weight as compress_bits stores it: rint(-shift), 32 for a zero sign.
+__device__ __forceinline__ float pack_shift(float shift, float sign) { return sign == 0.f ? 32.f : rintf(-shift); }
+
+// Largest right shift r[0], largest negated one r[1] (r starts at 0x80808080), r[2] = 1 when a value is no
+// integer of at most 24 bits (NaN, infinity).  HBM-bound: one read of both tensors.
+__global__ void __launch_bounds__(256) pack_range_kernel(const float* __restrict__ shift, const float* __restrict__ sign,
+                                                         long long n, int* r)
+{
+    int hi = INT_MIN, nlo = INT_MIN;
+    bool bad = false;
+    auto see = [&](float a, float g) {
+        const float v = pack_shift(a, g);
+        if (fabsf(v) <= 16777216.f) {
+            const int i = int(v);
+            hi = max(hi, i);
+            nlo = max(nlo, -i);
+        } else {
+            bad = true;
+        }
+    };
+    const long long t0 = blockIdx.x * 256ll + threadIdx.x, step = gridDim.x * 256ll;
+    const long long n4 = ((reinterpret_cast<uintptr_t>(shift) | reinterpret_cast<uintptr_t>(sign)) & 15u) == 0 ? n / 4 : 0;
+#pragma unroll 2
+    for (long long i = t0; i < n4; i += step) {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(shift) + i), g = __ldg(reinterpret_cast<const float4*>(sign) + i);
+        see(a.x, g.x);
+        see(a.y, g.y);
+        see(a.z, g.z);
+        see(a.w, g.w);
+    }
+    for (long long i = 4 * n4 + t0; i < n; i += step) see(__ldg(shift + i), __ldg(sign + i));
+    hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+    nlo = __reduce_max_sync(0xFFFFFFFFu, nlo);
+    const bool any = __any_sync(0xFFFFFFFFu, bad);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(r, hi);
+        atomicMax(r + 1, nlo);
+        if (any) r[2] = 1;
+    }
+}
+
+// One thread per output word: NUM neighbouring weights of a row, read as NUM / VEC vectors (rows of whole
+// vectors).  HBM-bound: one read of both tensors, one write of the words (4096 x 4096, 7-bit fields: 151 MB).
+template <int NUM, int VEC>
+__global__ void __launch_bounds__(256) pack_f32_kernel(const float* __restrict__ shift, const float* __restrict__ sign,
+                                                       int32_t* __restrict__ packed, long long words, int K, int bits,
+                                                       int base, int row_len)
+{
+    const long long i = blockIdx.x * 256ll + threadIdx.x;
+    if (i >= words) return;
+    const long long oc = i / row_len;
+    const int k0 = int(i - oc * row_len) * NUM;
+    const int len = min(NUM, K - k0);
+    const float* sp = shift + oc * K + k0;
+    const float* gp = sign + oc * K + k0;
+    float a[NUM], g[NUM];
+    if (VEC == 4 && len == NUM) {
+#pragma unroll
+        for (int j = 0; j < NUM / 4; ++j) {
+            *reinterpret_cast<float4*>(a + 4 * j) = __ldg(reinterpret_cast<const float4*>(sp) + j);
+            *reinterpret_cast<float4*>(g + 4 * j) = __ldg(reinterpret_cast<const float4*>(gp) + j);
+        }
+    } else if (VEC == 2 && len == NUM) {
+#pragma unroll
+        for (int j = 0; j < NUM / 2; ++j) {
+            const float2 x = __ldg(reinterpret_cast<const float2*>(sp) + j), y = __ldg(reinterpret_cast<const float2*>(gp) + j);
+            a[2 * j] = x.x;
+            a[2 * j + 1] = x.y;
+            g[2 * j] = y.x;
+            g[2 * j + 1] = y.y;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < NUM; ++j) {
+            a[j] = j < len ? __ldg(sp + j) : 0.f;
+            g[j] = j < len ? __ldg(gp + j) : 0.f;
+        }
+    }
+    uint32_t value = 0;
+#pragma unroll
+    for (int j = 0; j < NUM; ++j) {
+        if (j >= len) break;
+        const uint32_t field = uint32_t(int(pack_shift(a[j], g[j])) - base);
+        const uint32_t pos = (g[j] == 0.f || g[j] >= 1.f) ? 1u : 0u;  // int(sign) > 0, a zero sign counts as +1
+        value |= field << (j * (bits + 1)) | pos << (j * (bits + 1) + bits);
+    }
+    packed[i] = int32_t(value);
 }
 
 __global__ void quantize_kernel(const float* __restrict__ x, int32_t* __restrict__ out, long long n, int kind,
@@ -224,6 +315,49 @@ extern "C" int ds_compress(const int32_t* shiftp, const int32_t* sign, int32_t* 
     const int blocks = int(total / threads + 1 > 148 * 16 ? 148 * 16 : total / threads + 1);
     compress_kernel<<<blocks, threads, 0, static_cast<cudaStream_t>(stream)>>>(shiftp, sign, packed, OC, K, bits,
                                                                              base, num, row_len);
+    note_launch();
+    return cudaGetLastError() == cudaSuccess ? DS_OK : DS_ERR_CUDA;
+}
+
+extern "C" int ds_pack_range_f32(const float* shift, const float* sign, long long n, int* range, void* stream)
+{
+    if (!shift || !sign || !range || n <= 0) return DS_ERR_BAD_ARG;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (cudaMemsetAsync(range, 0x80, 3 * sizeof(int), st) != cudaSuccess) return DS_ERR_CUDA;
+    const long long want = (n / 4 + 255) / 256 + 1;
+    pack_range_kernel<<<unsigned(want > 148 * 8 ? 148 * 8 : want), 256, 0, st>>>(shift, sign, n, range);
+    note_launch();
+    return cudaGetLastError() == cudaSuccess ? DS_OK : DS_ERR_CUDA;
+}
+
+extern "C" int ds_pack_f32(const float* shift, const float* sign, int32_t* packed, int OC, int K, int bits, int base,
+                           void* stream)
+{
+    if (!shift || !sign || !packed || OC <= 0 || K <= 0) return DS_ERR_BAD_ARG;
+    if (bits < 1 || bits > 7) return DS_ERR_UNSUPPORTED;
+    const int num = 32 / (bits + 1);
+    const int row_len = (K + num - 1) / num;
+    const long long words = (long long)OC * row_len;
+    const long long blocks = (words + 255) / 256;
+    if (blocks > 2147483647ll) return DS_ERR_RANGE;
+    const uintptr_t at = reinterpret_cast<uintptr_t>(shift) | reinterpret_cast<uintptr_t>(sign);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    auto go = [&](auto num_tag) {
+        constexpr int NUM = decltype(num_tag)::value;
+        constexpr int V = NUM % 4 == 0 ? 4 : NUM % 2 == 0 ? 2 : 1;
+        if (V > 1 && K % V == 0 && (at & (4 * V - 1)) == 0)
+            pack_f32_kernel<NUM, V><<<unsigned(blocks), 256, 0, st>>>(shift, sign, packed, words, K, bits, base, row_len);
+        else
+            pack_f32_kernel<NUM, 1><<<unsigned(blocks), 256, 0, st>>>(shift, sign, packed, words, K, bits, base, row_len);
+    };
+    switch (num) {
+        case 4: go(std::integral_constant<int, 4>()); break;
+        case 5: go(std::integral_constant<int, 5>()); break;
+        case 6: go(std::integral_constant<int, 6>()); break;
+        case 8: go(std::integral_constant<int, 8>()); break;
+        case 10: go(std::integral_constant<int, 10>()); break;
+        default: go(std::integral_constant<int, 16>()); break;
+    }
     note_launch();
     return cudaGetLastError() == cudaSuccess ? DS_OK : DS_ERR_CUDA;
 }

@@ -265,6 +265,29 @@ def compress_sign_and_shift(shift, sign, comp_size, base, bits, row_length, num)
     return comp_weight
 
 
+def pack_range(shift, sign):
+    """(smallest, largest) right shift of fp32 parameters as ``compress_bits`` stores them, or None when they
+    are not all finite integers of at most 24 bits.  Synchronises (the packing geometry depends on it)."""
+    with torch.cuda.device(shift.device):
+        r = torch.empty(3, dtype=torch.int32, device=shift.device)
+        _ffi.check(_ffi.lib().ds_pack_range_f32(shift.data_ptr(), sign.data_ptr(), shift.numel(), r.data_ptr(),
+                                                _stream_ptr(shift.device)), "pack_range")
+    hi, nlo, bad = r.tolist()
+    return None if bad > 0 else (-nlo, hi)
+
+
+def pack_f32(shift, sign, bits, base):
+    """fp32 (shift, sign) [OC, ...] -> packed int32 words, in one pass."""
+    OC = shift.shape[0]
+    K = shift.numel() // OC
+    num = 32 // (bits + 1)
+    out = torch.empty([(K + num - 1) // num * OC], dtype=torch.int32, device=shift.device)
+    with torch.cuda.device(shift.device):
+        _ffi.check(_ffi.lib().ds_pack_f32(shift.data_ptr(), sign.data_ptr(), out.data_ptr(), OC, K, bits, base,
+                                          _stream_ptr(shift.device)), "pack_f32")
+    return out
+
+
 # ------------------------------------------------------------------------------------------------
 # Fused forms used by the modules and the integer pipeline (no counterpart in the reference,
 # which runs the quantise / convert / ReLU steps as separate torch passes).

@@ -189,6 +189,19 @@ int ds_compress(const int32_t *shiftp, const int32_t *sign, int32_t *packed, int
                 int bits, int base, void *stream);
 
 /*
+ * The same packing straight from a layer's fp32 parameters [OC,K] (utils.py:61-88 without its intermediate
+ * tensors).  A weight's right shift is rint(-shift), 32 where sign == 0; it counts as positive where
+ * sign == 0 or sign >= 1.
+ *   ds_pack_range_f32  range[0] = largest right shift, range[1] = minus the smallest, range[2] = 1 when a
+ *                      value is not an integer of at most 24 bits, else negative (device int32[3]): what the
+ *                      caller chooses bits and base from.
+ *   ds_pack_f32        the words.
+ */
+int ds_pack_range_f32(const float *shift, const float *sign, long long n, int *range, void *stream);
+int ds_pack_f32(const float *shift, const float *sign, int32_t *packed, int OC, int K, int bits, int base,
+                void *stream);
+
+/*
  * round_to_fixed(x, I, F) * 2^F as int32 (utils.py:7-21 + modules.py:153), one pass.
  * kind = DS_IN_F32_CONV (floor + clamp) or DS_IN_F32_LINEAR (trunc, no clamp, modules.py:25).
  */
