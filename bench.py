@@ -338,7 +338,7 @@ def run_ours(args, rank, world, local):
         raise SystemExit("a kernel gave up on a bounded wait during the timed regions: results are undefined")
 
     # ---- per-kernel times of one un-captured pass (CUDA events on the launching stream), for the
-    # roofline of the dominant kernel: the 3x3 convolutions on the warp-specialised FP32-pipe kernel
+    # roofline of the dominant kernel: the 3x3 convolutions on the tensor cores
     roofline = sweep = None
     if rank == 0:
         nograph = W.IntPipeline(net, ws, B, dev, use_graph=False)
@@ -384,19 +384,24 @@ def run_ours(args, rank, world, local):
         achieved = dom_ops / (dom_ms * 1e-3)
         peaks_path = os.path.join(ROOT, "MEASURED_PEAKS.json")
         hbm_peak, hbm_src = 6650.0, "of fallback"
+        bf16_peak, bf16_src = 1590.0, "of fallback"
         if os.path.exists(peaks_path):
             with open(peaks_path) as fh:
-                hbm_peak, hbm_src = float(json.load(fh)["hbm_gbs"]), "of measured"
+                peaks = json.load(fh)
+            hbm_peak, hbm_src = float(peaks["hbm_gbs"]), "of measured"
+            bf16_peak, bf16_src = float(peaks["bf16_tflops"]), "of measured"
+        peak_s8 = 2 * bf16_peak * 1e12 / 32
         roofline = {
-            # the kernel issues one FP32 FMA (round toward -inf) per shift-op: neither HBM nor the
-            # tensor cores bound it, the issue rate of the FMA pipe does
-            "bound": "fp32_fma_issue", "kernel": "3x3 convolutions (%d launches/step)" % dom_n,
-            "achieved": achieved / 1e12, "peak": peak_fma / 1e12, "unit": "Tshift-op/s (1 shift-op = 1 FFMA)",
-            "frac": achieved / peak_fma,
-            "peak_note": "measured live: register-only FFMA.RM probe (ds_pipe_peak mode 2)",
+            # sixteen u8 x s8 products with int32 accumulation per shift-accumulate (csrc/ds_tc.cuh): the rate of
+            # the 8-bit tensor-core MMA bounds it, twice the bf16 rate
+            "bound": "int8_tensor", "kernel": "3x3 convolutions (%d launches/step)" % dom_n,
+            "achieved": achieved / 1e12, "peak": peak_s8 / 1e12, "unit": "Tshift-op/s (1 shift-op = 16 8-bit MACs)",
+            "frac": achieved / peak_s8,
+            "peak_note": "2 x the bf16 GEMM rate (%.0f TFLOP/s, %s) / 32" % (bf16_peak, bf16_src),
+            "fma_issue_peak": peak_fma / 1e12, "fma_issue_frac": achieved / peak_fma,
             "int32_alu_peak": peak_alu / 1e12, "int32_alu_frac": achieved / peak_alu,
-            "int32_alu_note": "the INT32 shift+add probe (ds_pipe_peak mode 0) the target of the path is quoted "
-                              "against; the kernel does not run on that pipe",
+            "int32_alu_note": "the FFMA.RM and INT32 shift+add issue probes (ds_pipe_peak modes 2 and 0): what the "
+                              "same sum costs without tensor cores",
             "avg_launch_ms": dom_ms / dom_n,
             "hbm": {"achieved": dom_bytes / (dom_ms * 1e-3) / 1e9, "peak": hbm_peak, "unit": "GB/s",
                     "frac": dom_bytes / (dom_ms * 1e-3) / 1e9 / hbm_peak, "peak_source": hbm_src,
