@@ -32,6 +32,12 @@ class Staged(ctypes.Structure):
                 ("C", ctypes.c_int), ("halo", ctypes.c_int)]
 
 
+class Planes(ctypes.Structure):
+    """Mirror of ``ds_planes_t``."""
+    _fields_ = [("data", ctypes.c_void_p), ("B", ctypes.c_int), ("H", ctypes.c_int), ("W", ctypes.c_int),
+                ("C", ctypes.c_int), ("halo", ctypes.c_int)]
+
+
 class StagedOut(ctypes.Structure):
     """Mirror of ``ds_staged_out_t``."""
     _fields_ = [
@@ -56,6 +62,9 @@ _SIGNATURES = {
     "ds_tc_bytes": [_I] * 13 + [ctypes.POINTER(Fuse), _I, ctypes.POINTER(_LL), ctypes.POINTER(_LL)],
     "ds_tc_expand": [_VP] + [_I] * 13 + [_VP, _LL, _VP],
     "ds_tc_conv2d": [_VP, _VP, _VP, _VP] + [_I] * 13 + [ctypes.POINTER(Fuse), _VP, _LL, _VP, _LL, _VP],
+    "ds_planes_pack": [_VP, _I, _I, _I, ctypes.POINTER(Planes), _VP],
+    "ds_tc_conv2d_ex": [_VP, ctypes.POINTER(Planes), _VP, _VP, _VP, ctypes.POINTER(Planes)] + [_I] * 13 +
+                       [ctypes.POINTER(Fuse), _VP, _LL, _VP, _LL, _VP],
     "ds_compress": [_VP, _VP, _VP, _I, _I, _I, _I, _VP],
     "ds_pack_range_f32": [_VP, _VP, _LL, _VP, _VP],
     "ds_pack_f32": [_VP, _VP, _VP, _I, _I, _I, _I, _VP],
@@ -104,6 +113,8 @@ def lib():
         l.ds_version.restype = ctypes.c_int
         l.ds_launch_count.argtypes = []
         l.ds_launch_count.restype = ctypes.c_longlong
+        l.ds_planes_bytes.argtypes = [_I] * 5
+        l.ds_planes_bytes.restype = ctypes.c_longlong
         l.ds_staged_bytes.argtypes = [_I] * 5
         l.ds_staged_bytes.restype = ctypes.c_longlong
         _lib = l

@@ -45,7 +45,7 @@ struct TcTile {
 
 template <int BN>
 struct TcSmem {
-    alignas(1024) unsigned char b[TcTile<BN>::STAGES][TcTile<BN>::STAGE];
+    alignas(128) unsigned char b[TcTile<BN>::STAGES][TcTile<BN>::STAGE];
     alignas(8) unsigned long long bfull[TcTile<BN>::STAGES];
     unsigned long long bempty[TcTile<BN>::STAGES];
     unsigned long long afull[TcTile<BN>::WG];
@@ -139,7 +139,7 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 #define TC_R4(v, i) "r"(v[i]), "r"(v[i + 1]), "r"(v[i + 2]), "r"(v[i + 3])
 #define TC_W4(v, i) "=r"(v[i]), "=r"(v[i + 1]), "=r"(v[i + 2]), "=r"(v[i + 3])
 
-__device__ __forceinline__ void tmem_st32(unsigned addr, const unsigned (&v)[32])
+__device__ __forceinline__ void tmem_st32(unsigned addr, const unsigned* v)
 {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
@@ -174,7 +174,7 @@ __device__ __forceinline__ uint4 ld16(const unsigned char* a, int align)
 }
 
 // Planes 0-7 of four values (one byte each of l and h): word q of each plane.
-__device__ __forceinline__ void planes_low(unsigned l, unsigned h, unsigned (&v)[32], int q)
+__device__ __forceinline__ void planes_low(unsigned l, unsigned h, unsigned* v, int q)
 {
     const unsigned b7 = (l >> 7) & 0x01010101u, b15 = (h >> 7) & 0x01010101u;
     v[q] = (l & 0x7F7F7F7Fu) + b7 + 2u * (h & 0x01010101u);  // <= 130: no carry between bytes
@@ -187,7 +187,7 @@ __device__ __forceinline__ void planes_low(unsigned l, unsigned h, unsigned (&v)
     v[28 + q] = (h - b15) + b7;                               // 0..255: b15 set means h >= 128
 }
 
-__device__ __forceinline__ void planes_high(unsigned h, unsigned (&v)[32], int q)
+__device__ __forceinline__ void planes_high(unsigned h, unsigned* v, int q)
 {
     v[q] = h;
     v[4 + q] = (h >> 1) & 0x7F7F7F7Fu;
@@ -227,7 +227,11 @@ __device__ __forceinline__ Unit unit_of(const TcRun& p, int u)
 __device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 // Epilogue of 32 columns of one row: v (the int32 sums) at row m, columns n..n+31.
-__device__ __forceinline__ void tc_store(const TcRun& p, int (&v)[32], const int* colc, int m, int n, long long rowoff)
+// NEXT: the finished codes also (or only, when p.out is null) go into the byte planes of the next layer -- 32
+// channels of one pixel, 32 contiguous bytes per plane and thread.
+template <bool NEXT>
+__device__ __forceinline__ void tc_store(const TcRun& p, int (&v)[32], const int* colc, int m, int n, long long rowoff,
+                                         unsigned nextoff)
 {
     if (m >= p.M) return;
     int* oi = static_cast<int*>(p.out);
@@ -241,6 +245,38 @@ __device__ __forceinline__ void tc_store(const TcRun& p, int (&v)[32], const int
         return a;
     };
     const int live = min(32, p.N - n);
+    if (NEXT) {
+        long long o = rowoff + (long long)n * p.P;
+        unsigned char* nx = p.next + (nextoff + unsigned(n));
+#pragma unroll
+        for (int h = 0; h < 32; h += 16) {
+            if (h >= live) break;  // N is a multiple of 16 here
+            unsigned lw[4], hw[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                int c[4], r[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    r[e] = 0;
+                    const int* ra = p.residual + o + (long long)e * p.P;
+                    if (p.residual && DS_O_OK(p, p.residual, ra, 4)) r[e] = *ra;
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int a = finish(v[h + 4 * q + e] + colc[h + 4 * q + e], r[e]);
+                    if (oi && DS_O_OK(p, oi, oi + o, 4)) oi[o] = a;
+                    c[e] = min(max(a, p.next_lo), p.next_hi) + 32768;
+                    o += p.P;
+                }
+                const unsigned x = __byte_perm(c[0], c[1], 0x5140), y = __byte_perm(c[2], c[3], 0x5140);
+                lw[q] = __byte_perm(x, y, 0x5410);
+                hw[q] = __byte_perm(x, y, 0x7632);
+            }
+            *reinterpret_cast<uint4*>(nx + h) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+            *reinterpret_cast<uint4*>(nx + p.next_plane + h) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+        }
+        return;
+    }
     if (p.P == 1 && (p.N & 3) == 0) {
         const long long o0 = rowoff + n;
 #pragma unroll
@@ -288,12 +324,12 @@ __device__ __forceinline__ void tc_store(const TcRun& p, int (&v)[32], const int
     }
 }
 
-template <int BN, int S>
+template <int BN, int S, bool NEXT>
 __global__ void __launch_bounds__(TcTile<BN>::THREADS, 1) tc_run_kernel(const TcRun p)
 {
     using T = TcTile<BN>;
-    extern __shared__ unsigned char smem_raw[];
-    TcSmem<BN>& s = *reinterpret_cast<TcSmem<BN>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    TcSmem<BN>& s = *reinterpret_cast<TcSmem<BN>*>(smem_raw);
     if (p.gate && *p.gate != p.gate_want) return;  // the other arithmetic path serves this input
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     volatile int* err = &s.err;
@@ -323,15 +359,19 @@ __global__ void __launch_bounds__(TcTile<BN>::THREADS, 1) tc_run_kernel(const Tc
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem = *reinterpret_cast<volatile unsigned*>(&s.tmem);
-    const unsigned tmem_a = tmem + T::ACC_COLS;
+    // All 512 columns belong to this CTA, so its columns start at 0: as a constant the MMA operands' addresses
+    // are immediates.
+    constexpr unsigned tmem = 0;
+    constexpr unsigned tmem_a = tmem + T::ACC_COLS;
+    if (threadIdx.x == 0 && s.tmem != 0) s.err = 1;
+    constexpr bool FIX = S == T::WG;  // every warpgroup has its own row block
 
     if (warp < 4 * T::WG) {
         // ---- producers: expand activations into TMEM -------------------------------------------------
         const int wg = warp >> 2;
         const int row = threadIdx.x & 127;
         const unsigned lane_base = unsigned(warp & 3) << 21;  // TMEM lane (warp % 4) * 32 in bits 16-31
-        unsigned roff[S];
+        unsigned roff[FIX ? 1 : S];
         int u = blockIdx.x, sub = 0, g = 0, g1 = 0, j = 0, kh = 0;
         auto enter = [&]() {
             if (u >= p.units) return;
@@ -342,16 +382,18 @@ __global__ void __launch_bounds__(TcTile<BN>::THREADS, 1) tc_run_kernel(const Tc
             j = g - kh * p.J;
             sub = 0;
 #pragma unroll
-            for (int i = 0; i < S; ++i) {
-                const int m = min(un.m0 + i * TC_ROWS + row, p.M - 1);
+            for (int i = 0; i < (FIX ? 1 : S); ++i) {
+                const int m = min(un.m0 + (FIX ? wg : i) * TC_ROWS + row, p.M - 1);
                 const int b = m / p.P, pp = m - b * p.P;
                 const int oh = pp / p.OW, ow = pp - oh * p.OW;
                 roff[i] = unsigned(b) * p.img_bytes + unsigned(oh) * p.row_step + unsigned(ow) * p.col_step;
             }
         };
         auto step = [&]() {
-            if (++sub < S) return;
-            sub = 0;
+            if (!FIX) {
+                if (++sub < S) return;
+                sub = 0;
+            }
             if (++g == g1) {
                 u += gridDim.x;
                 enter();
@@ -364,37 +406,38 @@ __global__ void __launch_bounds__(TcTile<BN>::THREADS, 1) tc_run_kernel(const Tc
         auto fetch = [&]() {
             unsigned off = roff[0];
 #pragma unroll
-            for (int i = 1; i < S; ++i)
+            for (int i = 1; i < (FIX ? 1 : S); ++i)
                 if (sub == i) off = roff[i];
             const unsigned char* a = p.act + (off + unsigned(kh) * p.kh_step + unsigned(j) * 16u);
             nl = ld16(a, p.align);
             nh = ld16(a + p.plane, p.align);
         };
         enter();
-        for (int i = 0; i < wg && u < p.units; ++i) step();
+        for (int i = 0; !FIX && i < wg && u < p.units; ++i) step();
         if (u < p.units) fetch();
         for (unsigned round = 0; u < p.units;) {
             const uint4 l = nl, h = nh;
 #pragma unroll
-            for (int i = 0; i < T::WG; ++i)
+            for (int i = 0; i < (FIX ? 1 : T::WG); ++i)
                 if (u < p.units) step();
             if (u < p.units) fetch();
-            unsigned v[32];
+            unsigned v[64];
             planes_low(l.x, h.x, v, 0);
             planes_low(l.y, h.y, v, 1);
             planes_low(l.z, h.z, v, 2);
             planes_low(l.w, h.w, v, 3);
-            // one hand-shake per 16 values: two (a slot per eight planes) cost a third of the rate at 128 columns
+            planes_high(h.x, v + 32, 0);
+            planes_high(h.y, v + 32, 1);
+            planes_high(h.z, v + 32, 2);
+            planes_high(h.w, v + 32, 3);
+            // One hand-shake per 16 values (two, a slot per eight planes, cost a third of the rate at 128 columns),
+            // and nothing but the stores between the slot's release and its hand-over.
             if (round > 0 && !bar_wait(&s.aempty[wg], (round - 1) & 1u, err)) u = p.units;
             ++round;
             __syncwarp();
             tc_fence_after();
             tmem_st32(tmem_a + lane_base + wg * 64, v);
-            planes_high(h.x, v, 0);
-            planes_high(h.y, v, 1);
-            planes_high(h.z, v, 2);
-            planes_high(h.w, v, 3);
-            tmem_st32(tmem_a + lane_base + wg * 64 + 32, v);
+            tmem_st32(tmem_a + lane_base + wg * 64 + 32, v + 32);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             tc_fence_before();
             __syncwarp();
@@ -404,6 +447,11 @@ __global__ void __launch_bounds__(TcTile<BN>::THREADS, 1) tc_run_kernel(const Tc
         // ---- epilogue ----------------------------------------------------------------------------------
         const int row = threadIdx.x & 127;
         const unsigned lane_base = unsigned(warp & 3) << 21;
+        auto next_offset = [&](int b, int pp) -> unsigned {
+            if (!NEXT) return 0;
+            const int oh = pp / p.OW;
+            return unsigned(b) * p.next_img + unsigned(oh) * p.next_row + unsigned(pp - oh * p.OW) * p.next_px;
+        };
         unsigned acc = 0;
         int par = 0;
         bool bad = false;
@@ -427,6 +475,7 @@ __global__ void __launch_bounds__(TcTile<BN>::THREADS, 1) tc_run_kernel(const Tc
                 const int m = un.m0 + i * TC_ROWS + row;
                 const int b = m / p.P, pp = m - b * p.P;
                 const long long rowoff = (long long)b * p.OC * p.P + pp;
+                const unsigned nextoff = next_offset(b, pp);
 #pragma unroll 1
                 for (int c = 0; c < BN; c += 32) {
                     int v[32];
@@ -437,7 +486,7 @@ __global__ void __launch_bounds__(TcTile<BN>::THREADS, 1) tc_run_kernel(const Tc
                         if (lane == 0) bar_arrive(&s.accempty[slot]);
                     }
                     if (p.splits == 1) {
-                        tc_store(p, v, &s.colc[par][c], m, un.n0 + c, rowoff);
+                        tc_store<NEXT>(p, v, &s.colc[par][c], m, un.n0 + c, rowoff, nextoff);
                     } else {
                         int* dst = p.partials + ((long long)(un.tile * p.splits + un.sp) * S + i) * (BN * TC_ROWS) +
                                    c * TC_ROWS + row;
@@ -454,11 +503,13 @@ __global__ void __launch_bounds__(TcTile<BN>::THREADS, 1) tc_run_kernel(const Tc
                 epi_bar();
                 if (s.last_flag) {
                     __threadfence();
+                    if (row == 0) p.counters[un.tile] = 0;  // for the next launch
 #pragma unroll 1
                     for (int i = 0; i < S; ++i) {
                         const int m = un.m0 + i * TC_ROWS + row;
                         const int b = m / p.P, pp = m - b * p.P;
                         const long long rowoff = (long long)b * p.OC * p.P + pp;
+                        const unsigned nextoff = next_offset(b, pp);
 #pragma unroll 1
                         for (int c = 0; c < BN; c += 32) {
                             int v[32];
@@ -471,7 +522,7 @@ __global__ void __launch_bounds__(TcTile<BN>::THREADS, 1) tc_run_kernel(const Tc
 #pragma unroll
                                 for (int q = 0; q < 32; ++q) v[q] += __ldcg(src + q * TC_ROWS);
                             }
-                            tc_store(p, v, &s.colc[par][c], m, un.n0 + c, rowoff);
+                            tc_store<NEXT>(p, v, &s.colc[par][c], m, un.n0 + c, rowoff, nextoff);
                         }
                     }
                 }
@@ -511,21 +562,23 @@ __global__ void __launch_bounds__(TcTile<BN>::THREADS, 1) tc_run_kernel(const Tc
                 const unsigned long long bdesc = desc0 + st * unsigned(T::STAGE >> 4);
 #pragma unroll
                 for (int i = 0; i < S; ++i) {
-                    bar_wait(&s.afull[slot], aph, err);
+                    const unsigned sl = FIX ? unsigned(i) : slot;
+                    bar_wait(&s.afull[sl], aph, err);
                     tc_fence_after();
                     if (elect_one()) {
 #pragma unroll
                         for (int q = 0; q < 8; ++q)
-                            tc_mma_i8(d[i], tmem_a + slot * 64 + q * 8, bdesc + q * (2 * BN), idesc, q == 0 ? more : 1u);
-                        tc_commit(&s.aempty[slot]);
+                            tc_mma_i8(d[i], tmem_a + sl * 64 + q * 8, bdesc + q * (2 * BN), idesc, q == 0 ? more : 1u);
+                        tc_commit(&s.aempty[sl]);
                         if (i == S - 1) tc_commit(&s.bempty[st]);
                     }
                     __syncwarp();
-                    if (++slot == unsigned(T::WG)) {
+                    if (!FIX && ++slot == unsigned(T::WG)) {
                         slot = 0;
                         aph ^= 1u;
                     }
                 }
+                if (FIX) aph ^= 1u;
                 more = 1;
                 if (++st == unsigned(T::STAGES)) {
                     st = 0;
@@ -705,7 +758,7 @@ __global__ void __launch_bounds__(256) tc_pack_rows_kernel(const TcPack p)
 
 // ---- weights -> operand tiles -------------------------------------------------------------------------
 // Coefficient of plane f for a right shift r in 0..15 (ds_tc.cuh).
-__device__ __forceinline__ int tc_coef(int r, int f)
+constexpr int tc_coef(int r, int f)
 {
     if (r == 0) return f == 0 ? 1 : (f == 7 || f == 8 || f == 15) ? 127 : f == 9 ? 4 : 0;
     if (r == 1) return f == 1 ? 1 : (f == 7 || f == 8 || f == 15) ? 64 : 0;
@@ -713,6 +766,23 @@ __device__ __forceinline__ int tc_coef(int r, int f)
     if (r == 7) return (f == 7 || f == 8 || f == 15) ? 1 : 0;
     return f == r ? 1 : 0;
 }
+
+// [four planes][code]: the signed coefficients of four planes as the bytes of a word; code 32 is a zero weight.
+struct TcLut {
+    unsigned w[4 * 33];
+};
+constexpr TcLut tc_make_lut()
+{
+    TcLut t = {};
+    for (int q = 0; q < 4; ++q)
+        for (int c = 0; c < 33; ++c)
+            for (int e = 0; e < 4; ++e) {
+                const int v = c == 32 ? 0 : (c & 16 ? -1 : 1) * tc_coef(c & 15, 4 * q + e);
+                t.w[q * 33 + c] |= (unsigned(v) & 255u) << (8 * e);
+            }
+    return t;
+}
+__constant__ TcLut g_tc_lut = tc_make_lut();
 
 // Packed field of weight (n, k): r in 0..15 with bit 4 for a negative weight, or 32 for a zero weight.
 __device__ __forceinline__ int tc_code(const TcExpand& p, unsigned field)
@@ -754,33 +824,24 @@ __global__ void __launch_bounds__(256) tc_expand_kernel(const TcExpand p)
         if (lane == 0) p.colc[n] = int(sum);
         return;
     }
-    __shared__ unsigned lut[4][33];                // [four planes][code]
+    __shared__ unsigned lut[4][33];
     __shared__ __align__(16) unsigned char codes[128 * 16];
     const int g = blockIdx.x;
-    for (int i = threadIdx.x; i < 4 * 33; i += 256) {
-        const int q = i / 33, c = i - q * 33;
-        unsigned w = 0;
-        if (c < 32)
-            for (int e = 0; e < 4; ++e) {
-                int v = tc_coef(c & 15, 4 * q + e);
-                if (c & 16) v = -v;
-                w |= (unsigned(v) & 255u) << (8 * e);
-            }
-        lut[q][c] = w;
-    }
+    for (int i = threadIdx.x; i < 4 * 33; i += 256) lut[0][i] = g_tc_lut.w[i];
+    // a thread keeps its place in the group (and with it the word and the bit position) and walks the columns
     const int kh = g / p.J, j = g - kh * p.J;
-    for (int i = threadIdx.x; i < p.BN * 16; i += 256) {
-        const int e = i & 15, n = n0 + (i >> 4);
-        const int t = 16 * j + e;  // byte of the window row: (kw, c)
-        const int kw = t / p.Cp, c = t - kw * p.Cp;
+    const int t = 16 * j + (threadIdx.x & 15);  // byte of the window row: (kw, c)
+    const int kw = t / p.Cp, c = t - kw * p.Cp;
+    const bool live = kw < p.KW && c < p.C;
+    const int k = (c * p.KH + kh) * p.KW + kw;
+    const int w = k / p.dec.num, at = (k - w * p.dec.num) * p.dec.fw;
+    const int nl0 = threadIdx.x >> 4;
+    const int* src = p.packed + (long long)(n0 + nl0) * p.dec.row_len + w;
+#pragma unroll 8
+    for (int nl = nl0; nl < p.BN; nl += 16, src += 16ll * p.dec.row_len) {
         int code = 32;
-        if (n < p.N && kw < p.KW && c < p.C) {
-            const int k = (c * p.KH + kh) * p.KW + kw;
-            const int w = k / p.dec.num;
-            const int* src = p.packed + (long long)n * p.dec.row_len + w;
-            if (DS_W_OK(p, src, 4)) code = tc_code(p, (unsigned(__ldg(src)) >> ((k - w * p.dec.num) * p.dec.fw)) & fmask);
-        }
-        codes[i] = (unsigned char)code;
+        if (live && n0 + nl < p.N && DS_W_OK(p, src, 4)) code = tc_code(p, (unsigned(__ldg(src)) >> at) & fmask);
+        codes[nl * 16 + (threadIdx.x & 15)] = (unsigned char)code;
     }
     __syncthreads();
     uint4* out = reinterpret_cast<uint4*>(p.wexp + ((long long)blockIdx.y * p.G + g) * (p.BN * TC_PLANES * TC_KG));
@@ -806,15 +867,15 @@ __global__ void __launch_bounds__(256) tc_expand_kernel(const TcExpand p)
     }
 }
 
-template <int BN, int S>
+template <int BN, int S, bool NEXT>
 int run_cfg(const TcRun& p0, cudaStream_t st)
 {
     TcRun p = p0;
     p.err_flag = kernel_error_flag();
     const int dev = device_slot();
     if (!p.err_flag || dev < 0) return DS_ERR_CUDA;
-    auto kern = tc_run_kernel<BN, S>;
-    const size_t smem = sizeof(TcSmem<BN>) + 1024;
+    auto kern = tc_run_kernel<BN, S, NEXT>;
+    const size_t smem = sizeof(TcSmem<BN>);
     static bool done[kMaxDevices];  // per instantiation and device
     static int sms[kMaxDevices];
     if (!done[dev]) {
@@ -866,11 +927,17 @@ int tc_launch_expand(const TcExpand& p, int grid_n, cudaStream_t st)
     return cudaGetLastError() == cudaSuccess ? DS_OK : DS_ERR_CUDA;
 }
 
+template <bool NEXT>
+static int tc_launch_next(const TcRun& p, int BN, int S, cudaStream_t st)
+{
+    if (BN == 128) return S == 2 ? run_cfg<128, 2, NEXT>(p, st) : run_cfg<128, 1, NEXT>(p, st);
+    if (BN == 64) return S == 3 ? run_cfg<64, 3, NEXT>(p, st) : run_cfg<64, 1, NEXT>(p, st);
+    return S == 3 ? run_cfg<32, 3, NEXT>(p, st) : run_cfg<32, 1, NEXT>(p, st);
+}
+
 int tc_launch_run(const TcRun& p, int BN, int S, cudaStream_t st)
 {
-    if (BN == 128) return S == 2 ? run_cfg<128, 2>(p, st) : run_cfg<128, 1>(p, st);
-    if (BN == 64) return S == 2 ? run_cfg<64, 2>(p, st) : run_cfg<64, 1>(p, st);
-    return S == 3 ? run_cfg<32, 3>(p, st) : run_cfg<32, 1>(p, st);
+    return p.next ? tc_launch_next<true>(p, BN, S, st) : tc_launch_next<false>(p, BN, S, st);
 }
 
 }  // namespace ds

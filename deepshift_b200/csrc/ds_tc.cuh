@@ -28,6 +28,11 @@ namespace ds {
 constexpr int TC_ROWS = 128;    // rows (TMEM lanes) of one MMA
 constexpr int TC_PLANES = 16;   // functions f_p per value
 constexpr int TC_KG = 16;       // values of k per group: one 16-byte run of each plane
+// Scratch header: the range flag, then the arrival counters of split tiles (K is split only below 2 x 148
+// tiles).  At a fixed place, so that calls of different geometry may share a scratch buffer: the counters are
+// zero before and after every call.
+constexpr int TC_HEADER = 2048;
+constexpr int TC_MAX_SPLIT_TILES = (TC_HEADER - 16) / 4;
 
 // Geometry and tiling of one call; a pure function of its arguments (weights expanded for a geometry
 // fit every later call of the same geometry).
@@ -40,14 +45,14 @@ struct TcGeom {
     long long plane;     // bytes of one byte plane
     int BN, S;           // tile: S x 128 rows, BN columns
     int grid_m, grid_n, splits, gps;  // gps: groups per split
-    long long act_bytes;      // both planes, then counters, then partial sums
-    long long counters_off, partials_off;
+    long long act_bytes;      // scratch of one call: header, partial sums, both planes
+    long long planes_off;
     long long weight_bytes;   // expanded weights, then the column constants
     long long colc_off;
 };
 
 struct TcRun {
-    const unsigned char* act;
+    const unsigned char* act;   // pixel (0, -ph, -pw) of the l plane
     long long plane;
     const unsigned char* wexp;
     const int* colc;
@@ -57,6 +62,11 @@ struct TcRun {
     int M, N, P, OC, OW, G, J, align;
     unsigned img_bytes, row_step, col_step, kh_step;  // byte offsets inside a plane
     int grid_m, grid_n, splits, gps, units, m_fast;
+    // byte planes of the layer that reads this output (null: none); `next` is the pixel (0, 0, 0) of the l plane
+    unsigned char* next;
+    long long next_plane;
+    unsigned next_img, next_row, next_px;  // byte steps of an image, a row, a pixel
+    int next_lo, next_hi;                  // clamp of that layer's quantiser
     int* counters;
     int* partials;
     int out_kind, relu, requant, round_f32;

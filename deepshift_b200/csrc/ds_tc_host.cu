@@ -48,7 +48,7 @@ void choose_tile(TcGeom& g)
     const int bns[3] = {128, 64, 32};
     for (int bn : bns) {
         if (bn > 32 && g.N <= bn / 2) continue;
-        const int smax = bn == 32 ? 3 : 2;  // row blocks that share a weight tile, and that TMEM holds twice
+        const int smax = bn == 128 ? 2 : 3;  // row blocks that share a weight tile
         for (int s = 1; s <= smax; s += smax - 1) {
             const long long gm = (g.M + s * TC_ROWS - 1ll) / (s * TC_ROWS), gn = (g.N + bn - 1) / bn;
             const double epi = s * TC_ROWS * (double)bn * 4 / 23;
@@ -102,10 +102,9 @@ int tc_geometry(TcGeom& g, int B, int C, int H, int W, int OC, int KH, int KW, i
     choose_tile(g);
     const long long tiles = (long long)g.grid_m * g.grid_n;
     if (tiles * g.splits > limit || g.grid_n > 65535) return DS_ERR_UNSUPPORTED;
-    const long long counters = g.splits > 1 ? tiles : 0;
-    g.counters_off = 2 * g.plane;
-    g.partials_off = round16(g.counters_off + 16 + counters * 4);  // 16: the range flag comes first
-    g.act_bytes = g.partials_off + (g.splits > 1 ? tiles * g.splits * (long long)g.S * TC_ROWS * g.BN * 4 : 0);
+    if (g.splits > 1 && tiles > TC_MAX_SPLIT_TILES) return DS_ERR_UNSUPPORTED;
+    g.planes_off = TC_HEADER + (g.splits > 1 ? tiles * g.splits * (long long)g.S * TC_ROWS * g.BN * 4 : 0);
+    g.act_bytes = g.planes_off + 2 * g.plane;
     g.colc_off = (long long)g.grid_n * g.G * g.BN * TC_PLANES * TC_KG;
     g.weight_bytes = g.colc_off + round16(4ll * g.N);
     return DS_OK;
@@ -177,16 +176,76 @@ extern "C" int ds_tc_expand(const int32_t* packed, int B, int C, int H, int W, i
     return tc_launch_expand(p, g.grid_n, static_cast<cudaStream_t>(stream));
 }
 
-extern "C" int ds_tc_conv2d(const void* x, const int32_t* packed, const int32_t* bias, void* out, int B, int C, int H,
-                            int W, int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits, int base,
-                            const ds_fuse_t* fuse, void* act, long long act_bytes, const void* weights,
-                            long long weight_bytes, void* stream)
+namespace ds {
+namespace {
+
+// A ds_planes_t whose extent fits the 32-bit offsets of the kernels; its plane size in bytes, 0 if malformed.
+long long planes_plane(const ds_planes_t* t)
 {
-    if (!x || !packed || !out || !fuse || !act || !weights) return DS_ERR_BAD_ARG;
+    if (!t || t->B <= 0 || t->H <= 0 || t->W <= 0 || t->C <= 0 || t->C % 16 || t->halo < 0 || t->halo > 31) return 0;
+    const long long px = t->B * (t->H + 2ll * t->halo) * (t->W + 2ll * t->halo);
+    if (t->H > (1 << 20) || t->W > (1 << 20) || px > 0x7FFFFFFFll / t->C - 64) return 0;
+    return round16(px * t->C + 16);
+}
+
+TcPack pack_params(const GemmParams& q, const void* x, unsigned char* act, long long plane, int B, int C, int H, int W,
+                   int ph, int pw, int Cp)
+{
+    TcPack pk = {};
+    pk.x = x;
+    pk.act = act;
+    pk.plane = plane;
+    pk.B = B; pk.C = C; pk.H = H; pk.W = W; pk.ph = ph; pk.pw = pw; pk.Hp = H + 2 * ph; pk.Wp = W + 2 * pw; pk.Cp = Cp;
+    pk.Q = (long long)B * pk.Hp * pk.Wp;
+    pk.in_kind = q.in_kind;
+    pk.q = q.q;
+    pk.rq_lo = q.rq_lo; pk.rq_hi = q.rq_hi; pk.rq_mul = q.rq_mul; pk.rq_add = q.rq_add;
+    pk.chk_x_bytes = (long long)B * C * H * W * 4 - check_shrink_x();
+    pk.chk_status = bounds_status_ptr();
+    return pk;
+}
+
+}  // namespace
+}  // namespace ds
+
+extern "C" long long ds_planes_bytes(int B, int H, int W, int C, int halo)
+{
+    const ds_planes_t t = {nullptr, B, H, W, C, halo};
+    const long long plane = planes_plane(&t);
+    return plane ? 2 * plane : -1;
+}
+
+extern "C" int ds_planes_pack(const void* x, int in_kind, int I, int F, const ds_planes_t* dst, void* stream)
+{
+    const long long plane = planes_plane(dst);
+    if (!x || !plane || !dst->data) return DS_ERR_BAD_ARG;
+    if (reinterpret_cast<uintptr_t>(dst->data) & 15u) return DS_ERR_ALIGN;
+    ds_fuse_t f = {};
+    f.in_kind = in_kind;
+    f.act_integer_bits = I;
+    f.act_fraction_bits = F;
+    if ((in_kind != DS_IN_F32_CONV && in_kind != DS_IN_I32_CLAMP) || tc_mode(f, 1, 0) != TC_DIRECT) return DS_ERR_UNSUPPORTED;
+    GemmParams q = {};
+    bool fp = false;
+    q.K = 1;
+    const int rc = setup_common(q, 1, 0, &f, fp);
+    if (rc) return rc;
+    return tc_launch_pack(pack_params(q, x, static_cast<unsigned char*>(dst->data), plane, dst->B, dst->C, dst->H, dst->W,
+                                      dst->halo, dst->halo, dst->C),
+                          static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int ds_tc_conv2d_ex(const void* x, const ds_planes_t* xp, const int32_t* packed, const int32_t* bias, void* out,
+                               const ds_planes_t* next, int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw,
+                               int ph, int pw, int bits, int base, const ds_fuse_t* fuse, void* act, long long act_bytes,
+                               const void* weights, long long weight_bytes, void* stream)
+{
+    if ((!x && !xp) || (!out && !next) || !packed || !fuse || !act || !weights) return DS_ERR_BAD_ARG;
     if ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(act) | reinterpret_cast<uintptr_t>(weights)) & 15u)
         return DS_ERR_ALIGN;
-    const int mode = tc_mode(*fuse, bits, base);
-    if (mode == TC_NO) return DS_ERR_UNSUPPORTED;
+    if (base != 0) return DS_ERR_UNSUPPORTED;
+    const int mode = xp ? TC_DIRECT : tc_mode(*fuse, bits, base);
+    if (mode == TC_NO || (mode == TC_GATED && next)) return DS_ERR_UNSUPPORTED;
     TcGeom g;
     int rc = tc_geometry(g, B, C, H, W, OC, KH, KW, sh, sw, ph, pw);
     if (rc) return rc;
@@ -200,58 +259,82 @@ extern "C" int ds_tc_conv2d(const void* x, const int32_t* packed, const int32_t*
     if (fuse->residual && (reinterpret_cast<uintptr_t>(fuse->residual) & 3u)) return DS_ERR_ALIGN;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     unsigned char* a = static_cast<unsigned char*>(act);
-    int* flag = reinterpret_cast<int*>(a + g.counters_off);
+    int* flag = static_cast<int*>(act);
     int* counters = flag + 4;
-    const int ncounters = g.splits > 1 ? g.grid_m * g.grid_n : 0;
-
-    TcPack pk = {};
-    pk.x = x;
-    pk.act = a;
-    pk.plane = g.plane;
-    pk.B = g.B; pk.C = g.C; pk.H = g.H; pk.W = g.W; pk.ph = g.ph; pk.pw = g.pw; pk.Hp = g.Hp; pk.Wp = g.Wp; pk.Cp = g.Cp;
-    pk.Q = (long long)g.B * g.Hp * g.Wp;
-    pk.in_kind = q.in_kind;
-    pk.q = q.q;
-    pk.rq_lo = q.rq_lo; pk.rq_hi = q.rq_hi; pk.rq_mul = q.rq_mul; pk.rq_add = q.rq_add;
-    pk.counters = ncounters ? counters : nullptr;
-    pk.ncounters = ncounters;
-    pk.chk_x_bytes = (long long)g.B * g.C * g.H * g.W * 4 - check_shrink_x();
-    pk.chk_status = bounds_status_ptr();
-    if (mode == TC_GATED) {
-        if (cudaMemsetAsync(flag, 0, sizeof(int), st) != cudaSuccess) return DS_ERR_CUDA;
-        pk.flag = flag;
-    }
-    rc = tc_launch_pack(pk, st);
-    if (rc) return rc;
 
     TcRun p = {};
-    p.act = a;
-    p.plane = g.plane;
+    int Hp = g.Hp, Wp = g.Wp;
+    if (xp) {
+        const long long plane = planes_plane(xp);
+        if (!plane || !xp->data || xp->B != B || xp->C != C || xp->H != H || xp->W != W || xp->halo < ph || xp->halo < pw)
+            return DS_ERR_BAD_ARG;
+        if (reinterpret_cast<uintptr_t>(xp->data) & 15u) return DS_ERR_ALIGN;
+        Hp = H + 2 * xp->halo;
+        Wp = W + 2 * xp->halo;
+        p.act = static_cast<const unsigned char*>(xp->data) + ((long long)(xp->halo - ph) * Wp + (xp->halo - pw)) * C;
+        p.plane = plane;
+    } else {
+        p.act = a + g.planes_off;
+        p.plane = g.plane;
+        TcPack pk = pack_params(q, x, a + g.planes_off, g.plane, B, C, H, W, ph, pw, g.Cp);
+        pk.counters = g.splits > 1 ? counters : nullptr;
+        pk.ncounters = g.splits > 1 ? g.grid_m * g.grid_n : 0;
+        if (mode == TC_GATED) {
+            if (cudaMemsetAsync(flag, 0, sizeof(int), st) != cudaSuccess) return DS_ERR_CUDA;
+            p.gate = pk.flag = flag;
+        }
+        rc = tc_launch_pack(pk, st);
+        if (rc) return rc;
+    }
     p.wexp = static_cast<const unsigned char*>(weights);
     p.colc = reinterpret_cast<const int*>(p.wexp + g.colc_off);
     p.bias = bias;
     p.residual = fuse->residual;
     p.out = out;
     p.M = g.M; p.N = g.N; p.P = g.P; p.OC = g.OC; p.OW = g.OW; p.G = g.G; p.J = g.J; p.align = g.align;
-    p.kh_step = unsigned(g.Wp) * unsigned(g.Cp);
-    p.img_bytes = unsigned(g.Hp) * p.kh_step;
+    p.kh_step = unsigned(Wp) * unsigned(g.Cp);
+    p.img_bytes = unsigned(Hp) * p.kh_step;
     p.row_step = unsigned(g.sh) * p.kh_step;
     p.col_step = unsigned(g.sw) * unsigned(g.Cp);
+    if (next) {
+        const long long plane = planes_plane(next);
+        if (!plane || !next->data || next->B != B || next->C != OC || next->H != g.OH || next->W != g.OW) return DS_ERR_BAD_ARG;
+        if (reinterpret_cast<uintptr_t>(next->data) & 15u) return DS_ERR_ALIGN;
+        const int I = fuse->act_integer_bits, F = fuse->act_fraction_bits;
+        if (I < 2 || F < 0 || I + F > 16 || fuse->out_kind != DS_OUT_I32) return DS_ERR_UNSUPPORTED;
+        const unsigned nw = unsigned(next->W + 2 * next->halo), nh = unsigned(next->H + 2 * next->halo);
+        p.next_px = unsigned(OC);
+        p.next_row = nw * unsigned(OC);
+        p.next_img = nh * p.next_row;
+        p.next = static_cast<unsigned char*>(next->data) + ((long long)next->halo * nw + next->halo) * OC;
+        p.next_plane = plane;
+        p.next_lo = -(1 << (I - 1 + F));
+        p.next_hi = ((1 << (I - 1)) - 1) * (1 << F);
+    }
     p.grid_m = g.grid_m; p.grid_n = g.grid_n; p.splits = g.splits; p.gps = g.gps;
     p.units = g.grid_m * g.grid_n * g.splits;
     // neighbouring CTAs share the smaller operand's tiles through L2: rows fastest when the weights are the
     // larger one
     p.m_fast = g.weight_bytes > 2 * g.plane;
     p.counters = counters;
-    p.partials = reinterpret_cast<int*>(a + g.partials_off);
+    p.partials = reinterpret_cast<int*>(a + TC_HEADER);
     p.out_kind = q.out_kind; p.relu = q.relu; p.requant = q.requant; p.round_f32 = q.round_f32;
     p.rq_lo = q.rq_lo; p.rq_hi = q.rq_hi; p.rq_mul = q.rq_mul; p.rq_add = q.rq_add;
     p.inv_scale = q.inv_scale;
-    p.gate = pk.flag;
     p.gate_want = 0;
     p.chk_o_bytes = (long long)g.M * g.N * 4;
     p.chk_status = bounds_status_ptr();
     rc = tc_launch_run(p, g.BN, g.S, st);
     if (rc || mode != TC_GATED) return rc;
     return launch_gated_int(x, packed, bias, out, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, bits, base, fuse, flag, 1, st);
+}
+
+extern "C" int ds_tc_conv2d(const void* x, const int32_t* packed, const int32_t* bias, void* out, int B, int C, int H,
+                            int W, int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits, int base,
+                            const ds_fuse_t* fuse, void* act, long long act_bytes, const void* weights,
+                            long long weight_bytes, void* stream)
+{
+    if (!x || !out) return DS_ERR_BAD_ARG;
+    return ds_tc_conv2d_ex(x, nullptr, packed, bias, out, nullptr, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, bits, base, fuse,
+                           act, act_bytes, weights, weight_bytes, stream);
 }

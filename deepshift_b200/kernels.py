@@ -180,6 +180,19 @@ def tc_serves_fp32_conv(input_shape, weight_shape, stride, padding, conc_weight,
     return tc_bytes(geometry, conc_weight, f)[0] > 0
 
 
+class Planes:
+    """Activations [B, C, H, W] as the byte planes the tensor-core convolutions read (ds_planes_t): C a multiple
+    of 16, ``halo`` border pixels of code 0 (filled here once; layers only write the interior)."""
+
+    def __init__(self, B, C, H, W, halo, device):
+        n = _ffi.lib().ds_planes_bytes(B, H, W, C, halo)
+        if n < 0:
+            raise RuntimeError("no byte planes for shape %s, halo %d" % ((B, C, H, W), halo))
+        self.data = torch.zeros(n, dtype=torch.uint8, device=device)
+        self.data[n // 2:] = 128   # code 0 is 2^15: l = 0, h = 128
+        self.c = _ffi.Planes(self.data.data_ptr(), B, H, W, C, halo)
+
+
 ACT_BITS_AUTO = -1   # DS_ACT_BITS_AUTO: the library measures the range of the activations on the device
 
 

@@ -344,7 +344,6 @@ class IntPipeline(_Pipeline):
         t = {'x': self.x_in}
         fp32 = {'x': True}
         self.calls = []
-        self.tc = {}   # index of a call -> (geometry, scratch bytes, expanded weights)
         n_shift = sum(1 for s in net.steps if s[0] in ('conv', 'linear'))
         seen = 0
         for st in net.steps:
@@ -379,15 +378,15 @@ class IntPipeline(_Pipeline):
                 fuse = kernels._fuse(in_kind, _ffi.OUT_F32 if lastlayer else _ffi.OUT_I32, self.I, self.F,
                                      relu=bool(o.get('relu')), requant=False, residual=res,
                                      round_f32=not lastlayer, workspace=self.workspace)
-                self.calls.append((op, xin, li, L, out, fuse, res))
                 geometry = tuple(xin.shape) + (L.cout, L.k, L.k, L.stride, L.stride, L.pad, L.pad)
                 if op == 'linear':
                     geometry = (xin.shape[0], xin.shape[1], 1, 1, L.cout, 1, 1, 1, 1, 0, 0)
                 act_bytes, weight_bytes = kernels.tc_bytes(geometry, self.packed[li], fuse)
-                if act_bytes:
-                    # tensor cores: weights expanded once, one scratch buffer for all layers of the pass
-                    self.tc[len(self.calls) - 1] = (geometry, act_bytes, kernels.tc_expand(
-                        geometry, self.packed[li], weight_bytes, dev))
+                tc = None
+                if act_bytes:   # tensor cores: weights expanded once for all passes
+                    tc = dict(geometry=geometry, act_bytes=act_bytes, src=None, next=None,
+                              weights=kernels.tc_expand(geometry, self.packed[li], weight_bytes, dev))
+                self.calls.append((op, xin, li, L, out, fuse, res, tc))
                 dst = o.get('dst', 'x')
                 t[dst], fp32[dst] = out, lastlayer
             elif op == 'maxpool':
@@ -416,23 +415,68 @@ class IntPipeline(_Pipeline):
                 self.calls.append(('shortcutA', xin, out, pad))
                 t[st[2]], fp32[st[2]] = out, False
         self.out = t['x']
-        self.tc_act = torch.empty(max([v[1] for v in self.tc.values()], default=0), dtype=torch.uint8, device=dev)
+        self._chain()
+
+    def _chain(self):
+        """Hands activations from one tensor-core convolution to the next as byte planes: a convolution whose
+        output feeds others writes their (clamped) planes in its epilogue, any other producer is followed by one
+        packing pass for all its readers, and int32 codes are only written where something else reads them."""
+        layers = [c for c in self.calls if c[0] in ('conv', 'linear')]
+        # one scratch buffer for all layers of the pass; its header starts at zero and is left at zero
+        self.tc_act = torch.zeros(max([c[7]['act_bytes'] for c in layers if c[7]], default=0), dtype=torch.uint8,
+                                  device=self.device)
+        producer, codes_read, readers = {}, {self.out.data_ptr()}, {}
+        for i, c in enumerate(self.calls):
+            if c[0] in ('conv', 'linear'):
+                _, xin, _, L, out, fuse, res, tc = c
+                if tc and c[0] == 'conv' and L.cin % 16 == 0 and self.I >= 2 and fuse.in_kind == _ffi.IN_I32_CLAMP:
+                    readers.setdefault(xin.data_ptr(), (xin, []))[1].append(i)
+                else:
+                    codes_read.add(xin.data_ptr())
+                if res is not None:
+                    codes_read.add(res.data_ptr())
+            else:
+                out = c[5] if c[0] == 'maxpool' else c[2]
+                codes_read.add(c[1].data_ptr())
+            producer[out.data_ptr()] = i
+        pack_after = {}
+        for ptr, (xin, users) in readers.items():
+            B, C, H, W = xin.shape
+            planes = kernels.Planes(B, C, H, W, max(self.calls[i][3].pad for i in users), self.device)
+            for i in users:
+                c = self.calls[i]
+                c[7]['src'] = planes
+                self.calls[i] = c[:1] + (None,) + c[2:]
+            src = producer[ptr]
+            c = self.calls[src]
+            if c[0] == 'conv' and c[7]:
+                c[7]['next'] = planes
+                if ptr not in codes_read:   # nothing reads the int32 tensor: give it back
+                    self.calls[src] = c[:4] + (None,) + c[5:]
+            else:
+                pack_after[src] = ('planes', xin, planes)
+        calls, self.calls = self.calls, []
+        for i, c in enumerate(calls):
+            self.calls.append(c)
+            if i in pack_after:
+                self.calls.append(pack_after[i])
 
     def _launch_all(self):
         lib = _ffi.lib()
         stream = torch.cuda.current_stream(self.device).cuda_stream
-        for i, c in enumerate(self.calls):
+        for c in self.calls:
             op = c[0]
-            if i in self.tc:
-                _, xin, li, L, out, fuse, _res = c
-                cw = self.packed[li]
-                geometry, act_bytes, wt = self.tc[i]
-                rc = lib.ds_tc_conv2d(xin.data_ptr(), cw.data.data_ptr(), self.bias[li].data_ptr(), out.data_ptr(),
-                                      *geometry, cw.bits, cw.base, fuse, self.tc_act.data_ptr(), act_bytes,
-                                      wt.data_ptr(), wt.numel(), stream)
+            if op in ('conv', 'linear') and c[7]:
+                _, xin, li, _L, out, fuse, _res, tc = c
+                cw, src, nxt, wt = self.packed[li], tc['src'], tc['next'], tc['weights']
+                rc = lib.ds_tc_conv2d_ex(xin.data_ptr() if src is None else None, src.c if src else None,
+                                         cw.data.data_ptr(), self.bias[li].data_ptr(),
+                                         out.data_ptr() if out is not None else None, nxt.c if nxt else None,
+                                         *tc['geometry'], cw.bits, cw.base, fuse, self.tc_act.data_ptr(),
+                                         tc['act_bytes'], wt.data_ptr(), wt.numel(), stream)
                 _ffi.check(rc, "tc_conv2d")
             elif op == 'conv':
-                _, xin, li, L, out, fuse, _res = c
+                _, xin, li, L, out, fuse, _res, _tc = c
                 B, C, H, W = xin.shape
                 cw = self.packed[li]
                 if fuse.prepared is None and fuse.prepared_bytes == 0:
@@ -448,7 +492,7 @@ class IntPipeline(_Pipeline):
                                       cw.base, fuse, stream)
                 _ffi.check(rc, "conv2d_ex")
             elif op == 'linear':
-                _, xin, li, L, out, fuse, _res = c
+                _, xin, li, L, out, fuse, _res, _tc = c
                 cw = self.packed[li]
                 rc = lib.ds_linear_ex(xin.data_ptr(), cw.data.data_ptr(), self.bias[li].data_ptr(), out.data_ptr(),
                                       xin.shape[0], xin.shape[1], L.cout, cw.bits, cw.base, fuse, stream)
@@ -470,6 +514,10 @@ class IntPipeline(_Pipeline):
             elif op == 'shortcutA':
                 _, xin, out, pad = c
                 out[:, pad:pad + xin.shape[1]].copy_(xin[:, :, ::2, ::2])
+            elif op == 'planes':
+                _, xin, planes = c
+                _ffi.check(lib.ds_planes_pack(xin.data_ptr(), _ffi.IN_I32_CLAMP, self.I, self.F, planes.c, stream),
+                           "planes_pack")
 
 
 

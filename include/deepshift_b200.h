@@ -295,6 +295,30 @@ int ds_tc_conv2d(const void *x, const int32_t *packed, const int32_t *bias, void
                  void *act, long long act_bytes, const void *weights, long long weight_bytes, void *stream);
 
 /*
+ * Chains of layers keep their activations as byte planes: the l and h bytes of code + 2^15 after the quantiser
+ * clamp of the layer that reads them, pixel-major, with `halo` border pixels of code 0.  Two planes of
+ * ds_planes_bytes / 2 bytes each.  C must be a multiple of 16; I + F <= 16 and I >= 2.
+ *   ds_planes_pack   fills a tensor, border included, from NCHW (DS_IN_F32_CONV or DS_IN_I32_CLAMP).
+ *   ds_tc_conv2d_ex  ds_tc_conv2d that reads planes (`xp`, halo >= ph, pw) instead of packing `x`, and / or
+ *                    writes the interior of the planes the next layer reads (`next`, clamped with I and F of
+ *                    `fuse`; the border must have been filled once, e.g. by ds_planes_pack of anything).  `out`
+ *                    may be NULL when `next` is given.  With `xp` the first 2048 bytes of `act` must be zero
+ *                    before the first call; every call leaves them zero.
+ */
+typedef struct {
+    void *data;
+    int B, H, W, C, halo;
+} ds_planes_t;
+
+long long ds_planes_bytes(int B, int H, int W, int C, int halo);
+int ds_planes_pack(const void *x, int in_kind, int act_integer_bits, int act_fraction_bits, const ds_planes_t *dst,
+                   void *stream);
+int ds_tc_conv2d_ex(const void *x, const ds_planes_t *xp, const int32_t *packed, const int32_t *bias, void *out,
+                    const ds_planes_t *next, int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw, int ph,
+                    int pw, int bits, int base, const ds_fuse_t *fuse, void *act, long long act_bytes,
+                    const void *weights, long long weight_bytes, void *stream);
+
+/*
  * ---- Staged activations: the TMA-fed convolution path (no counterpart in the reference) ----------
  *
  * For a chain of shift layers (a whole network) the activations can stay in the form the FP32-pipe

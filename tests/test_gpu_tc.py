@@ -153,3 +153,53 @@ def test_sizes_and_refusals(cuda_device):
     x = torch.zeros(geo[:4], dtype=torch.int32, device=cuda_device)
     assert _ffi.lib().ds_tc_conv2d(x.data_ptr(), cw.data.data_ptr(), None, x.data_ptr(), *geo, cw.bits, 0, f, buf.data_ptr(),
                                    act - 1, buf.data_ptr(), wt, st) == 6
+
+
+@pytest.mark.parametrize("geo", [(3, 16, 9, 11, 48, 3, 1, 1, 1), (2, 64, 14, 14, 32, 1, 2, 0, 1), (2, 512, 7, 7, 16, 3, 1, 1, 2),
+                                 (5, 32, 8, 8, 144, 3, 2, 1, 1)])
+@pytest.mark.parametrize("codes", [True, False])
+def test_planes_in_and_out(oracle, cuda_device, geo, codes):
+    """Planes packed with a border wider than the padding, read by a convolution that writes the next layer's
+    planes; a second convolution reads those.  The border of the second tensor stays as it was filled."""
+    from deepshift_b200 import _ffi, kernels, utils
+    B, C, H, W, OC, k, s, p, halo = geo
+    rng = np.random.default_rng(sum(geo))
+    x = acts_wide(rng, (B, C, H, W), 17)
+    shift, sign = weights(rng, (OC, C, k, k))
+    bias = rng.integers(-2000, 2000, OC).astype(np.int32)
+    OH, OW = (H + 2 * p - k) // s + 1, (W + 2 * p - k) // s + 1
+    res = rng.integers(-50000, 50000, (B, OC, OH, OW)).astype(np.int32)
+    s2, g2 = weights(rng, (20, OC, 3, 3))
+    lib, st = _ffi.lib(), torch.cuda.current_stream(cuda_device).cuda_stream
+    cw = utils.compress_bits(torch.from_numpy(shift).float(), torch.from_numpy(sign).float(), device=cuda_device)
+    cw2 = utils.compress_bits(torch.from_numpy(s2).float(), torch.from_numpy(g2).float(), device=cuda_device)
+    xt, bt, rt = (torch.from_numpy(a).to(cuda_device) for a in (x, bias, res))
+    src, nxt = kernels.Planes(B, C, H, W, halo, cuda_device), kernels.Planes(B, OC, OH, OW, 1, cuda_device)
+    assert lib.ds_planes_pack(xt.data_ptr(), _ffi.IN_I32_CLAMP, 4, 12, src.c, st) == 0
+    f = kernels._fuse(_ffi.IN_I32_CLAMP, 0, 4, 12, relu=True, residual=rt, round_f32=True)
+    g1 = (B, C, H, W, OC, k, k, s, s, p, p)
+    gg2 = (B, OC, OH, OW, 20, 3, 3, 1, 1, 1, 1)
+    a1, w1 = kernels.tc_bytes(g1, cw, f, any_size=True)
+    a2, w2 = kernels.tc_bytes(gg2, cw2, f, any_size=True)
+    act = torch.zeros(max(a1, a2), dtype=torch.uint8, device=cuda_device)
+    out = torch.full((B, OC, OH, OW), -7, dtype=torch.int32, device=cuda_device)
+    out2 = torch.empty((B, 20, OH, OW), dtype=torch.int32, device=cuda_device)
+    e1, e2 = kernels.tc_expand(g1, cw, w1, cuda_device), kernels.tc_expand(gg2, cw2, w2, cuda_device)
+    f2 = kernels._fuse(_ffi.IN_I32_CLAMP, 0, 4, 12)
+    for _ in range(2):   # the second pass finds the scratch header as the first left it
+        rc = lib.ds_tc_conv2d_ex(None, src.c, cw.data.data_ptr(), bt.data_ptr(), out.data_ptr() if codes else None, nxt.c, *g1,
+                                 cw.bits, 0, f, act.data_ptr(), a1, e1.data_ptr(), w1, st)
+        assert rc == 0
+        rc = lib.ds_tc_conv2d_ex(None, nxt.c, cw2.data.data_ptr(), None, out2.data_ptr(), None, *gg2, cw2.bits, 0, f2,
+                                 act.data_ptr(), a2, e2.data_ptr(), w2, st)
+        assert rc == 0
+    torch.cuda.synchronize(cuda_device)
+    assert kernels.last_kernel_error() == 0
+    acc = oracle.conv2d(np.clip(x, -32768, 28672), shift, sign, bias, (s, s), (p, p))
+    v = np.maximum((acc.astype(np.float32) + res.astype(np.float32)).astype(np.int32), 0)
+    if codes:
+        assert np.array_equal(out.cpu().numpy(), v)
+    else:
+        assert bool((out == -7).all())
+    assert np.array_equal(out2.cpu().numpy(), oracle.conv2d(np.clip(v, -32768, 28672), s2, g2, None, (1, 1), (1, 1)))
+    assert int(act[:2048].sum()) == 0
