@@ -33,23 +33,26 @@ constexpr int TC_TMEM_COLS = 512;
 // bytes; a slot shared between warpgroups could not be guarded by a phase parity, since a warpgroup may be two
 // phases away from it), and as many accumulator slots as the remaining columns hold.  Two warpgroups keep up with the MMAs
 // of 128 columns (512 cycles per 128 rows x 16 values), three are needed for 64 (256 cycles).
-template <int BN>
+template <int BN, bool WIDE>
 struct TcTile {
-    static constexpr int WG = BN == 128 ? 2 : 3;
+    static constexpr int WG = WIDE || BN == 128 ? 2 : 3;
+    static constexpr int PLANES = WIDE ? TC_PLANES_WIDE : TC_PLANES;
+    static constexpr int ASTRIDE = WIDE ? 96 : 64;   // columns from one A slot to the next
+    static constexpr int ACC = WIDE ? 2 * BN : BN;   // columns of an accumulator slot (wide: sums of weight 2^8 behind)
     static constexpr int THREADS = (4 * WG + 6) * 32;  // + 4 epilogue warps + MMA warp + loader warp
-    static constexpr int ACC_COLS = TC_TMEM_COLS - 64 * WG;
-    static constexpr int NACC = ACC_COLS / BN < 6 ? ACC_COLS / BN : 6;
-    static constexpr int STAGE = BN * TC_PLANES * TC_KG;
+    static constexpr int ACC_COLS = TC_TMEM_COLS - ASTRIDE * WG;
+    static constexpr int NACC = ACC_COLS / ACC < 6 ? ACC_COLS / ACC : 6;
+    static constexpr int STAGE = BN * PLANES * TC_KG;
     static constexpr int STAGES = BN == 128 ? 6 : 8;
 };
 
-template <int BN>
+template <int BN, bool WIDE>
 struct TcSmem {
-    alignas(128) unsigned char b[TcTile<BN>::STAGES][TcTile<BN>::STAGE];
-    alignas(8) unsigned long long bfull[TcTile<BN>::STAGES];
-    unsigned long long bempty[TcTile<BN>::STAGES];
-    unsigned long long afull[TcTile<BN>::WG];
-    unsigned long long aempty[TcTile<BN>::WG];
+    alignas(128) unsigned char b[TcTile<BN, WIDE>::STAGES][TcTile<BN, WIDE>::STAGE];
+    alignas(8) unsigned long long bfull[TcTile<BN, WIDE>::STAGES];
+    unsigned long long bempty[TcTile<BN, WIDE>::STAGES];
+    unsigned long long afull[TcTile<BN, WIDE>::WG];
+    unsigned long long aempty[TcTile<BN, WIDE>::WG];
     unsigned long long accfull[6];
     unsigned long long accempty[6];
     unsigned long long done;
@@ -155,6 +158,14 @@ __device__ __forceinline__ void tmem_ld32(unsigned addr, int (&v)[32])
         "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n\ttcgen05.wait::ld.sync.aligned;"
         : TC_W4(v, 0), TC_W4(v, 4), TC_W4(v, 8), TC_W4(v, 12), TC_W4(v, 16), TC_W4(v, 20), TC_W4(v, 24), TC_W4(v, 28)
         : "r"(addr)
+        : "memory");
+}
+
+__device__ __forceinline__ void tmem_st16(unsigned addr, const unsigned* v)
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(addr),
+        TC_R4(v, 0), TC_R4(v, 4), TC_R4(v, 8), TC_R4(v, 12)
         : "memory");
 }
 
@@ -324,12 +335,12 @@ __device__ __forceinline__ void tc_store(const TcRun& p, int (&v)[32], const int
     }
 }
 
-template <int BN, int S, bool NEXT>
-__global__ void __launch_bounds__(TcTile<BN>::THREADS, 1) tc_run_kernel(const TcRun p)
+template <int BN, int S, bool NEXT, bool WIDE>
+__global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(const TcRun p)
 {
-    using T = TcTile<BN>;
+    using T = TcTile<BN, WIDE>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    TcSmem<BN>& s = *reinterpret_cast<TcSmem<BN>*>(smem_raw);
+    TcSmem<BN, WIDE>& s = *reinterpret_cast<TcSmem<BN, WIDE>*>(smem_raw);
     if (p.gate && *p.gate != p.gate_want) return;  // the other arithmetic path serves this input
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     volatile int* err = &s.err;
@@ -402,7 +413,7 @@ __global__ void __launch_bounds__(TcTile<BN>::THREADS, 1) tc_run_kernel(const Tc
                 ++kh;
             }
         };
-        uint4 nl = make_uint4(0, 0, 0, 0), nh = nl;
+        uint4 nl = make_uint4(0, 0, 0, 0), nh = nl, nt = nl;
         auto fetch = [&]() {
             unsigned off = roff[0];
 #pragma unroll
@@ -411,12 +422,13 @@ __global__ void __launch_bounds__(TcTile<BN>::THREADS, 1) tc_run_kernel(const Tc
             const unsigned char* a = p.act + (off + unsigned(kh) * p.kh_step + unsigned(j) * 16u);
             nl = ld16(a, p.align);
             nh = ld16(a + p.plane, p.align);
+            if (WIDE) nt = ld16(a + 2 * p.plane, p.align);
         };
         enter();
         for (int i = 0; !FIX && i < wg && u < p.units; ++i) step();
         if (u < p.units) fetch();
         for (unsigned round = 0; u < p.units;) {
-            const uint4 l = nl, h = nh;
+            const uint4 l = nl, h = nh, t = nt;
 #pragma unroll
             for (int i = 0; i < (FIX ? 1 : T::WG); ++i)
                 if (u < p.units) step();
@@ -436,8 +448,12 @@ __global__ void __launch_bounds__(TcTile<BN>::THREADS, 1) tc_run_kernel(const Tc
             ++round;
             __syncwarp();
             tc_fence_after();
-            tmem_st32(tmem_a + lane_base + wg * 64, v);
-            tmem_st32(tmem_a + lane_base + wg * 64 + 32, v + 32);
+            tmem_st32(tmem_a + lane_base + wg * T::ASTRIDE, v);
+            tmem_st32(tmem_a + lane_base + wg * T::ASTRIDE + 32, v + 32);
+            if (WIDE) {
+                const unsigned w[16] = {t.x, t.y, t.z, t.w, t.x, t.y, t.z, t.w, t.x, t.y, t.z, t.w, t.x, t.y, t.z, t.w};
+                tmem_st16(tmem_a + lane_base + wg * T::ASTRIDE + 64, w);
+            }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             tc_fence_before();
             __syncwarp();
@@ -479,7 +495,13 @@ __global__ void __launch_bounds__(TcTile<BN>::THREADS, 1) tc_run_kernel(const Tc
 #pragma unroll 1
                 for (int c = 0; c < BN; c += 32) {
                     int v[32];
-                    tmem_ld32(tmem + lane_base + slot * BN + c, v);
+                    tmem_ld32(tmem + lane_base + slot * T::ACC + c, v);
+                    if (WIDE) {
+                        int w[32];
+                        tmem_ld32(tmem + lane_base + slot * T::ACC + BN + c, w);
+#pragma unroll
+                        for (int q = 0; q < 32; ++q) v[q] += int(unsigned(w[q]) << 8);
+                    }
                     if (c + 32 >= BN) {
                         tc_fence_before();
                         __syncwarp();
@@ -549,7 +571,7 @@ __global__ void __launch_bounds__(TcTile<BN>::THREADS, 1) tc_run_kernel(const Tc
 #pragma unroll
             for (int i = 0; i < S; ++i) {
                 accs[i] = aslot;
-                d[i] = tmem + aslot * BN;
+                d[i] = tmem + aslot * T::ACC;
                 bar_wait(&s.accempty[aslot], accph, err);  // the first round finds the slots free
                 if (++aslot == unsigned(T::NACC)) {
                     aslot = 0;
@@ -568,7 +590,13 @@ __global__ void __launch_bounds__(TcTile<BN>::THREADS, 1) tc_run_kernel(const Tc
                     if (elect_one()) {
 #pragma unroll
                         for (int q = 0; q < 8; ++q)
-                            tc_mma_i8(d[i], tmem_a + sl * 64 + q * 8, bdesc + q * (2 * BN), idesc, q == 0 ? more : 1u);
+                            tc_mma_i8(d[i], tmem_a + sl * T::ASTRIDE + q * 8, bdesc + q * (2 * BN), idesc, q == 0 ? more : 1u);
+                        if (WIDE) {
+                            const unsigned at = tmem_a + sl * T::ASTRIDE + 64;
+                            tc_mma_i8(d[i], at, bdesc + 8 * (2 * BN), idesc, 1u);
+                            tc_mma_i8(d[i] + BN, at, bdesc + 9 * (2 * BN), idesc, more);
+                            tc_mma_i8(d[i] + BN, at + 8, bdesc + 10 * (2 * BN), idesc, 1u);
+                        }
                         tc_commit(&s.aempty[sl]);
                         if (i == S - 1) tc_commit(&s.bempty[st]);
                     }
@@ -684,9 +712,9 @@ __global__ void __launch_bounds__(256) tc_pack_nchw_kernel(const TcPack p, int c
         if (q < p.Q) {
             const unsigned qi = unsigned(q);
             const unsigned rowi = qi / unsigned(p.Wp);
-            const int w = int(qi - rowi * unsigned(p.Wp)) - p.pw;
+            const int w = (int(qi - rowi * unsigned(p.Wp)) - p.pw) * p.sub_w;
             const unsigned b = rowi / unsigned(p.Hp);
-            const int h = int(rowi - b * unsigned(p.Hp)) - p.ph;
+            const int h = (int(rowi - b * unsigned(p.Hp)) - p.ph) * p.sub_h;
             if (unsigned(h) < unsigned(p.H) && unsigned(w) < unsigned(p.W)) {
                 const int c = 4 * (cw0 + cw);
                 const int* src = x + ((long long)b * p.C + c) * hw + (long long)h * p.W + w;
@@ -720,7 +748,7 @@ __global__ void __launch_bounds__(256) tc_pack_nchw_kernel(const TcPack p, int c
 }
 
 // Rows of a matrix [Q, C]: 4 values of a row per thread.
-template <int INK>
+template <int INK, bool WIDE>
 __global__ void __launch_bounds__(256) tc_pack_rows_kernel(const TcPack p)
 {
     const unsigned words = unsigned(p.Cp) >> 2;
@@ -729,7 +757,7 @@ __global__ void __launch_bounds__(256) tc_pack_rows_kernel(const TcPack p)
     const unsigned i0 = blockIdx.x * 256u + threadIdx.x;
     if (p.counters)
         for (unsigned i = i0; i < unsigned(p.ncounters); i += gridDim.x * 256u) p.counters[i] = 0;
-    bool over = false;
+    bool over = i0 == 0 && p.refuse && *p.refuse;
     for (unsigned i = i0; i < total; i += gridDim.x * 256u) {
         const unsigned m = i / words, w = i - m * words;
         const int k = int(4 * w);
@@ -748,8 +776,19 @@ __global__ void __launch_bounds__(256) tc_pack_rows_kernel(const TcPack p)
 #pragma unroll
         for (int e = 0; e < 4; ++e) c4[e] = k + e < p.C ? pack_code<INK>(p, raw[e]) : 0;
         unsigned l, h;
-        pack4(c4, l, h, over);
         unsigned* dst = reinterpret_cast<unsigned*>(p.act) + i;
+        if (WIDE) {
+            unsigned y[4], t = 0;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                y[e] = unsigned(c4[e]) + (1u << 23);
+                over |= y[e] >> 24 != 0;
+                t |= ((y[e] >> 16) & 255u) << (8 * e);
+                c4[e] = int(y[e] & 0xFFFFu) - 32768;
+            }
+            *reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(dst) + 2 * p.plane) = t;
+        }
+        pack4(c4, l, h, over);
         *dst = l;
         *reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(dst) + p.plane) = h;
     }
@@ -767,17 +806,29 @@ constexpr int tc_coef(int r, int f)
     return f == r ? 1 : 0;
 }
 
+// Planes 16-21 of a 24-bit value, all copies of t: 2^(16-r) for r >= 9 in planes 16 and 17, 2^(8-r) in planes
+// 18-21 (the accumulator of weight 2^8) for r <= 8.
+constexpr int tc_coef_t(int r, int f)
+{
+    if (f >= 22) return 0;
+    if (f == 16) return r == 9 ? 64 : r > 9 ? 1 << (16 - r) : 0;
+    if (f == 17) return r == 9 ? 64 : 0;
+    if (r == 0) return 64;
+    if (r == 1) return f <= 19 ? 64 : 0;
+    return f == 18 && r <= 8 ? 1 << (8 - r) : 0;
+}
+
 // [four planes][code]: the signed coefficients of four planes as the bytes of a word; code 32 is a zero weight.
 struct TcLut {
-    unsigned w[4 * 33];
+    unsigned w[6 * 33];
 };
 constexpr TcLut tc_make_lut()
 {
     TcLut t = {};
-    for (int q = 0; q < 4; ++q)
+    for (int q = 0; q < 6; ++q)
         for (int c = 0; c < 33; ++c)
             for (int e = 0; e < 4; ++e) {
-                const int v = c == 32 ? 0 : (c & 16 ? -1 : 1) * tc_coef(c & 15, 4 * q + e);
+                const int v = c == 32 ? 0 : (c & 16 ? -1 : 1) * (q < 4 ? tc_coef(c & 15, 4 * q + e) : tc_coef_t(c & 15, 4 * q + e));
                 t.w[q * 33 + c] |= (unsigned(v) & 255u) << (8 * e);
             }
     return t;
@@ -814,7 +865,8 @@ __global__ void __launch_bounds__(256) tc_expand_kernel(const TcExpand p)
             for (int i = 0; i < p.dec.num && k + i < p.K; ++i, word >>= p.dec.fw) {
                 const int c = tc_code(p, word & fmask);
                 if (c < 32) {
-                    const unsigned v = 1u << (15 - (c & 15));
+                    if (p.wide && (word & fmask & ((1u << p.dec.bits) - 1u)) >= 16u) p.colc[p.N] = 1;
+                    const unsigned v = 1u << ((p.wide ? 23 : 15) - (c & 15));
                     sum += (c & 16) ? v : 0u - v;
                 }
             }
@@ -824,10 +876,10 @@ __global__ void __launch_bounds__(256) tc_expand_kernel(const TcExpand p)
         if (lane == 0) p.colc[n] = int(sum);
         return;
     }
-    __shared__ unsigned lut[4][33];
+    __shared__ unsigned lut[6][33];
     __shared__ __align__(16) unsigned char codes[128 * 16];
     const int g = blockIdx.x;
-    for (int i = threadIdx.x; i < 4 * 33; i += 256) lut[0][i] = g_tc_lut.w[i];
+    for (int i = threadIdx.x; i < 6 * 33; i += 256) (&lut[0][0])[i] = g_tc_lut.w[i];
     // a thread keeps its place in the group (and with it the word and the bit position) and walks the columns
     const int kh = g / p.J, j = g - kh * p.J;
     const int t = 16 * j + (threadIdx.x & 15);  // byte of the window row: (kw, c)
@@ -844,8 +896,8 @@ __global__ void __launch_bounds__(256) tc_expand_kernel(const TcExpand p)
         codes[nl * 16 + (threadIdx.x & 15)] = (unsigned char)code;
     }
     __syncthreads();
-    uint4* out = reinterpret_cast<uint4*>(p.wexp + ((long long)blockIdx.y * p.G + g) * (p.BN * TC_PLANES * TC_KG));
-    for (int i = threadIdx.x; i < p.BN * 4; i += 256) {
+    uint4* out = reinterpret_cast<uint4*>(p.wexp + ((long long)blockIdx.y * p.G + g) * (p.BN * (p.wide ? TC_PLANES_WIDE : TC_PLANES) * TC_KG));
+    for (int i = threadIdx.x; i < p.BN * (p.wide ? 6 : 4); i += 256) {
         const int n = i & (p.BN - 1), q = i / p.BN;
         const uint4 cw = *reinterpret_cast<const uint4*>(codes + n * 16);
         const unsigned cws[4] = {cw.x, cw.y, cw.z, cw.w};
@@ -863,19 +915,20 @@ __global__ void __launch_bounds__(256) tc_expand_kernel(const TcExpand p)
             o[3][w] = __byte_perm(y01, y23, 0x7632);
         }
 #pragma unroll
-        for (int f = 0; f < 4; ++f) out[(4 * q + f) * p.BN + n] = make_uint4(o[f][0], o[f][1], o[f][2], o[f][3]);
+        for (int f = 0; f < 4; ++f)
+            if (4 * q + f < TC_PLANES_WIDE) out[(4 * q + f) * p.BN + n] = make_uint4(o[f][0], o[f][1], o[f][2], o[f][3]);
     }
 }
 
-template <int BN, int S, bool NEXT>
+template <int BN, int S, bool NEXT, bool WIDE>
 int run_cfg(const TcRun& p0, cudaStream_t st)
 {
     TcRun p = p0;
     p.err_flag = kernel_error_flag();
     const int dev = device_slot();
     if (!p.err_flag || dev < 0) return DS_ERR_CUDA;
-    auto kern = tc_run_kernel<BN, S, NEXT>;
-    const size_t smem = sizeof(TcSmem<BN>);
+    auto kern = tc_run_kernel<BN, S, NEXT, WIDE>;
+    const size_t smem = sizeof(TcSmem<BN, WIDE>);
     static bool done[kMaxDevices];  // per instantiation and device
     static int sms[kMaxDevices];
     if (!done[dev]) {
@@ -889,18 +942,20 @@ int run_cfg(const TcRun& p0, cudaStream_t st)
         done[dev] = true;
     }
     const int grid = p.units < sms[dev] ? p.units : sms[dev];
-    kern<<<grid, TcTile<BN>::THREADS, smem, st>>>(p);
+    kern<<<grid, TcTile<BN, WIDE>::THREADS, smem, st>>>(p);
     note_launch();
     return cudaGetLastError() == cudaSuccess ? DS_OK : DS_ERR_CUDA;
 }
 
 }  // namespace
 
-int tc_launch_pack(const TcPack& p, cudaStream_t st)
+int tc_launch_pack(const TcPack& p, bool wide, cudaStream_t st)
 {
     auto rows = [&](auto ink) {
         const long long want = (p.Q * (p.Cp / 4) + 255) / 256;
-        tc_pack_rows_kernel<decltype(ink)::value><<<unsigned(want > 148 * 64 ? 148 * 64 : want), 256, 0, st>>>(p);
+        const unsigned grid = unsigned(want > 148 * 64 ? 148 * 64 : want);
+        if (wide) tc_pack_rows_kernel<decltype(ink)::value, true><<<grid, 256, 0, st>>>(p);
+        else tc_pack_rows_kernel<decltype(ink)::value, false><<<grid, 256, 0, st>>>(p);
     };
     auto nchw = [&](auto ink) {
         int lg = 0;
@@ -910,7 +965,7 @@ int tc_launch_pack(const TcPack& p, cudaStream_t st)
         tc_pack_nchw_kernel<decltype(ink)::value><<<grid, 256, 0, st>>>(p, lg);
     };
     auto go = [&](auto ink) {
-        if (p.Hp == 1 && p.Wp == 1) rows(ink);
+        if (p.Hp == 1 && p.Wp == 1 && p.H == 1 && p.W == 1) rows(ink);
         else nchw(ink);
     };
     if (p.in_kind == DS_IN_I32) go(std::integral_constant<int, INK_I32>());
@@ -922,6 +977,7 @@ int tc_launch_pack(const TcPack& p, cudaStream_t st)
 
 int tc_launch_expand(const TcExpand& p, int grid_n, cudaStream_t st)
 {
+    if (p.wide && cudaMemsetAsync(p.colc + p.N, 0, sizeof(int), st) != cudaSuccess) return DS_ERR_CUDA;
     tc_expand_kernel<<<dim3(unsigned(p.G + TC_COLC_BLOCKS), unsigned(grid_n)), 256, 0, st>>>(p);
     note_launch();
     return cudaGetLastError() == cudaSuccess ? DS_OK : DS_ERR_CUDA;
@@ -930,13 +986,14 @@ int tc_launch_expand(const TcExpand& p, int grid_n, cudaStream_t st)
 template <bool NEXT>
 static int tc_launch_next(const TcRun& p, int BN, int S, cudaStream_t st)
 {
-    if (BN == 128) return S == 2 ? run_cfg<128, 2, NEXT>(p, st) : run_cfg<128, 1, NEXT>(p, st);
-    if (BN == 64) return S == 3 ? run_cfg<64, 3, NEXT>(p, st) : run_cfg<64, 1, NEXT>(p, st);
-    return S == 3 ? run_cfg<32, 3, NEXT>(p, st) : run_cfg<32, 1, NEXT>(p, st);
+    if (BN == 128) return S == 2 ? run_cfg<128, 2, NEXT, false>(p, st) : run_cfg<128, 1, NEXT, false>(p, st);
+    if (BN == 64) return S == 3 ? run_cfg<64, 3, NEXT, false>(p, st) : run_cfg<64, 1, NEXT, false>(p, st);
+    return S == 3 ? run_cfg<32, 3, NEXT, false>(p, st) : run_cfg<32, 1, NEXT, false>(p, st);
 }
 
-int tc_launch_run(const TcRun& p, int BN, int S, cudaStream_t st)
+int tc_launch_run(const TcRun& p, int BN, int S, bool wide, cudaStream_t st)
 {
+    if (wide) return run_cfg<64, 1, false, true>(p, st);
     return p.next ? tc_launch_next<true>(p, BN, S, st) : tc_launch_next<false>(p, BN, S, st);
 }
 

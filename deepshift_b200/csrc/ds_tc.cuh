@@ -20,6 +20,11 @@
 // 256 of the high byte (r = 0) does not fit an s8 operand; f_0, f_7 and f_9 are chosen so that two nearly
 // equal high-byte functions carry 127 each.  r in 16..31 equals r = 15 for 16-bit x, r >= 32 is a zero
 // weight.
+//
+// Wider codes (linear layers with unclamped activations): for |x| < 2^23, y = x + 2^23 has a third byte t and
+//     y >> r = ((256 h + l) >> r) + 2^(16-r) t       (r = 0..15),
+// so two more products with plane t go into the same sum (r >= 9: coefficients up to 128 as 64 + 64) and four
+// into a second accumulator of weight 2^8 (r <= 8: up to 256 as four times 64).
 #pragma once
 #include "ds_gemm_common.cuh"
 
@@ -27,6 +32,7 @@ namespace ds {
 
 constexpr int TC_ROWS = 128;    // rows (TMEM lanes) of one MMA
 constexpr int TC_PLANES = 16;   // functions f_p per value
+constexpr int TC_PLANES_WIDE = 22;  // ... of one 24-bit value: planes 16-21 are copies of t
 constexpr int TC_KG = 16;       // values of k per group: one 16-byte run of each plane
 // Scratch header: the range flag, then the arrival counters of split tiles (K is split only below 2 x 148
 // tiles).  At a fixed place, so that calls of different geometry may share a scratch buffer: the counters are
@@ -39,10 +45,12 @@ constexpr int TC_MAX_SPLIT_TILES = (TC_HEADER - 16) / 4;
 struct TcGeom {
     int B, C, H, W, OC, KH, KW, sh, sw, ph, pw, OH, OW;
     int M, N, K, P;
+    int sub_h, sub_w;    // packing takes every sub-th pixel: the strides of a 1x1 window, else 1
     int Hp, Wp, Cp;      // padded image and bytes per pixel of one byte plane (l or h) of the activations
     int J, G;            // groups per window row: ceil(KW * Cp / 16); groups in all: KH * J
     int align;           // every load starts at a multiple of this: 16, 8 or 4
     long long plane;     // bytes of one byte plane
+    int wide;            // 24-bit codes: three byte planes
     int BN, S;           // tile: S x 128 rows, BN columns
     int grid_m, grid_n, splits, gps;  // gps: groups per split
     long long act_bytes;      // scratch of one call: header, partial sums, both planes
@@ -84,11 +92,13 @@ struct TcPack {
     unsigned char* act;
     long long plane;
     int B, C, H, W, ph, pw, Hp, Wp, Cp;
+    int sub_h, sub_w;    // source pixel of (h, w): (h * sub_h, w * sub_w)
     long long Q;         // padded pixels
     int in_kind;
     Quant q;
     int rq_lo, rq_hi, rq_mul, rq_add;
-    int* flag;           // set to 1 when a code does not fit 16 bits; null = no check
+    int* flag;           // set to 1 when a code does not fit 16 (24) bits; null = no check
+    const int* refuse;   // wide: not zero when the weights hold a shift of 16..31; null = no such word
     int* counters;       // zeroed here for the launch behind
     int ncounters;
     long long chk_x_bytes;
@@ -101,6 +111,7 @@ struct TcExpand {
     int* colc;
     Decode dec;
     int C, KH, KW, Cp, J, G, N, K, BN;
+    int wide;            // 22 planes; colc[N] is set when a weight has a shift of 16..31
     long long chk_w_bytes;
     int* chk_status;
 };
@@ -113,8 +124,8 @@ int launch_gated_int(const void* x, const int32_t* packed, const int32_t* bias, 
                      const int* gate, int want, cudaStream_t st);
 long long check_shrink_x();
 
-int tc_launch_pack(const TcPack& p, cudaStream_t st);
+int tc_launch_pack(const TcPack& p, bool wide, cudaStream_t st);
 int tc_launch_expand(const TcExpand& p, int grid_n, cudaStream_t st);
-int tc_launch_run(const TcRun& p, int BN, int S, cudaStream_t st);
+int tc_launch_run(const TcRun& p, int BN, int S, bool wide, cudaStream_t st);
 
 }  // namespace ds

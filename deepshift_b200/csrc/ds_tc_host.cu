@@ -32,12 +32,11 @@ void choose_pixel(TcGeom& g)
     while (g.align > 4 && ((g.Cp * g.sw) % g.align || ((long long)g.Wp * g.Cp) % g.align)) g.align >>= 1;
 }
 
-// Clock cycles of one (group, 128 rows) item: eight MMAs of BN / 2 cycles, or what the producers need for
-// one item when that is longer.
-double item_cycles(int bn, int s)
+// Clock cycles of one (group, 128 rows) item: eight MMAs (eleven when wide).
+double item_cycles(int bn, int s, bool wide)
 {
-    if (bn == 128) return s == 1 ? 640 : 530;  // one row block: the weight tile comes from L2 for 128 rows only
-    return bn == 64 ? 290 : 240;
+    if (wide) return 800;
+    return bn == 128 ? 810 : 690;  // measured; 64 and 32 columns cost the same
 }
 
 // Tile and split with the smallest estimated time: waves of units over the SMs, a unit being the longer of
@@ -47,9 +46,10 @@ void choose_tile(TcGeom& g)
     double best = 1e30;
     const int bns[3] = {128, 64, 32};
     for (int bn : bns) {
-        if (bn > 32 && g.N <= bn / 2) continue;
+        if (g.wide ? bn != 64 : bn > 32 && g.N <= bn / 2) continue;
         const int smax = bn == 128 ? 2 : 3;  // row blocks that share a weight tile
         for (int s = 1; s <= smax; s += smax - 1) {
+            if (g.wide && s > 1) continue;  // two accumulators per row block
             const long long gm = (g.M + s * TC_ROWS - 1ll) / (s * TC_ROWS), gn = (g.N + bn - 1) / bn;
             const double epi = s * TC_ROWS * (double)bn * 4 / 23;
             for (int sp = 1; sp <= 16; ++sp) {
@@ -58,9 +58,9 @@ void choose_tile(TcGeom& g)
                 if (sp > 1 && gm * gn >= 2 * kSms) break;
                 const long long units = gm * gn * sp;
                 const double waves = double((units + kSms - 1) / kSms);
-                const double main = gps * s * item_cycles(bn, s) + 400;
+                const double main = gps * s * item_cycles(bn, s, g.wide) + 1500;  // ... and the pipeline's fill
                 double cost = waves * (main > epi ? main : epi) + (main > epi ? epi : main) + 3000;
-                if (sp > 1) cost += 2500 + sp * epi * 0.5;
+                if (sp > 1) cost += 3000 + 800.0 * sp * s * (bn / 32);  // the last CTA reads all partial sums
                 if (cost < best) {
                     best = cost;
                     g.BN = bn;
@@ -76,7 +76,7 @@ void choose_tile(TcGeom& g)
 }
 
 // Fills the geometry; DS_ERR_UNSUPPORTED when 32-bit offsets do not reach.
-int tc_geometry(TcGeom& g, int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw, int ph, int pw)
+int tc_geometry(TcGeom& g, int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw, int ph, int pw, bool wide)
 {
     if (B < 0 || C <= 0 || H <= 0 || W <= 0 || OC <= 0 || KH <= 0 || KW <= 0 || sh <= 0 || sw <= 0 || ph < 0 || pw < 0)
         return DS_ERR_BAD_ARG;
@@ -84,9 +84,20 @@ int tc_geometry(TcGeom& g, int B, int C, int H, int W, int OC, int KH, int KW, i
     if ((long long)H + 2ll * ph < KH || (long long)W + 2ll * pw < KW) return DS_ERR_BAD_ARG;
     if (B == 0) return DS_ERR_UNSUPPORTED;
     g = TcGeom{};
+    g.wide = wide;
+    if (wide && !(H == 1 && W == 1 && KH == 1 && KW == 1 && ph == 0 && pw == 0)) return DS_ERR_UNSUPPORTED;  // linear layers
     g.B = B; g.C = C; g.H = H; g.W = W; g.OC = OC; g.KH = KH; g.KW = KW; g.sh = sh; g.sw = sw; g.ph = ph; g.pw = pw;
-    const long long hp = (long long)H + 2ll * ph, wp = (long long)W + 2ll * pw;
+    long long hp = (long long)H + 2ll * ph, wp = (long long)W + 2ll * pw;
     const long long oh = (hp - KH) / sh + 1, ow = (wp - KW) / sw + 1;
+    g.sub_h = g.sub_w = 1;
+    if (KH == 1 && KW == 1 && ph == 0 && pw == 0) {
+        // a strided 1x1 window reads only these pixels (256 x 64 x 56 x 56, stride 2: 252 us with all packed)
+        g.sub_h = sh;
+        g.sub_w = sw;
+        g.sh = g.sw = 1;
+        hp = oh;
+        wp = ow;
+    }
     if (hp > (1 << 20) || wp > (1 << 20) || (long long)C * KH * KW > (1ll << 30)) return DS_ERR_UNSUPPORTED;
     const long long M = B * oh * ow, K = (long long)C * KH * KW;
     // what ds_conv2d_ex refuses with DS_ERR_RANGE stays with it
@@ -104,16 +115,17 @@ int tc_geometry(TcGeom& g, int B, int C, int H, int W, int OC, int KH, int KW, i
     if (tiles * g.splits > limit || g.grid_n > 65535) return DS_ERR_UNSUPPORTED;
     if (g.splits > 1 && tiles > TC_MAX_SPLIT_TILES) return DS_ERR_UNSUPPORTED;
     g.planes_off = TC_HEADER + (g.splits > 1 ? tiles * g.splits * (long long)g.S * TC_ROWS * g.BN * 4 : 0);
-    g.act_bytes = g.planes_off + 2 * g.plane;
-    g.colc_off = (long long)g.grid_n * g.G * g.BN * TC_PLANES * TC_KG;
-    g.weight_bytes = g.colc_off + round16(4ll * g.N);
+    g.act_bytes = g.planes_off + (wide ? 3 : 2) * g.plane;
+    g.colc_off = (long long)g.grid_n * g.G * g.BN * (wide ? TC_PLANES_WIDE : TC_PLANES) * TC_KG;
+    g.weight_bytes = g.colc_off + round16(4ll * g.N + 4);  // the word behind: a shift of 16..31 exists (wide)
     return DS_OK;
 }
 
 enum { TC_NO = 0, TC_DIRECT, TC_GATED };
 
 // Whether the activations of this call are known to fit 16 bits (TC_DIRECT), may fit (TC_GATED: measured on
-// the device while packing, the integer path stands behind) or cannot be served.
+// the device while packing, the integer path stands behind) or cannot be served.  LinearShift's entry conversion
+// does not clamp, so its codes pass 16 bits as soon as |x| >= 2^(15-F): they take the 24-bit form.
 int tc_mode(const ds_fuse_t& f, int bits, int base)
 {
     if (base != 0 || bits < 1 || bits > 7) return TC_NO;
@@ -125,9 +137,28 @@ int tc_mode(const ds_fuse_t& f, int bits, int base)
             return f.act_bits >= 1 && f.act_bits <= 15 ? TC_DIRECT : TC_NO;  // 16 promises |x| <= 2^15, one too many
         case DS_IN_F32_CONV:
         case DS_IN_I32_CLAMP: return I >= 1 && F >= 0 && code_bits <= 16 ? TC_DIRECT : TC_NO;
-        case DS_IN_F32_LINEAR: return I >= 1 && F >= 0 && I + F <= 16 ? TC_GATED : TC_NO;
+        case DS_IN_F32_LINEAR: return F >= 0 && F <= 30 ? TC_GATED : TC_NO;
         default: return TC_NO;
     }
+}
+
+// Whether the tensor cores beat the other paths, packing included.  Measured, us, other path -> this one:
+//   linear, fp32 input (weights expanded once): 64 x 784 -> 512 120 -> 19, 17 x 512 -> 512 83 -> 18, 1024 x 500
+//     -> 10 80 -> 19: the integer path behind it runs one CTA per 64 x 128 outputs over all of K, 0.16 us per k.
+//     Up to 16 rows the small-batch kernel takes 10 to 15.
+//   linear, int32 input (expanded per call): 256 x 512 -> 1000 86 -> 28, 1024 x 800 -> 500 108 -> 37; up to 64 rows
+//     the integer path splits K and is faster (64 x 784 -> 512 21 -> 26).
+//   convolution: 128 -> 128 channels, 28 x 28, one image 103 -> 19; 1x1 stride 2, 64 -> 128, one image 32 -> 12:
+//     few 256-row tiles leave the other path's SMs idle.  With many tiles it pays from about 2^26 shift-accumulates
+//     (16 -> 16 channels, 32 x 32, 64 images 40 -> 24), and not where most of the padded product is padding
+//     (1 -> 20 channels, 5x5: a tenth is live, 110 -> 135).
+bool worthwhile(const TcGeom& g, int in_kind)
+{
+    const double ops = (double)g.M * g.N * g.K;
+    if (g.H == 1 && g.W == 1 && g.KH == 1 && g.KW == 1) return g.K >= 128 && g.M > (in_kind == DS_IN_F32_LINEAR ? 16 : 64);
+    const long long tiles = ((g.M + 255ll) / 256) * ((g.N + 127) / 128);
+    const double padded = (double)g.grid_m * g.S * TC_ROWS * g.grid_n * g.BN * g.G * TC_KG;
+    return tiles <= 16 ? ops >= 6e6 : ops >= double(1 << 26) && ops * 5 >= padded;
 }
 
 }  // namespace
@@ -142,23 +173,24 @@ extern "C" int ds_tc_bytes(int B, int C, int H, int W, int OC, int KH, int KW, i
     *act_bytes = *weight_bytes = 0;
     if (tc_mode(*fuse, bits, base) == TC_NO) return DS_OK;
     TcGeom g;
-    const int rc = tc_geometry(g, B, C, H, W, OC, KH, KW, sh, sw, ph, pw);
+    const int rc = tc_geometry(g, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, fuse->in_kind == DS_IN_F32_LINEAR);
     if (rc == DS_ERR_UNSUPPORTED) return DS_OK;
     if (rc) return rc;
-    if (!any_size && ((double)g.M * g.N * g.K < double(1 << 26) || g.M <= 64)) return DS_OK;
+    if (!any_size && !worthwhile(g, fuse->in_kind)) return DS_OK;
     *act_bytes = g.act_bytes;
     *weight_bytes = g.weight_bytes;
     return DS_OK;
 }
 
 extern "C" int ds_tc_expand(const int32_t* packed, int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw,
-                            int ph, int pw, int bits, int base, void* weights, long long weight_bytes, void* stream)
+                            int ph, int pw, int bits, int base, const ds_fuse_t* fuse, void* weights,
+                            long long weight_bytes, void* stream)
 {
-    if (!packed || !weights) return DS_ERR_BAD_ARG;
+    if (!packed || !weights || !fuse) return DS_ERR_BAD_ARG;
     if (base != 0 || bits < 1 || bits > 7) return DS_ERR_UNSUPPORTED;
     if (reinterpret_cast<uintptr_t>(weights) & 15u) return DS_ERR_ALIGN;
     TcGeom g;
-    const int rc = tc_geometry(g, B, C, H, W, OC, KH, KW, sh, sw, ph, pw);
+    const int rc = tc_geometry(g, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, fuse->in_kind == DS_IN_F32_LINEAR);
     if (rc) return rc;
     if (weight_bytes < g.weight_bytes) return DS_ERR_SCRATCH;
     TcExpand p = {};
@@ -171,6 +203,7 @@ extern "C" int ds_tc_expand(const int32_t* packed, int B, int C, int H, int W, i
     p.dec.base = 0;
     p.dec.row_len = (g.K + p.dec.num - 1) / p.dec.num;
     p.C = g.C; p.KH = g.KH; p.KW = g.KW; p.Cp = g.Cp; p.J = g.J; p.G = g.G; p.N = g.N; p.K = g.K; p.BN = g.BN;
+    p.wide = g.wide;
     p.chk_w_bytes = (long long)g.N * p.dec.row_len * 4;
     p.chk_status = bounds_status_ptr();
     return tc_launch_expand(p, g.grid_n, static_cast<cudaStream_t>(stream));
@@ -189,13 +222,14 @@ long long planes_plane(const ds_planes_t* t)
 }
 
 TcPack pack_params(const GemmParams& q, const void* x, unsigned char* act, long long plane, int B, int C, int H, int W,
-                   int ph, int pw, int Cp)
+                   int ph, int pw, int Hp, int Wp, int Cp, int sub_h, int sub_w)
 {
     TcPack pk = {};
     pk.x = x;
     pk.act = act;
     pk.plane = plane;
-    pk.B = B; pk.C = C; pk.H = H; pk.W = W; pk.ph = ph; pk.pw = pw; pk.Hp = H + 2 * ph; pk.Wp = W + 2 * pw; pk.Cp = Cp;
+    pk.B = B; pk.C = C; pk.H = H; pk.W = W; pk.ph = ph; pk.pw = pw; pk.Hp = Hp; pk.Wp = Wp; pk.Cp = Cp;
+    pk.sub_h = sub_h; pk.sub_w = sub_w;
     pk.Q = (long long)B * pk.Hp * pk.Wp;
     pk.in_kind = q.in_kind;
     pk.q = q.q;
@@ -231,8 +265,8 @@ extern "C" int ds_planes_pack(const void* x, int in_kind, int I, int F, const ds
     const int rc = setup_common(q, 1, 0, &f, fp);
     if (rc) return rc;
     return tc_launch_pack(pack_params(q, x, static_cast<unsigned char*>(dst->data), plane, dst->B, dst->C, dst->H, dst->W,
-                                      dst->halo, dst->halo, dst->C),
-                          static_cast<cudaStream_t>(stream));
+                                      dst->halo, dst->halo, dst->H + 2 * dst->halo, dst->W + 2 * dst->halo, dst->C, 1, 1),
+                          false, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int ds_tc_conv2d_ex(const void* x, const ds_planes_t* xp, const int32_t* packed, const int32_t* bias, void* out,
@@ -245,9 +279,10 @@ extern "C" int ds_tc_conv2d_ex(const void* x, const ds_planes_t* xp, const int32
         return DS_ERR_ALIGN;
     if (base != 0) return DS_ERR_UNSUPPORTED;
     const int mode = xp ? TC_DIRECT : tc_mode(*fuse, bits, base);
-    if (mode == TC_NO || (mode == TC_GATED && next)) return DS_ERR_UNSUPPORTED;
+    if (mode == TC_NO || (mode == TC_GATED && next) || (xp && fuse->in_kind == DS_IN_F32_LINEAR)) return DS_ERR_UNSUPPORTED;
     TcGeom g;
-    int rc = tc_geometry(g, B, C, H, W, OC, KH, KW, sh, sw, ph, pw);
+    const bool wide = !xp && fuse->in_kind == DS_IN_F32_LINEAR;
+    int rc = tc_geometry(g, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, wide);
     if (rc) return rc;
     if (act_bytes < g.act_bytes || weight_bytes < g.weight_bytes) return DS_ERR_SCRATCH;
     // the quantiser and clamp constants, checked as for every other path
@@ -259,11 +294,14 @@ extern "C" int ds_tc_conv2d_ex(const void* x, const ds_planes_t* xp, const int32
     if (fuse->residual && (reinterpret_cast<uintptr_t>(fuse->residual) & 3u)) return DS_ERR_ALIGN;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     unsigned char* a = static_cast<unsigned char*>(act);
+    int* counters = static_cast<int*>(act) + 4;
+    // the range flag: the last counter word of the workspace, as for the other paths, else the scratch's first word
     int* flag = static_cast<int*>(act);
-    int* counters = flag + 4;
+    if (fuse->workspace && fuse->workspace_bytes >= (long long)kWorkspaceCounters * 4)
+        flag = static_cast<int*>(fuse->workspace) + kWorkspaceGateSlot;
 
     TcRun p = {};
-    int Hp = g.Hp, Wp = g.Wp;
+    int Hp = g.Hp, Wp = g.Wp, step_h = g.sh, step_w = g.sw;
     if (xp) {
         const long long plane = planes_plane(xp);
         if (!plane || !xp->data || xp->B != B || xp->C != C || xp->H != H || xp->W != W || xp->halo < ph || xp->halo < pw)
@@ -271,19 +309,22 @@ extern "C" int ds_tc_conv2d_ex(const void* x, const ds_planes_t* xp, const int32
         if (reinterpret_cast<uintptr_t>(xp->data) & 15u) return DS_ERR_ALIGN;
         Hp = H + 2 * xp->halo;
         Wp = W + 2 * xp->halo;
+        step_h = sh;
+        step_w = sw;
         p.act = static_cast<const unsigned char*>(xp->data) + ((long long)(xp->halo - ph) * Wp + (xp->halo - pw)) * C;
         p.plane = plane;
     } else {
         p.act = a + g.planes_off;
         p.plane = g.plane;
-        TcPack pk = pack_params(q, x, a + g.planes_off, g.plane, B, C, H, W, ph, pw, g.Cp);
+        TcPack pk = pack_params(q, x, a + g.planes_off, g.plane, B, C, H, W, ph, pw, g.Hp, g.Wp, g.Cp, g.sub_h, g.sub_w);
         pk.counters = g.splits > 1 ? counters : nullptr;
         pk.ncounters = g.splits > 1 ? g.grid_m * g.grid_n : 0;
         if (mode == TC_GATED) {
             if (cudaMemsetAsync(flag, 0, sizeof(int), st) != cudaSuccess) return DS_ERR_CUDA;
             p.gate = pk.flag = flag;
         }
-        rc = tc_launch_pack(pk, st);
+        if (wide) pk.refuse = reinterpret_cast<const int*>(static_cast<const unsigned char*>(weights) + g.colc_off) + g.N;
+        rc = tc_launch_pack(pk, wide, st);
         if (rc) return rc;
     }
     p.wexp = static_cast<const unsigned char*>(weights);
@@ -294,8 +335,8 @@ extern "C" int ds_tc_conv2d_ex(const void* x, const ds_planes_t* xp, const int32
     p.M = g.M; p.N = g.N; p.P = g.P; p.OC = g.OC; p.OW = g.OW; p.G = g.G; p.J = g.J; p.align = g.align;
     p.kh_step = unsigned(Wp) * unsigned(g.Cp);
     p.img_bytes = unsigned(Hp) * p.kh_step;
-    p.row_step = unsigned(g.sh) * p.kh_step;
-    p.col_step = unsigned(g.sw) * unsigned(g.Cp);
+    p.row_step = unsigned(step_h) * p.kh_step;
+    p.col_step = unsigned(step_w) * unsigned(g.Cp);
     if (next) {
         const long long plane = planes_plane(next);
         if (!plane || !next->data || next->B != B || next->C != OC || next->H != g.OH || next->W != g.OW) return DS_ERR_BAD_ARG;
@@ -324,7 +365,7 @@ extern "C" int ds_tc_conv2d_ex(const void* x, const ds_planes_t* xp, const int32
     p.gate_want = 0;
     p.chk_o_bytes = (long long)g.M * g.N * 4;
     p.chk_status = bounds_status_ptr();
-    rc = tc_launch_run(p, g.BN, g.S, st);
+    rc = tc_launch_run(p, g.BN, g.S, wide, st);
     if (rc || mode != TC_GATED) return rc;
     return launch_gated_int(x, packed, bias, out, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, bits, base, fuse, flag, 1, st);
 }

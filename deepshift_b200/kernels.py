@@ -104,7 +104,7 @@ def _fuse(in_kind=0, out_kind=0, act_integer_bits=0, act_fraction_bits=0, relu=F
 
 
 # ------------------------------------------------------------------------------------------------
-# Tensor-core path (ds_tc_*): 16-bit activations, right shifts.  A geometry is (B, C, H, W, OC, KH, KW, sh,
+# Tensor-core path (ds_tc_*): 16-bit activations (24-bit ones for linear layers on fp32), right shifts.  A geometry is (B, C, H, W, OC, KH, KW, sh,
 # sw, ph, pw); a linear layer [M,K] x [N,K] is the 1x1 convolution (M, K, 1, 1, N, 1, 1, 1, 1, 0, 0).
 
 def tc_bytes(geometry, conc_weight, fuse, any_size=False):
@@ -116,26 +116,26 @@ def tc_bytes(geometry, conc_weight, fuse, any_size=False):
     return act.value, wt.value
 
 
-def tc_expand(geometry, conc_weight, nbytes, device):
-    """The layer's weights as the operand tiles of this geometry, in a new buffer."""
+def tc_expand(geometry, conc_weight, fuse, nbytes, device):
+    """The layer's weights as the operand tiles of this geometry and input kind, in a new buffer."""
     buf = torch.empty(nbytes, dtype=torch.uint8, device=device)
     _ffi.check(_ffi.lib().ds_tc_expand(conc_weight.data.data_ptr(), *geometry, conc_weight.bits, conc_weight.base,
-                                       buf.data_ptr(), nbytes, _stream_ptr(device)), "tc_expand")
+                                       fuse, buf.data_ptr(), nbytes, _stream_ptr(device)), "tc_expand")
     return buf
 
 
-def _tc_weights(geometry, conc_weight, nbytes, device):
+def _tc_weights(geometry, conc_weight, fuse, nbytes, device):
     """Expanded weights kept on the ``ConcWeight`` they were made from, as ``_prepared_weights`` keeps its
     own.  The buffer is filled on the stream of the first call; calls on other streams wait for that.  While
     a stream is being captured nothing is kept, and a buffer not known to be complete is not used (an event
     from outside a capture cannot be waited for inside): the expansion becomes part of the graph."""
     cache = conc_weight.__dict__.setdefault("_tc", {})
-    key = geometry + (conc_weight.bits, conc_weight.base, conc_weight.data.data_ptr(), str(device))
+    key = geometry + (fuse.in_kind == _ffi.IN_F32_LINEAR, conc_weight.bits, conc_weight.base, conc_weight.data.data_ptr(), str(device))
     entry = cache.get(key)
     stream = torch.cuda.current_stream(device)
     capturing = torch.cuda.is_current_stream_capturing()
     if entry is None:
-        buf = tc_expand(geometry, conc_weight, nbytes, device)
+        buf = tc_expand(geometry, conc_weight, fuse, nbytes, device)
         if not capturing:
             event = torch.cuda.Event()
             event.record(stream)
@@ -143,7 +143,7 @@ def _tc_weights(geometry, conc_weight, nbytes, device):
         return buf
     if not entry["ready"]:
         if capturing:
-            return tc_expand(geometry, conc_weight, nbytes, device)
+            return tc_expand(geometry, conc_weight, fuse, nbytes, device)
         if entry["event"].query():
             entry["ready"] = True
         else:
@@ -159,9 +159,9 @@ def _tc_run(x, conc_weight, bias, out, geometry, fuse, keep_weights):
         return False
     device = x.device
     if keep_weights:
-        wt = _tc_weights(geometry, conc_weight, weight_bytes, device)
+        wt = _tc_weights(geometry, conc_weight, fuse, weight_bytes, device)
     else:
-        wt = tc_expand(geometry, conc_weight, weight_bytes, device)
+        wt = tc_expand(geometry, conc_weight, fuse, weight_bytes, device)
     act = torch.empty(act_bytes, dtype=torch.uint8, device=device)
     rc = _ffi.lib().ds_tc_conv2d(x.data_ptr(), conc_weight.data.data_ptr(),
                                  bias.data_ptr() if bias is not None else None, out.data_ptr(), *geometry,

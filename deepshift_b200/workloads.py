@@ -381,11 +381,13 @@ class IntPipeline(_Pipeline):
                 geometry = tuple(xin.shape) + (L.cout, L.k, L.k, L.stride, L.stride, L.pad, L.pad)
                 if op == 'linear':
                     geometry = (xin.shape[0], xin.shape[1], 1, 1, L.cout, 1, 1, 1, 1, 0, 0)
-                act_bytes, weight_bytes = kernels.tc_bytes(geometry, self.packed[li], fuse)
+                # codes that can travel as byte planes need no packing: the tensor cores win at any size
+                chained = op == 'conv' and in_kind == _ffi.IN_I32_CLAMP and L.cin % 16 == 0 and self.I >= 2
+                act_bytes, weight_bytes = kernels.tc_bytes(geometry, self.packed[li], fuse, any_size=chained)
                 tc = None
                 if act_bytes:   # tensor cores: weights expanded once for all passes
                     tc = dict(geometry=geometry, act_bytes=act_bytes, src=None, next=None,
-                              weights=kernels.tc_expand(geometry, self.packed[li], weight_bytes, dev))
+                              weights=kernels.tc_expand(geometry, self.packed[li], fuse, weight_bytes, dev))
                 self.calls.append((op, xin, li, L, out, fuse, res, tc))
                 dst = o.get('dst', 'x')
                 t[dst], fp32[dst] = out, lastlayer

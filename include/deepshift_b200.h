@@ -272,24 +272,24 @@ int ds_conv2d_prepare(const int32_t *packed, int B, int C, int H, int W, int OC,
  * expanded to 16 bytes each (`weights`, about 16 * KH * ceil16(KW * C) * ceil(OC / tile) * tile bytes), and
  * sixteen byte products per shift-accumulate replace the shift (see csrc/ds_tc.cuh).
  *
- * Activations must be known or found to fit 16 bits:
+ * Activations must be known or found to fit 16 bits (24 for DS_IN_F32_LINEAR):
  *   DS_IN_F32_CONV, DS_IN_I32_CLAMP   with I + F <= 16 (F + 2 <= 16 when I == 1);
  *   DS_IN_I32                         with act_bits 1..15, or DS_ACT_BITS_AUTO;
- *   DS_IN_F32_LINEAR                  with I + F <= 16.
+ *   DS_IN_F32_LINEAR                  linear layers, codes of up to 24 bits (22 byte products instead of 16).
  * For the last two the packing pass looks at every code; when one does not fit, the tensor-core launch
- * returns at once and the integer-path launch enqueued behind it does the work.  fuse->workspace and
- * fuse->prepared are not used.
+ * returns at once and the integer-path launch enqueued behind it does the work.  Of
+ * fuse->workspace only the last counter word is used (the range flag, see DS_ACT_BITS_AUTO); fuse->prepared is not.
  *
  * ds_tc_bytes     sizes of `act` (scratch of one call, any contents, reusable in stream order) and `weights`;
  *                 both 0 when the call is not served, or, unless any_size, has too little work to be worth it.
- * ds_tc_expand    fills `weights` for one geometry; may be kept as long as the packed weights do not change.
+ * ds_tc_expand    fills `weights` for one geometry and input kind (fuse->in_kind); may be kept as long as the packed weights do not change.
  * ds_tc_conv2d    the call.  Both buffers 16-byte aligned and at least as long as ds_tc_bytes said.  Enqueues
  *                 two kernels (four with the measured range); works under stream capture.
  */
 int ds_tc_bytes(int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits, int base,
                 const ds_fuse_t *fuse, int any_size, long long *act_bytes, long long *weight_bytes);
 int ds_tc_expand(const int32_t *packed, int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw, int ph,
-                 int pw, int bits, int base, void *weights, long long weight_bytes, void *stream);
+                 int pw, int bits, int base, const ds_fuse_t *fuse, void *weights, long long weight_bytes, void *stream);
 int ds_tc_conv2d(const void *x, const int32_t *packed, const int32_t *bias, void *out, int B, int C, int H, int W,
                  int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits, int base, const ds_fuse_t *fuse,
                  void *act, long long act_bytes, const void *weights, long long weight_bytes, void *stream);

@@ -25,7 +25,7 @@ def _run(dev, x, shift, sign, bias, s, p, *, in_kind=0, act_bits=15, out_f32=Fal
     f = kernels._fuse(in_kind, 1 if out_f32 else 0, I, F, relu=relu, act_bits=act_bits, residual=rt, round_f32=round_f32)
     act, wt = kernels.tc_bytes(geo, cw, f, any_size=True)
     assert act > 0 and wt > 0
-    weights_ = kernels.tc_expand(geo, cw, wt, dev)
+    weights_ = kernels.tc_expand(geo, cw, f, wt, dev)
     scratch = torch.full((act + 64,), 0xA5, dtype=torch.uint8, device=dev)
     out = torch.full((B * OC * OH * OW + 16,), 0x5EADBEE, dtype=torch.int32, device=dev)
     rc = _ffi.lib().ds_tc_conv2d(xt.data_ptr(), cw.data.data_ptr(), bt.data_ptr() if bt is not None else None,
@@ -138,9 +138,10 @@ def test_sizes_and_refusals(cuda_device):
     cw = utils.compress_bits(torch.from_numpy(shift).float(), torch.from_numpy(sign).float(), device=cuda_device)
     geo = (8, 64, 28, 28, 64, 3, 3, 1, 1, 1, 1)
     assert kernels.tc_bytes(geo, cw, kernels._fuse(0, 0, act_bits=-1))[0] > 0
-    assert kernels.tc_bytes((1,) + geo[1:], cw, kernels._fuse(0, 0, act_bits=-1))[0] == 0      # too little work
+    tiny = (1, 64, 7, 7, 64, 3, 3, 2, 2, 1, 1)
+    assert kernels.tc_bytes(tiny, cw, kernels._fuse(0, 0, act_bits=-1))[0] == 0      # too little work
     for f in (kernels._fuse(0, 0, act_bits=16), kernels._fuse(0, 0, act_bits=0), kernels._fuse(3, 0, 5, 12),
-              kernels._fuse(2, 0, 16, 16)):
+              kernels._fuse(2, 0, 16, 16)):   # 24-bit codes: linear layers only
         assert kernels.tc_bytes(geo, cw, f, any_size=True) == (0, 0)
     left = utils.ConcWeight(cw.data, -1, cw.bits)
     assert kernels.tc_bytes(geo, left, kernels._fuse(0, 0, act_bits=-1), any_size=True) == (0, 0)
@@ -148,8 +149,8 @@ def test_sizes_and_refusals(cuda_device):
     act, wt = kernels.tc_bytes(geo, cw, f)
     buf = torch.empty(max(act, wt), dtype=torch.uint8, device=cuda_device)
     st = torch.cuda.current_stream(cuda_device).cuda_stream
-    assert _ffi.lib().ds_tc_expand(cw.data.data_ptr(), *geo, cw.bits, 0, buf.data_ptr(), wt - 1, st) == 6
-    assert _ffi.lib().ds_tc_expand(cw.data.data_ptr(), *geo, cw.bits, -1, buf.data_ptr(), wt, st) == 2
+    assert _ffi.lib().ds_tc_expand(cw.data.data_ptr(), *geo, cw.bits, 0, f, buf.data_ptr(), wt - 1, st) == 6
+    assert _ffi.lib().ds_tc_expand(cw.data.data_ptr(), *geo, cw.bits, -1, f, buf.data_ptr(), wt, st) == 2
     x = torch.zeros(geo[:4], dtype=torch.int32, device=cuda_device)
     assert _ffi.lib().ds_tc_conv2d(x.data_ptr(), cw.data.data_ptr(), None, x.data_ptr(), *geo, cw.bits, 0, f, buf.data_ptr(),
                                    act - 1, buf.data_ptr(), wt, st) == 6
@@ -184,7 +185,7 @@ def test_planes_in_and_out(oracle, cuda_device, geo, codes):
     act = torch.zeros(max(a1, a2), dtype=torch.uint8, device=cuda_device)
     out = torch.full((B, OC, OH, OW), -7, dtype=torch.int32, device=cuda_device)
     out2 = torch.empty((B, 20, OH, OW), dtype=torch.int32, device=cuda_device)
-    e1, e2 = kernels.tc_expand(g1, cw, w1, cuda_device), kernels.tc_expand(gg2, cw2, w2, cuda_device)
+    e1, e2 = kernels.tc_expand(g1, cw, f, w1, cuda_device), kernels.tc_expand(gg2, cw2, f, w2, cuda_device)
     f2 = kernels._fuse(_ffi.IN_I32_CLAMP, 0, 4, 12)
     for _ in range(2):   # the second pass finds the scratch header as the first left it
         rc = lib.ds_tc_conv2d_ex(None, src.c, cw.data.data_ptr(), bt.data_ptr(), out.data_ptr() if codes else None, nxt.c, *g1,
@@ -203,3 +204,37 @@ def test_planes_in_and_out(oracle, cuda_device, geo, codes):
         assert bool((out == -7).all())
     assert np.array_equal(out2.cpu().numpy(), oracle.conv2d(np.clip(v, -32768, 28672), s2, g2, None, (1, 1), (1, 1)))
     assert int(act[:2048].sum()) == 0
+
+
+@pytest.mark.parametrize("mkn", [(17, 128, 10), (64, 784, 512), (128, 2047, 65), (130, 300, 64), (1000, 513, 130)])
+@pytest.mark.parametrize("scale", [1.0, 3e4, 1.27e5])
+def test_linear_fp32_input_24_bit_codes(oracle, cuda_device, mkn, scale):
+    """16.16 codes of up to 24 bits, both ends of the range among them; fp32 output and ReLU."""
+    M, K, N = mkn
+    rng = np.random.default_rng(M + K + N)
+    x = (rng.uniform(-1, 1, (M, K, 1, 1)) * scale / 1e3).astype(np.float32)
+    x.flat[::17], x.flat[5::31] = -128.0, np.float32(8388607 / 65536)
+    shift, sign = weights(rng, (N, K, 1, 1))
+    bias = rng.integers(-2000, 2000, N).astype(np.int32)
+    got = _run(cuda_device, x, shift, sign, bias, (1, 1), (0, 0), in_kind=2, act_bits=0, I=16, F=16, relu=True)
+    codes = np.trunc(x.astype(np.float64) * 65536).astype(np.int32).reshape(M, K)
+    want = np.maximum(oracle.linear(codes, shift.reshape(N, K), sign.reshape(N, K), bias), 0)
+    assert np.array_equal(got.reshape(M, N), want)
+
+
+@pytest.mark.parametrize("what", ["code", "shift"])
+def test_linear_fp32_input_falls_back(oracle, cuda_device, what):
+    """A code beyond 24 bits, or a right shift of 16..31 somewhere in the weights: the integer path."""
+    rng = np.random.default_rng(8)
+    M, K, N = 90, 200, 70
+    x = rng.normal(0, 1, (M, K, 1, 1)).astype(np.float32)
+    shift, sign = weights(rng, (N, K, 1, 1))
+    sign[sign == 0] = 1
+    sign[0, 0] = 0
+    if what == "code":
+        x[89, 199] = 128.0
+    else:
+        shift[69, 199] = -17
+    got = _run(cuda_device, x, shift, sign, None, (1, 1), (0, 0), in_kind=2, act_bits=0, I=16, F=16)
+    codes = np.trunc(x.astype(np.float64) * 65536).astype(np.int32).reshape(M, K)
+    assert np.array_equal(got.reshape(M, N), oracle.linear(codes, shift.reshape(N, K), sign.reshape(N, K), None))
