@@ -144,10 +144,11 @@ int tc_mode(const ds_fuse_t& f, int bits, int base)
 
 // Whether the tensor cores beat the other paths, packing included.  Measured, us, other path -> this one:
 //   linear, fp32 input (weights expanded once): 64 x 784 -> 512 120 -> 19, 17 x 512 -> 512 83 -> 18, 1024 x 500
-//     -> 10 80 -> 19: the integer path behind it runs one CTA per 64 x 128 outputs over all of K, 0.16 us per k.
-//     Up to 16 rows the small-batch kernel takes 10 to 15.
+//     -> 10 80 -> 19: the integer path behind it runs one CTA per 64 x 128 outputs over all of K, 0.16 us per k, so
+//     the two meet near K = 150.  Up to 16 rows the small-batch kernel takes 10 to 15.
 //   linear, int32 input (expanded per call): 256 x 512 -> 1000 86 -> 28, 1024 x 800 -> 500 108 -> 37; up to 64 rows
-//     the integer path splits K and is faster (64 x 784 -> 512 21 -> 26).
+//     the integer path splits K and is faster (64 x 784 -> 512 21 -> 26).  With the launch of the expansion the two
+//     meet near K = 200.
 //   convolution: 128 -> 128 channels, 28 x 28, one image 103 -> 19; 1x1 stride 2, 64 -> 128, one image 32 -> 12:
 //     few 256-row tiles leave the other path's SMs idle.  With many tiles it pays from about 2^26 shift-accumulates
 //     (16 -> 16 channels, 32 x 32, 64 images 40 -> 24), and not where most of the padded product is padding
@@ -155,7 +156,7 @@ int tc_mode(const ds_fuse_t& f, int bits, int base)
 bool worthwhile(const TcGeom& g, int in_kind)
 {
     const double ops = (double)g.M * g.N * g.K;
-    if (g.H == 1 && g.W == 1 && g.KH == 1 && g.KW == 1) return g.K >= 128 && g.M > (in_kind == DS_IN_F32_LINEAR ? 16 : 64);
+    if (g.H == 1 && g.W == 1 && g.KH == 1 && g.KW == 1) return in_kind == DS_IN_F32_LINEAR ? g.M > 16 && g.K >= 192 : g.M > 64 && g.K >= 256;
     const long long tiles = ((g.M + 255ll) / 256) * ((g.N + 127) / 128);
     const double padded = (double)g.grid_m * g.S * TC_ROWS * g.grid_n * g.BN * g.G * TC_KG;
     return tiles <= 16 ? ops >= 6e6 : ops >= double(1 << 26) && ops * 5 >= padded;

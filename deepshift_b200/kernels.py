@@ -139,8 +139,10 @@ def _tc_weights(geometry, conc_weight, fuse, nbytes, device):
         if not capturing:
             event = torch.cuda.Event()
             event.record(stream)
-            cache[key] = dict(buf=buf, event=event, ready=False)
+            cache[key] = dict(buf=buf, event=event, ready=False, stream=stream)
         return buf
+    if entry["stream"] != stream and not capturing:
+        entry["buf"].record_stream(stream)   # freed only after this stream's uses
     if not entry["ready"]:
         if capturing:
             return tc_expand(geometry, conc_weight, fuse, nbytes, device)
@@ -151,9 +153,15 @@ def _tc_weights(geometry, conc_weight, fuse, nbytes, device):
     return entry["buf"]
 
 
+_TC_MIN_OPS = 4_000_000   # below this ds_tc_bytes never takes a call: not worth asking
+
+
 def _tc_run(x, conc_weight, bias, out, geometry, fuse, keep_weights):
     """Runs the call on the tensor cores if it is one for them; False otherwise.  Scratch comes from torch's
     allocator, whose blocks are reused in stream order."""
+    _, C, _, _, _, KH, KW = geometry[:7]
+    if KH * KW > 1 and out.numel() * C * KH * KW < _TC_MIN_OPS:
+        return False
     act_bytes, weight_bytes = tc_bytes(geometry, conc_weight, fuse)
     if act_bytes == 0:
         return False

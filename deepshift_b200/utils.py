@@ -82,6 +82,13 @@ class ConcWeight():
         self.base = base
         self.bits = bits
 
+    def __getstate__(self):
+        # a copy or a saved module starts without the expanded operand tiles (kernels._tc_weights): they hold a
+        # CUDA event and are made again on first use
+        state = dict(self.__dict__)
+        state.pop('_tc', None)
+        return state
+
 
 def compress_bits(shift, sign, device=None):
     """utils.py:61-88: packs a layer's (shift, sign) parameters into a ``ConcWeight``.
