@@ -145,7 +145,7 @@ int tc_mode(const ds_fuse_t& f, int bits, int base)
 // Whether the tensor cores beat the other paths, packing included.  Measured, us, other path -> this one:
 //   linear, fp32 input (weights expanded once): 64 x 784 -> 512 120 -> 19, 17 x 512 -> 512 83 -> 18, 1024 x 500
 //     -> 10 80 -> 19: the integer path behind it runs one CTA per 64 x 128 outputs over all of K, 0.16 us per k, so
-//     the two meet near K = 150.  Up to 16 rows the small-batch kernel takes 10 to 15.
+//     the GPU times meet near K = 150, with the host's four launches (about 45 us a call) near 300.  Up to 16 rows the small-batch kernel takes 10 to 15.
 //   linear, int32 input (expanded per call): 256 x 512 -> 1000 86 -> 28, 1024 x 800 -> 500 108 -> 37; up to 64 rows
 //     the integer path splits K and is faster (64 x 784 -> 512 21 -> 26).  With the launch of the expansion the two
 //     meet near K = 200.
@@ -156,8 +156,15 @@ int tc_mode(const ds_fuse_t& f, int bits, int base)
 bool worthwhile(const TcGeom& g, int in_kind)
 {
     const double ops = (double)g.M * g.N * g.K;
-    if (g.H == 1 && g.W == 1 && g.KH == 1 && g.KW == 1) return in_kind == DS_IN_F32_LINEAR ? g.M > 16 && g.K >= 192 : g.M > 64 && g.K >= 256;
+    if (g.H == 1 && g.W == 1 && g.KH == 1 && g.KW == 1) return in_kind == DS_IN_F32_LINEAR ? g.M > 16 && g.K >= 320 : g.M > 64 && g.K >= 256;
     const long long tiles = ((g.M + 255ll) / 256) * ((g.N + 127) / 128);
+    if (in_kind == DS_IN_I32) {
+        // Weights expanded per call: five launches, 45 us of host time.  The other path takes about 20 us and 0.23 us
+        // per k and wave of 256 x 128 tiles (0.13 at 64 columns), up to four CTAs sharing a tile along K: 37 images of
+        // 45 channels, 31 x 29, stride 2, -> 70: 85 -> 45; one image, 64 channels, 56 x 56 stays.
+        const double waves = tiles >= kSms ? double((tiles + kSms - 1) / kSms) : tiles * 4 >= kSms ? (double)tiles / kSms : 0.25;
+        if (waves * g.K * (g.N > 64 ? 0.23 : 0.13) < 20) return false;
+    }
     const double padded = (double)g.grid_m * g.S * TC_ROWS * g.grid_n * g.BN * g.G * TC_KG;
     return tiles <= 16 ? ops >= 6e6 : ops >= double(1 << 26) && ops * 5 >= padded;
 }

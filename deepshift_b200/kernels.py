@@ -17,6 +17,7 @@ Differences from the reference, all deliberate:
   * ``dilation != 1`` or ``groups != 1`` raises instead of being ignored (kernels.py:28).
 """
 import ctypes
+import functools
 
 import torch
 
@@ -110,9 +111,16 @@ def _fuse(in_kind=0, out_kind=0, act_integer_bits=0, act_fraction_bits=0, relu=F
 def tc_bytes(geometry, conc_weight, fuse, any_size=False):
     """(scratch bytes, expanded-weight bytes) of a call on the tensor cores; (0, 0) when the call is served
     by the other paths (left shifts, activations wider than 16 bits, too little work to pay the packing)."""
+    return _tc_bytes(tuple(geometry), conc_weight.bits, conc_weight.base, fuse.in_kind, fuse.act_bits, fuse.act_integer_bits,
+                     fuse.act_fraction_bits, int(any_size))
+
+
+@functools.lru_cache(maxsize=4096)
+def _tc_bytes(geometry, bits, base, in_kind, act_bits, integer_bits, fraction_bits, any_size):
+    # a function of these numbers alone: 3 us of ctypes otherwise, on every call
     act, wt = ctypes.c_longlong(0), ctypes.c_longlong(0)
-    _ffi.check(_ffi.lib().ds_tc_bytes(*geometry, conc_weight.bits, conc_weight.base, fuse, int(any_size),
-                                      ctypes.byref(act), ctypes.byref(wt)), "tc_bytes")
+    f = _fuse(in_kind, 0, integer_bits, fraction_bits, act_bits=act_bits)
+    _ffi.check(_ffi.lib().ds_tc_bytes(*geometry, bits, base, f, any_size, ctypes.byref(act), ctypes.byref(wt)), "tc_bytes")
     return act.value, wt.value
 
 

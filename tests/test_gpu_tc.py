@@ -136,7 +136,7 @@ def test_sizes_and_refusals(cuda_device):
     rng = np.random.default_rng(1)
     shift, sign = weights(rng, (64, 64, 3, 3))
     cw = utils.compress_bits(torch.from_numpy(shift).float(), torch.from_numpy(sign).float(), device=cuda_device)
-    geo = (8, 64, 28, 28, 64, 3, 3, 1, 1, 1, 1)
+    geo = (64, 64, 28, 28, 64, 3, 3, 1, 1, 1, 1)
     assert kernels.tc_bytes(geo, cw, kernels._fuse(0, 0, act_bits=-1))[0] > 0
     tiny = (1, 64, 7, 7, 64, 3, 3, 2, 2, 1, 1)
     assert kernels.tc_bytes(tiny, cw, kernels._fuse(0, 0, act_bits=-1))[0] == 0      # too little work

@@ -18,9 +18,10 @@ def _linear(M, K, N):
 
 @pytest.mark.parametrize("geo,in_kind,act_bits,served", [
     (_linear(8192, 4096, 4096), 0, -1, True), (_linear(65, 256, 10), 0, -1, True), (_linear(64, 4096, 4096), 0, -1, False),
-    (_linear(8192, 255, 4096), 0, -1, False), (_linear(17, 192, 10), 2, 0, True), (_linear(16, 4096, 4096), 2, 0, False),
+    (_linear(8192, 255, 4096), 0, -1, False), (_linear(17, 320, 10), 2, 0, True), (_linear(17, 319, 10), 2, 0, False), (_linear(16, 4096, 4096), 2, 0, False),
     (_linear(8192, 4096, 4096), 0, 16, False), (_linear(8192, 4096, 4096), 0, 15, True), (_linear(8192, 4096, 4096), 0, 0, False),
-    ((256, 64, 56, 56, 64, 3, 3, 1, 1, 1, 1), 3, 0, True), ((1, 64, 56, 56, 128, 1, 1, 2, 2, 0, 0), 3, 0, True),
+    ((256, 64, 56, 56, 64, 3, 3, 1, 1, 1, 1), 3, 0, True), ((64, 64, 28, 28, 64, 1, 1, 1, 1, 0, 0), 0, -1, False),
+    ((37, 45, 31, 29, 70, 3, 3, 2, 2, 1, 1), 0, -1, True), ((1, 64, 56, 56, 64, 3, 3, 1, 1, 1, 1), 0, -1, False), ((1, 64, 56, 56, 128, 1, 1, 2, 2, 0, 0), 3, 0, True),
     ((12, 16, 28, 28, 40, 3, 3, 1, 1, 1, 1), 3, 0, False), ((1024, 1, 28, 28, 20, 5, 5, 1, 1, 0, 0), 1, 0, False)])
 def test_which_calls_are_served(geo, in_kind, act_bits, served):
     assert (_bytes(geo, in_kind, act_bits)[0] > 0) == served
