@@ -14,10 +14,12 @@
 //                   next         one thread issues the MMAs: 128 x BN x 32 bytes, A from TMEM, B from shared memory.
 //                   last         one thread fetches weight tiles with cp.async.bulk into a ring.
 //                 TMEM: a ring of BN-column accumulator slots, so that the epilogue of a tile overlaps the next tile's
-//                 MMAs, and one A slot per producer warpgroup (sixteen planes x 16 bytes x 128 rows).
+//                 MMAs, and two A slots per producer warpgroup (sixteen planes x 16 bytes x 128 rows each).
 //
 // What bounds it: the s8 MMA rate, 16 byte-products per shift-accumulate (8192 per SM and clock: 144 T
-// shift-op/s at 1.9 GHz).  A from TMEM because shared memory could not carry both operands: at BN = 64 an
+// shift-op/s at 1.9 GHz), of which 63 % are in use at 128 columns and 41 % at 64.  Measured, packing included: 8192 x
+// 4096 x 4096 1.50 ms = 92 T shift-op/s (6.69 ms on the FP32 pipe); 3x3 on 64 / 128 / 256 / 512 channels, 256 images,
+// 48 / 74 / 73 / 75 T (20.5 / 24 / 21.5 / 20.9).  A from TMEM because shared memory could not carry both operands: at BN = 64 an
 // MMA of 32 cycles would read 4 KiB of A and 2 KiB of B, 192 bytes per cycle where 128 are available.
 #include "ds_tc.cuh"
 
@@ -29,10 +31,13 @@ namespace {
 
 constexpr int TC_TMEM_COLS = 512;
 
-// Per column width: WG producer warpgroups, each with an operand slot of its own (64 columns: sixteen planes x 16
+// Per column width: WG producer warpgroups, each with two A slots of its own (64 columns: sixteen planes x 16
 // bytes; a slot shared between warpgroups could not be guarded by a phase parity, since a warpgroup may be two
-// phases away from it), and as many accumulator slots as the remaining columns hold.  Two warpgroups keep up with the MMAs
-// of 128 columns (512 cycles per 128 rows x 16 values), three are needed for 64 (256 cycles).
+// phases away from it), and as many accumulator slots as the remaining columns hold: two of 128 or 64 columns, so
+// that the epilogue of a tile overlaps the next tile's MMAs.  With one A slot per warpgroup the refill sat in the
+// MMAs' way (813 cycles per 128 rows x 16 values at 128 columns, 675 at 64, where the MMAs alone take 640 and 450).
+// The price: no two row blocks share a weight tile any more (512 channels, 256 images: 348 -> 392 us; 64 channels
+// 640 -> 613).
 template <int BN, bool WIDE>
 struct TcTile {
     static constexpr int WG = WIDE || BN == 128 ? 2 : 3;
@@ -40,7 +45,8 @@ struct TcTile {
     static constexpr int ASTRIDE = WIDE ? 96 : 64;   // columns from one A slot to the next
     static constexpr int ACC = WIDE ? 2 * BN : BN;   // columns of an accumulator slot (wide: sums of weight 2^8 behind)
     static constexpr int THREADS = (4 * WG + 6) * 32;  // + 4 epilogue warps + MMA warp + loader warp
-    static constexpr int ACC_COLS = TC_TMEM_COLS - ASTRIDE * WG;
+    static constexpr int SLOTS = (WIDE ? 1 : 2) * WG;  // A slots, handed out round robin: item i fills slot i % SLOTS
+    static constexpr int ACC_COLS = TC_TMEM_COLS - ASTRIDE * SLOTS;
     static constexpr int NACC = ACC_COLS / ACC < 6 ? ACC_COLS / ACC : 6;
     static constexpr int STAGE = BN * PLANES * TC_KG;
     static constexpr int STAGES = BN == 128 ? 6 : 8;
@@ -51,8 +57,8 @@ struct TcSmem {
     alignas(128) unsigned char b[TcTile<BN, WIDE>::STAGES][TcTile<BN, WIDE>::STAGE];
     alignas(8) unsigned long long bfull[TcTile<BN, WIDE>::STAGES];
     unsigned long long bempty[TcTile<BN, WIDE>::STAGES];
-    unsigned long long afull[TcTile<BN, WIDE>::WG];
-    unsigned long long aempty[TcTile<BN, WIDE>::WG];
+    unsigned long long afull[TcTile<BN, WIDE>::SLOTS];
+    unsigned long long aempty[TcTile<BN, WIDE>::SLOTS];
     unsigned long long accfull[6];
     unsigned long long accempty[6];
     unsigned long long done;
@@ -214,7 +220,7 @@ struct Unit {
     int tile, sp, m0, n0, nt, g0, g1;
 };
 
-template <int BN, int S>
+template <int BN>
 __device__ __forceinline__ Unit unit_of(const TcRun& p, int u)
 {
     Unit r;
@@ -228,7 +234,7 @@ __device__ __forceinline__ Unit unit_of(const TcRun& p, int u)
         mt = r.tile / p.grid_n;
         r.nt = r.tile - mt * p.grid_n;
     }
-    r.m0 = mt * (S * TC_ROWS);
+    r.m0 = mt * TC_ROWS;
     r.n0 = r.nt * BN;
     r.g0 = r.sp * p.gps;
     r.g1 = min(p.G, r.g0 + p.gps);
@@ -245,19 +251,63 @@ __device__ __forceinline__ void tc_store(const TcRun& p, int (&v)[32], const int
                                          unsigned nextoff)
 {
     if (m >= p.M) return;
-    int* oi = static_cast<int*>(p.out);
-    float* of = static_cast<float*>(p.out);
-    const bool f32 = p.out_kind == DS_OUT_F32;
-    auto finish = [&](int a, int r) -> int {
-        if (p.residual) a = __float2int_rn(__int2float_rn(a) + __int2float_rn(r));
-        if (p.relu) a = max(a, 0);
-        if (p.requant) a = min(max(a, p.rq_lo), p.rq_hi) * p.rq_mul + p.rq_add;
-        if (p.round_f32) a = __float2int_rn(__int2float_rn(a));
-        return a;
-    };
     const int live = min(32, p.N - n);
+    int* oi = static_cast<int*>(p.out);
+    // Step by step over all 32 columns, each step's condition tested once: with the conditions inside the loop over
+    // the columns the epilogue of a 1x1 layer took longer than its MMAs.
+#pragma unroll
+    for (int c = 0; c < 32; c += 4) {
+        const int4 cc = *reinterpret_cast<const int4*>(colc + c);
+        v[c] += cc.x;
+        v[c + 1] += cc.y;
+        v[c + 2] += cc.z;
+        v[c + 3] += cc.w;
+    }
+    const long long o0 = rowoff + (long long)n * p.P;
+    if (p.residual) {
+        const int* ra = p.residual + o0;
+#pragma unroll
+        for (int h = 0; h < 32; h += 16) {
+            int r[16];
+#pragma unroll
+            for (int c = 0; c < 16; ++c) {
+                const int* q = ra + (long long)(h + c) * p.P;
+                r[c] = (h + c < live && DS_O_OK(p, p.residual, q, 4)) ? *q : 0;
+            }
+#pragma unroll
+            for (int c = 0; c < 16; ++c) v[h + c] = __float2int_rn(__int2float_rn(v[h + c]) + __int2float_rn(r[c]));
+        }
+    }
+    if (p.relu) {
+#pragma unroll
+        for (int c = 0; c < 32; ++c) v[c] = max(v[c], 0);
+    }
+    if (p.requant) {
+#pragma unroll
+        for (int c = 0; c < 32; ++c) v[c] = min(max(v[c], p.rq_lo), p.rq_hi) * p.rq_mul + p.rq_add;
+    }
+    if (p.round_f32) {
+#pragma unroll
+        for (int c = 0; c < 32; ++c) v[c] = __float2int_rn(__int2float_rn(v[c]));
+    }
+    if (p.out) {
+        if (p.out_kind == DS_OUT_F32) {
+#pragma unroll
+            for (int c = 0; c < 32; ++c) v[c] = __float_as_int(__int2float_rn(v[c]) * p.inv_scale);
+        }
+        if (p.P == 1 && (p.N & 3) == 0) {
+#pragma unroll
+            for (int c = 0; c < 32; c += 4)
+                if (c < live && DS_O_OK(p, oi, oi + o0 + c, 16))
+                    *reinterpret_cast<int4*>(oi + o0 + c) = make_int4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+        } else {
+            int* o = oi + o0;
+#pragma unroll
+            for (int c = 0; c < 32; ++c, o += p.P)
+                if (c < live && DS_O_OK(p, oi, o, 4)) *o = v[c];
+        }
+    }
     if (NEXT) {
-        long long o = rowoff + (long long)n * p.P;
         unsigned char* nx = p.next + (nextoff + unsigned(n));
 #pragma unroll
         for (int h = 0; h < 32; h += 16) {
@@ -265,20 +315,9 @@ __device__ __forceinline__ void tc_store(const TcRun& p, int (&v)[32], const int
             unsigned lw[4], hw[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                int c[4], r[4];
+                unsigned c[4];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    r[e] = 0;
-                    const int* ra = p.residual + o + (long long)e * p.P;
-                    if (p.residual && DS_O_OK(p, p.residual, ra, 4)) r[e] = *ra;
-                }
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int a = finish(v[h + 4 * q + e] + colc[h + 4 * q + e], r[e]);
-                    if (oi && DS_O_OK(p, oi, oi + o, 4)) oi[o] = a;
-                    c[e] = min(max(a, p.next_lo), p.next_hi) + 32768;
-                    o += p.P;
-                }
+                for (int e = 0; e < 4; ++e) c[e] = unsigned(min(max(v[h + 4 * q + e], p.next_lo), p.next_hi)) + 32768u;
                 const unsigned x = __byte_perm(c[0], c[1], 0x5140), y = __byte_perm(c[2], c[3], 0x5140);
                 lw[q] = __byte_perm(x, y, 0x5410);
                 hw[q] = __byte_perm(x, y, 0x7632);
@@ -286,56 +325,10 @@ __device__ __forceinline__ void tc_store(const TcRun& p, int (&v)[32], const int
             *reinterpret_cast<uint4*>(nx + h) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
             *reinterpret_cast<uint4*>(nx + p.next_plane + h) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
         }
-        return;
-    }
-    if (p.P == 1 && (p.N & 3) == 0) {
-        const long long o0 = rowoff + n;
-#pragma unroll
-        for (int c = 0; c < 32; c += 4) {
-            if (c >= live) break;
-            const int4 cc = *reinterpret_cast<const int4*>(colc + c);
-            int4 r = make_int4(0, 0, 0, 0);
-            if (p.residual && DS_O_OK(p, p.residual, p.residual + o0 + c, 16))
-                r = make_int4(p.residual[o0 + c], p.residual[o0 + c + 1], p.residual[o0 + c + 2], p.residual[o0 + c + 3]);
-            const int a = finish(v[c] + cc.x, r.x), b = finish(v[c + 1] + cc.y, r.y), d = finish(v[c + 2] + cc.z, r.z),
-                      e = finish(v[c + 3] + cc.w, r.w);
-            if (!f32) {
-                if (DS_O_OK(p, oi, oi + o0 + c, 16)) *reinterpret_cast<int4*>(oi + o0 + c) = make_int4(a, b, d, e);
-            } else if (DS_O_OK(p, of, of + o0 + c, 16)) {
-                *reinterpret_cast<float4*>(of + o0 + c) =
-                    make_float4(__int2float_rn(a) * p.inv_scale, __int2float_rn(b) * p.inv_scale,
-                                __int2float_rn(d) * p.inv_scale, __int2float_rn(e) * p.inv_scale);
-            }
-        }
-        return;
-    }
-    long long o = rowoff + (long long)n * p.P;
-#pragma unroll
-    for (int c0 = 0; c0 < 32; c0 += 8) {
-        if (c0 >= live) break;
-        int r[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            r[c] = 0;
-            const int* ra = p.residual + o + (long long)c * p.P;
-            if (p.residual && c0 + c < live && DS_O_OK(p, p.residual, ra, 4)) r[c] = *ra;
-        }
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            if (c0 + c < live) {
-                const int a = finish(v[c0 + c] + colc[c0 + c], r[c]);
-                if (!f32) {
-                    if (DS_O_OK(p, oi, oi + o, 4)) oi[o] = a;
-                } else if (DS_O_OK(p, of, of + o, 4)) {
-                    of[o] = __int2float_rn(a) * p.inv_scale;
-                }
-            }
-            o += p.P;
-        }
     }
 }
 
-template <int BN, int S, bool NEXT, bool WIDE>
+template <int BN, bool NEXT, bool WIDE>
 __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(const TcRun p)
 {
     using T = TcTile<BN, WIDE>;
@@ -351,7 +344,7 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
             bar_init(&s.bfull[i], 1);
             bar_init(&s.bempty[i], 1);
         }
-        for (int i = 0; i < T::WG; ++i) {
+        for (int i = 0; i < T::SLOTS; ++i) {
             bar_init(&s.afull[i], 4);
             bar_init(&s.aempty[i], 1);
         }
@@ -375,63 +368,58 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
     constexpr unsigned tmem = 0;
     constexpr unsigned tmem_a = tmem + T::ACC_COLS;
     if (threadIdx.x == 0 && s.tmem != 0) s.err = 1;
-    constexpr bool FIX = S == T::WG;  // every warpgroup has its own row block
 
     if (warp < 4 * T::WG) {
         // ---- producers: expand activations into TMEM -------------------------------------------------
         const int wg = warp >> 2;
         const int row = threadIdx.x & 127;
         const unsigned lane_base = unsigned(warp & 3) << 21;  // TMEM lane (warp % 4) * 32 in bits 16-31
-        unsigned roff[FIX ? 1 : S];
-        int u = blockIdx.x, sub = 0, g = 0, g1 = 0, j = 0, kh = 0;
-        auto enter = [&]() {
-            if (u >= p.units) return;
-            const Unit un = unit_of<BN, S>(p, u);
-            g = un.g0;
-            g1 = un.g1;
-            kh = g / p.J;
-            j = g - kh * p.J;
-            sub = 0;
-#pragma unroll
-            for (int i = 0; i < (FIX ? 1 : S); ++i) {
-                const int m = min(un.m0 + (FIX ? wg : i) * TC_ROWS + row, p.M - 1);
-                const int b = m / p.P, pp = m - b * p.P;
-                const int oh = pp / p.OW, ow = pp - oh * p.OW;
-                roff[i] = unsigned(b) * p.img_bytes + unsigned(oh) * p.row_step + unsigned(ow) * p.col_step;
+        unsigned roff = 0;
+        int u = blockIdx.x, g = 0, g1 = 0, j = 0, kh = 0;
+        // Unit u, `skip` groups in; units too short for that are passed over.
+        auto enter = [&](int skip) {
+            for (; u < p.units; u += gridDim.x) {
+                const Unit un = unit_of<BN>(p, u);
+                g = un.g0 + skip;
+                g1 = un.g1;
+                if (g < g1) {
+                    kh = g / p.J;
+                    j = g - kh * p.J;
+                    const int m = min(un.m0 + row, p.M - 1);
+                    const int b = m / p.P, pp = m - b * p.P;
+                    const int oh = pp / p.OW, ow = pp - oh * p.OW;
+                    roff = unsigned(b) * p.img_bytes + unsigned(oh) * p.row_step + unsigned(ow) * p.col_step;
+                    return;
+                }
+                skip = g - g1;
             }
         };
+        // this warpgroup's next item
         auto step = [&]() {
-            if (!FIX) {
-                if (++sub < S) return;
-                sub = 0;
-            }
-            if (++g == g1) {
+            g += T::WG;
+            if (g >= g1) {
                 u += gridDim.x;
-                enter();
-            } else if (++j == p.J) {
-                j = 0;
-                ++kh;
+                enter(g - g1);
+            } else {
+                j += T::WG;
+                while (j >= p.J) {
+                    j -= p.J;
+                    ++kh;
+                }
             }
         };
         uint4 nl = make_uint4(0, 0, 0, 0), nh = nl, nt = nl;
         auto fetch = [&]() {
-            unsigned off = roff[0];
-#pragma unroll
-            for (int i = 1; i < (FIX ? 1 : S); ++i)
-                if (sub == i) off = roff[i];
-            const unsigned char* a = p.act + (off + unsigned(kh) * p.kh_step + unsigned(j) * 16u);
+            const unsigned char* a = p.act + (roff + unsigned(kh) * p.kh_step + unsigned(j) * 16u);
             nl = ld16(a, p.align);
             nh = ld16(a + p.plane, p.align);
             if (WIDE) nt = ld16(a + 2 * p.plane, p.align);
         };
-        enter();
-        for (int i = 0; !FIX && i < wg && u < p.units; ++i) step();
+        enter(wg);
         if (u < p.units) fetch();
         for (unsigned round = 0; u < p.units;) {
             const uint4 l = nl, h = nh, t = nt;
-#pragma unroll
-            for (int i = 0; i < (FIX ? 1 : T::WG); ++i)
-                if (u < p.units) step();
+            step();
             if (u < p.units) fetch();
             unsigned v[64];
             planes_low(l.x, h.x, v, 0);
@@ -444,20 +432,22 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
             planes_high(h.w, v + 32, 3);
             // One hand-shake per 16 values (two, a slot per eight planes, cost a third of the rate at 128 columns),
             // and nothing but the stores between the slot's release and its hand-over.
-            if (round > 0 && !bar_wait(&s.aempty[wg], (round - 1) & 1u, err)) u = p.units;
+            constexpr int PER = T::SLOTS / T::WG;  // slots of this warpgroup, used in turn
+            const unsigned slot = wg + T::WG * (round % PER), use = round / PER;
+            if (use > 0 && !bar_wait(&s.aempty[slot], (use - 1) & 1u, err)) u = p.units;
             ++round;
             __syncwarp();
             tc_fence_after();
-            tmem_st32(tmem_a + lane_base + wg * T::ASTRIDE, v);
-            tmem_st32(tmem_a + lane_base + wg * T::ASTRIDE + 32, v + 32);
+            tmem_st32(tmem_a + lane_base + slot * T::ASTRIDE, v);
+            tmem_st32(tmem_a + lane_base + slot * T::ASTRIDE + 32, v + 32);
             if (WIDE) {
                 const unsigned w[16] = {t.x, t.y, t.z, t.w, t.x, t.y, t.z, t.w, t.x, t.y, t.z, t.w, t.x, t.y, t.z, t.w};
-                tmem_st16(tmem_a + lane_base + wg * T::ASTRIDE + 64, w);
+                tmem_st16(tmem_a + lane_base + slot * T::ASTRIDE + 64, w);
             }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) bar_arrive(&s.afull[wg]);
+            if (lane == 0) bar_arrive(&s.afull[slot]);
         }
     } else if (warp < 4 * T::WG + 4) {
         // ---- epilogue ----------------------------------------------------------------------------------
@@ -471,24 +461,23 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
         unsigned acc = 0;
         int par = 0;
         bool bad = false;
-        for (int u = blockIdx.x; u < p.units && !bad; u += gridDim.x, acc += S, par ^= 1) {
-            const Unit un = unit_of<BN, S>(p, u);
+        for (int u = blockIdx.x; u < p.units && !bad; u += gridDim.x, ++acc, par ^= 1) {
+            const Unit un = unit_of<BN>(p, u);
             // column constants of this tile; two copies, so a slow warp still reads the previous tile's
             if (row < BN) {
                 const int n = un.n0 + row;
                 s.colc[par][row] = n < p.N ? __ldg(p.colc + n) + (p.bias ? __ldg(p.bias + n) : 0) : 0;
             }
             epi_bar();
-#pragma unroll 1
-            for (int i = 0; i < S; ++i) {
-                const unsigned a = acc + i, slot = a % T::NACC;
-                if (!bar_wait(&s.accfull[slot], (a / T::NACC) & 1u, err)) {
+            {
+                const unsigned slot = acc % T::NACC;
+                if (!bar_wait(&s.accfull[slot], (acc / T::NACC) & 1u, err)) {
                     bad = true;
                     break;
                 }
                 __syncwarp();
                 tc_fence_after();
-                const int m = un.m0 + i * TC_ROWS + row;
+                const int m = un.m0 + row;
                 const int b = m / p.P, pp = m - b * p.P;
                 const long long rowoff = (long long)b * p.OC * p.P + pp;
                 const unsigned nextoff = next_offset(b, pp);
@@ -510,7 +499,7 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
                     if (p.splits == 1) {
                         tc_store<NEXT>(p, v, &s.colc[par][c], m, un.n0 + c, rowoff, nextoff);
                     } else {
-                        int* dst = p.partials + ((long long)(un.tile * p.splits + un.sp) * S + i) * (BN * TC_ROWS) +
+                        int* dst = p.partials + (long long)(un.tile * p.splits + un.sp) * (BN * TC_ROWS) +
                                    c * TC_ROWS + row;
 #pragma unroll
                         for (int q = 0; q < 32; ++q) __stcg(dst + q * TC_ROWS, v[q]);
@@ -526,9 +515,8 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
                 if (s.last_flag) {
                     __threadfence();
                     if (row == 0) p.counters[un.tile] = 0;  // for the next launch
-#pragma unroll 1
-                    for (int i = 0; i < S; ++i) {
-                        const int m = un.m0 + i * TC_ROWS + row;
+                    {
+                        const int m = un.m0 + row;
                         const int b = m / p.P, pp = m - b * p.P;
                         const long long rowoff = (long long)b * p.OC * p.P + pp;
                         const unsigned nextoff = next_offset(b, pp);
@@ -539,7 +527,7 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
                             for (int q = 0; q < 32; ++q) v[q] = 0;
 #pragma unroll 1
                             for (int k = 0; k < p.splits; ++k) {
-                                const int* src = p.partials + ((long long)(un.tile * p.splits + k) * S + i) * (BN * TC_ROWS) +
+                                const int* src = p.partials + (long long)(un.tile * p.splits + k) * (BN * TC_ROWS) +
                                                  c * TC_ROWS + row;
 #pragma unroll
                                 for (int q = 0; q < 32; ++q) v[q] += __ldcg(src + q * TC_ROWS);
@@ -566,57 +554,45 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
             (1ull << 46) | (8ull << 32) | ((unsigned long long)BN << 16) | (s32(&s.b[0][0]) >> 4);
         unsigned slot = 0, aph = 0, st = 0, bph = 0, aslot = 0, accph = 1;
         for (int u = blockIdx.x; u < p.units; u += gridDim.x) {
-            const Unit un = unit_of<BN, S>(p, u);
-            unsigned d[S], accs[S];
-#pragma unroll
-            for (int i = 0; i < S; ++i) {
-                accs[i] = aslot;
-                d[i] = tmem + aslot * T::ACC;
-                bar_wait(&s.accempty[aslot], accph, err);  // the first round finds the slots free
-                if (++aslot == unsigned(T::NACC)) {
-                    aslot = 0;
-                    accph ^= 1u;
-                }
+            const Unit un = unit_of<BN>(p, u);
+            const unsigned d = tmem + aslot * T::ACC;
+            unsigned long long* accfull = &s.accfull[aslot];
+            bar_wait(&s.accempty[aslot], accph, err);  // the first round finds the slots free
+            if (++aslot == unsigned(T::NACC)) {
+                aslot = 0;
+                accph ^= 1u;
             }
             unsigned more = 0;  // the first MMA of a unit overwrites the accumulator
             for (int g = un.g0; g < un.g1; ++g) {
                 bar_wait(&s.bfull[st], bph, err);
                 const unsigned long long bdesc = desc0 + st * unsigned(T::STAGE >> 4);
+                bar_wait(&s.afull[slot], aph, err);
+                tc_fence_after();
+                if (elect_one()) {
 #pragma unroll
-                for (int i = 0; i < S; ++i) {
-                    const unsigned sl = FIX ? unsigned(i) : slot;
-                    bar_wait(&s.afull[sl], aph, err);
-                    tc_fence_after();
-                    if (elect_one()) {
-#pragma unroll
-                        for (int q = 0; q < 8; ++q)
-                            tc_mma_i8(d[i], tmem_a + sl * T::ASTRIDE + q * 8, bdesc + q * (2 * BN), idesc, q == 0 ? more : 1u);
-                        if (WIDE) {
-                            const unsigned at = tmem_a + sl * T::ASTRIDE + 64;
-                            tc_mma_i8(d[i], at, bdesc + 8 * (2 * BN), idesc, 1u);
-                            tc_mma_i8(d[i] + BN, at, bdesc + 9 * (2 * BN), idesc, more);
-                            tc_mma_i8(d[i] + BN, at + 8, bdesc + 10 * (2 * BN), idesc, 1u);
-                        }
-                        tc_commit(&s.aempty[sl]);
-                        if (i == S - 1) tc_commit(&s.bempty[st]);
+                    for (int q = 0; q < 8; ++q)
+                        tc_mma_i8(d, tmem_a + slot * T::ASTRIDE + q * 8, bdesc + q * (2 * BN), idesc, q == 0 ? more : 1u);
+                    if (WIDE) {
+                        const unsigned at = tmem_a + slot * T::ASTRIDE + 64;
+                        tc_mma_i8(d, at, bdesc + 8 * (2 * BN), idesc, 1u);
+                        tc_mma_i8(d + BN, at, bdesc + 9 * (2 * BN), idesc, more);
+                        tc_mma_i8(d + BN, at + 8, bdesc + 10 * (2 * BN), idesc, 1u);
                     }
-                    __syncwarp();
-                    if (!FIX && ++slot == unsigned(T::WG)) {
-                        slot = 0;
-                        aph ^= 1u;
-                    }
+                    tc_commit(&s.aempty[slot]);
+                    tc_commit(&s.bempty[st]);
                 }
-                if (FIX) aph ^= 1u;
+                __syncwarp();
+                if (++slot == unsigned(T::SLOTS)) {
+                    slot = 0;
+                    aph ^= 1u;
+                }
                 more = 1;
                 if (++st == unsigned(T::STAGES)) {
                     st = 0;
                     bph ^= 1u;
                 }
             }
-            if (elect_one()) {
-#pragma unroll
-                for (int i = 0; i < S; ++i) tc_commit(&s.accfull[accs[i]]);
-            }
+            if (elect_one()) tc_commit(accfull);
             __syncwarp();
         }
         if (elect_one()) tc_commit(&s.done);  // nothing of this CTA is in flight when the columns go back
@@ -629,7 +605,7 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
             unsigned bs = 0;
             bool ok = true;
             for (int u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
-                const Unit un = unit_of<BN, S>(p, u);
+                const Unit un = unit_of<BN>(p, u);
                 const unsigned char* src = p.wexp + ((long long)un.nt * p.G + un.g0) * T::STAGE;
                 for (int g = un.g0; g < un.g1; ++g, ++bs, src += T::STAGE) {
                     const unsigned st = bs % T::STAGES;
@@ -920,14 +896,14 @@ __global__ void __launch_bounds__(256) tc_expand_kernel(const TcExpand p)
     }
 }
 
-template <int BN, int S, bool NEXT, bool WIDE>
+template <int BN, bool NEXT, bool WIDE>
 int run_cfg(const TcRun& p0, cudaStream_t st)
 {
     TcRun p = p0;
     p.err_flag = kernel_error_flag();
     const int dev = device_slot();
     if (!p.err_flag || dev < 0) return DS_ERR_CUDA;
-    auto kern = tc_run_kernel<BN, S, NEXT, WIDE>;
+    auto kern = tc_run_kernel<BN, NEXT, WIDE>;
     const size_t smem = sizeof(TcSmem<BN, WIDE>);
     static bool done[kMaxDevices];  // per instantiation and device
     static int sms[kMaxDevices];
@@ -983,18 +959,11 @@ int tc_launch_expand(const TcExpand& p, int grid_n, cudaStream_t st)
     return cudaGetLastError() == cudaSuccess ? DS_OK : DS_ERR_CUDA;
 }
 
-template <bool NEXT>
-static int tc_launch_next(const TcRun& p, int BN, int S, cudaStream_t st)
+int tc_launch_run(const TcRun& p, int BN, bool wide, cudaStream_t st)
 {
-    if (BN == 128) return S == 2 ? run_cfg<128, 2, NEXT, false>(p, st) : run_cfg<128, 1, NEXT, false>(p, st);
-    if (BN == 64) return S == 3 ? run_cfg<64, 3, NEXT, false>(p, st) : run_cfg<64, 1, NEXT, false>(p, st);
-    return S == 3 ? run_cfg<32, 3, NEXT, false>(p, st) : run_cfg<32, 1, NEXT, false>(p, st);
-}
-
-int tc_launch_run(const TcRun& p, int BN, int S, bool wide, cudaStream_t st)
-{
-    if (wide) return run_cfg<64, 1, false, true>(p, st);
-    return p.next ? tc_launch_next<true>(p, BN, S, st) : tc_launch_next<false>(p, BN, S, st);
+    if (wide) return run_cfg<64, false, true>(p, st);
+    if (p.next) return BN == 128 ? run_cfg<128, true, false>(p, st) : BN == 64 ? run_cfg<64, true, false>(p, st) : run_cfg<32, true, false>(p, st);
+    return BN == 128 ? run_cfg<128, false, false>(p, st) : BN == 64 ? run_cfg<64, false, false>(p, st) : run_cfg<32, false, false>(p, st);
 }
 
 }  // namespace ds

@@ -51,7 +51,7 @@ struct TcGeom {
     int align;           // every load starts at a multiple of this: 16, 8 or 4
     long long plane;     // bytes of one byte plane
     int wide;            // 24-bit codes: three byte planes
-    int BN, S;           // tile: S x 128 rows, BN columns
+    int BN;              // tile: 128 rows, BN columns
     int grid_m, grid_n, splits, gps;  // gps: groups per split
     long long act_bytes;      // scratch of one call: header, partial sums, both planes
     long long planes_off;
@@ -126,6 +126,6 @@ long long check_shrink_x();
 
 int tc_launch_pack(const TcPack& p, bool wide, cudaStream_t st);
 int tc_launch_expand(const TcExpand& p, int grid_n, cudaStream_t st);
-int tc_launch_run(const TcRun& p, int BN, int S, bool wide, cudaStream_t st);
+int tc_launch_run(const TcRun& p, int BN, bool wide, cudaStream_t st);
 
 }  // namespace ds

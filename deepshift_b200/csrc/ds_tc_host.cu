@@ -33,10 +33,10 @@ void choose_pixel(TcGeom& g)
 }
 
 // Clock cycles of one (group, 128 rows) item: eight MMAs (eleven when wide).
-double item_cycles(int bn, int s, bool wide)
+double item_cycles(int bn, bool wide)
 {
-    if (wide) return 800;
-    return bn == 128 ? 810 : 690;  // measured; 64 and 32 columns cost the same
+    if (wide) return 1000;
+    return bn == 128 ? 700 : bn == 64 ? 520 : 480;
 }
 
 // Tile and split with the smallest estimated time: waves of units over the SMs, a unit being the longer of
@@ -47,29 +47,24 @@ void choose_tile(TcGeom& g)
     const int bns[3] = {128, 64, 32};
     for (int bn : bns) {
         if (g.wide ? bn != 64 : bn > 32 && g.N <= bn / 2) continue;
-        const int smax = bn == 128 ? 2 : 3;  // row blocks that share a weight tile
-        for (int s = 1; s <= smax; s += smax - 1) {
-            if (g.wide && s > 1) continue;  // two accumulators per row block
-            const long long gm = (g.M + s * TC_ROWS - 1ll) / (s * TC_ROWS), gn = (g.N + bn - 1) / bn;
-            const double epi = s * TC_ROWS * (double)bn * 4 / 23;
-            for (int sp = 1; sp <= 16; ++sp) {
-                const int gps = (g.G + sp - 1) / sp;
-                if (sp > 1 && (gps < 4 || (g.G + gps - 1) / gps != sp)) continue;
-                if (sp > 1 && gm * gn >= 2 * kSms) break;
-                const long long units = gm * gn * sp;
-                const double waves = double((units + kSms - 1) / kSms);
-                const double main = gps * s * item_cycles(bn, s, g.wide) + 1500;  // ... and the pipeline's fill
-                double cost = waves * (main > epi ? main : epi) + (main > epi ? epi : main) + 3000;
-                if (sp > 1) cost += 3000 + 800.0 * sp * s * (bn / 32);  // the last CTA reads all partial sums
-                if (cost < best) {
-                    best = cost;
-                    g.BN = bn;
-                    g.S = s;
-                    g.grid_m = int(gm);
-                    g.grid_n = int(gn);
-                    g.splits = sp;
-                    g.gps = gps;
-                }
+        const long long gm = (g.M + TC_ROWS - 1ll) / TC_ROWS, gn = (g.N + bn - 1) / bn;
+        const double epi = TC_ROWS * (double)bn * 4 / 23;
+        for (int sp = 1; sp <= 16; ++sp) {
+            const int gps = (g.G + sp - 1) / sp;
+            if (sp > 1 && (gps < 4 || (g.G + gps - 1) / gps != sp)) continue;
+            if (sp > 1 && gm * gn >= 2 * kSms) break;
+            const long long units = gm * gn * sp;
+            const double waves = double((units + kSms - 1) / kSms);
+            const double main = gps * item_cycles(bn, g.wide) + 300;
+            double cost = waves * (main > epi ? main : epi) + (main > epi ? epi : main) + 3000;  // ... and the pipeline's fill
+            if (sp > 1) cost += 3000 + 800.0 * sp * (bn / 32);  // the last CTA reads all partial sums
+            if (cost < best) {
+                best = cost;
+                g.BN = bn;
+                g.grid_m = int(gm);
+                g.grid_n = int(gn);
+                g.splits = sp;
+                g.gps = gps;
             }
         }
     }
@@ -114,7 +109,7 @@ int tc_geometry(TcGeom& g, int B, int C, int H, int W, int OC, int KH, int KW, i
     const long long tiles = (long long)g.grid_m * g.grid_n;
     if (tiles * g.splits > limit || g.grid_n > 65535) return DS_ERR_UNSUPPORTED;
     if (g.splits > 1 && tiles > TC_MAX_SPLIT_TILES) return DS_ERR_UNSUPPORTED;
-    g.planes_off = TC_HEADER + (g.splits > 1 ? tiles * g.splits * (long long)g.S * TC_ROWS * g.BN * 4 : 0);
+    g.planes_off = TC_HEADER + (g.splits > 1 ? tiles * g.splits * TC_ROWS * g.BN * 4 : 0);
     g.act_bytes = g.planes_off + (wide ? 3 : 2) * g.plane;
     g.colc_off = (long long)g.grid_n * g.G * g.BN * (wide ? TC_PLANES_WIDE : TC_PLANES) * TC_KG;
     g.weight_bytes = g.colc_off + round16(4ll * g.N + 4);  // the word behind: a shift of 16..31 exists (wide)
@@ -165,7 +160,7 @@ bool worthwhile(const TcGeom& g, int in_kind)
         const double waves = tiles >= kSms ? double((tiles + kSms - 1) / kSms) : tiles * 4 >= kSms ? (double)tiles / kSms : 0.25;
         if (waves * g.K * (g.N > 64 ? 0.23 : 0.13) < 20) return false;
     }
-    const double padded = (double)g.grid_m * g.S * TC_ROWS * g.grid_n * g.BN * g.G * TC_KG;
+    const double padded = (double)g.grid_m * TC_ROWS * g.grid_n * g.BN * g.G * TC_KG;
     return tiles <= 16 ? ops >= 6e6 : ops >= double(1 << 26) && ops * 5 >= padded;
 }
 
@@ -373,7 +368,7 @@ extern "C" int ds_tc_conv2d_ex(const void* x, const ds_planes_t* xp, const int32
     p.gate_want = 0;
     p.chk_o_bytes = (long long)g.M * g.N * 4;
     p.chk_status = bounds_status_ptr();
-    rc = tc_launch_run(p, g.BN, g.S, wide, st);
+    rc = tc_launch_run(p, g.BN, wide, st);
     if (rc || mode != TC_GATED) return rc;
     return launch_gated_int(x, packed, bias, out, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, bits, base, fuse, flag, 1, st);
 }
