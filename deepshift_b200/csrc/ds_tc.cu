@@ -1,10 +1,11 @@
 // Tensor-core shift GEMM / convolution (tcgen05, kind::i8).  The arithmetic is described in ds_tc.cuh.
 //
-// Three kernels per call:
+// Three kernels:
 //   tc_pack_*     x (int32 or fp32, quantised here) -> two byte planes l and h, pixel-major with a physical
 //                 zero border.  One pass over x; from here on a filter tap is an address offset.
 //   tc_expand     packed weights -> s8 operand tiles in the order the MMA reads them, and const[n].  Once per
-//                 layer for callers that keep it.
+//                 layer for callers that keep it and never change the weights; where they may change, tc_pack looks
+//                 after a kept buffer.
 //   tc_run        the product.  Persistent, one CTA per SM, warp-specialised:
 //                   warps 0-     two or three producer warpgroups, thread = output row = TMEM lane.  A thread loads 16
 //                                values (16 bytes of l, 16 of h) and turns them into the sixteen planes with
@@ -639,138 +640,6 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
     if (threadIdx.x == 0 && s.err) *p.err_flag = 1;
 }
 
-// ---- activations -> byte planes -----------------------------------------------------------------------
-// Code of the raw word `v` of x, as operand_of defines it for the integer path.
-template <int INK>
-__device__ __forceinline__ int pack_code(const TcPack& p, int v)
-{
-    if (INK == INK_I32) return v;
-    if (INK == INK_I32_CLAMP) return min(max(v, p.rq_lo), p.rq_hi) * p.rq_mul + p.rq_add;
-    if (p.in_kind == DS_IN_F32_CONV) return __float2int_rz(quant_conv_f(__int_as_float(v), p.q));
-    return __float2int_rz(truncf(__int_as_float(v) * p.q.scale));
-}
-
-// Bytes l and h of four codes; notes a code that does not fit 16 bits.
-__device__ __forceinline__ void pack4(const int (&c)[4], unsigned& l, unsigned& h, bool& over)
-{
-    unsigned y[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        y[e] = unsigned(c[e]) + 32768u;
-        over |= y[e] > 65535u;
-    }
-    const unsigned a = __byte_perm(y[0], y[1], 0x5140), b = __byte_perm(y[2], y[3], 0x5140);  // l0 l1 h0 h1
-    l = __byte_perm(a, b, 0x5410);
-    h = __byte_perm(a, b, 0x7632);
-}
-
-// NCHW -> pixel-major planes.  A block takes 1024 / CW padded pixels x 4 CW channels: lanes run over pixels
-// when reading (coalesced in x), over channels when writing (coalesced in the planes).  HBM-bound: 4 bytes
-// read and 2 written per value.
-template <int INK>
-__global__ void __launch_bounds__(256) tc_pack_nchw_kernel(const TcPack p, int cw_log)
-{
-    __shared__ unsigned sl[2048], sh[2048];
-    const int CW = 1 << cw_log, PIX = 1024 >> cw_log;
-    const long long q0 = (long long)blockIdx.x * PIX;
-    const int cw0 = blockIdx.y << cw_log;
-    if (p.counters && blockIdx.y == 0)
-        for (long long i = blockIdx.x * 256ll + threadIdx.x; i < p.ncounters; i += gridDim.x * 256ll) p.counters[i] = 0;
-    const long long hw = (long long)p.H * p.W;
-    const int* x = static_cast<const int*>(p.x);
-    bool over = false;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int i = threadIdx.x + 256 * k;
-        const int pix = i & (PIX - 1), cw = i >> (10 - cw_log);
-        const long long q = q0 + pix;
-        int c4[4] = {0, 0, 0, 0};
-        if (q < p.Q) {
-            const unsigned qi = unsigned(q);
-            const unsigned rowi = qi / unsigned(p.Wp);
-            const int w = (int(qi - rowi * unsigned(p.Wp)) - p.pw) * p.sub_w;
-            const unsigned b = rowi / unsigned(p.Hp);
-            const int h = (int(rowi - b * unsigned(p.Hp)) - p.ph) * p.sub_h;
-            if (unsigned(h) < unsigned(p.H) && unsigned(w) < unsigned(p.W)) {
-                const int c = 4 * (cw0 + cw);
-                const int* src = x + ((long long)b * p.C + c) * hw + (long long)h * p.W + w;
-                int raw[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) raw[e] = (c + e < p.C && DS_X_OK(p, src + e * hw, 4)) ? __ldg(src + e * hw) : 0;
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (c + e < p.C) c4[e] = pack_code<INK>(p, raw[e]);
-            }
-        }
-        unsigned l, h;
-        pack4(c4, l, h, over);
-        sl[pix * (CW + 1) + cw] = l;
-        sh[pix * (CW + 1) + cw] = h;
-    }
-    if (over && p.flag) *p.flag = 1;
-    __syncthreads();
-    const int cwords = p.Cp >> 2;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int i = threadIdx.x + 256 * k;
-        const int cw = i & (CW - 1), pix = i >> cw_log;
-        const long long q = q0 + pix;
-        if (q < p.Q && cw0 + cw < cwords) {
-            unsigned* dst = reinterpret_cast<unsigned*>(p.act + q * p.Cp) + cw0 + cw;
-            *dst = sl[pix * (CW + 1) + cw];
-            *reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(dst) + p.plane) = sh[pix * (CW + 1) + cw];
-        }
-    }
-}
-
-// Rows of a matrix [Q, C]: 4 values of a row per thread.
-template <int INK, bool WIDE>
-__global__ void __launch_bounds__(256) tc_pack_rows_kernel(const TcPack p)
-{
-    const unsigned words = unsigned(p.Cp) >> 2;
-    const unsigned total = unsigned(p.Q) * words;  // plane bytes < 2^31, so this fits
-    const bool vec = p.C % 4 == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15u) == 0;
-    const unsigned i0 = blockIdx.x * 256u + threadIdx.x;
-    if (p.counters)
-        for (unsigned i = i0; i < unsigned(p.ncounters); i += gridDim.x * 256u) p.counters[i] = 0;
-    bool over = i0 == 0 && p.refuse && *p.refuse;
-    for (unsigned i = i0; i < total; i += gridDim.x * 256u) {
-        const unsigned m = i / words, w = i - m * words;
-        const int k = int(4 * w);
-        const int* src = static_cast<const int*>(p.x) + (long long)m * p.C + k;
-        int raw[4] = {0, 0, 0, 0}, c4[4];
-        if (vec && k + 4 <= p.C) {
-            if (DS_X_OK(p, src, 16)) {
-                const int4 v = __ldg(reinterpret_cast<const int4*>(src));
-                raw[0] = v.x; raw[1] = v.y; raw[2] = v.z; raw[3] = v.w;
-            }
-        } else {
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-                if (k + e < p.C && DS_X_OK(p, src + e, 4)) raw[e] = __ldg(src + e);
-        }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) c4[e] = k + e < p.C ? pack_code<INK>(p, raw[e]) : 0;
-        unsigned l, h;
-        unsigned* dst = reinterpret_cast<unsigned*>(p.act) + i;
-        if (WIDE) {
-            unsigned y[4], t = 0;
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                y[e] = unsigned(c4[e]) + (1u << 23);
-                over |= y[e] >> 24 != 0;
-                t |= ((y[e] >> 16) & 255u) << (8 * e);
-                c4[e] = int(y[e] & 0xFFFFu) - 32768;
-            }
-            *reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(dst) + 2 * p.plane) = t;
-        }
-        pack4(c4, l, h, over);
-        *dst = l;
-        *reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(dst) + p.plane) = h;
-    }
-    if (over && p.flag) *p.flag = 1;
-}
-
 // ---- weights -> operand tiles -------------------------------------------------------------------------
 // Coefficient of plane f for a right shift r in 0..15 (ds_tc.cuh).
 constexpr int tc_coef(int r, int f)
@@ -819,29 +688,36 @@ __device__ __forceinline__ int tc_code(const TcExpand& p, unsigned field)
     return min(r, 15) | (((field >> p.dec.bits) & 1u) ? 0 : 16);
 }
 
-constexpr int TC_COLC_BLOCKS = 16;  // blocks per column tile that compute const[n]
+constexpr int TC_KEEP_WAIT = 1 << 22;  // rounds of at least 64 ns
 
-// Block (g, nt): the operand tile of group g, columns nt * BN.. -- [16 planes][BN][16 bytes].  A thread makes
+struct ExpandSmem {
+    unsigned lut[6][33];
+    int stale;
+    alignas(16) unsigned char codes[128 * 16];
+};
+
+// Block (nt, g): the operand tile of group g, columns nt * BN.. -- [16 planes][BN][16 bytes].  A thread makes
 // four planes of one column: 16 table words (four planes each, sign applied), transposed 4 x 4 bytes.
 // Blocks g = G.. compute the column constants -sum s 2^(15-r).
-__global__ void __launch_bounds__(256) tc_expand_kernel(const TcExpand p)
+__device__ __forceinline__ void expand_block(const TcExpand& p, int nt, int g, ExpandSmem& sm)
 {
-    const int n0 = blockIdx.y * p.BN;
+    const int n0 = nt * p.BN;
     const unsigned fmask = (1u << p.dec.fw) - 1u;
-    if (int(blockIdx.x) >= p.G) {
+    if (g >= p.G) {
         const int per = p.BN / TC_COLC_BLOCKS;  // 2, 4 or 8 columns: one per warp
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const int n = n0 + (int(blockIdx.x) - p.G) * per + warp;
+        const int n = n0 + (g - p.G) * per + warp;
         if (warp >= per || n >= p.N) return;
         const int* src = p.packed + (long long)n * p.dec.row_len;
         unsigned sum = 0;
+        bool far = false;
         for (int w = lane; w < p.dec.row_len; w += 32) {
             unsigned word = DS_W_OK(p, src + w, 4) ? unsigned(__ldg(src + w)) : 0u;
             const int k = w * p.dec.num;
             for (int i = 0; i < p.dec.num && k + i < p.K; ++i, word >>= p.dec.fw) {
                 const int c = tc_code(p, word & fmask);
                 if (c < 32) {
-                    if (p.wide && (word & fmask & ((1u << p.dec.bits) - 1u)) >= 16u) p.colc[p.N] = 1;
+                    if (p.wide) far |= (word & fmask & ((1u << p.dec.bits) - 1u)) >= 16u;
                     const unsigned v = 1u << ((p.wide ? 23 : 15) - (c & 15));
                     sum += (c & 16) ? v : 0u - v;
                 }
@@ -849,13 +725,14 @@ __global__ void __launch_bounds__(256) tc_expand_kernel(const TcExpand p)
         }
 #pragma unroll
         for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+        if (p.wide && __any_sync(0xFFFFFFFFu, far) && lane == 0) {
+            p.colc[p.N] = 1;
+            if (p.range_flag) *p.range_flag = 1;
+        }
         if (lane == 0) p.colc[n] = int(sum);
         return;
     }
-    __shared__ unsigned lut[6][33];
-    __shared__ __align__(16) unsigned char codes[128 * 16];
-    const int g = blockIdx.x;
-    for (int i = threadIdx.x; i < 6 * 33; i += 256) (&lut[0][0])[i] = g_tc_lut.w[i];
+    for (int i = threadIdx.x; i < 6 * 33; i += 256) (&sm.lut[0][0])[i] = g_tc_lut.w[i];
     // a thread keeps its place in the group (and with it the word and the bit position) and walks the columns
     const int kh = g / p.J, j = g - kh * p.J;
     const int t = 16 * j + (threadIdx.x & 15);  // byte of the window row: (kw, c)
@@ -869,20 +746,20 @@ __global__ void __launch_bounds__(256) tc_expand_kernel(const TcExpand p)
     for (int nl = nl0; nl < p.BN; nl += 16, src += 16ll * p.dec.row_len) {
         int code = 32;
         if (live && n0 + nl < p.N && DS_W_OK(p, src, 4)) code = tc_code(p, (unsigned(__ldg(src)) >> at) & fmask);
-        codes[nl * 16 + (threadIdx.x & 15)] = (unsigned char)code;
+        sm.codes[nl * 16 + (threadIdx.x & 15)] = (unsigned char)code;
     }
     __syncthreads();
-    uint4* out = reinterpret_cast<uint4*>(p.wexp + ((long long)blockIdx.y * p.G + g) * (p.BN * (p.wide ? TC_PLANES_WIDE : TC_PLANES) * TC_KG));
+    uint4* out = reinterpret_cast<uint4*>(p.wexp + ((long long)nt * p.G + g) * (p.BN * (p.wide ? TC_PLANES_WIDE : TC_PLANES) * TC_KG));
     for (int i = threadIdx.x; i < p.BN * (p.wide ? 6 : 4); i += 256) {
         const int n = i & (p.BN - 1), q = i / p.BN;
-        const uint4 cw = *reinterpret_cast<const uint4*>(codes + n * 16);
+        const uint4 cw = *reinterpret_cast<const uint4*>(sm.codes + n * 16);
         const unsigned cws[4] = {cw.x, cw.y, cw.z, cw.w};
         unsigned o[4][4];  // [plane][word]
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
             unsigned a[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) a[e] = lut[q][(cws[w] >> (8 * e)) & 255u];
+            for (int e = 0; e < 4; ++e) a[e] = sm.lut[q][(cws[w] >> (8 * e)) & 255u];
             const unsigned x01 = __byte_perm(a[0], a[1], 0x5140), y01 = __byte_perm(a[0], a[1], 0x7362);
             const unsigned x23 = __byte_perm(a[2], a[3], 0x5140), y23 = __byte_perm(a[2], a[3], 0x7362);
             o[0][w] = __byte_perm(x01, x23, 0x5410);
@@ -894,6 +771,241 @@ __global__ void __launch_bounds__(256) tc_expand_kernel(const TcExpand p)
         for (int f = 0; f < 4; ++f)
             if (4 * q + f < TC_PLANES_WIDE) out[(4 * q + f) * p.BN + n] = make_uint4(o[f][0], o[f][1], o[f][2], o[f][3]);
     }
+}
+
+__global__ void __launch_bounds__(256) tc_expand_kernel(const TcExpand p)
+{
+    __shared__ ExpandSmem sm;
+    expand_block(p, blockIdx.y, blockIdx.x, sm);
+}
+
+// Kept buffers.  The tiles stay with the packed words they were made from, and the packing launch of every call looks
+// after them: its first blocks compare the copy with the words of the moment (4096 x 4096 weights: 34 MB, 9 us; a
+// convolution's disappear in the packing pass), its last ones wait for those and make the tiles again if a word
+// differs.  Weights changed by any means take effect with the next call, and no launch is added for it (comparing
+// tile by tile inside the expansion took 45 us for 4096 x 4096, a launch of its own 5 us per layer).
+__device__ __forceinline__ void keep_compare(const TcExpand& p, unsigned block)
+{
+    const long long i0 = block * 256ll + threadIdx.x, step = p.cmp_blocks * 256ll;
+    const long long n4 = (reinterpret_cast<uintptr_t>(p.packed) & 15u) == 0 ? p.nwords / 4 : 0;
+    bool differs = p.fresh != 0;
+#pragma unroll 2
+    for (long long i = i0; i < n4; i += step) {
+        const int4* src = reinterpret_cast<const int4*>(p.packed) + i;
+        int4* dst = reinterpret_cast<int4*>(p.words) + i;
+        if (!DS_W_OK(p, src, 16)) continue;
+        const int4 a = __ldg(src), b = __ldcg(dst);
+        if (p.fresh || ((a.x ^ b.x) | (a.y ^ b.y) | (a.z ^ b.z) | (a.w ^ b.w)) != 0) {
+            *dst = a;
+            differs = true;
+        }
+    }
+    for (long long i = 4 * n4 + i0; i < p.nwords; i += step) {
+        if (!DS_W_OK(p, p.packed + i, 4)) continue;
+        const int a = __ldg(p.packed + i);
+        if (p.fresh || a != __ldcg(p.words + i)) {
+            p.words[i] = a;
+            differs = true;
+        }
+    }
+    if (differs) {
+        p.colc[p.N] = 0;  // found again, if it holds, when the tiles are made
+        p.state[0] = 1;
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) atomicAdd(p.state + 1, 1);
+}
+
+// The wait ends: the blocks waited for depend on nothing, and exp_blocks never fill the GPU.  (Bounded all the same.)
+__device__ __forceinline__ void keep_expand(const TcExpand& p, int block, ExpandSmem& sm)
+{
+    if (threadIdx.x == 0) {
+        int done = 0;
+        for (int i = 0; i < TC_KEEP_WAIT && !done; ++i) {
+            done = *(volatile const int*)(p.state + 1) >= p.cmp_blocks;
+            if (!done) __nanosleep(64);
+        }
+        if (!done) *p.err_flag = 1;
+        __threadfence();
+        sm.stale = *(volatile const int*)p.state;
+    }
+    __syncthreads();
+    if (sm.stale) {
+        const int per_tile = p.G + TC_COLC_BLOCKS;
+        for (int b = block; b < p.total; b += p.exp_blocks) {
+            const int nt = b / per_tile;
+            expand_block(p, nt, b - nt * per_tile, sm);
+            __syncthreads();
+        }
+    }
+    if (threadIdx.x == 0 && atomicAdd(p.state + 2, 1) == p.exp_blocks - 1) {
+        // all others have read the state
+        p.state[0] = 0;
+        p.state[1] = 0;
+        p.state[2] = 0;
+    }
+}
+
+// Blocks of a packing launch that look after the weights; false for the others, whose index among themselves goes
+// to `block`.
+__device__ __forceinline__ bool keep_weights(const TcExpand& p, unsigned& block, ExpandSmem& sm)
+{
+    if (blockIdx.x < unsigned(p.cmp_blocks)) {
+        keep_compare(p, blockIdx.x);
+        return true;
+    }
+    const int left = int(gridDim.x - blockIdx.x);
+    if (left <= p.exp_blocks) {
+        keep_expand(p, left - 1, sm);
+        return true;
+    }
+    block = blockIdx.x - unsigned(p.cmp_blocks);
+    return false;
+}
+
+// ---- activations -> byte planes -----------------------------------------------------------------------
+// Code of the raw word `v` of x, as operand_of defines it for the integer path.
+template <int INK>
+__device__ __forceinline__ int pack_code(const TcPack& p, int v)
+{
+    if (INK == INK_I32) return v;
+    if (INK == INK_I32_CLAMP) return min(max(v, p.rq_lo), p.rq_hi) * p.rq_mul + p.rq_add;
+    if (p.in_kind == DS_IN_F32_CONV) return __float2int_rz(quant_conv_f(__int_as_float(v), p.q));
+    return __float2int_rz(truncf(__int_as_float(v) * p.q.scale));
+}
+
+// Bytes l and h of four codes; notes a code that does not fit 16 bits.
+__device__ __forceinline__ void pack4(const int (&c)[4], unsigned& l, unsigned& h, bool& over)
+{
+    unsigned y[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        y[e] = unsigned(c[e]) + 32768u;
+        over |= y[e] > 65535u;
+    }
+    const unsigned a = __byte_perm(y[0], y[1], 0x5140), b = __byte_perm(y[2], y[3], 0x5140);  // l0 l1 h0 h1
+    l = __byte_perm(a, b, 0x5410);
+    h = __byte_perm(a, b, 0x7632);
+}
+
+// NCHW -> pixel-major planes.  A block takes 1024 / CW padded pixels x 4 CW channels: lanes run over pixels
+// when reading (coalesced in x), over channels when writing (coalesced in the planes).  HBM-bound: 4 bytes
+// read and 2 written per value.  `nx` blocks side by side along the pixels, one row of them per 4 CW channels.
+// KEPT: further blocks look after the weights; eight blocks per SM as without them (at the 40 registers the
+// expansion would like, 64 x 64 x 56 x 56 takes 34 us instead of 29).
+template <int INK, bool KEPT>
+__global__ void __launch_bounds__(256, 8) tc_pack_nchw_kernel(const TcPack p, const TcExpand e, int cw_log, unsigned nx)
+{
+    __shared__ __align__(16) unsigned words[2][2048];
+    unsigned block = blockIdx.x;
+    if (KEPT && keep_weights(e, block, *reinterpret_cast<ExpandSmem*>(&words[0][0]))) return;
+    unsigned *sl = words[0], *sh = words[1];
+    const unsigned by = block / nx, bx = block - by * nx;
+    const int CW = 1 << cw_log, PIX = 1024 >> cw_log;
+    const long long q0 = (long long)bx * PIX;
+    const int cw0 = int(by << cw_log);
+    if (p.counters && by == 0)
+        for (long long i = bx * 256ll + threadIdx.x; i < p.ncounters; i += nx * 256ll) p.counters[i] = 0;
+    const long long hw = (long long)p.H * p.W;
+    const int* x = static_cast<const int*>(p.x);
+    bool over = false;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int i = threadIdx.x + 256 * k;
+        const int pix = i & (PIX - 1), cw = i >> (10 - cw_log);
+        const long long q = q0 + pix;
+        int c4[4] = {0, 0, 0, 0};
+        if (q < p.Q) {
+            const unsigned qi = unsigned(q);
+            const unsigned rowi = qi / unsigned(p.Wp);
+            const int w = (int(qi - rowi * unsigned(p.Wp)) - p.pw) * p.sub_w;
+            const unsigned b = rowi / unsigned(p.Hp);
+            const int h = (int(rowi - b * unsigned(p.Hp)) - p.ph) * p.sub_h;
+            if (unsigned(h) < unsigned(p.H) && unsigned(w) < unsigned(p.W)) {
+                const int c = 4 * (cw0 + cw);
+                const int* src = x + ((long long)b * p.C + c) * hw + (long long)h * p.W + w;
+                int raw[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) raw[e] = (c + e < p.C && DS_X_OK(p, src + e * hw, 4)) ? __ldg(src + e * hw) : 0;
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (c + e < p.C) c4[e] = pack_code<INK>(p, raw[e]);
+            }
+        }
+        unsigned l, h;
+        pack4(c4, l, h, over);
+        sl[pix * (CW + 1) + cw] = l;
+        sh[pix * (CW + 1) + cw] = h;
+    }
+    if (over && p.flag) *p.flag = 1;
+    __syncthreads();
+    const int cwords = p.Cp >> 2;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int i = threadIdx.x + 256 * k;
+        const int cw = i & (CW - 1), pix = i >> cw_log;
+        const long long q = q0 + pix;
+        if (q < p.Q && cw0 + cw < cwords) {
+            unsigned* dst = reinterpret_cast<unsigned*>(p.act + q * p.Cp) + cw0 + cw;
+            *dst = sl[pix * (CW + 1) + cw];
+            *reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(dst) + p.plane) = sh[pix * (CW + 1) + cw];
+        }
+    }
+}
+
+// Rows of a matrix [Q, C]: 4 values of a row per thread.  KEPT as above.
+template <int INK, bool WIDE, bool KEPT>
+__global__ void __launch_bounds__(256, 8) tc_pack_rows_kernel(const TcPack p, const TcExpand e)
+{
+    unsigned block = blockIdx.x, blocks = gridDim.x;
+    if constexpr (KEPT) {
+        __shared__ ExpandSmem sm;
+        if (keep_weights(e, block, sm)) return;
+        blocks -= unsigned(e.cmp_blocks + e.exp_blocks);
+    }
+    const unsigned words = unsigned(p.Cp) >> 2;
+    const unsigned total = unsigned(p.Q) * words;  // plane bytes < 2^31, so this fits
+    const bool vec = p.C % 4 == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15u) == 0;
+    const unsigned i0 = block * 256u + threadIdx.x;
+    if (p.counters)
+        for (unsigned i = i0; i < unsigned(p.ncounters); i += blocks * 256u) p.counters[i] = 0;
+    bool over = i0 == 0 && p.refuse && *p.refuse;
+    for (unsigned i = i0; i < total; i += blocks * 256u) {
+        const unsigned m = i / words, w = i - m * words;
+        const int k = int(4 * w);
+        const int* src = static_cast<const int*>(p.x) + (long long)m * p.C + k;
+        int raw[4] = {0, 0, 0, 0}, c4[4];
+        if (vec && k + 4 <= p.C) {
+            if (DS_X_OK(p, src, 16)) {
+                const int4 v = __ldg(reinterpret_cast<const int4*>(src));
+                raw[0] = v.x; raw[1] = v.y; raw[2] = v.z; raw[3] = v.w;
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (k + e < p.C && DS_X_OK(p, src + e, 4)) raw[e] = __ldg(src + e);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) c4[e] = k + e < p.C ? pack_code<INK>(p, raw[e]) : 0;
+        unsigned l, h;
+        unsigned* dst = reinterpret_cast<unsigned*>(p.act) + i;
+        if (WIDE) {
+            unsigned y[4], t = 0;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                y[e] = unsigned(c4[e]) + (1u << 23);
+                over |= y[e] >> 24 != 0;
+                t |= ((y[e] >> 16) & 255u) << (8 * e);
+                c4[e] = int(y[e] & 0xFFFFu) - 32768;
+            }
+            *reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(dst) + 2 * p.plane) = t;
+        }
+        pack4(c4, l, h, over);
+        *dst = l;
+        *reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(dst) + p.plane) = h;
+    }
+    if (over && p.flag) *p.flag = 1;
 }
 
 template <int BN, bool NEXT, bool WIDE>
@@ -925,20 +1037,35 @@ int run_cfg(const TcRun& p0, cudaStream_t st)
 
 }  // namespace
 
-int tc_launch_pack(const TcPack& p, bool wide, cudaStream_t st)
+int tc_launch_pack(const TcPack& p, const TcExpand* e0, bool wide, cudaStream_t st)
 {
+    TcExpand e = e0 ? *e0 : TcExpand{};
+    if (e0) {
+        e.err_flag = kernel_error_flag();
+        if (!e.err_flag) return DS_ERR_CUDA;
+        const long long want = (e.nwords + 2047) / 2048;
+        e.cmp_blocks = int(want > 148 * 4 ? 148 * 4 : want);
+        e.exp_blocks = e.total < 148 ? e.total : 148;
+    }
+    const unsigned more = unsigned(e.cmp_blocks + e.exp_blocks);
     auto rows = [&](auto ink) {
         const long long want = (p.Q * (p.Cp / 4) + 255) / 256;
-        const unsigned grid = unsigned(want > 148 * 64 ? 148 * 64 : want);
-        if (wide) tc_pack_rows_kernel<decltype(ink)::value, true><<<grid, 256, 0, st>>>(p);
-        else tc_pack_rows_kernel<decltype(ink)::value, false><<<grid, 256, 0, st>>>(p);
+        const unsigned grid = unsigned(want > 148 * 64 ? 148 * 64 : want) + more;
+        constexpr int K = decltype(ink)::value;
+        if (wide && e0) tc_pack_rows_kernel<K, true, true><<<grid, 256, 0, st>>>(p, e);
+        else if (wide) tc_pack_rows_kernel<K, true, false><<<grid, 256, 0, st>>>(p, e);
+        else if (e0) tc_pack_rows_kernel<K, false, true><<<grid, 256, 0, st>>>(p, e);
+        else tc_pack_rows_kernel<K, false, false><<<grid, 256, 0, st>>>(p, e);
     };
     auto nchw = [&](auto ink) {
         int lg = 0;
         while (lg < 4 && (4 << lg) < p.Cp) ++lg;
         const int pix = 1024 >> lg;
-        const dim3 grid(unsigned((p.Q + pix - 1) / pix), unsigned((p.Cp / 4 + (1 << lg) - 1) >> lg));
-        tc_pack_nchw_kernel<decltype(ink)::value><<<grid, 256, 0, st>>>(p, lg);
+        const unsigned nx = unsigned((p.Q + pix - 1) / pix);
+        const unsigned grid = nx * unsigned((p.Cp / 4 + (1 << lg) - 1) >> lg) + more;
+        constexpr int K = decltype(ink)::value;
+        if (e0) tc_pack_nchw_kernel<K, true><<<grid, 256, 0, st>>>(p, e, lg, nx);
+        else tc_pack_nchw_kernel<K, false><<<grid, 256, 0, st>>>(p, e, lg, nx);
     };
     auto go = [&](auto ink) {
         if (p.Hp == 1 && p.Wp == 1 && p.H == 1 && p.W == 1) rows(ink);
@@ -951,10 +1078,10 @@ int tc_launch_pack(const TcPack& p, bool wide, cudaStream_t st)
     return cudaGetLastError() == cudaSuccess ? DS_OK : DS_ERR_CUDA;
 }
 
-int tc_launch_expand(const TcExpand& p, int grid_n, cudaStream_t st)
+int tc_launch_expand(const TcExpand& p, cudaStream_t st)
 {
     if (p.wide && cudaMemsetAsync(p.colc + p.N, 0, sizeof(int), st) != cudaSuccess) return DS_ERR_CUDA;
-    tc_expand_kernel<<<dim3(unsigned(p.G + TC_COLC_BLOCKS), unsigned(grid_n)), 256, 0, st>>>(p);
+    tc_expand_kernel<<<dim3(unsigned(p.G + TC_COLC_BLOCKS), unsigned(p.total / (p.G + TC_COLC_BLOCKS))), 256, 0, st>>>(p);
     note_launch();
     return cudaGetLastError() == cudaSuccess ? DS_OK : DS_ERR_CUDA;
 }

@@ -34,6 +34,7 @@ constexpr int TC_ROWS = 128;    // rows (TMEM lanes) of one MMA
 constexpr int TC_PLANES = 16;   // functions f_p per value
 constexpr int TC_PLANES_WIDE = 22;  // ... of one 24-bit value: planes 16-21 are copies of t
 constexpr int TC_KG = 16;       // values of k per group: one 16-byte run of each plane
+constexpr int TC_COLC_BLOCKS = 16;  // expansion blocks per column tile that compute const[n]
 // Scratch header: the range flag, then the arrival counters of split tiles (K is split only below 2 x 148
 // tiles).  At a fixed place, so that calls of different geometry may share a scratch buffer: the counters are
 // zero before and after every call.
@@ -55,8 +56,8 @@ struct TcGeom {
     int grid_m, grid_n, splits, gps;  // gps: groups per split
     long long act_bytes;      // scratch of one call: header, partial sums, both planes
     long long planes_off;
-    long long weight_bytes;   // expanded weights, then the column constants
-    long long colc_off;
+    long long weight_bytes;   // expanded weights, the column constants, then what a kept buffer is checked by:
+    long long colc_off, state_off, words_off;  // two state words and a copy of the packed words
 };
 
 struct TcRun {
@@ -112,6 +113,16 @@ struct TcExpand {
     Decode dec;
     int C, KH, KW, Cp, J, G, N, K, BN;
     int wide;            // 22 planes; colc[N] is set when a weight has a shift of 16..31
+    int total;           // blocks of work: (G + TC_COLC_BLOCKS) per column tile
+    // A kept buffer, looked after by blocks of the packing launch (tc_keep_*):
+    int* words;          // copy of the packed words that its tiles were made from
+    int* state;          // three words, zero between calls: words differ; comparing, expanding blocks that are done
+    long long nwords;
+    int fresh;           // nothing is in the buffer yet
+    int cmp_blocks;      // the first blocks of the launch compare, the last `exp_blocks` make stale tiles again
+    int exp_blocks;
+    int* range_flag;     // set with colc[N]; null = none
+    int* err_flag;
     long long chk_w_bytes;
     int* chk_status;
 };
@@ -124,8 +135,9 @@ int launch_gated_int(const void* x, const int32_t* packed, const int32_t* bias, 
                      const int* gate, int want, cudaStream_t st);
 long long check_shrink_x();
 
-int tc_launch_pack(const TcPack& p, bool wide, cudaStream_t st);
-int tc_launch_expand(const TcExpand& p, int grid_n, cudaStream_t st);
+// `e` (may be null): a kept buffer of expanded weights to look after in the same launch.
+int tc_launch_pack(const TcPack& p, const TcExpand* e, bool wide, cudaStream_t st);
+int tc_launch_expand(const TcExpand& p, cudaStream_t st);
 int tc_launch_run(const TcRun& p, int BN, bool wide, cudaStream_t st);
 
 }  // namespace ds

@@ -71,7 +71,8 @@ void choose_tile(TcGeom& g)
 }
 
 // Fills the geometry; DS_ERR_UNSUPPORTED when 32-bit offsets do not reach.
-int tc_geometry(TcGeom& g, int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw, int ph, int pw, bool wide)
+int tc_geometry(TcGeom& g, int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits,
+                bool wide)
 {
     if (B < 0 || C <= 0 || H <= 0 || W <= 0 || OC <= 0 || KH <= 0 || KW <= 0 || sh <= 0 || sw <= 0 || ph < 0 || pw < 0)
         return DS_ERR_BAD_ARG;
@@ -112,7 +113,11 @@ int tc_geometry(TcGeom& g, int B, int C, int H, int W, int OC, int KH, int KW, i
     g.planes_off = TC_HEADER + (g.splits > 1 ? tiles * g.splits * TC_ROWS * g.BN * 4 : 0);
     g.act_bytes = g.planes_off + (wide ? 3 : 2) * g.plane;
     g.colc_off = (long long)g.grid_n * g.G * g.BN * (wide ? TC_PLANES_WIDE : TC_PLANES) * TC_KG;
-    g.weight_bytes = g.colc_off + round16(4ll * g.N + 4);  // the word behind: a shift of 16..31 exists (wide)
+    g.state_off = g.colc_off + round16(4ll * g.N + 4);  // the word behind: a shift of 16..31 exists (wide)
+    g.words_off = g.state_off + 16;
+    const int num = 32 / (bits + 1);
+    g.weight_bytes = g.words_off + round16(4ll * g.N * ((g.K + num - 1) / num));
+    if ((long long)g.grid_n * (g.G + TC_COLC_BLOCKS) > limit) return DS_ERR_UNSUPPORTED;  // blocks of the expansion
     return DS_OK;
 }
 
@@ -176,7 +181,7 @@ extern "C" int ds_tc_bytes(int B, int C, int H, int W, int OC, int KH, int KW, i
     *act_bytes = *weight_bytes = 0;
     if (tc_mode(*fuse, bits, base) == TC_NO) return DS_OK;
     TcGeom g;
-    const int rc = tc_geometry(g, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, fuse->in_kind == DS_IN_F32_LINEAR);
+    const int rc = tc_geometry(g, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, bits, fuse->in_kind == DS_IN_F32_LINEAR);
     if (rc == DS_ERR_UNSUPPORTED) return DS_OK;
     if (rc) return rc;
     if (!any_size && !worthwhile(g, fuse->in_kind)) return DS_OK;
@@ -184,6 +189,34 @@ extern "C" int ds_tc_bytes(int B, int C, int H, int W, int OC, int KH, int KW, i
     *weight_bytes = g.weight_bytes;
     return DS_OK;
 }
+
+namespace ds {
+namespace {
+
+TcExpand expand_params(const TcGeom& g, const int32_t* packed, int bits, void* weights)
+{
+    TcExpand p = {};
+    p.packed = packed;
+    p.wexp = static_cast<unsigned char*>(weights);
+    p.colc = reinterpret_cast<int*>(p.wexp + g.colc_off);
+    p.state = reinterpret_cast<int*>(p.wexp + g.state_off);
+    p.words = reinterpret_cast<int*>(p.wexp + g.words_off);
+    p.total = g.grid_n * (g.G + TC_COLC_BLOCKS);
+    p.dec.bits = bits;
+    p.dec.fw = bits + 1;
+    p.dec.num = 32 / (bits + 1);
+    p.dec.base = 0;
+    p.dec.row_len = (g.K + p.dec.num - 1) / p.dec.num;
+    p.C = g.C; p.KH = g.KH; p.KW = g.KW; p.Cp = g.Cp; p.J = g.J; p.G = g.G; p.N = g.N; p.K = g.K; p.BN = g.BN;
+    p.wide = g.wide;
+    p.nwords = (long long)g.N * p.dec.row_len;
+    p.chk_w_bytes = p.nwords * 4;
+    p.chk_status = bounds_status_ptr();
+    return p;
+}
+
+}  // namespace
+}  // namespace ds
 
 extern "C" int ds_tc_expand(const int32_t* packed, int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw,
                             int ph, int pw, int bits, int base, const ds_fuse_t* fuse, void* weights,
@@ -193,23 +226,10 @@ extern "C" int ds_tc_expand(const int32_t* packed, int B, int C, int H, int W, i
     if (base != 0 || bits < 1 || bits > 7) return DS_ERR_UNSUPPORTED;
     if (reinterpret_cast<uintptr_t>(weights) & 15u) return DS_ERR_ALIGN;
     TcGeom g;
-    const int rc = tc_geometry(g, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, fuse->in_kind == DS_IN_F32_LINEAR);
+    const int rc = tc_geometry(g, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, bits, fuse->in_kind == DS_IN_F32_LINEAR);
     if (rc) return rc;
     if (weight_bytes < g.weight_bytes) return DS_ERR_SCRATCH;
-    TcExpand p = {};
-    p.packed = packed;
-    p.wexp = static_cast<unsigned char*>(weights);
-    p.colc = reinterpret_cast<int*>(p.wexp + g.colc_off);
-    p.dec.bits = bits;
-    p.dec.fw = bits + 1;
-    p.dec.num = 32 / (bits + 1);
-    p.dec.base = 0;
-    p.dec.row_len = (g.K + p.dec.num - 1) / p.dec.num;
-    p.C = g.C; p.KH = g.KH; p.KW = g.KW; p.Cp = g.Cp; p.J = g.J; p.G = g.G; p.N = g.N; p.K = g.K; p.BN = g.BN;
-    p.wide = g.wide;
-    p.chk_w_bytes = (long long)g.N * p.dec.row_len * 4;
-    p.chk_status = bounds_status_ptr();
-    return tc_launch_expand(p, g.grid_n, static_cast<cudaStream_t>(stream));
+    return tc_launch_expand(expand_params(g, packed, bits, weights), static_cast<cudaStream_t>(stream));
 }
 
 namespace ds {
@@ -269,13 +289,20 @@ extern "C" int ds_planes_pack(const void* x, int in_kind, int I, int F, const ds
     if (rc) return rc;
     return tc_launch_pack(pack_params(q, x, static_cast<unsigned char*>(dst->data), plane, dst->B, dst->C, dst->H, dst->W,
                                       dst->halo, dst->halo, dst->H + 2 * dst->halo, dst->W + 2 * dst->halo, dst->C, 1, 1),
-                          false, static_cast<cudaStream_t>(stream));
+                          nullptr, false, static_cast<cudaStream_t>(stream));
 }
 
-extern "C" int ds_tc_conv2d_ex(const void* x, const ds_planes_t* xp, const int32_t* packed, const int32_t* bias, void* out,
-                               const ds_planes_t* next, int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw,
-                               int ph, int pw, int bits, int base, const ds_fuse_t* fuse, void* act, long long act_bytes,
-                               const void* weights, long long weight_bytes, void* stream)
+namespace ds {
+namespace {
+
+// What `weights` is: scratch of this call; a buffer to be kept, with nothing in it yet; one that an earlier call
+// has filled, from whatever words `packed` held then; tiles of these packed words.
+enum { TILES_SCRATCH = 0, TILES_FRESH, TILES_KEPT, TILES_READY };
+
+int tc_conv2d(const void* x, const ds_planes_t* xp, const int32_t* packed, const int32_t* bias, void* out,
+              const ds_planes_t* next, int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw, int ph, int pw,
+              int bits, int base, const ds_fuse_t* fuse, void* act, long long act_bytes, void* weights,
+              long long weight_bytes, int tiles, cudaStream_t st)
 {
     if ((!x && !xp) || (!out && !next) || !packed || !fuse || !act || !weights) return DS_ERR_BAD_ARG;
     if ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(act) | reinterpret_cast<uintptr_t>(weights)) & 15u)
@@ -285,7 +312,7 @@ extern "C" int ds_tc_conv2d_ex(const void* x, const ds_planes_t* xp, const int32
     if (mode == TC_NO || (mode == TC_GATED && next) || (xp && fuse->in_kind == DS_IN_F32_LINEAR)) return DS_ERR_UNSUPPORTED;
     TcGeom g;
     const bool wide = !xp && fuse->in_kind == DS_IN_F32_LINEAR;
-    int rc = tc_geometry(g, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, wide);
+    int rc = tc_geometry(g, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, bits, wide);
     if (rc) return rc;
     if (act_bytes < g.act_bytes || weight_bytes < g.weight_bytes) return DS_ERR_SCRATCH;
     // the quantiser and clamp constants, checked as for every other path
@@ -295,7 +322,6 @@ extern "C" int ds_tc_conv2d_ex(const void* x, const ds_planes_t* xp, const int32
     rc = setup_common(q, bits, base, fuse, fp);
     if (rc) return rc;
     if (fuse->residual && (reinterpret_cast<uintptr_t>(fuse->residual) & 3u)) return DS_ERR_ALIGN;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
     unsigned char* a = static_cast<unsigned char*>(act);
     int* counters = static_cast<int*>(act) + 4;
     // the range flag: the last counter word of the workspace, as for the other paths, else the scratch's first word
@@ -322,12 +348,17 @@ extern "C" int ds_tc_conv2d_ex(const void* x, const ds_planes_t* xp, const int32
         TcPack pk = pack_params(q, x, a + g.planes_off, g.plane, B, C, H, W, ph, pw, g.Hp, g.Wp, g.Cp, g.sub_h, g.sub_w);
         pk.counters = g.splits > 1 ? counters : nullptr;
         pk.ncounters = g.splits > 1 ? g.grid_m * g.grid_n : 0;
-        if (mode == TC_GATED) {
-            if (cudaMemsetAsync(flag, 0, sizeof(int), st) != cudaSuccess) return DS_ERR_CUDA;
-            p.gate = pk.flag = flag;
-        }
-        if (wide) pk.refuse = reinterpret_cast<const int*>(static_cast<const unsigned char*>(weights) + g.colc_off) + g.N;
-        rc = tc_launch_pack(pk, wide, st);
+        if (mode == TC_GATED) p.gate = pk.flag = flag;
+        if (pk.flag && cudaMemsetAsync(flag, 0, sizeof(int), st) != cudaSuccess) return DS_ERR_CUDA;
+        const bool kept = tiles == TILES_FRESH || tiles == TILES_KEPT;
+        TcExpand e = expand_params(g, packed, bits, weights);
+        e.fresh = tiles == TILES_FRESH;
+        e.range_flag = pk.flag;
+        if (e.fresh && cudaMemsetAsync(e.state, 0, 16, st) != cudaSuccess) return DS_ERR_CUDA;
+        if (tiles == TILES_SCRATCH) rc = tc_launch_expand(e, st);
+        if (rc) return rc;
+        if (wide) pk.refuse = e.colc + g.N;
+        rc = tc_launch_pack(pk, kept ? &e : nullptr, wide, st);
         if (rc) return rc;
     }
     p.wexp = static_cast<const unsigned char*>(weights);
@@ -359,7 +390,7 @@ extern "C" int ds_tc_conv2d_ex(const void* x, const ds_planes_t* xp, const int32
     p.units = g.grid_m * g.grid_n * g.splits;
     // neighbouring CTAs share the smaller operand's tiles through L2: rows fastest when the weights are the
     // larger one
-    p.m_fast = g.weight_bytes > 2 * g.plane;
+    p.m_fast = g.colc_off > 2 * g.plane;
     p.counters = counters;
     p.partials = reinterpret_cast<int*>(a + TC_HEADER);
     p.out_kind = q.out_kind; p.relu = q.relu; p.requant = q.requant; p.round_f32 = q.round_f32;
@@ -371,6 +402,28 @@ extern "C" int ds_tc_conv2d_ex(const void* x, const ds_planes_t* xp, const int32
     rc = tc_launch_run(p, g.BN, wide, st);
     if (rc || mode != TC_GATED) return rc;
     return launch_gated_int(x, packed, bias, out, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, bits, base, fuse, flag, 1, st);
+}
+
+}  // namespace
+}  // namespace ds
+
+extern "C" int ds_tc_conv2d_ex(const void* x, const ds_planes_t* xp, const int32_t* packed, const int32_t* bias, void* out,
+                               const ds_planes_t* next, int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw,
+                               int ph, int pw, int bits, int base, const ds_fuse_t* fuse, void* act, long long act_bytes,
+                               const void* weights, long long weight_bytes, void* stream)
+{
+    return tc_conv2d(x, xp, packed, bias, out, next, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, bits, base, fuse, act,
+                     act_bytes, const_cast<void*>(weights), weight_bytes, TILES_READY, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int ds_tc_conv2d_packed(const void* x, const int32_t* packed, const int32_t* bias, void* out, int B, int C, int H,
+                                   int W, int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits, int base,
+                                   const ds_fuse_t* fuse, void* act, long long act_bytes, void* weights,
+                                   long long weight_bytes, int kept, void* stream)
+{
+    if (!x || !out || kept < TILES_SCRATCH || kept > TILES_KEPT) return DS_ERR_BAD_ARG;
+    return tc_conv2d(x, nullptr, packed, bias, out, nullptr, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, bits, base, fuse, act,
+                     act_bytes, weights, weight_bytes, kept, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int ds_tc_conv2d(const void* x, const int32_t* packed, const int32_t* bias, void* out, int B, int C, int H,

@@ -132,41 +132,18 @@ def tc_expand(geometry, conc_weight, fuse, nbytes, device):
     return buf
 
 
-def _tc_weights(geometry, conc_weight, fuse, nbytes, device):
-    """Expanded weights kept on the ``ConcWeight`` they were made from, as ``_prepared_weights`` keeps its
-    own.  The buffer is filled on the stream of the first call; calls on other streams wait for that.  While
-    a stream is being captured nothing is kept, and a buffer not known to be complete is not used (an event
-    from outside a capture cannot be waited for inside): the expansion becomes part of the graph."""
-    cache = conc_weight.__dict__.setdefault("_tc", {})
-    key = geometry + (fuse.in_kind == _ffi.IN_F32_LINEAR, conc_weight.bits, conc_weight.base, conc_weight.data.data_ptr(), str(device))
-    entry = cache.get(key)
-    stream = torch.cuda.current_stream(device)
-    capturing = torch.cuda.is_current_stream_capturing()
-    if entry is None:
-        buf = tc_expand(geometry, conc_weight, fuse, nbytes, device)
-        if not capturing:
-            event = torch.cuda.Event()
-            event.record(stream)
-            cache[key] = dict(buf=buf, event=event, ready=False, stream=stream)
-        return buf
-    if entry["stream"] != stream and not capturing:
-        entry["buf"].record_stream(stream)   # freed only after this stream's uses
-    if not entry["ready"]:
-        if capturing:
-            return tc_expand(geometry, conc_weight, fuse, nbytes, device)
-        if entry["event"].query():
-            entry["ready"] = True
-        else:
-            stream.wait_event(entry["event"])
-    return entry["buf"]
-
-
 _TC_MIN_OPS = 4_000_000   # below this ds_tc_bytes never takes a call: not worth asking
 
 
 def _tc_run(x, conc_weight, bias, out, geometry, fuse, keep_weights):
     """Runs the call on the tensor cores if it is one for them; False otherwise.  Scratch comes from torch's
-    allocator, whose blocks are reused in stream order."""
+    allocator, whose blocks are reused in stream order.
+
+    ``keep_weights``: the expanded weights stay on the ``ConcWeight``, one buffer per stream (calls on one stream
+    never overlap).  Every later call compares the packed words they were made from with the words of the moment, on
+    the device, and makes them again if they differ, so a change of ``conc_weight.data``, in place or not, by whatever means, takes effect with the next call as it
+    does on the paths that decode in the kernel.  Under stream capture nothing is kept: the expansion is part of
+    the graph, whose replays read the packed words as they are then."""
     _, C, _, _, _, KH, KW = geometry[:7]
     if KH * KW > 1 and out.numel() * C * KH * KW < _TC_MIN_OPS:
         return False
@@ -174,16 +151,25 @@ def _tc_run(x, conc_weight, bias, out, geometry, fuse, keep_weights):
     if act_bytes == 0:
         return False
     device = x.device
-    if keep_weights:
-        wt = _tc_weights(geometry, conc_weight, fuse, weight_bytes, device)
-    else:
-        wt = tc_expand(geometry, conc_weight, fuse, weight_bytes, device)
-    act = torch.empty(act_bytes, dtype=torch.uint8, device=device)
-    rc = _ffi.lib().ds_tc_conv2d(x.data_ptr(), conc_weight.data.data_ptr(),
-                                 bias.data_ptr() if bias is not None else None, out.data_ptr(), *geometry,
-                                 conc_weight.bits, conc_weight.base, fuse, act.data_ptr(), act_bytes, wt.data_ptr(),
-                                 weight_bytes, _stream_ptr(device))
+    stream = _stream_ptr(device)
+    tiles = kept = None
+    if keep_weights and not torch.cuda.is_current_stream_capturing():
+        kept = conc_weight.__dict__.setdefault("_tc", {})
+        key = (geometry, fuse.in_kind == _ffi.IN_F32_LINEAR, conc_weight.bits, device, stream)
+        tiles = kept.get(key)
+    state = 0 if kept is None else 1 if tiles is None else 2
+    if state == 1:
+        tiles = torch.empty(weight_bytes, dtype=torch.uint8, device=device)
+    scratch = torch.empty(act_bytes if tiles is not None else act_bytes + weight_bytes, dtype=torch.uint8, device=device)
+    act = scratch.data_ptr()
+    rc = _ffi.lib().ds_tc_conv2d_packed(x.data_ptr(), conc_weight.data.data_ptr(),
+                                        bias.data_ptr() if bias is not None else None, out.data_ptr(), *geometry,
+                                        conc_weight.bits, conc_weight.base, fuse, act, act_bytes,
+                                        tiles.data_ptr() if tiles is not None else act + act_bytes, weight_bytes,
+                                        state, stream)
     _ffi.check(rc, "tc_conv2d")
+    if state == 1:
+        kept[key] = tiles   # only once the call that fills it is in the stream
     return True
 
 

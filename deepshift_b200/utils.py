@@ -83,8 +83,8 @@ class ConcWeight():
         self.bits = bits
 
     def __getstate__(self):
-        # a copy or a saved module starts without the expanded operand tiles (kernels._tc_weights): they hold a
-        # CUDA event and are made again on first use
+        # a copy or a saved module starts without the expanded operand tiles (kernels._tc_run): they belong to
+        # streams of this process and are made again on first use
         state = dict(self.__dict__)
         state.pop('_tc', None)
         return state

@@ -282,9 +282,15 @@ int ds_conv2d_prepare(const int32_t *packed, int B, int C, int H, int W, int OC,
  *
  * ds_tc_bytes     sizes of `act` (scratch of one call, any contents, reusable in stream order) and `weights`;
  *                 both 0 when the call is not served, or, unless any_size, has too little work to be worth it.
- * ds_tc_expand    fills `weights` for one geometry and input kind (fuse->in_kind); may be kept as long as the packed weights do not change.
+ * ds_tc_expand    fills `weights` for one geometry and input kind (fuse->in_kind); may be kept as long as the packed
+ *                 weights do not change.
  * ds_tc_conv2d    the call.  Both buffers 16-byte aligned and at least as long as ds_tc_bytes said.  Enqueues
  *                 two kernels (four with the measured range); works under stream capture.
+ * ds_tc_conv2d_packed  the same without ds_tc_expand.  `kept` = 0: `weights` is scratch of this call.  1: a buffer
+ *                 that the caller keeps, with nothing in it yet.  2: a kept buffer that an earlier call of the same
+ *                 geometry, kind and `bits` has filled, ordered before this one: it is compared on the device with
+ *                 the packed words as they are now and made again if they differ, so it never goes stale.  Calls
+ *                 that may overlap on the GPU need buffers of their own.
  */
 int ds_tc_bytes(int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits, int base,
                 const ds_fuse_t *fuse, int any_size, long long *act_bytes, long long *weight_bytes);
@@ -293,6 +299,10 @@ int ds_tc_expand(const int32_t *packed, int B, int C, int H, int W, int OC, int 
 int ds_tc_conv2d(const void *x, const int32_t *packed, const int32_t *bias, void *out, int B, int C, int H, int W,
                  int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits, int base, const ds_fuse_t *fuse,
                  void *act, long long act_bytes, const void *weights, long long weight_bytes, void *stream);
+
+int ds_tc_conv2d_packed(const void *x, const int32_t *packed, const int32_t *bias, void *out, int B, int C, int H, int W,
+                        int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits, int base, const ds_fuse_t *fuse,
+                        void *act, long long act_bytes, void *weights, long long weight_bytes, int kept, void *stream);
 
 /*
  * Chains of layers keep their activations as byte planes: the l and h bytes of code + 2^15 after the quantiser
