@@ -60,6 +60,7 @@ _SIGNATURES = {
     "ds_conv2d_noalloc": [_VP, _VP, _VP, _VP] + [_I] * 13 + [ctypes.POINTER(Fuse), _VP],
     "ds_conv2d_prepare": [_VP] + [_I] * 13 + [ctypes.POINTER(Fuse), ctypes.POINTER(ctypes.c_longlong), _VP],
     "ds_tc_bytes": [_I] * 13 + [ctypes.POINTER(Fuse), _I, ctypes.POINTER(_LL), ctypes.POINTER(_LL)],
+    "ds_tc_columns": [_I] * 13 + [ctypes.POINTER(Fuse)],
     "ds_tc_expand": [_VP] + [_I] * 13 + [ctypes.POINTER(Fuse), _VP, _LL, _VP],
     "ds_tc_conv2d": [_VP, _VP, _VP, _VP] + [_I] * 13 + [ctypes.POINTER(Fuse), _VP, _LL, _VP, _LL, _VP],
     "ds_tc_conv2d_packed": [_VP, _VP, _VP, _VP] + [_I] * 13 + [ctypes.POINTER(Fuse), _VP, _LL, _VP, _LL, _I, _VP],

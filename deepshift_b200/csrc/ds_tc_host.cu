@@ -190,6 +190,16 @@ extern "C" int ds_tc_bytes(int B, int C, int H, int W, int OC, int KH, int KW, i
     return DS_OK;
 }
 
+extern "C" int ds_tc_columns(int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits,
+                             int base, const ds_fuse_t* fuse)
+{
+    TcGeom g;
+    if (!fuse || tc_mode(*fuse, bits, base) == TC_NO ||
+        tc_geometry(g, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, bits, fuse->in_kind == DS_IN_F32_LINEAR) != DS_OK)
+        return 0;
+    return g.BN;
+}
+
 namespace ds {
 namespace {
 

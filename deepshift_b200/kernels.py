@@ -18,6 +18,8 @@ Differences from the reference, all deliberate:
 """
 import ctypes
 import functools
+import threading
+import weakref
 
 import torch
 
@@ -112,16 +114,17 @@ def tc_bytes(geometry, conc_weight, fuse, any_size=False):
     """(scratch bytes, expanded-weight bytes) of a call on the tensor cores; (0, 0) when the call is served
     by the other paths (left shifts, activations wider than 16 bits, too little work to pay the packing)."""
     return _tc_bytes(tuple(geometry), conc_weight.bits, conc_weight.base, fuse.in_kind, fuse.act_bits, fuse.act_integer_bits,
-                     fuse.act_fraction_bits, int(any_size))
+                     fuse.act_fraction_bits, int(any_size))[:2]
 
 
 @functools.lru_cache(maxsize=4096)
 def _tc_bytes(geometry, bits, base, in_kind, act_bits, integer_bits, fraction_bits, any_size):
-    # a function of these numbers alone: 3 us of ctypes otherwise, on every call
+    # ... and the columns of the weight tiles.  A function of these numbers alone: 3 us of ctypes otherwise, on every
+    # call
     act, wt = ctypes.c_longlong(0), ctypes.c_longlong(0)
     f = _fuse(in_kind, 0, integer_bits, fraction_bits, act_bits=act_bits)
     _ffi.check(_ffi.lib().ds_tc_bytes(*geometry, bits, base, f, any_size, ctypes.byref(act), ctypes.byref(wt)), "tc_bytes")
-    return act.value, wt.value
+    return act.value, wt.value, _ffi.lib().ds_tc_columns(*geometry, bits, base, f) if act.value else 0
 
 
 def tc_expand(geometry, conc_weight, fuse, nbytes, device):
@@ -134,38 +137,71 @@ def tc_expand(geometry, conc_weight, fuse, nbytes, device):
 
 _TC_MIN_OPS = 4_000_000   # below this ds_tc_bytes never takes a call: not worth asking
 
+_TC_KEEP_SHARE = 16       # expanded weights of all layers may keep one part in this many of a GPU's memory
+
+
+class _Tiles:
+    """Expanded weights of one layer, layout and stream, owned by the ``ConcWeight``."""
+    __slots__ = ("buf", "__weakref__")
+
+    def __init__(self, buf):
+        self.buf = buf
+
+
+_TC_KEPT = weakref.WeakSet()   # every _Tiles alive
+_TC_KEPT_LOCK = threading.Lock()
+
+
+def _new_tiles(nbytes, device):
+    """A buffer to keep, or None when the layers already keep their share of the memory: 16 to 22 bytes per weight
+    would else crowd out models whose packed weights (a byte each) fit."""
+    limit = torch.cuda.get_device_properties(device).total_memory // _TC_KEEP_SHARE
+    with _TC_KEPT_LOCK:
+        if nbytes + sum(t.buf.numel() for t in _TC_KEPT if t.buf.device == device) > limit:
+            return None
+        tiles = _Tiles(torch.empty(nbytes, dtype=torch.uint8, device=device))
+        _TC_KEPT.add(tiles)
+    return tiles
+
 
 def _tc_run(x, conc_weight, bias, out, geometry, fuse, keep_weights):
     """Runs the call on the tensor cores if it is one for them; False otherwise.  Scratch comes from torch's
-    allocator, whose blocks are reused in stream order.
+    allocator, whose blocks are reused in stream order; a call that does not get it is left to the other paths.
 
-    ``keep_weights``: the expanded weights stay on the ``ConcWeight``, one buffer per stream (calls on one stream
-    never overlap).  Every later call compares the packed words they were made from with the words of the moment, on
-    the device, and makes them again if they differ, so a change of ``conc_weight.data``, in place or not, by whatever means, takes effect with the next call as it
-    does on the paths that decode in the kernel.  Under stream capture nothing is kept: the expansion is part of
-    the graph, whose replays read the packed words as they are then."""
-    _, C, _, _, _, KH, KW = geometry[:7]
+    ``keep_weights``: the expanded weights stay on the ``ConcWeight``, one buffer per layout and stream (calls on one
+    stream never overlap) while ``_new_tiles`` grants it.  Every later call compares the packed words they were made
+    from with the words of the moment, on the device, and makes them again if they differ, so a change of
+    ``conc_weight.data``, in place or not, by whatever means, takes effect with the next call as it does on the paths
+    that decode in the kernel.  Under stream capture nothing is kept: the expansion is part of the graph, whose
+    replays read the packed words as they are then."""
+    _, C, _, _, OC, KH, KW = geometry[:7]
     if KH * KW > 1 and out.numel() * C * KH * KW < _TC_MIN_OPS:
         return False
-    act_bytes, weight_bytes = tc_bytes(geometry, conc_weight, fuse)
+    act_bytes, weight_bytes, columns = _tc_bytes(geometry, conc_weight.bits, conc_weight.base, fuse.in_kind, fuse.act_bits,
+                                                 fuse.act_integer_bits, fuse.act_fraction_bits, 0)
     if act_bytes == 0:
         return False
     device = x.device
     stream = _stream_ptr(device)
-    tiles = kept = None
-    if keep_weights and not torch.cuda.is_current_stream_capturing():
-        kept = conc_weight.__dict__.setdefault("_tc", {})
-        key = (geometry, fuse.in_kind == _ffi.IN_F32_LINEAR, conc_weight.bits, device, stream)
-        tiles = kept.get(key)
-    state = 0 if kept is None else 1 if tiles is None else 2
-    if state == 1:
-        tiles = torch.empty(weight_bytes, dtype=torch.uint8, device=device)
-    scratch = torch.empty(act_bytes if tiles is not None else act_bytes + weight_bytes, dtype=torch.uint8, device=device)
+    tiles, state = None, 0
+    try:
+        if keep_weights and not torch.cuda.is_current_stream_capturing():
+            kept = conc_weight.__dict__.setdefault("_tc", {})
+            # what the layout depends on (ds_tc_columns), then what separates calls that may overlap
+            key = (C, OC, KH, KW, columns, fuse.in_kind == _ffi.IN_F32_LINEAR, conc_weight.bits, device, stream)
+            tiles = kept.get(key)
+            state = 2
+            if tiles is None:
+                tiles = _new_tiles(weight_bytes, device)
+                state = 0 if tiles is None else 1
+        scratch = torch.empty(act_bytes if tiles is not None else act_bytes + weight_bytes, dtype=torch.uint8, device=device)
+    except torch.OutOfMemoryError:
+        return False
     act = scratch.data_ptr()
     rc = _ffi.lib().ds_tc_conv2d_packed(x.data_ptr(), conc_weight.data.data_ptr(),
                                         bias.data_ptr() if bias is not None else None, out.data_ptr(), *geometry,
                                         conc_weight.bits, conc_weight.base, fuse, act, act_bytes,
-                                        tiles.data_ptr() if tiles is not None else act + act_bytes, weight_bytes,
+                                        tiles.buf.data_ptr() if tiles is not None else act + act_bytes, weight_bytes,
                                         state, stream)
     _ffi.check(rc, "tc_conv2d")
     if state == 1:

@@ -288,12 +288,17 @@ int ds_conv2d_prepare(const int32_t *packed, int B, int C, int H, int W, int OC,
  *                 two kernels (four with the measured range); works under stream capture.
  * ds_tc_conv2d_packed  the same without ds_tc_expand.  `kept` = 0: `weights` is scratch of this call.  1: a buffer
  *                 that the caller keeps, with nothing in it yet.  2: a kept buffer that an earlier call of the same
- *                 geometry, kind and `bits` has filled, ordered before this one: it is compared on the device with
- *                 the packed words as they are now and made again if they differ, so it never goes stale.  Calls
- *                 that may overlap on the GPU need buffers of their own.
+ *                 layout has filled, ordered before this one: it is compared on the device with the packed words as
+ *                 they are now and made again if they differ, so it never goes stale.  Calls that may overlap on the
+ *                 GPU need buffers of their own.
+ * ds_tc_columns   columns of the call's weight tiles (32, 64 or 128; 0: not served).  What ds_tc_expand writes, and a
+ *                 kept buffer holds, depends on this number, C, OC, KH, KW, `bits` and on whether fuse->in_kind is
+ *                 DS_IN_F32_LINEAR: calls that agree in these have one layout, whatever their batch and image size.
  */
 int ds_tc_bytes(int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits, int base,
                 const ds_fuse_t *fuse, int any_size, long long *act_bytes, long long *weight_bytes);
+int ds_tc_columns(int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits, int base,
+                  const ds_fuse_t *fuse);
 int ds_tc_expand(const int32_t *packed, int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw, int ph,
                  int pw, int bits, int base, const ds_fuse_t *fuse, void *weights, long long weight_bytes, void *stream);
 int ds_tc_conv2d(const void *x, const int32_t *packed, const int32_t *bias, void *out, int B, int C, int H, int W,

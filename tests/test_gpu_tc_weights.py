@@ -110,3 +110,57 @@ def test_streams_do_not_share_what_a_call_may_rewrite(oracle, cuda_device, kind)
             a.check(o)
         cw, a.want = a.make()
         a.cw.data.copy_(cw.data)
+
+
+def test_batch_sizes_share_one_buffer(oracle, cuda_device):
+    """A new number of rows, or of images, finds the tiles of the layout: no new buffer, at most one per tile width."""
+    lin = Layer(oracle, cuda_device, "linear")
+    for rows in (17, 40, 64, 200, 33):
+        b = Layer(oracle, cuda_device, "linear", rows)
+        lin.x, lin.cw.data = b.x, b.cw.data
+        lin.check(lin.run(), b.want)
+        assert len(lin.cw.__dict__["_tc"]) == 1
+    conv = Layer(oracle, cuda_device, "conv", 1)
+    for images in (1, 2, 3, 5, 9, 17, 33, 40):
+        b = Layer(oracle, cuda_device, "conv", images)
+        conv.x, conv.cw.data = b.x, b.cw.data
+        conv.check(conv.run(), b.want)
+        assert len(conv.cw.__dict__["_tc"]) <= 3
+    before = torch.cuda.memory_allocated()
+    conv.run()
+    assert torch.cuda.memory_allocated() == before
+
+
+def test_kept_tiles_are_bounded_and_given_back(oracle, cuda_device, monkeypatch):
+    from deepshift_b200 import kernels
+    a = Layer(oracle, cuda_device, "linear")
+    a.check(a.run())
+    size = next(iter(a.cw.__dict__["_tc"].values())).buf.numel()
+    used = sum(t.buf.numel() for t in list(kernels._TC_KEPT))
+    assert used >= size
+    total = torch.cuda.get_device_properties(cuda_device).total_memory
+    monkeypatch.setattr(kernels, "_TC_KEEP_SHARE", total // (used + size // 2))   # no room for one more of this size
+    b = Layer(oracle, cuda_device, "linear", seed=2)
+    for _ in range(2):
+        b.check(b.run())
+    assert not b.cw.__dict__["_tc"]
+    a.check(a.run())                    # what is there stays in use
+    del a.cw                            # ... and what is given up makes room
+    b.check(b.run())
+    assert len(b.cw.__dict__["_tc"]) == 1
+
+
+@pytest.mark.parametrize("kind", ["linear", "conv"])
+def test_without_memory_for_tiles_the_other_paths_serve_the_call(oracle, cuda_device, kind, monkeypatch):
+    a = Layer(oracle, cuda_device, kind)
+    empty = torch.empty
+
+    def no_bytes(*args, **kwargs):
+        if kwargs.get("dtype") == torch.uint8:
+            raise torch.OutOfMemoryError("no memory (test)")
+        return empty(*args, **kwargs)
+
+    monkeypatch.setattr(torch, "empty", no_bytes)
+    a.check(a.run())
+    monkeypatch.undo()
+    a.check(a.run())

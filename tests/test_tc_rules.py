@@ -44,3 +44,12 @@ def test_copies_of_packed_weights_leave_the_expanded_tiles_behind():
     for other in (copy.deepcopy(cw), pickle.loads(pickle.dumps(cw)), copy.copy(cw)):
         assert torch.equal(other.data, cw.data) and (other.base, other.bits) == (-2, 5) and "_tc" not in other.__dict__
     assert "_tc" in cw.__dict__
+
+
+def test_layout_of_the_weights_does_not_depend_on_the_batch():
+    """24-bit linear layers have one width of tile; convolutions at most three, whatever the batch."""
+    from deepshift_b200 import _ffi, kernels
+    columns = lambda geo, kind: kernels._tc_bytes(geo, 6, 0, kind, 0, 4, 12, 1)[1:]
+    assert len({columns(_linear(m, 4096, 4096), _ffi.IN_F32_LINEAR) for m in (17, 64, 1000, 20000)}) == 1
+    sizes = {columns((b, 64, 28, 28, 128, 3, 3, 1, 1, 1, 1), _ffi.IN_F32_CONV) for b in range(1, 400, 7)}
+    assert {c for _, c in sizes} <= {32, 64, 128} and len(sizes) <= 3
