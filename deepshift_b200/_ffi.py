@@ -79,6 +79,7 @@ _SIGNATURES = {
     "ds_last_kernel_error": [ctypes.POINTER(ctypes.c_int)],
     "ds_bounds_status": [ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)],
     "ds_bounds_debug_shrink_x": [_LL],
+    "ds_tc_debug_waits": [_LL, _I],
     "ds_unopt_linear_f32": [_VP, _VP, _VP, _VP, _I, _I, _I, _VP],
     "ds_unopt_conv2d_f32": [_VP, _VP, _VP, _VP] + [_I] * 11 + [_VP],
     "ds_staged_fill": [ctypes.POINTER(Staged), _VP],

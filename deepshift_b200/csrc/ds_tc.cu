@@ -69,8 +69,9 @@ struct TcSmem {
     alignas(16) int colc[2][128];
 };
 
-constexpr int TC_WAIT_LIMIT = 1 << 17;     // rounds of one wait before giving up (about half a second)
+constexpr int TC_WAIT_ROUNDS = 1 << 22;    // rounds of one wait, each up to TC_WAIT_NS
 constexpr unsigned TC_WAIT_NS = 1000000;   // suspend hint of one round
+constexpr unsigned long long TC_DRAIN_NS = 2000000000ull;  // limit on what a CTA has in flight when it ends
 
 __device__ __forceinline__ unsigned s32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
@@ -106,20 +107,64 @@ __device__ __forceinline__ bool bar_try_long(unsigned long long* b, unsigned par
     return ok != 0;
 }
 
-// Bounded wait; whoever gives up sets the CTA's error word, and every wait that finds it set gives up too.
+__device__ __forceinline__ bool bar_test(unsigned long long* b, unsigned parity)
+{
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(s32(b)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
+__device__ __forceinline__ unsigned long long now_ns()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// Wait of at most limit_ns; whoever gives up sets the CTA's error word, and every wait that finds it set and its
+// barrier not ready returns at once.  The longest wait of a correct run is the epilogue's for one unit of K: planes
+// stay below 2^31 bytes and tiles in 180 GB, which leaves at most 2^19 groups of half a microsecond.
 // The first rounds carry no suspend hint: with one, a wait between warps of the main loop wakes up later
 // (7 % of the whole kernel).
-__device__ __forceinline__ bool bar_wait(unsigned long long* b, unsigned parity, volatile int* err)
+__device__ __forceinline__ bool bar_wait(unsigned long long* b, unsigned parity, volatile int* err, unsigned limit_ns)
 {
-    for (int i = 0; i < 32; ++i)
+    if (bar_test(b, parity)) return true;
+    for (int i = 0; i < 32; ++i) {
+        if (*err) return false;
         if (bar_try(b, parity)) return true;
-    for (int i = 0; i < TC_WAIT_LIMIT; ++i) {
+    }
+    const unsigned long long t0 = now_ns();
+    for (int i = 0; i < TC_WAIT_ROUNDS; ++i) {
         if (bar_try_long(b, parity)) return true;
         if (*err) return false;
+        if (now_ns() - t0 > limit_ns) break;
     }
     *err = 1;
     return false;
 }
+
+// Wait for this CTA's own copies or MMAs in flight, error or not.
+__device__ __forceinline__ bool bar_drain(unsigned long long* b, unsigned parity)
+{
+    if (bar_try(b, parity)) return true;
+    const unsigned long long t0 = now_ns();
+    for (int i = 0; i < TC_WAIT_ROUNDS; ++i) {
+        if (bar_try_long(b, parity)) return true;
+        if (now_ns() - t0 > TC_DRAIN_NS) break;
+    }
+    return false;
+}
+
+// Checked build: parts of the kernel that ds_tc_debug_waits keeps from doing their work, so that waits run out.
+#ifdef DS_BOUNDS_CHECK
+#define TC_HELD(p, bit) (((p).hold & (bit)) != 0)
+#else
+#define TC_HELD(p, bit) false
+#endif
 
 __device__ __forceinline__ void tc_commit(unsigned long long* b)
 {
@@ -435,9 +480,9 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
             // and nothing but the stores between the slot's release and its hand-over.
             constexpr int PER = T::SLOTS / T::WG;  // slots of this warpgroup, used in turn
             const unsigned slot = wg + T::WG * (round % PER), use = round / PER;
-            if (use > 0 && !bar_wait(&s.aempty[slot], (use - 1) & 1u, err)) u = p.units;
+            const bool ok = use == 0 || bar_wait(&s.aempty[slot], (use - 1) & 1u, err, p.wait_ns);
             ++round;
-            __syncwarp();
+            if (!__all_sync(0xFFFFFFFFu, ok) || TC_HELD(p, 2)) break;  // the whole warp, or none of it
             tc_fence_after();
             tmem_st32(tmem_a + lane_base + slot * T::ASTRIDE, v);
             tmem_st32(tmem_a + lane_base + slot * T::ASTRIDE + 32, v + 32);
@@ -461,8 +506,8 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
         };
         unsigned acc = 0;
         int par = 0;
-        bool bad = false;
-        for (int u = blockIdx.x; u < p.units && !bad; u += gridDim.x, ++acc, par ^= 1) {
+        // A warp whose wait gives up walks on without the unit's sums: the named barriers below need all four.
+        for (int u = blockIdx.x; u < p.units; u += gridDim.x, ++acc, par ^= 1) {
             const Unit un = unit_of<BN>(p, u);
             // column constants of this tile; two copies, so a slow warp still reads the previous tile's
             if (row < BN) {
@@ -470,13 +515,8 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
                 s.colc[par][row] = n < p.N ? __ldg(p.colc + n) + (p.bias ? __ldg(p.bias + n) : 0) : 0;
             }
             epi_bar();
-            {
-                const unsigned slot = acc % T::NACC;
-                if (!bar_wait(&s.accfull[slot], (acc / T::NACC) & 1u, err)) {
-                    bad = true;
-                    break;
-                }
-                __syncwarp();
+            const unsigned slot = acc % T::NACC;
+            if (__all_sync(0xFFFFFFFFu, bar_wait(&s.accfull[slot], (acc / T::NACC) & 1u, err, p.wait_ns))) {
                 tc_fence_after();
                 const int m = un.m0 + row;
                 const int b = m / p.P, pp = m - b * p.P;
@@ -495,7 +535,7 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
                     if (c + 32 >= BN) {
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) bar_arrive(&s.accempty[slot]);
+                        if (lane == 0 && !TC_HELD(p, 4)) bar_arrive(&s.accempty[slot]);
                     }
                     if (p.splits == 1) {
                         tc_store<NEXT>(p, v, &s.colc[par][c], m, un.n0 + c, rowoff, nextoff);
@@ -507,7 +547,7 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
                     }
                 }
             }
-            if (p.splits > 1 && !bad) {
+            if (p.splits > 1) {
                 // the split that arrives last adds all partial sums in order and applies the epilogue
                 __threadfence();
                 epi_bar();
@@ -558,16 +598,16 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
             const Unit un = unit_of<BN>(p, u);
             const unsigned d = tmem + aslot * T::ACC;
             unsigned long long* accfull = &s.accfull[aslot];
-            bar_wait(&s.accempty[aslot], accph, err);  // the first round finds the slots free
+            bar_wait(&s.accempty[aslot], accph, err, p.wait_ns);  // the first round finds the slots free
             if (++aslot == unsigned(T::NACC)) {
                 aslot = 0;
                 accph ^= 1u;
             }
             unsigned more = 0;  // the first MMA of a unit overwrites the accumulator
             for (int g = un.g0; g < un.g1; ++g) {
-                bar_wait(&s.bfull[st], bph, err);
+                bar_wait(&s.bfull[st], bph, err, p.wait_ns);
                 const unsigned long long bdesc = desc0 + st * unsigned(T::STAGE >> 4);
-                bar_wait(&s.afull[slot], aph, err);
+                bar_wait(&s.afull[slot], aph, err, p.wait_ns);
                 tc_fence_after();
                 if (elect_one()) {
 #pragma unroll
@@ -597,21 +637,20 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
             __syncwarp();
         }
         if (elect_one()) tc_commit(&s.done);  // nothing of this CTA is in flight when the columns go back
-        for (int i = 0; i < TC_WAIT_LIMIT; ++i)
-            if (bar_try(&s.done, 0)) break;
+        if (!bar_drain(&s.done, 0)) *err = 1;
         __syncwarp();
     } else {
         // ---- weight tiles: one thread ------------------------------------------------------------------
         if (lane == 0) {
             unsigned bs = 0;
             bool ok = true;
-            for (int u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
+            for (int u = blockIdx.x; u < p.units && ok && !TC_HELD(p, 1); u += gridDim.x) {
                 const Unit un = unit_of<BN>(p, u);
                 const unsigned char* src = p.wexp + ((long long)un.nt * p.G + un.g0) * T::STAGE;
                 for (int g = un.g0; g < un.g1; ++g, ++bs, src += T::STAGE) {
                     const unsigned st = bs % T::STAGES;
                     if (bs >= unsigned(T::STAGES)) {
-                        ok = bar_wait(&s.bempty[st], (bs / T::STAGES - 1) & 1u, err);
+                        ok = bar_wait(&s.bempty[st], (bs / T::STAGES - 1) & 1u, err, p.wait_ns);
                         if (!ok) break;
                     }
                     asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(
@@ -627,8 +666,7 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
             // Let every copy land before the CTA ends (the MMA thread has waited for all of them unless a
             // wait gave up).
             for (unsigned k = bs > unsigned(T::STAGES) ? bs - T::STAGES : 0; k < bs; ++k)
-                for (int i = 0; i < 64; ++i)
-                    if (bar_try(&s.bfull[k % T::STAGES], (k / T::STAGES) & 1u)) break;
+                if (!bar_drain(&s.bfull[k % T::STAGES], (k / T::STAGES) & 1u)) *err = 1;
         }
         __syncwarp();
     }

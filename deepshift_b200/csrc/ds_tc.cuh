@@ -83,6 +83,8 @@ struct TcRun {
     float inv_scale;
     const int* gate;
     int gate_want;
+    unsigned wait_ns;    // limit of every wait
+    int hold;            // checked build: see ds_tc_debug_waits
     int* err_flag;
     long long chk_o_bytes;
     int* chk_status;

@@ -9,6 +9,10 @@ namespace {
 
 constexpr int kSms = 148;
 
+constexpr unsigned kWaitNs = 2000000000u;  // two seconds; correct runs stay below a third of one
+unsigned g_wait_ns = kWaitNs;              // changed by ds_tc_debug_waits only
+int g_hold = 0;
+
 long long round16(long long v) { return (v + 15) & ~15ll; }
 
 // Bytes per pixel and plane, and the groups per window row that follow.  The (kw, c) run of one window row
@@ -407,6 +411,8 @@ int tc_conv2d(const void* x, const ds_planes_t* xp, const int32_t* packed, const
     p.rq_lo = q.rq_lo; p.rq_hi = q.rq_hi; p.rq_mul = q.rq_mul; p.rq_add = q.rq_add;
     p.inv_scale = q.inv_scale;
     p.gate_want = 0;
+    p.wait_ns = g_wait_ns;
+    p.hold = g_hold;
     p.chk_o_bytes = (long long)g.M * g.N * 4;
     p.chk_status = bounds_status_ptr();
     rc = tc_launch_run(p, g.BN, wide, st);
@@ -444,4 +450,20 @@ extern "C" int ds_tc_conv2d(const void* x, const int32_t* packed, const int32_t*
     if (!x || !out) return DS_ERR_BAD_ARG;
     return ds_tc_conv2d_ex(x, nullptr, packed, bias, out, nullptr, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, bits, base, fuse,
                            act, act_bytes, weights, weight_bytes, stream);
+}
+
+// Checked build only: limit of the kernel's waits in nanoseconds (0 restores the normal one) and the parts of it that
+// do not do their work, so that a test can watch waits run out.  DS_ERR_UNSUPPORTED in a normal build.
+extern "C" int ds_tc_debug_waits(long long limit_ns, int hold)
+{
+#ifdef DS_BOUNDS_CHECK
+    if (limit_ns < 0 || limit_ns > kWaitNs || hold < 0 || hold > 7) return DS_ERR_BAD_ARG;
+    ds::g_wait_ns = limit_ns ? unsigned(limit_ns) : kWaitNs;
+    ds::g_hold = hold;
+    return DS_OK;
+#else
+    (void)limit_ns;
+    (void)hold;
+    return DS_ERR_UNSUPPORTED;
+#endif
 }

@@ -23,6 +23,41 @@ def status(lib):
     return st.value, ck.value
 
 
+def waits_that_run_out(lib, dev, O, cw_of, rng):
+    """Parts of the tensor-core kernel hold still, so that each kind of wait runs out: the launch ends by itself, says
+    so, leaves the scratch header as it found it, and the next launch is exact again.  A linear layer with four units
+    per CTA, a convolution with few tiles whose K is split."""
+    from deepshift_b200 import kernels
+    for (B, C, H, OC, k, p, holds) in [(60000, 64, 1, 33, 1, 0, (1, 2, 4, 7)), (2, 512, 7, 512, 3, 1, (1, 2))]:
+        x = acts_q16(rng, (B, C, H, H))
+        shift, sign = weights(rng, (OC, C, k, k))
+        cw = cw_of(shift, sign)
+        geo = (B, C, H, H, OC, k, k, 1, 1, p, p)
+        f = kernels._fuse(act_bits=15)
+        act, wt = kernels.tc_bytes(geo, cw, f, any_size=True)
+        xt = torch.from_numpy(x).to(dev) // 2      # 15 bits
+        wexp = kernels.tc_expand(geo, cw, f, wt, dev)
+        want = O.conv2d(x // 2, shift, sign, None, (1, 1), (p, p))
+        out = torch.empty(want.shape, dtype=torch.int32, device=dev)
+        scratch = torch.zeros(act, dtype=torch.uint8, device=dev)
+
+        def call():
+            assert lib.ds_tc_conv2d(xt.data_ptr(), cw.data.data_ptr(), None, out.data_ptr(), *geo, cw.bits, cw.base, f,
+                                    scratch.data_ptr(), act, wexp.data_ptr(), wt, torch.cuda.current_stream().cuda_stream) == 0
+            torch.cuda.synchronize()
+            return kernels.last_kernel_error()
+
+        assert call() == 0 and np.array_equal(out.cpu().numpy(), want)
+        for hold in holds:
+            assert lib.ds_tc_debug_waits(5_000_000, hold) == 0
+            assert call() == 1, hold
+            assert lib.ds_tc_debug_waits(0, 0) == 0
+            assert int(scratch[:2048].sum()) == 0, hold
+            out.fill_(7)
+            assert call() == 0 and np.array_equal(out.cpu().numpy(), want), hold
+    assert lib.ds_tc_debug_waits(1 << 40, 0) != 0
+
+
 def main():
     from deepshift_b200 import _ffi, kernels, utils
     from oracle import oracle as O
@@ -53,6 +88,8 @@ def main():
             out = kernels.linear(torch.from_numpy(x).to(dev), torch.from_numpy(shift).to(dev), None, None, cw, act_bits=ab)
             assert np.array_equal(out.cpu().numpy(), O.linear(x, shift, sign, None)), (M, K, N, ab)
     assert status(lib) == (0, 1), "an access left its extent"
+    waits_that_run_out(lib, dev, O, cw_of, rng)
+    assert status(lib) == (0, 1)
     # the checks fire: x declared 64 bytes short, nothing leaves the real buffer
     B, C, H, OC = 2, 8, 12, 20
     shift, sign = weights(rng, (OC, C, 3, 3))
