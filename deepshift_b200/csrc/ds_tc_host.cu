@@ -146,21 +146,45 @@ int tc_mode(const ds_fuse_t& f, int bits, int base)
     }
 }
 
+// int32 codes with a promise: the FP32-pipe path takes one launch and splits K while nothing is fused, so a call
+// costs it 20 us of host time or 8 us and 0.09 us per 10^6 products of its 64 x 128 tiles.  Here the weights are
+// expanded per call: three launches, 28 us, or 22 us, 5 us per 1000 of K (the column constants) and 6.5 us per 10^6
+// weights.  Measured, us, that path -> this one: 128 x 2048 -> 1000 32 -> 47, 256 x 2048 -> 1000 57 -> 51, 512 x 700 ->
+// 1000 43 -> 35, 512 x 2048 -> 256 32 -> 37, 1024 x 2048 -> 256 57 -> 43, 65 x 256 -> 10 19 -> 28; the 15 % keep calls at
+// the crossing where they were.
+bool promised_linear(const TcGeom& g)
+{
+    const double eff = (double)((g.M + 63) / 64 * 64) * g.K * ((g.N + 127) / 128 * 128);
+    const double there = 8 + 0.09e-6 * eff, here = 22 + 0.005 * g.K + 6.5e-6 * g.N * (double)g.K;
+    return there > 1.15 * (here > 28.5 ? here : 28.5);
+}
+
 // Whether the tensor cores beat the other paths, packing included.  Measured, us, other path -> this one:
-//   linear, fp32 input (weights expanded once): 64 x 784 -> 512 120 -> 19, 17 x 512 -> 512 83 -> 18, 1024 x 500
-//     -> 10 80 -> 19: the integer path behind it runs one CTA per 64 x 128 outputs over all of K, 0.16 us per k, so
-//     the GPU times meet near K = 150, with the host's four launches (about 45 us a call) near 300.  Up to 16 rows the small-batch kernel takes 10 to 15.
-//   linear, int32 input (expanded per call): 256 x 512 -> 1000 86 -> 28, 1024 x 800 -> 500 108 -> 37; up to 64 rows
-//     the integer path splits K and is faster (64 x 784 -> 512 21 -> 26).  With the launch of the expansion the two
-//     meet near K = 200.
+//   linear, fp32 input (weights kept): 64 x 784 -> 512 120 -> 19, 17 x 512 -> 512 83 -> 18, 1024 x 500 -> 10 80 -> 19:
+//     the integer path behind it runs one CTA per 64 x 128 outputs over all of K, 0.16 us per k, so the GPU times meet
+//     near K = 150, with the host's four launches (about 45 us a call) near 300.  That is one wave of CTAs: with many
+//     rows and columns this path also wins below (8192 x 256 -> 256 88 -> 30), which the rule leaves out.  Up to 16
+//     rows the small-batch kernel takes 10 to 15.
+//   linear, int32 input without a promise (expanded per call): 256 x 512 -> 1000 86 -> 28, 1024 x 800 -> 500 108 -> 37;
+//     up to 64 rows the integer path splits K and is faster (64 x 784 -> 512 21 -> 26).  With the launch of the
+//     expansion the two meet near K = 200.
+//   linear, int32 input with a promise: promised_linear; with a fused epilogue the other path does not split K, 0.1 us
+//     per k, and the two meet at K = 400 (quantised fp32 input, 320: 43 -> 51, 512: 62 -> 51).
 //   convolution: 128 -> 128 channels, 28 x 28, one image 103 -> 19; 1x1 stride 2, 64 -> 128, one image 32 -> 12:
 //     few 256-row tiles leave the other path's SMs idle.  With many tiles it pays from about 2^26 shift-accumulates
 //     (16 -> 16 channels, 32 x 32, 64 images 40 -> 24), and not where most of the padded product is padding
 //     (1 -> 20 channels, 5x5: a tenth is live, 110 -> 135).
-bool worthwhile(const TcGeom& g, int in_kind)
+bool worthwhile(const TcGeom& g, const ds_fuse_t& f)
 {
+    const int in_kind = f.in_kind;
     const double ops = (double)g.M * g.N * g.K;
-    if (g.H == 1 && g.W == 1 && g.KH == 1 && g.KW == 1) return in_kind == DS_IN_F32_LINEAR ? g.M > 16 && g.K >= 320 : g.M > 64 && g.K >= 256;
+    if (g.H == 1 && g.W == 1 && g.KH == 1 && g.KW == 1) {
+        if (in_kind == DS_IN_F32_LINEAR) return g.M > 16 && g.K >= 320;
+        if (g.M <= 64 || g.K < 256) return false;
+        if (in_kind != DS_IN_I32 || f.act_bits < 1) return true;
+        const bool plain = f.out_kind == DS_OUT_I32 && !f.relu && !f.requant && !f.round_f32 && !f.residual;
+        return plain ? promised_linear(g) : g.K >= 400;
+    }
     const long long tiles = ((g.M + 255ll) / 256) * ((g.N + 127) / 128);
     if (in_kind == DS_IN_I32) {
         // Weights expanded per call: five launches, 45 us of host time.  The other path takes about 20 us and 0.23 us
@@ -188,7 +212,7 @@ extern "C" int ds_tc_bytes(int B, int C, int H, int W, int OC, int KH, int KW, i
     const int rc = tc_geometry(g, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, bits, fuse->in_kind == DS_IN_F32_LINEAR);
     if (rc == DS_ERR_UNSUPPORTED) return DS_OK;
     if (rc) return rc;
-    if (!any_size && !worthwhile(g, fuse->in_kind)) return DS_OK;
+    if (!any_size && !worthwhile(g, *fuse)) return DS_OK;
     *act_bytes = g.act_bytes;
     *weight_bytes = g.weight_bytes;
     return DS_OK;

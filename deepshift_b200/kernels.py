@@ -114,15 +114,19 @@ def tc_bytes(geometry, conc_weight, fuse, any_size=False):
     """(scratch bytes, expanded-weight bytes) of a call on the tensor cores; (0, 0) when the call is served
     by the other paths (left shifts, activations wider than 16 bits, too little work to pay the packing)."""
     return _tc_bytes(tuple(geometry), conc_weight.bits, conc_weight.base, fuse.in_kind, fuse.act_bits, fuse.act_integer_bits,
-                     fuse.act_fraction_bits, int(any_size))[:2]
+                     fuse.act_fraction_bits, _plain(fuse), int(any_size))[:2]
+
+
+def _plain(fuse):
+    return not (fuse.out_kind or fuse.relu or fuse.requant or fuse.round_f32 or fuse.residual)
 
 
 @functools.lru_cache(maxsize=4096)
-def _tc_bytes(geometry, bits, base, in_kind, act_bits, integer_bits, fraction_bits, any_size):
+def _tc_bytes(geometry, bits, base, in_kind, act_bits, integer_bits, fraction_bits, plain, any_size):
     # ... and the columns of the weight tiles.  A function of these numbers alone: 3 us of ctypes otherwise, on every
     # call
     act, wt = ctypes.c_longlong(0), ctypes.c_longlong(0)
-    f = _fuse(in_kind, 0, integer_bits, fraction_bits, act_bits=act_bits)
+    f = _fuse(in_kind, _ffi.OUT_I32, integer_bits, fraction_bits, relu=not plain, act_bits=act_bits)
     _ffi.check(_ffi.lib().ds_tc_bytes(*geometry, bits, base, f, any_size, ctypes.byref(act), ctypes.byref(wt)), "tc_bytes")
     return act.value, wt.value, _ffi.lib().ds_tc_columns(*geometry, bits, base, f) if act.value else 0
 
@@ -178,7 +182,7 @@ def _tc_run(x, conc_weight, bias, out, geometry, fuse, keep_weights):
     if KH * KW > 1 and out.numel() * C * KH * KW < _TC_MIN_OPS:
         return False
     act_bytes, weight_bytes, columns = _tc_bytes(geometry, conc_weight.bits, conc_weight.base, fuse.in_kind, fuse.act_bits,
-                                                 fuse.act_integer_bits, fuse.act_fraction_bits, 0)
+                                                 fuse.act_integer_bits, fuse.act_fraction_bits, _plain(fuse), 0)
     if act_bytes == 0:
         return False
     device = x.device

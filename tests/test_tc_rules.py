@@ -49,7 +49,19 @@ def test_copies_of_packed_weights_leave_the_expanded_tiles_behind():
 def test_layout_of_the_weights_does_not_depend_on_the_batch():
     """24-bit linear layers have one width of tile; convolutions at most three, whatever the batch."""
     from deepshift_b200 import _ffi, kernels
-    columns = lambda geo, kind: kernels._tc_bytes(geo, 6, 0, kind, 0, 4, 12, 1)[1:]
+    columns = lambda geo, kind: kernels._tc_bytes(geo, 6, 0, kind, 0, 4, 12, True, 1)[1:]
     assert len({columns(_linear(m, 4096, 4096), _ffi.IN_F32_LINEAR) for m in (17, 64, 1000, 20000)}) == 1
     sizes = {columns((b, 64, 28, 28, 128, 3, 3, 1, 1, 1, 1), _ffi.IN_F32_CONV) for b in range(1, 400, 7)}
     assert {c for _, c in sizes} <= {32, 64, 128} and len(sizes) <= 3
+
+
+@pytest.mark.parametrize("geo,plain,served", [
+    ((65, 256, 10), True, False), ((128, 2048, 1000), True, False), ((256, 2048, 1000), True, True),
+    ((512, 2048, 256), True, False), ((1024, 2048, 256), True, True), ((512, 4096, 256), True, False),
+    ((512, 700, 1000), True, True), ((4096, 1024, 10), True, True), ((128, 4096, 1000), True, False),
+    ((65, 320, 10), False, False), ((65, 400, 10), False, True), ((4096, 399, 4096), False, False)])
+def test_promised_codes_move_only_where_it_is_faster(geo, plain, served):
+    """Linear layers whose caller bounds the codes: the FP32-pipe path needs one launch, so small ones stay there."""
+    from deepshift_b200 import kernels, utils
+    f = kernels._fuse(0, 0 if plain else 1, 4, 8, act_bits=12)
+    assert (kernels.tc_bytes(_linear(*geo), utils.ConcWeight(None, 0, 6), f)[0] > 0) == served
