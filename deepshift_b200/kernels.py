@@ -41,6 +41,8 @@ def _check_tensor(t, name, dtype=None):
 
 
 def _pair(v):
+    if type(v) is tuple and len(v) == 2 and type(v[0]) is int and type(v[1]) is int:
+        return v   # what the modules hold
     if isinstance(v, int):
         return (v, v)
     v = tuple(int(e) for e in v)
@@ -178,11 +180,18 @@ def _tc_run(x, conc_weight, bias, out, geometry, fuse, keep_weights):
     ``conc_weight.data``, in place or not, by whatever means, takes effect with the next call as it does on the paths
     that decode in the kernel.  Under stream capture nothing is kept: the expansion is part of the graph, whose
     replays read the packed words as they are then."""
-    _, C, _, _, OC, KH, KW = geometry[:7]
-    if KH * KW > 1 and out.numel() * C * KH * KW < _TC_MIN_OPS:
+    C, OC, KH, KW = geometry[1], geometry[4], geometry[5], geometry[6]
+    in_kind = fuse.in_kind
+    # calls that ds_tc_bytes never takes, told apart before anything is put together: most are small, and every
+    # microsecond of the question would count
+    if conc_weight.base != 0 or (KH * KW > 1 and out.numel() * C * KH * KW < _TC_MIN_OPS):
         return False
-    act_bytes, weight_bytes, columns = _tc_bytes(geometry, conc_weight.bits, conc_weight.base, fuse.in_kind, fuse.act_bits,
-                                                 fuse.act_integer_bits, fuse.act_fraction_bits, _plain(fuse), 0)
+    act_bits = fuse.act_bits
+    if in_kind == _ffi.IN_I32 and not (act_bits == ACT_BITS_AUTO or 1 <= act_bits <= 15):
+        return False
+    plain = in_kind != _ffi.IN_I32 or _plain(fuse)   # an epilogue matters to promised codes only
+    act_bytes, weight_bytes, columns = _tc_bytes(geometry, conc_weight.bits, 0, in_kind, act_bits, fuse.act_integer_bits,
+                                                 fuse.act_fraction_bits, plain, 0)
     if act_bytes == 0:
         return False
     device = x.device
@@ -192,7 +201,7 @@ def _tc_run(x, conc_weight, bias, out, geometry, fuse, keep_weights):
         if keep_weights and not torch.cuda.is_current_stream_capturing():
             kept = conc_weight.__dict__.setdefault("_tc", {})
             # what the layout depends on (ds_tc_columns), then what separates calls that may overlap
-            key = (C, OC, KH, KW, columns, fuse.in_kind == _ffi.IN_F32_LINEAR, conc_weight.bits, device, stream)
+            key = (C, OC, KH, KW, columns, in_kind == _ffi.IN_F32_LINEAR, conc_weight.bits, device, stream)
             tiles = kept.get(key)
             state = 2
             if tiles is None:
@@ -217,9 +226,15 @@ def tc_serves_fp32_conv(input_shape, weight_shape, stride, padding, conc_weight,
     """Whether a shift convolution with fp32 input of these sizes runs on the tensor cores, which quantise
     every value once: no quantising pass is needed in front."""
     B, C, H, W = input_shape
-    geometry = (B, C, H, W, weight_shape[0], weight_shape[2], weight_shape[3]) + _pair(stride) + _pair(padding)
-    f = _fuse(_ffi.IN_F32_CONV, _ffi.OUT_F32, act_integer_bits, act_fraction_bits)
-    return tc_bytes(geometry, conc_weight, f)[0] > 0
+    OC, _, KH, KW = weight_shape
+    sh, sw = _pair(stride)
+    ph, pw = _pair(padding)
+    if conc_weight.base != 0:
+        return False
+    if KH * KW > 1 and B * ((H + 2 * ph - KH) // sh + 1) * ((W + 2 * pw - KW) // sw + 1) * OC * C * KH * KW < _TC_MIN_OPS:
+        return False
+    return _tc_bytes((B, C, H, W, OC, KH, KW, sh, sw, ph, pw), conc_weight.bits, 0, _ffi.IN_F32_CONV, 0, act_integer_bits,
+                     act_fraction_bits, True, 0)[0] > 0
 
 
 class Planes:
