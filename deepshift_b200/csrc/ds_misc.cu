@@ -41,18 +41,21 @@ __global__ void compress_kernel(const int32_t* __restrict__ shiftp, const int32_
 __device__ __forceinline__ float pack_shift(float shift, float sign) { return sign == 0.f ? 32.f : rintf(-shift); }
 
 // Largest right shift r[0], largest negated one r[1] (r starts at 0x80808080), r[2] = 1 when a value is no
-// integer of at most 24 bits (NaN, infinity).  HBM-bound: one read of both tensors.
-__global__ void __launch_bounds__(256) pack_range_kernel(const float* __restrict__ shift, const float* __restrict__ sign,
+// integer of at most 24 bits (NaN, infinity), else 0 when one lies in 16..31 (or 80..95, ..).
+// HBM-bound: one read of both tensors; eight blocks per SM, so 32 registers (4096 x 4096: 33 us, 35 us with 34).
+__global__ void __launch_bounds__(256, 8) pack_range_kernel(const float* __restrict__ shift, const float* __restrict__ sign,
                                                          long long n, int* r)
 {
     int hi = INT_MIN, nlo = INT_MIN;
     bool bad = false;
+    int far = 0;  // bit 4: set without bit 5 in some shift
     auto see = [&](float a, float g) {
         const float v = pack_shift(a, g);
         if (fabsf(v) <= 16777216.f) {
             const int i = int(v);
             hi = max(hi, i);
             nlo = max(nlo, -i);
+            far |= i & ~(i >> 1);
         } else {
             bad = true;
         }
@@ -70,11 +73,11 @@ __global__ void __launch_bounds__(256) pack_range_kernel(const float* __restrict
     for (long long i = 4 * n4 + t0; i < n; i += step) see(__ldg(shift + i), __ldg(sign + i));
     hi = __reduce_max_sync(0xFFFFFFFFu, hi);
     nlo = __reduce_max_sync(0xFFFFFFFFu, nlo);
-    const bool any = __any_sync(0xFFFFFFFFu, bad);
+    const bool any = __any_sync(0xFFFFFFFFu, bad), anyfar = __any_sync(0xFFFFFFFFu, (far & 16) != 0);
     if ((threadIdx.x & 31) == 0) {
         atomicMax(r, hi);
         atomicMax(r + 1, nlo);
-        if (any) r[2] = 1;
+        if (any || anyfar) atomicMax(r + 2, any ? 1 : 0);
     }
 }
 

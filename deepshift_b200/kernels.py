@@ -186,6 +186,8 @@ def _tc_run(x, conc_weight, bias, out, geometry, fuse, keep_weights):
     # microsecond of the question would count
     if conc_weight.base != 0 or (KH * KW > 1 and out.numel() * C * KH * KW < _TC_MIN_OPS):
         return False
+    if in_kind == _ffi.IN_F32_LINEAR and getattr(conc_weight, "far_shifts", False):
+        return False   # the 24-bit form would find a shift of 16..31 and leave the call to the integer path
     act_bits = fuse.act_bits
     if in_kind == _ffi.IN_I32 and not (act_bits == ACT_BITS_AUTO or 1 <= act_bits <= 15):
         return False
@@ -336,14 +338,15 @@ def compress_sign_and_shift(shift, sign, comp_size, base, bits, row_length, num)
 
 
 def pack_range(shift, sign):
-    """(smallest, largest) right shift of fp32 parameters as ``compress_bits`` stores them, or None when they
-    are not all finite integers of at most 24 bits.  Synchronises (the packing geometry depends on it)."""
+    """(smallest, largest, one in 16..31?) of the right shifts of fp32 parameters as ``compress_bits`` stores them, or
+    None when they are not all finite integers of at most 24 bits.  Synchronises (the packing geometry depends on
+    it)."""
     with torch.cuda.device(shift.device):
         r = torch.empty(3, dtype=torch.int32, device=shift.device)
         _ffi.check(_ffi.lib().ds_pack_range_f32(shift.data_ptr(), sign.data_ptr(), shift.numel(), r.data_ptr(),
                                                 _stream_ptr(shift.device)), "pack_range")
     hi, nlo, bad = r.tolist()
-    return None if bad > 0 else (-nlo, hi)
+    return None if bad > 0 else (-nlo, hi, bad == 0)
 
 
 def pack_f32(shift, sign, bits, base):

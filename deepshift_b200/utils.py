@@ -75,12 +75,15 @@ def _same_device(device, have):
 
 
 class ConcWeight():
-    """utils.py:54-58: packed weights, the (non-positive) shift base and the field width."""
+    """utils.py:54-58: packed weights, the (non-positive) shift base and the field width.  ``far_shifts``: whether a
+    right shift of 16..31 was among the weights when they were packed (a hint about the faster path, never about the
+    result)."""
 
     def __init__(self, data=None, base=0, bits=8):
         self.data = data
         self.base = base
         self.bits = bits
+        self.far_shifts = False
 
     def __getstate__(self):
         # a copy or a saved module starts without the expanded operand tiles (kernels._tc_run): they belong to
@@ -112,6 +115,7 @@ def compress_bits(shift, sign, device=None):
             bits = max(1, (span[1] - base).bit_length())
             if bits <= 7:
                 conc_weight.base, conc_weight.bits = base, bits
+                conc_weight.far_shifts = base == 0 and span[2]
                 conc_weight.data = kernels.pack_f32(sh, sg, bits, base)
                 return conc_weight
     shift = shift.detach().clone()
@@ -126,6 +130,7 @@ def compress_bits(shift, sign, device=None):
 
     shift = (shift * -1).round().to(torch.int64)          # right shift as the default
     minimum, maximum = int(shift.min()), int(shift.max())
+    conc_weight.far_shifts = minimum >= 0 and maximum >= 16 and bool(((shift >= 16) & (shift < 32)).any())
     conc_weight.base = minimum if minimum < 0 else 0
     # ceil(log2(max + 1)) of utils.py:72 in exact integer arithmetic, on the stored field
     conc_weight.bits = max(1, (maximum - conc_weight.base).bit_length())

@@ -193,8 +193,8 @@ int ds_compress(const int32_t *shiftp, const int32_t *sign, int32_t *packed, int
  * tensors).  A weight's right shift is rint(-shift), 32 where sign == 0; it counts as positive where
  * sign == 0 or sign >= 1.
  *   ds_pack_range_f32  range[0] = largest right shift, range[1] = minus the smallest, range[2] = 1 when a
- *                      value is not an integer of at most 24 bits, else negative (device int32[3]): what the
- *                      caller chooses bits and base from.
+ *                      value is not an integer of at most 24 bits, else 0 when a shift modulo 64 lies in
+ *                      16..31, else negative (device int32[3]): what the caller chooses bits and base from.
  *   ds_pack_f32        the words.
  */
 int ds_pack_range_f32(const float *shift, const float *sign, long long n, int *range, void *stream);

@@ -37,3 +37,36 @@ def test_unrounded_parameters_and_views(cuda_device):
                  (shift.t(), sign.t())):
         fast, slow = utils.compress_bits(s, q), utils.compress_bits(s.double(), q.double())
         assert (fast.base, fast.bits) == (slow.base, slow.bits) and torch.equal(fast.data, slow.data)
+
+
+@pytest.mark.parametrize("lo,hi,odd,far", [(-15, 0, None, False), (-15, 0, -16, True), (-15, 0, -31, True), (-15, 0, -32, False),
+                                           (-60, -32, None, False), (-15, 2, -20, False)])
+def test_shifts_of_16_to_31_are_noted(cuda_device, lo, hi, odd, far):
+    """On both routes; zero weights (stored as 32) are none, and with left shifts (base < 0) nobody asks."""
+    from deepshift_b200 import utils
+    g = torch.Generator(device=cuda_device).manual_seed(5)
+    shift = torch.randint(lo, hi + 1, (40, 61), generator=g, device=cuda_device).float()
+    shift[0, 0] = hi
+    sign = torch.where(torch.rand((40, 61), generator=g, device=cuda_device) < 0.5, -1.0, 1.0)
+    sign[3, 3:9] = 0
+    if odd is not None:
+        shift[39, 60] = odd
+    assert utils.compress_bits(shift, sign).far_shifts == far
+    assert utils.compress_bits(shift.double(), sign.double()).far_shifts == far
+
+
+@pytest.mark.parametrize("seen", [True, False])
+def test_linear_layer_with_far_shifts_is_exact_on_either_path(oracle, cuda_device, seen):
+    """The integer path when the packing saw them; found on the device when the packed words came otherwise."""
+    from deepshift_b200 import _ffi, kernels, utils
+    rng = np.random.default_rng(6)
+    shift, sign = weights(rng, (70, 400), lo=-30)
+    x = rng.normal(0, 1, (40, 400)).astype(np.float32)
+    cw = utils.compress_bits(torch.from_numpy(shift).float(), torch.from_numpy(sign).float(), device=cuda_device)
+    assert cw.far_shifts
+    cw.far_shifts = seen
+    want = oracle.linear(np.trunc(x.astype(np.float64) * 65536).astype(np.int32), shift, sign, None)
+    for _ in range(2):
+        got = kernels.linear_fused(torch.from_numpy(x).to(cuda_device), 70, None, cw, in_kind=_ffi.IN_F32_LINEAR)
+        assert np.array_equal(got.cpu().numpy(), want)
+    assert bool(cw.__dict__.get("_tc")) != seen
