@@ -362,10 +362,8 @@ int tc_conv2d(const void* x, const ds_planes_t* xp, const int32_t* packed, const
     if (fuse->residual && (reinterpret_cast<uintptr_t>(fuse->residual) & 3u)) return DS_ERR_ALIGN;
     unsigned char* a = static_cast<unsigned char*>(act);
     int* counters = static_cast<int*>(act) + 4;
-    // the range flag: the last counter word of the workspace, as for the other paths, else the scratch's first word
+    // the range flag, in this call's own scratch: other calls may enqueue launches of theirs between these
     int* flag = static_cast<int*>(act);
-    if (fuse->workspace && fuse->workspace_bytes >= (long long)kWorkspaceCounters * 4)
-        flag = static_cast<int*>(fuse->workspace) + kWorkspaceGateSlot;
 
     TcRun p = {};
     int Hp = g.Hp, Wp = g.Wp, step_h = g.sh, step_w = g.sw;

@@ -238,3 +238,32 @@ def test_linear_fp32_input_falls_back(oracle, cuda_device, what):
     got = _run(cuda_device, x, shift, sign, None, (1, 1), (0, 0), in_kind=2, act_bits=0, I=16, F=16)
     codes = np.trunc(x.astype(np.float64) * 65536).astype(np.int32).reshape(M, K)
     assert np.array_equal(got.reshape(M, N), oracle.linear(codes, shift.reshape(N, K), sign.reshape(N, K), None))
+
+
+def test_the_range_flag_belongs_to_the_call(oracle, cuda_device):
+    """Threads may enqueue calls on one stream at once, launch by launch in any order; the workspace is the stream's,
+    so a flag there would be cleared by one call between the packing and the product of another."""
+    from deepshift_b200 import _ffi, kernels, utils
+    rng = np.random.default_rng(9)
+    M, K, N = 70, 400, 60
+    shift, sign = weights(rng, (N, K))
+    cw = utils.compress_bits(torch.from_numpy(shift).float(), torch.from_numpy(sign).float(), device=cuda_device)
+    geo = (M, K, 1, 1, N, 1, 1, 1, 1, 0, 0)
+    ws = torch.full((16384,), 77, dtype=torch.int32, device=cuda_device)
+    f = kernels._fuse(_ffi.IN_F32_LINEAR, 0, 16, 16, workspace=ws)
+    act, wt = kernels.tc_bytes(geo, cw, f, any_size=True)
+    tiles = kernels.tc_expand(geo, cw, f, wt, cuda_device)
+    scratch = torch.empty(act, dtype=torch.uint8, device=cuda_device)
+    out = torch.empty((M, N), dtype=torch.int32, device=cuda_device)
+    for wide in (0, 1):
+        x = rng.normal(0, 1, (M, K)).astype(np.float32)
+        if wide:
+            x[M - 1, K - 1] = 200.0
+        xt = torch.from_numpy(x).to(cuda_device)
+        assert _ffi.lib().ds_tc_conv2d(xt.data_ptr(), cw.data.data_ptr(), None, out.data_ptr(), *geo, cw.bits, 0, f,
+                                       scratch.data_ptr(), act, tiles.data_ptr(), wt,
+                                       torch.cuda.current_stream(cuda_device).cuda_stream) == 0
+        codes = np.trunc(x.astype(np.float64) * 65536).astype(np.int32)
+        assert np.array_equal(out.cpu().numpy(), oracle.linear(codes, shift, sign, None))
+        assert int(scratch[:4].view(torch.int32)) == wide
+        assert bool((ws == 77).all())
