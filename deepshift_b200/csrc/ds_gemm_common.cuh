@@ -117,10 +117,14 @@ __device__ __forceinline__ bool bounds_ok(int* status, const void* base, long lo
 #define DS_X_OK(p, ptr, bytes) bounds_ok((p).chk_status, (p).x, (p).chk_x_bytes, ptr, bytes, 1)
 #define DS_W_OK(p, ptr, bytes) bounds_ok((p).chk_status, (p).packed, (p).chk_w_bytes, ptr, bytes, 2)
 #define DS_O_OK(p, base, ptr, bytes) bounds_ok((p).chk_status, base, (p).chk_o_bytes, ptr, bytes, 3)
+#define DS_A_OK(p, ptr, bytes) bounds_ok((p).chk_status, (p).chk_act, (p).chk_act_bytes, ptr, bytes, 4)
+#define DS_N_OK(p, ptr, bytes) bounds_ok((p).chk_status, (p).chk_next, (p).chk_next_bytes, ptr, bytes, 5)
 #else
 #define DS_X_OK(p, ptr, bytes) true
 #define DS_W_OK(p, ptr, bytes) true
 #define DS_O_OK(p, base, ptr, bytes) true
+#define DS_A_OK(p, ptr, bytes) true
+#define DS_N_OK(p, ptr, bytes) true
 #endif
 int* bounds_status_ptr();  // device address of the status word (ds_gemm_ws.cu), null on failure
 

@@ -368,8 +368,9 @@ __device__ __forceinline__ void tc_store(const TcRun& p, int (&v)[32], const int
                 lw[q] = __byte_perm(x, y, 0x5410);
                 hw[q] = __byte_perm(x, y, 0x7632);
             }
-            *reinterpret_cast<uint4*>(nx + h) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
-            *reinterpret_cast<uint4*>(nx + p.next_plane + h) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+            if (DS_N_OK(p, nx + h, 16)) *reinterpret_cast<uint4*>(nx + h) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+            if (DS_N_OK(p, nx + p.next_plane + h, 16))
+                *reinterpret_cast<uint4*>(nx + p.next_plane + h) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
         }
     }
 }
@@ -457,9 +458,9 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
         uint4 nl = make_uint4(0, 0, 0, 0), nh = nl, nt = nl;
         auto fetch = [&]() {
             const unsigned char* a = p.act + (roff + unsigned(kh) * p.kh_step + unsigned(j) * 16u);
-            nl = ld16(a, p.align);
-            nh = ld16(a + p.plane, p.align);
-            if (WIDE) nt = ld16(a + 2 * p.plane, p.align);
+            if (DS_A_OK(p, a, 16)) nl = ld16(a, p.align);
+            if (DS_A_OK(p, a + p.plane, 16)) nh = ld16(a + p.plane, p.align);
+            if (WIDE && DS_A_OK(p, a + 2 * p.plane, 16)) nt = ld16(a + 2 * p.plane, p.align);
         };
         enter(wg);
         if (u < p.units) fetch();
@@ -986,8 +987,9 @@ __global__ void __launch_bounds__(256, 8) tc_pack_nchw_kernel(const TcPack p, co
         const long long q = q0 + pix;
         if (q < p.Q && cw0 + cw < cwords) {
             unsigned* dst = reinterpret_cast<unsigned*>(p.act + q * p.Cp) + cw0 + cw;
-            *dst = sl[pix * (CW + 1) + cw];
-            *reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(dst) + p.plane) = sh[pix * (CW + 1) + cw];
+            unsigned* dsth = reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(dst) + p.plane);
+            if (DS_A_OK(p, dst, 4)) *dst = sl[pix * (CW + 1) + cw];
+            if (DS_A_OK(p, dsth, 4)) *dsth = sh[pix * (CW + 1) + cw];
         }
     }
 }
@@ -1037,11 +1039,13 @@ __global__ void __launch_bounds__(256, 8) tc_pack_rows_kernel(const TcPack p, co
                 t |= ((y[e] >> 16) & 255u) << (8 * e);
                 c4[e] = int(y[e] & 0xFFFFu) - 32768;
             }
-            *reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(dst) + 2 * p.plane) = t;
+            unsigned* dstt = reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(dst) + 2 * p.plane);
+            if (DS_A_OK(p, dstt, 4)) *dstt = t;
         }
         pack4(c4, l, h, over);
-        *dst = l;
-        *reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(dst) + p.plane) = h;
+        unsigned* dsth = reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(dst) + p.plane);
+        if (DS_A_OK(p, dst, 4)) *dst = l;
+        if (DS_A_OK(p, dsth, 4)) *dsth = h;
     }
     if (over && p.flag) *p.flag = 1;
 }

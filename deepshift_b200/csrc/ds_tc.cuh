@@ -86,7 +86,10 @@ struct TcRun {
     unsigned wait_ns;    // limit of every wait
     int hold;            // checked build: see ds_tc_debug_waits
     int* err_flag;
+    // checked build: extents of the output, of the planes read and of the planes written
     long long chk_o_bytes;
+    const unsigned char *chk_act, *chk_next;
+    long long chk_act_bytes, chk_next_bytes;
     int* chk_status;
 };
 
@@ -105,6 +108,8 @@ struct TcPack {
     int* counters;       // zeroed here for the launch behind
     int ncounters;
     long long chk_x_bytes;
+    const unsigned char* chk_act;  // checked build: the planes
+    long long chk_act_bytes;
     int* chk_status;
 };
 

@@ -295,6 +295,8 @@ TcPack pack_params(const GemmParams& q, const void* x, unsigned char* act, long 
     pk.in_kind = q.in_kind;
     pk.q = q.q;
     pk.rq_lo = q.rq_lo; pk.rq_hi = q.rq_hi; pk.rq_mul = q.rq_mul; pk.rq_add = q.rq_add;
+    pk.chk_act = act;
+    pk.chk_act_bytes = (q.in_kind == DS_IN_F32_LINEAR ? 3 : 2) * plane;
     pk.chk_x_bytes = (long long)B * C * H * W * 4 - check_shrink_x();
     pk.chk_status = bounds_status_ptr();
     return pk;
@@ -378,9 +380,13 @@ int tc_conv2d(const void* x, const ds_planes_t* xp, const int32_t* packed, const
         step_w = sw;
         p.act = static_cast<const unsigned char*>(xp->data) + ((long long)(xp->halo - ph) * Wp + (xp->halo - pw)) * C;
         p.plane = plane;
+        p.chk_act = static_cast<const unsigned char*>(xp->data);
+        p.chk_act_bytes = 2 * plane;
     } else {
         p.act = a + g.planes_off;
         p.plane = g.plane;
+        p.chk_act = p.act;
+        p.chk_act_bytes = (wide ? 3 : 2) * g.plane;
         TcPack pk = pack_params(q, x, a + g.planes_off, g.plane, B, C, H, W, ph, pw, g.Hp, g.Wp, g.Cp, g.sub_h, g.sub_w);
         pk.counters = g.splits > 1 ? counters : nullptr;
         pk.ncounters = g.splits > 1 ? g.grid_m * g.grid_n : 0;
@@ -419,6 +425,8 @@ int tc_conv2d(const void* x, const ds_planes_t* xp, const int32_t* packed, const
         p.next_img = nh * p.next_row;
         p.next = static_cast<unsigned char*>(next->data) + ((long long)next->halo * nw + next->halo) * OC;
         p.next_plane = plane;
+        p.chk_next = static_cast<const unsigned char*>(next->data);
+        p.chk_next_bytes = 2 * plane;
         p.next_lo = -(1 << (I - 1 + F));
         p.next_hi = ((1 << (I - 1)) - 1) * (1 << F);
     }

@@ -432,7 +432,7 @@ int ds_last_kernel_error(int *flag);
  * packed weights and residual and of every global store in the linear / convolution kernels against
  * the extents implied by the call's arguments.  An access outside is skipped, never performed, and
  * the first one leaves its kind in a status word: 1 activations, 2 packed weights, 3 output /
- * residual.  Nothing traps.  (The TMA-fed staged kernel is not instrumented: the
+ * residual, 4 byte planes packed and read by a call, 5 byte planes of the layer behind it.  Nothing traps.  (The TMA-fed staged kernel is not instrumented: the
  * tensor map bounds its loads in hardware.)
  *   ds_bounds_status        reads and clears the status word (synchronises the device); *checked
  *                           says whether this library was built with the checks.

@@ -87,6 +87,39 @@ def main():
             x = acts_q16(rng, (M, K))
             out = kernels.linear(torch.from_numpy(x).to(dev), torch.from_numpy(shift).to(dev), None, None, cw, act_bits=ab)
             assert np.array_equal(out.cpu().numpy(), O.linear(x, shift, sign, None)), (M, K, N, ab)
+    # ... on the tensor cores: rows packed from measured int32 codes, 24-bit codes of fp32 input (kept tiles, used twice),
+    # byte planes from layer to layer
+    for (M, K, N) in [(66, 1031, 300), (300, 512, 200), (1000, 401, 129)]:
+        shift, sign = weights(rng, (N, K))
+        cw = cw_of(shift, sign)
+        st, x = torch.from_numpy(shift).to(dev), acts_q16(rng, (M, K))
+        assert kernels.tc_bytes((M, K, 1, 1, N, 1, 1, 1, 1, 0, 0), cw, kernels._fuse(act_bits=-1))[0] > 0
+        out = kernels.linear(torch.from_numpy(x).to(dev), st, None, None, cw)
+        assert np.array_equal(out.cpu().numpy(), O.linear(x, shift, sign, None)), (M, K, N)
+        xf = rng.normal(0, 1, (M, K)).astype(np.float32)
+        want = O.linear(np.trunc(xf.astype(np.float64) * 65536).astype(np.int32), shift, sign, None)
+        for _ in range(2):
+            out = kernels.linear_fused(torch.from_numpy(xf).to(dev), N, None, cw, in_kind=_ffi.IN_F32_LINEAR)
+            assert np.array_equal(out.cpu().numpy(), want), (M, K, N)
+    for (B, C, H, OC, halo) in [(3, 16, 9, 48, 1), (2, 64, 14, 144, 2), (2, 512, 7, 16, 1)]:
+        shift, sign = weights(rng, (OC, C, 3, 3))
+        s2, g2 = weights(rng, (20, OC, 1, 1))
+        x = acts_q16(rng, (B, C, H, H))
+        src, nxt = kernels.Planes(B, C, H, H, halo, dev), kernels.Planes(B, OC, H, H, 0, dev)
+        cur = torch.cuda.current_stream().cuda_stream
+        f, xt = kernels._fuse(_ffi.IN_I32_CLAMP, 0, 4, 12), torch.from_numpy(x).to(dev)
+        assert lib.ds_planes_pack(xt.data_ptr(), _ffi.IN_I32_CLAMP, 4, 12, src.c, cur) == 0
+        out = torch.empty((B, 20, H, H), dtype=torch.int32, device=dev)
+        for cw, geo, a, b, o in ((cw_of(shift, sign), (B, C, H, H, OC, 3, 3, 1, 1, 1, 1), src.c, nxt.c, None),
+                                 (cw_of(s2, g2), (B, OC, H, H, 20, 1, 1, 1, 1, 0, 0), nxt.c, None, out)):
+            na, nw = kernels.tc_bytes(geo, cw, f, any_size=True)
+            act = torch.zeros(na, dtype=torch.uint8, device=dev)
+            tiles = kernels.tc_expand(geo, cw, f, nw, dev)
+            assert lib.ds_tc_conv2d_ex(None, a, cw.data.data_ptr(), None, o.data_ptr() if o is not None else None, b, *geo,
+                                       cw.bits, 0, f, act.data_ptr(), na, tiles.data_ptr(), nw, cur) == 0
+            torch.cuda.synchronize()
+        v = np.clip(O.conv2d(np.clip(x, -32768, 28672), shift, sign, None, (1, 1), (1, 1)), -32768, 28672)
+        assert np.array_equal(out.cpu().numpy(), O.conv2d(v, s2, g2, None, (1, 1), (0, 0))), (B, C, H, OC)
     assert status(lib) == (0, 1), "an access left its extent"
     waits_that_run_out(lib, dev, O, cw_of, rng)
     assert status(lib) == (0, 1)

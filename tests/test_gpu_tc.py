@@ -11,8 +11,9 @@ pytestmark = pytest.mark.gpu
 
 
 def _run(dev, x, shift, sign, bias, s, p, *, in_kind=0, act_bits=15, out_f32=False, relu=False, residual=None, I=4, F=12,
-         round_f32=False):
-    """One call of any size through the C ABI, scratch and weights in buffers of exactly the asked size."""
+         round_f32=False, falls_back=None):
+    """One call of any size through the C ABI, scratch and weights in buffers of exactly the asked size.
+    ``falls_back`` (calls whose range is measured): whether the integer path must have given the answer."""
     from deepshift_b200 import _ffi, kernels, utils
     B, C, H, W = x.shape
     OC, _, KH, KW = shift.shape
@@ -35,6 +36,8 @@ def _run(dev, x, shift, sign, bias, s, p, *, in_kind=0, act_bits=15, out_f32=Fal
     torch.cuda.synchronize(dev)
     assert kernels.last_kernel_error() == 0
     assert bool((scratch[act:] == 0xA5).all()) and bool((out[-16:] == 0x5EADBEE).all())
+    if falls_back is not None:   # the range flag, first word of the scratch
+        assert int(scratch[:4].view(torch.int32)) == int(falls_back)
     y = out[:-16].reshape(B, OC, OH, OW)
     return (y.view(torch.float32) if out_f32 else y).cpu().numpy()
 
@@ -70,9 +73,32 @@ def test_linear_full_16_bit_range(oracle, cuda_device, mkn):
     x.flat[::7] = -32768
     x.flat[3::11] = 32767
     shift, sign = weights(rng, (N, K, 1, 1))
-    got = _run(cuda_device, x, shift, sign, None, (1, 1), (0, 0), act_bits=-1)
+    got = _run(cuda_device, x, shift, sign, None, (1, 1), (0, 0), act_bits=-1, falls_back=False)
     want = oracle.linear(x.reshape(M, K), shift.reshape(N, K), sign.reshape(N, K), None)
     assert np.array_equal(got.reshape(M, N), want)
+
+
+@pytest.mark.parametrize("rows", [1, 130])
+@pytest.mark.parametrize("fp32", [False, True])
+def test_sums_wrap_around_like_int32(oracle, cuda_device, fp32, rows):
+    """Partial sums of one sign that leave int32: 16-bit codes reach 2^31 after 2^16 products without a shift, 24-bit
+    codes after 2^8.  The accumulators must wrap, not saturate."""
+    rng = np.random.default_rng(rows)
+    K, N = 150_000, 33
+    x = np.full((rows, K, 1, 1), -128.0 if fp32 else -32768, np.float32 if fp32 else np.int32)
+    x.flat[::5] = 127.5 if fp32 else -32767
+    shift = np.zeros((N, K, 1, 1), np.int32)
+    sign = np.ones((N, K, 1, 1), np.int32)
+    sign[1::2] = -1
+    shift[3, ::2] = -1
+    shift[4] = -rng.integers(0, 16, (K, 1, 1))
+    got = _run(cuda_device, x, shift, sign, None, (1, 1), (0, 0), in_kind=2 if fp32 else 0, act_bits=0 if fp32 else -1, I=16,
+               F=16, falls_back=False)
+    codes = (x.astype(np.float64) * (65536 if fp32 else 1)).astype(np.int64).reshape(rows, K)
+    w, r = sign.reshape(N, K).astype(np.int64), -shift.reshape(N, K).astype(np.int64)
+    exact = np.stack([((codes >> r[n]) * w[n]).sum(1) for n in range(N)], 1)
+    assert np.abs(exact).max() > 2 ** 32
+    assert np.array_equal(got.reshape(rows, N), exact.astype(np.int32))
 
 
 @pytest.mark.parametrize("value", [32768, -32769, 1 << 30])
@@ -81,12 +107,12 @@ def test_one_wide_code_sends_the_call_to_the_integer_path(oracle, cuda_device, v
     x = acts_q16(rng, (3, 20, 9, 10))
     x[2, 19, 8, 9] = value
     shift, sign = weights(rng, (40, 20, 3, 3))
-    got = _run(cuda_device, x, shift, sign, None, (1, 1), (1, 1), act_bits=-1)
+    got = _run(cuda_device, x, shift, sign, None, (1, 1), (1, 1), act_bits=-1, falls_back=True)
     assert np.array_equal(got, oracle.conv2d(x, shift, sign, None, (1, 1), (1, 1)))
     xl = acts_q16(rng, (90, 70, 1, 1))
     xl[89, 69] = value
     sl, gl = weights(rng, (33, 70, 1, 1))
-    got = _run(cuda_device, xl, sl, gl, None, (1, 1), (0, 0), act_bits=-1)
+    got = _run(cuda_device, xl, sl, gl, None, (1, 1), (0, 0), act_bits=-1, falls_back=True)
     assert np.array_equal(got.reshape(90, 33), oracle.linear(xl.reshape(90, 70), sl.reshape(33, 70), gl.reshape(33, 70), None))
 
 
@@ -127,7 +153,7 @@ def test_every_packing(oracle, cuda_device, bits):
     shift = -rng.integers(0, 2 ** bits, (48, 96, 1, 1)).astype(np.int32)
     sign = rng.choice([-1, 1], (48, 96, 1, 1)).astype(np.int32)
     shift[0, 0] = -(2 ** bits - 1)
-    got = _run(cuda_device, x, shift, sign, None, (1, 1), (0, 0), act_bits=-1)
+    got = _run(cuda_device, x, shift, sign, None, (1, 1), (0, 0), act_bits=-1, falls_back=False)
     assert np.array_equal(got.reshape(70, 48), oracle.linear(x.reshape(70, 96), shift.reshape(48, 96), sign.reshape(48, 96), None))
 
 
@@ -216,7 +242,8 @@ def test_linear_fp32_input_24_bit_codes(oracle, cuda_device, mkn, scale):
     x.flat[::17], x.flat[5::31] = -128.0, np.float32(8388607 / 65536)
     shift, sign = weights(rng, (N, K, 1, 1))
     bias = rng.integers(-2000, 2000, N).astype(np.int32)
-    got = _run(cuda_device, x, shift, sign, bias, (1, 1), (0, 0), in_kind=2, act_bits=0, I=16, F=16, relu=True)
+    got = _run(cuda_device, x, shift, sign, bias, (1, 1), (0, 0), in_kind=2, act_bits=0, I=16, F=16, relu=True,
+               falls_back=False)
     codes = np.trunc(x.astype(np.float64) * 65536).astype(np.int32).reshape(M, K)
     want = np.maximum(oracle.linear(codes, shift.reshape(N, K), sign.reshape(N, K), bias), 0)
     assert np.array_equal(got.reshape(M, N), want)
@@ -235,7 +262,7 @@ def test_linear_fp32_input_falls_back(oracle, cuda_device, what):
         x[89, 199] = 128.0
     else:
         shift[69, 199] = -17
-    got = _run(cuda_device, x, shift, sign, None, (1, 1), (0, 0), in_kind=2, act_bits=0, I=16, F=16)
+    got = _run(cuda_device, x, shift, sign, None, (1, 1), (0, 0), in_kind=2, act_bits=0, I=16, F=16, falls_back=True)
     codes = np.trunc(x.astype(np.float64) * 65536).astype(np.int32).reshape(M, K)
     assert np.array_equal(got.reshape(M, N), oracle.linear(codes, shift.reshape(N, K), sign.reshape(N, K), None))
 
@@ -267,3 +294,34 @@ def test_the_range_flag_belongs_to_the_call(oracle, cuda_device):
         assert np.array_equal(out.cpu().numpy(), oracle.linear(codes, shift, sign, None))
         assert int(scratch[:4].view(torch.int32)) == wide
         assert bool((ws == 77).all())
+
+
+@pytest.mark.parametrize("what", ["fits", "code", "shift"])
+@pytest.mark.parametrize("kind", ["linear", "conv", "linear fp32"])
+def test_calls_that_expand_their_weights(oracle, cuda_device, kind, what):
+    """Weights expanded in the call, which may itself send it to the integer path (24-bit form, a shift of 16..31).  The
+    scratch comes filled, as an allocator hands it out."""
+    from deepshift_b200 import _ffi, kernels, utils
+    rng = np.random.default_rng(3)
+    fp32 = kind == "linear fp32"
+    B, C, H, OC, k = (3, 40, 9, 70, 3) if kind == "conv" else (90, 400, 1, 70, 1)
+    shift, sign = weights(rng, (OC, C, k, k))
+    sign.flat[0] = 0
+    if what == "shift":
+        sign[OC - 1, C - 1], shift[OC - 1, C - 1] = 1, -17
+    cw = utils.compress_bits(torch.from_numpy(shift).float(), torch.from_numpy(sign).float(), device=cuda_device)
+    geo = (B, C, H, H, OC, k, k, 1, 1, k // 2, k // 2)
+    f = kernels._fuse(_ffi.IN_F32_LINEAR, 0, 16, 16) if fp32 else kernels._fuse(act_bits=-1)
+    act, wt = kernels.tc_bytes(geo, cw, f, any_size=True)
+    scratch = torch.full((act + wt,), 0xA5, dtype=torch.uint8, device=cuda_device)
+    out = torch.empty((B, OC, H, H), dtype=torch.int32, device=cuda_device)
+    x = rng.normal(0, 1, (B, C, H, H)).astype(np.float32)
+    if what == "code":
+        x.flat[-1] = 200.0
+    codes = np.trunc(x.astype(np.float64) * (65536 if fp32 else 4096)).astype(np.int32)
+    xt = torch.from_numpy(x if fp32 else codes).to(cuda_device)
+    assert _ffi.lib().ds_tc_conv2d_packed(xt.data_ptr(), cw.data.data_ptr(), None, out.data_ptr(), *geo, cw.bits, 0, f,
+                                          scratch.data_ptr(), act, scratch.data_ptr() + act, wt, 0,
+                                          torch.cuda.current_stream(cuda_device).cuda_stream) == 0
+    assert np.array_equal(out.cpu().numpy(), oracle.conv2d(codes, shift, sign, None, (1, 1), (k // 2, k // 2)))
+    assert int(scratch[:4].view(torch.int32)) == int(what == "code" or (fp32 and what == "shift"))
