@@ -18,9 +18,9 @@
 //                 MMAs, and two A slots per producer warpgroup (sixteen planes x 16 bytes x 128 rows each).
 //
 // What bounds it: the s8 MMA rate, 16 byte-products per shift-accumulate (8192 per SM and clock: 144 T
-// shift-op/s at 1.9 GHz), of which 63 % are in use at 128 columns and 41 % at 64.  Measured, packing included: 8192 x
-// 4096 x 4096 1.50 ms = 92 T shift-op/s (6.69 ms on the FP32 pipe); 3x3 on 64 / 128 / 256 / 512 channels, 256 images,
-// 48 / 74 / 73 / 75 T (20.5 / 24 / 21.5 / 20.9).  A from TMEM because shared memory could not carry both operands: at BN = 64 an
+// shift-op/s at 1.9 GHz), of which 63 % are in use at 128 columns and 41 % at 64.  Measured: 8192 x 4096 x 4096, packing
+// and expansion in the call, 1.72 ms = 80 T shift-op/s (6.69 ms on the FP32 pipe); the sixteen 3x3 convolutions of a
+// ResNet-18 on 256 images, planes from layer to layer, 74 T together, 57 T at 64 channels to 82 T (20.5 to 24).  A from TMEM because shared memory could not carry both operands: at BN = 64 an
 // MMA of 32 cycles would read 4 KiB of A and 2 KiB of B, 192 bytes per cycle where 128 are available.
 #include "ds_tc.cuh"
 
@@ -856,7 +856,8 @@ __device__ __forceinline__ void keep_compare(const TcExpand& p, unsigned block)
     if (threadIdx.x == 0) atomicAdd(p.state + 1, 1);
 }
 
-// The wait ends: the blocks waited for depend on nothing, and exp_blocks never fill the GPU.  (Bounded all the same.)
+// The wait ends: the blocks waited for depend on nothing and come first in the launch, and exp_blocks, an eighth of
+// what is resident, never fill the GPU.  (Bounded all the same.)
 __device__ __forceinline__ void keep_expand(const TcExpand& p, int block, ExpandSmem& sm)
 {
     if (threadIdx.x == 0) {
