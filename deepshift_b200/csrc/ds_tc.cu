@@ -18,10 +18,11 @@
 //                 MMAs, and two A slots per producer warpgroup (sixteen planes x 16 bytes x 128 rows each).
 //
 // What bounds it: the s8 MMA rate, 16 byte-products per shift-accumulate (8192 per SM and clock: 144 T
-// shift-op/s at 1.9 GHz), of which 63 % are in use at 128 columns and 41 % at 64.  Measured: 8192 x 4096 x 4096, packing
-// and expansion in the call, 1.72 ms = 80 T shift-op/s (6.69 ms on the FP32 pipe); the sixteen 3x3 convolutions of a
-// ResNet-18 on 256 images, planes from layer to layer, 74 T together, 57 T at 64 channels to 82 T (20.5 to 24).  A from TMEM because shared memory could not carry both operands: at BN = 64 an
-// MMA of 32 cycles would read 4 KiB of A and 2 KiB of B, 192 bytes per cycle where 128 are available.
+// shift-op/s at 1.9 GHz).  A takes N / 2 cycles per MMA from tensor memory, whatever N; from shared memory 40 + N / 8
+// up to 128 columns, which could not carry both operands.  At 128 columns 78 to 85 % of the rate are in use (8192 x 4096 x
+// 4096: 1124 us = 122 T; 128 to 512 channels 3x3, 256 images: 260 to 268 us = 112 T, 317 to 341 before the
+// hand-shake below).  At 64 columns it is the producers: 177 instructions per item and scheduler on a pipe that takes
+// one every other cycle, 550 cycles per item where the MMAs take 256.
 #include "ds_tc.cuh"
 
 namespace ds {
@@ -32,34 +33,30 @@ namespace {
 
 constexpr int TC_TMEM_COLS = 512;
 
-// Per column width: WG producer warpgroups, each with two A slots of its own (64 columns: sixteen planes x 16
+// Per column width: WG producer warpgroups, each with A slots of its own (64 columns: sixteen planes x 16
 // bytes; a slot shared between warpgroups could not be guarded by a phase parity, since a warpgroup may be two
 // phases away from it), and as many accumulator slots as the remaining columns hold: two of 128 or 64 columns, so
-// that the epilogue of a tile overlaps the next tile's MMAs.  With one A slot per warpgroup the refill sat in the
-// MMAs' way (813 cycles per 128 rows x 16 values at 128 columns, 675 at 64, where the MMAs alone take 640 and 450).
-// The price: no two row blocks share a weight tile any more (512 channels, 256 images: 348 -> 392 us; 64 channels
-// 640 -> 613).
+// that the epilogue of a tile overlaps the next tile's MMAs.
 template <int BN, bool WIDE>
 struct TcTile {
-    static constexpr int WG = WIDE || BN == 128 ? 2 : 3;
+    static constexpr int WG = WIDE ? 2 : 3;
     static constexpr int PLANES = WIDE ? TC_PLANES_WIDE : TC_PLANES;
     static constexpr int ASTRIDE = WIDE ? 96 : 64;   // columns from one A slot to the next
     static constexpr int ACC = WIDE ? 2 * BN : BN;   // columns of an accumulator slot (wide: sums of weight 2^8 behind)
     static constexpr int THREADS = (4 * WG + 6) * 32;  // + 4 epilogue warps + MMA warp + loader warp
-    static constexpr int SLOTS = (WIDE ? 1 : 2) * WG;  // A slots, handed out round robin: item i fills slot i % SLOTS
+    static constexpr int SLOTS = (WIDE || BN == 128 ? 1 : 2) * WG;  // A slots, handed out round robin: item i fills slot i % SLOTS
     static constexpr int ACC_COLS = TC_TMEM_COLS - ASTRIDE * SLOTS;
     static constexpr int NACC = ACC_COLS / ACC < 6 ? ACC_COLS / ACC : 6;
     static constexpr int STAGE = BN * PLANES * TC_KG;
-    static constexpr int STAGES = BN == 128 ? 6 : 8;
+    static constexpr int STAGES = BN == 128 ? 6 : WIDE ? 8 : 12;  // weight tiles in shared memory, more than A slots
 };
 
 template <int BN, bool WIDE>
 struct TcSmem {
     alignas(128) unsigned char b[TcTile<BN, WIDE>::STAGES][TcTile<BN, WIDE>::STAGE];
     alignas(8) unsigned long long bfull[TcTile<BN, WIDE>::STAGES];
-    unsigned long long bempty[TcTile<BN, WIDE>::STAGES];
-    unsigned long long afull[TcTile<BN, WIDE>::SLOTS];
-    unsigned long long aempty[TcTile<BN, WIDE>::SLOTS];
+    unsigned long long full[TcTile<BN, WIDE>::SLOTS];   // both operands of the item in this slot are there
+    unsigned long long empty[TcTile<BN, WIDE>::SLOTS];  // its MMAs are done
     unsigned long long accfull[6];
     unsigned long long accempty[6];
     unsigned long long done;
@@ -287,6 +284,14 @@ __device__ __forceinline__ Unit unit_of(const TcRun& p, int u)
     return r;
 }
 
+// Groups of unit u.
+__device__ __forceinline__ int unit_groups(const TcRun& p, int u)
+{
+    if (p.splits == 1) return p.G;
+    const int g0 = u % p.splits * p.gps;
+    return min(p.G, g0 + p.gps) - g0;
+}
+
 __device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 // Epilogue of 32 columns of one row: v (the int32 sums) at row m, columns n..n+31.
@@ -387,13 +392,10 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
 
     if (threadIdx.x == 0) {
         s.err = 0;
-        for (int i = 0; i < T::STAGES; ++i) {
-            bar_init(&s.bfull[i], 1);
-            bar_init(&s.bempty[i], 1);
-        }
+        for (int i = 0; i < T::STAGES; ++i) bar_init(&s.bfull[i], 1);
         for (int i = 0; i < T::SLOTS; ++i) {
-            bar_init(&s.afull[i], 4);
-            bar_init(&s.aempty[i], 1);
+            bar_init(&s.full[i], 5);  // four producer warps and the loader
+            bar_init(&s.empty[i], 1);
         }
         for (int i = 0; i < T::NACC; ++i) {
             bar_init(&s.accfull[i], 1);
@@ -481,7 +483,7 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
             // and nothing but the stores between the slot's release and its hand-over.
             constexpr int PER = T::SLOTS / T::WG;  // slots of this warpgroup, used in turn
             const unsigned slot = wg + T::WG * (round % PER), use = round / PER;
-            const bool ok = use == 0 || bar_wait(&s.aempty[slot], (use - 1) & 1u, err, p.wait_ns);
+            const bool ok = use == 0 || bar_wait(&s.empty[slot], (use - 1) & 1u, err, p.wait_ns);
             ++round;
             if (!__all_sync(0xFFFFFFFFu, ok) || TC_HELD(p, 2)) break;  // the whole warp, or none of it
             tc_fence_after();
@@ -494,7 +496,7 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) bar_arrive(&s.afull[slot]);
+            if (lane == 0) bar_arrive(&s.full[slot]);
         }
     } else if (warp < 4 * T::WG + 4) {
         // ---- epilogue ----------------------------------------------------------------------------------
@@ -583,9 +585,11 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
         }
     } else if (warp == 4 * T::WG + 4) {
         // ---- MMA issue ---------------------------------------------------------------------------------
-        // The whole warp walks the loop and an elected lane issues: control flow and addresses stay
-        // warp-uniform, and every ring index is a counter that wraps.  (One divergent lane with indices by
-        // division took 1100 cycles per four MMAs, whatever their width: 42 T shift-op/s at M = 8192.)
+        // One elected lane walks the whole loop.  Its instructions are in one queue with the MMAs and, on its
+        // scheduler, with the producers' stores to tensor memory: a wait costs 150 to 300 cycles even when what it
+        // waits for is there (64 columns, MMAs alone 256 cycles per item: two waits, two commits and an election per
+        // item 620 cycles, one wait of which the answer is asked for before the previous item's MMAs 367).  So an item
+        // has one barrier for both operands, asked ahead, and one commit.
         // A wait that gives up does not leave the loop: the error word makes all later ones return at once,
         // and every access stays inside shared and tensor memory.
         // D s32, A u8, B s8, both K-major, N = BN, M = 128
@@ -594,80 +598,102 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
         // plane (BN * 16 bytes) along K
         const unsigned long long desc0 =
             (1ull << 46) | (8ull << 32) | ((unsigned long long)BN << 16) | (s32(&s.b[0][0]) >> 4);
-        unsigned slot = 0, aph = 0, st = 0, bph = 0, aslot = 0, accph = 1;
-        for (int u = blockIdx.x; u < p.units; u += gridDim.x) {
-            const Unit un = unit_of<BN>(p, u);
-            const unsigned d = tmem + aslot * T::ACC;
-            unsigned long long* accfull = &s.accfull[aslot];
-            bar_wait(&s.accempty[aslot], accph, err, p.wait_ns);  // the first round finds the slots free
-            if (++aslot == unsigned(T::NACC)) {
-                aslot = 0;
-                accph ^= 1u;
-            }
-            unsigned more = 0;  // the first MMA of a unit overwrites the accumulator
-            for (int g = un.g0; g < un.g1; ++g) {
-                bar_wait(&s.bfull[st], bph, err, p.wait_ns);
-                const unsigned long long bdesc = desc0 + st * unsigned(T::STAGE >> 4);
-                bar_wait(&s.afull[slot], aph, err, p.wait_ns);
-                tc_fence_after();
-                if (elect_one()) {
-#pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        tc_mma_i8(d, tmem_a + slot * T::ASTRIDE + q * 8, bdesc + q * (2 * BN), idesc, q == 0 ? more : 1u);
-                    if (WIDE) {
-                        const unsigned at = tmem_a + slot * T::ASTRIDE + 64;
-                        tc_mma_i8(d, at, bdesc + 8 * (2 * BN), idesc, 1u);
-                        tc_mma_i8(d + BN, at, bdesc + 9 * (2 * BN), idesc, more);
-                        tc_mma_i8(d + BN, at + 8, bdesc + 10 * (2 * BN), idesc, 1u);
-                    }
-                    tc_commit(&s.aempty[slot]);
-                    tc_commit(&s.bempty[st]);
+        if (elect_one()) {
+            unsigned slot = 0, ph = 0, st = 0, aslot = 0, accph = 1;
+            bool ready = false, acc_ready = true;  // the first round finds the accumulator slots free
+            for (int u = blockIdx.x; u < p.units; u += gridDim.x) {
+                const unsigned d = tmem + aslot * T::ACC;
+                if (!acc_ready) bar_wait(&s.accempty[aslot], accph, err, p.wait_ns);
+                unsigned long long* accfull = &s.accfull[aslot];
+                if (++aslot == unsigned(T::NACC)) {
+                    aslot = 0;
+                    accph ^= 1u;
                 }
-                __syncwarp();
+                unsigned more = 0;  // the first MMA of a unit overwrites the accumulator
+                for (int left = unit_groups(p, u); left > 0; --left) {
+                    if (!ready) bar_wait(&s.full[slot], ph, err, p.wait_ns);
+                    const unsigned cur = slot;
+                    if (++slot == unsigned(T::SLOTS)) {
+                        slot = 0;
+                        ph ^= 1u;
+                    }
+                    ready = bar_test(&s.full[slot], ph);
+                    if (left == 1) acc_ready = bar_test(&s.accempty[aslot], accph);
+                    const unsigned long long bdesc = desc0 + st * unsigned(T::STAGE >> 4);
+                    const unsigned at = tmem_a + cur * T::ASTRIDE;
+                    tc_fence_after();
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) tc_mma_i8(d, at + q * 8, bdesc + q * (2 * BN), idesc, q == 0 ? more : 1u);
+                    if (WIDE) {
+                        tc_mma_i8(d, at + 64, bdesc + 8 * (2 * BN), idesc, 1u);
+                        tc_mma_i8(d + BN, at + 64, bdesc + 9 * (2 * BN), idesc, more);
+                        tc_mma_i8(d + BN, at + 72, bdesc + 10 * (2 * BN), idesc, 1u);
+                    }
+                    tc_commit(&s.empty[cur]);
+                    more = 1;
+                    if (++st == unsigned(T::STAGES)) st = 0;
+                }
+                tc_commit(accfull);
+            }
+            tc_commit(&s.done);  // nothing of this CTA is in flight when the columns go back
+            if (!bar_drain(&s.done, 0)) *err = 1;
+        }
+        __syncwarp();
+    } else {
+        // ---- weight tiles: one thread ------------------------------------------------------------------
+        // It keeps STAGES tiles in flight or in use, and takes part in each item's barrier once its tile has landed:
+        // the stage of item i is free again when item i's MMAs are done, which is also when slot i % SLOTS is.
+        if (lane == 0) {
+            int lu = blockIdx.x, lleft = 0;  // what to fetch next
+            const unsigned char* src = nullptr;
+            unsigned lst = 0, issued = 0;
+            auto fetch = [&]() {
+                while (lleft == 0) {
+                    if (lu >= p.units || TC_HELD(p, 1)) return;
+                    const Unit un = unit_of<BN>(p, lu);
+                    src = p.wexp + ((long long)un.nt * p.G + un.g0) * T::STAGE;
+                    lleft = un.g1 - un.g0;
+                    lu += gridDim.x;
+                }
+                asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(
+                                 s32(&s.bfull[lst])),
+                             "r"(unsigned(T::STAGE))
+                             : "memory");
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                 s32(&s.b[lst][0])),
+                             "l"(src), "r"(unsigned(T::STAGE)), "r"(s32(&s.bfull[lst]))
+                             : "memory");
+                src += T::STAGE;
+                --lleft;
+                ++issued;
+                if (++lst == unsigned(T::STAGES)) lst = 0;
+            };
+            for (int i = 0; i < T::STAGES; ++i) fetch();
+            unsigned i = 0, st = 0, bph = 0, slot = 0, ph = 1;
+            for (; i < issued; ++i) {
+                if (i >= unsigned(T::SLOTS)) {
+                    if (!bar_wait(&s.empty[slot], ph, err, p.wait_ns)) break;
+                    fetch();
+                }
+                if (!bar_wait(&s.bfull[st], bph, err, p.wait_ns)) break;
+                bar_arrive(&s.full[slot]);
                 if (++slot == unsigned(T::SLOTS)) {
                     slot = 0;
-                    aph ^= 1u;
+                    ph ^= 1u;
                 }
-                more = 1;
                 if (++st == unsigned(T::STAGES)) {
                     st = 0;
                     bph ^= 1u;
                 }
             }
-            if (elect_one()) tc_commit(accfull);
-            __syncwarp();
-        }
-        if (elect_one()) tc_commit(&s.done);  // nothing of this CTA is in flight when the columns go back
-        if (!bar_drain(&s.done, 0)) *err = 1;
-        __syncwarp();
-    } else {
-        // ---- weight tiles: one thread ------------------------------------------------------------------
-        if (lane == 0) {
-            unsigned bs = 0;
-            bool ok = true;
-            for (int u = blockIdx.x; u < p.units && ok && !TC_HELD(p, 1); u += gridDim.x) {
-                const Unit un = unit_of<BN>(p, u);
-                const unsigned char* src = p.wexp + ((long long)un.nt * p.G + un.g0) * T::STAGE;
-                for (int g = un.g0; g < un.g1; ++g, ++bs, src += T::STAGE) {
-                    const unsigned st = bs % T::STAGES;
-                    if (bs >= unsigned(T::STAGES)) {
-                        ok = bar_wait(&s.bempty[st], (bs / T::STAGES - 1) & 1u, err, p.wait_ns);
-                        if (!ok) break;
-                    }
-                    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(
-                                     s32(&s.bfull[st])),
-                                 "r"(unsigned(T::STAGE))
-                                 : "memory");
-                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                                     s32(&s.b[st][0])),
-                                 "l"(src), "r"(unsigned(T::STAGE)), "r"(s32(&s.bfull[st]))
-                                 : "memory");
+            // Every copy has landed before the CTA ends, also when a wait gave up.
+            for (; i < issued; ++i) {
+                if (!bar_drain(&s.bfull[st], bph)) *err = 1;
+                if (++st == unsigned(T::STAGES)) {
+                    st = 0;
+                    bph ^= 1u;
                 }
             }
-            // Let every copy land before the CTA ends (the MMA thread has waited for all of them unless a
-            // wait gave up).
-            for (unsigned k = bs > unsigned(T::STAGES) ? bs - T::STAGES : 0; k < bs; ++k)
-                if (!bar_drain(&s.bfull[k % T::STAGES], (k / T::STAGES) & 1u)) *err = 1;
         }
         __syncwarp();
     }
