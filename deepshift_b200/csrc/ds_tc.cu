@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
         };
         uint4 nl = make_uint4(0, 0, 0, 0), nh = nl, nt = nl;
         auto fetch = [&]() {
-            const unsigned char* a = p.act + (roff + unsigned(kh) * p.kh_step + unsigned(j) * 16u);
+            const unsigned char* a = p.act + (roff + unsigned(kh) * p.kh_step + unsigned(j) * p.j_step);
             if (DS_A_OK(p, a, 16)) nl = ld16(a, p.align);
             if (DS_A_OK(p, a + p.plane, 16)) nh = ld16(a + p.plane, p.align);
             if (WIDE && DS_A_OK(p, a + 2 * p.plane, 16)) nt = ld16(a + 2 * p.plane, p.align);
@@ -1021,7 +1021,9 @@ __global__ void __launch_bounds__(256, 8) tc_pack_nchw_kernel(const TcPack p, co
     }
 }
 
-// Rows of a matrix [Q, C]: 4 values of a row per thread.  KEPT as above.
+// Rows of a matrix [Q, C]: 4 values of a row per thread, 16 values of 8 rows per warp.  The planes come out pixel-major
+// (row_bytes = Cp, group_bytes = 16) or, for the product behind, as [16 values][row]: its threads are rows, and 16 bytes
+// at the row's pitch from each cost the load unit a wavefront per thread.  KEPT as above.
 template <int INK, bool WIDE, bool KEPT>
 __global__ void __launch_bounds__(256, 8) tc_pack_rows_kernel(const TcPack p, const TcExpand e)
 {
@@ -1031,16 +1033,18 @@ __global__ void __launch_bounds__(256, 8) tc_pack_rows_kernel(const TcPack p, co
         if (keep_weights(e, block, sm)) return;
         blocks -= unsigned(e.cmp_blocks + e.exp_blocks);
     }
-    const unsigned words = unsigned(p.Cp) >> 2;
-    const unsigned total = unsigned(p.Q) * words;  // plane bytes < 2^31, so this fits
+    const unsigned groups = (unsigned(p.Cp) + 15u) >> 4;
+    const unsigned total = (unsigned(p.Q) + 7u) / 8u * groups * 32u;  // checked by the launch
     const bool vec = p.C % 4 == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15u) == 0;
     const unsigned i0 = block * 256u + threadIdx.x;
     if (p.counters)
         for (unsigned i = i0; i < unsigned(p.ncounters); i += blocks * 256u) p.counters[i] = 0;
     bool over = i0 == 0 && p.refuse && *p.refuse;
     for (unsigned i = i0; i < total; i += blocks * 256u) {
-        const unsigned m = i / words, w = i - m * words;
-        const int k = int(4 * w);
+        const unsigned t = i >> 5, mb = t / groups, j = t - mb * groups;
+        const unsigned m = 8 * mb + ((i >> 2) & 7u);
+        const int k = int(16 * j + 4 * (i & 3u));
+        if (m >= unsigned(p.Q) || k >= p.Cp) continue;
         const int* src = static_cast<const int*>(p.x) + (long long)m * p.C + k;
         int raw[4] = {0, 0, 0, 0}, c4[4];
         if (vec && k + 4 <= p.C) {
@@ -1056,7 +1060,7 @@ __global__ void __launch_bounds__(256, 8) tc_pack_rows_kernel(const TcPack p, co
 #pragma unroll
         for (int e = 0; e < 4; ++e) c4[e] = k + e < p.C ? pack_code<INK>(p, raw[e]) : 0;
         unsigned l, h;
-        unsigned* dst = reinterpret_cast<unsigned*>(p.act) + i;
+        unsigned* dst = reinterpret_cast<unsigned*>(p.act + (m * p.row_bytes + j * p.group_bytes + 4 * (i & 3u)));
         if (WIDE) {
             unsigned y[4], t = 0;
 #pragma unroll
@@ -1118,7 +1122,7 @@ int tc_launch_pack(const TcPack& p, const TcExpand* e0, bool wide, cudaStream_t 
     }
     const unsigned more = unsigned(e.cmp_blocks + e.exp_blocks);
     auto rows = [&](auto ink) {
-        const long long want = (p.Q * (p.Cp / 4) + 255) / 256;
+        const long long want = ((p.Q + 7) / 8 * ((p.Cp + 15) / 16) * 32 + 255) / 256;
         const unsigned grid = unsigned(want > 148 * 64 ? 148 * 64 : want) + more;
         constexpr int K = decltype(ink)::value;
         if (wide && e0) tc_pack_rows_kernel<K, true, true><<<grid, 256, 0, st>>>(p, e);

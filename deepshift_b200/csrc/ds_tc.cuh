@@ -69,7 +69,7 @@ struct TcRun {
     const int* residual;
     void* out;
     int M, N, P, OC, OW, G, J, align;
-    unsigned img_bytes, row_step, col_step, kh_step;  // byte offsets inside a plane
+    unsigned img_bytes, row_step, col_step, kh_step, j_step;  // byte offsets inside a plane
     int grid_m, grid_n, splits, gps, units, m_fast;
     // byte planes of the layer that reads this output (null: none); `next` is the pixel (0, 0, 0) of the l plane
     unsigned char* next;
@@ -100,6 +100,7 @@ struct TcPack {
     int B, C, H, W, ph, pw, Hp, Wp, Cp;
     int sub_h, sub_w;    // source pixel of (h, w): (h * sub_h, w * sub_w)
     long long Q;         // padded pixels
+    unsigned row_bytes, group_bytes;  // tc_pack_rows: from one row, or group of 16 values, to the next
     int in_kind;
     Quant q;
     int rq_lo, rq_hi, rq_mul, rq_add;

@@ -292,6 +292,8 @@ TcPack pack_params(const GemmParams& q, const void* x, unsigned char* act, long 
     pk.B = B; pk.C = C; pk.H = H; pk.W = W; pk.ph = ph; pk.pw = pw; pk.Hp = Hp; pk.Wp = Wp; pk.Cp = Cp;
     pk.sub_h = sub_h; pk.sub_w = sub_w;
     pk.Q = (long long)B * pk.Hp * pk.Wp;
+    pk.row_bytes = unsigned(Cp);
+    pk.group_bytes = 16;
     pk.in_kind = q.in_kind;
     pk.q = q.q;
     pk.rq_lo = q.rq_lo; pk.rq_hi = q.rq_hi; pk.rq_mul = q.rq_mul; pk.rq_add = q.rq_add;
@@ -367,6 +369,7 @@ int tc_conv2d(const void* x, const ds_planes_t* xp, const int32_t* packed, const
     // the range flag, in this call's own scratch: other calls may enqueue launches of theirs between these
     int* flag = static_cast<int*>(act);
 
+    const bool rows = !xp && H == 1 && W == 1 && g.Hp == 1 && g.Wp == 1;  // a matrix: its planes lie group by group
     TcRun p = {};
     int Hp = g.Hp, Wp = g.Wp, step_h = g.sh, step_w = g.sw;
     if (xp) {
@@ -388,6 +391,10 @@ int tc_conv2d(const void* x, const ds_planes_t* xp, const int32_t* packed, const
         p.chk_act = p.act;
         p.chk_act_bytes = (wide ? 3 : 2) * g.plane;
         TcPack pk = pack_params(q, x, a + g.planes_off, g.plane, B, C, H, W, ph, pw, g.Hp, g.Wp, g.Cp, g.sub_h, g.sub_w);
+        if (rows) {
+            pk.row_bytes = 16;
+            pk.group_bytes = 16u * unsigned(g.M);
+        }
         pk.counters = g.splits > 1 ? counters : nullptr;
         pk.ncounters = g.splits > 1 ? g.grid_m * g.grid_n : 0;
         if (mode == TC_GATED) p.gate = pk.flag = flag;
@@ -410,7 +417,8 @@ int tc_conv2d(const void* x, const ds_planes_t* xp, const int32_t* packed, const
     p.out = out;
     p.M = g.M; p.N = g.N; p.P = g.P; p.OC = g.OC; p.OW = g.OW; p.G = g.G; p.J = g.J; p.align = g.align;
     p.kh_step = unsigned(Wp) * unsigned(g.Cp);
-    p.img_bytes = unsigned(Hp) * p.kh_step;
+    p.img_bytes = rows ? 16u : unsigned(Hp) * p.kh_step;
+    p.j_step = rows ? 16u * unsigned(g.M) : 16u;
     p.row_step = unsigned(step_h) * p.kh_step;
     p.col_step = unsigned(step_w) * unsigned(g.Cp);
     if (next) {
