@@ -19,10 +19,12 @@
 //
 // What bounds it: the s8 MMA rate, 16 byte-products per shift-accumulate (8192 per SM and clock: 144 T
 // shift-op/s at 1.9 GHz).  A takes N / 2 cycles per MMA from tensor memory, whatever N; from shared memory 40 + N / 8
-// up to 128 columns, which could not carry both operands.  At 128 columns 78 to 85 % of the rate are in use (8192 x 4096 x
-// 4096: 1124 us = 122 T; 128 to 512 channels 3x3, 256 images: 260 to 268 us = 112 T, 317 to 341 before the
-// hand-shake below).  At 64 columns it is the producers: 177 instructions per item and scheduler on a pipe that takes
-// one every other cycle, 550 cycles per item where the MMAs take 256.
+// up to 128 columns, which could not carry both operands.  At 128 and 192 columns 74 to 85 % of the rate are in use (8192 x
+// 4096 x 4096: 1124 us = 122 T; 3x3 on 256 images, 64 channels 278 us = 106 T, 128 to 512 channels 253 to 257 us = 115 T).
+// Narrower tiles are bound by the producers, 177 ALU instructions per item and scheduler on a pipe that takes one every
+// other cycle (550 cycles per item of a plain tile of 64 columns, whose MMAs take 256): hence the folded windows.  Folded
+// tiles of 16 channels: 4096 images of 32 x 32, 313 us, 393 with residuals and codes; 2700 cycles for three items, of
+// which the MMAs take 576 and the ALU pipe 1440.
 #include "ds_tc.cuh"
 
 namespace ds {
@@ -35,20 +37,30 @@ constexpr int TC_TMEM_COLS = 512;
 
 // Per column width: WG producer warpgroups, each with A slots of its own (64 columns: sixteen planes x 16
 // bytes; a slot shared between warpgroups could not be guarded by a phase parity, since a warpgroup may be two
-// phases away from it), and as many accumulator slots as the remaining columns hold: two of 128 or 64 columns, so
-// that the epilogue of a tile overlaps the next tile's MMAs.
+// phases away from it), and as many accumulator slots as the remaining columns hold: at least two, so
+// that the epilogue of a tile overlaps the next tile's MMAs.  Tiles of 192, 96 and 48 columns are 64, 32 and 16 channels of
+// a folded window.
 template <int BN, bool WIDE>
 struct TcTile {
-    static constexpr int WG = WIDE ? 2 : 3;
+    static constexpr int FOLD = BN % 3 == 0 ? TC_FOLD : 1;
+    static constexpr int CH = BN / FOLD;             // channels
+    static constexpr int WG = WIDE || BN == 192 || BN == 48 ? 2 : 3;
+    // Epilogue warpgroups, which take the tiles in turn: a folded tile of 16 channels may have three items only (4096
+    // images, 32 x 32, with residual and codes: 498 -> 396 us; three and two warpgroups leave 80 registers, 819 us).
+    static constexpr int EWG = BN == 48 ? 2 : 1;
     static constexpr int PLANES = WIDE ? TC_PLANES_WIDE : TC_PLANES;
     static constexpr int ASTRIDE = WIDE ? 96 : 64;   // columns from one A slot to the next
     static constexpr int ACC = WIDE ? 2 * BN : BN;   // columns of an accumulator slot (wide: sums of weight 2^8 behind)
-    static constexpr int THREADS = (4 * WG + 6) * 32;  // + 4 epilogue warps + MMA warp + loader warp
-    static constexpr int SLOTS = (WIDE || BN == 128 ? 1 : 2) * WG;  // A slots, handed out round robin: item i fills slot i % SLOTS
+    static constexpr int THREADS = (4 * WG + 4 * EWG + 2) * 32;  // + MMA warp + loader warp
+    static constexpr int MMA_WARP = 4 * WG + 4 * EWG;
+    // A slots, handed out round robin: item i fills slot i % SLOTS
+    static constexpr int SLOTS = (WIDE || BN >= 96 ? 1 : 2) * WG;
     static constexpr int ACC_COLS = TC_TMEM_COLS - ASTRIDE * SLOTS;
-    static constexpr int NACC = ACC_COLS / ACC < 6 ? ACC_COLS / ACC : 6;
+    static constexpr int NACC = ACC_COLS / ACC < 4 ? ACC_COLS / ACC : 4;
     static constexpr int STAGE = BN * PLANES * TC_KG;
-    static constexpr int STAGES = BN == 128 ? 6 : WIDE ? 8 : 12;  // weight tiles in shared memory, more than A slots
+    // weight tiles in shared memory, more than A slots
+    static constexpr int STAGES = BN == 192 ? 4 : BN == 128 ? 6 : WIDE || BN == 96 ? 8 : 12;
+    static_assert(NACC >= 2 && NACC % EWG == 0 && STAGES > SLOTS, "slots");
 };
 
 template <int BN, bool WIDE>
@@ -62,8 +74,8 @@ struct TcSmem {
     unsigned long long done;
     unsigned tmem;
     int err;
-    int last_flag;
-    alignas(16) int colc[2][128];
+    int last_flag[2];
+    alignas(16) int colc[TcTile<BN, WIDE>::EWG][2][BN];
 };
 
 constexpr int TC_WAIT_ROUNDS = 1 << 22;    // rounds of one wait, each up to TC_WAIT_NS
@@ -200,12 +212,12 @@ __device__ __forceinline__ void tmem_st32(unsigned addr, const unsigned* v)
         : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld32(unsigned addr, int (&v)[32])
+__device__ __forceinline__ void tmem_ld(unsigned addr, int (&v)[16])
 {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
-        "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n\ttcgen05.wait::ld.sync.aligned;"
-        : TC_W4(v, 0), TC_W4(v, 4), TC_W4(v, 8), TC_W4(v, 12), TC_W4(v, 16), TC_W4(v, 20), TC_W4(v, 24), TC_W4(v, 28)
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : TC_W4(v, 0), TC_W4(v, 4), TC_W4(v, 8), TC_W4(v, 12)
         : "r"(addr)
         : "memory");
 }
@@ -259,28 +271,51 @@ __device__ __forceinline__ void planes_high(unsigned h, unsigned* v, int q)
     v[28 + q] = (h >> 7) & 0x01010101u;
 }
 
+__device__ __forceinline__ unsigned fdiv(unsigned n, FastDiv d) { return d.mul ? __umulhi(n, d.mul) >> d.sh : n; }
+
 struct Unit {
-    int tile, sp, m0, n0, nt, g0, g1;
+    int tile, sp, mt, n0, nt, g0, g1;
 };
 
-template <int BN>
+template <int CH>
 __device__ __forceinline__ Unit unit_of(const TcRun& p, int u)
 {
     Unit r;
-    r.tile = u / p.splits;
+    r.tile = int(fdiv(u, p.by_splits));
     r.sp = u - r.tile * p.splits;
-    int mt;
     if (p.m_fast) {
-        r.nt = r.tile / p.grid_m;
-        mt = r.tile - r.nt * p.grid_m;
+        r.nt = int(fdiv(r.tile, p.by_tile));
+        r.mt = r.tile - r.nt * p.grid_m;
     } else {
-        mt = r.tile / p.grid_n;
-        r.nt = r.tile - mt * p.grid_n;
+        r.mt = int(fdiv(r.tile, p.by_tile));
+        r.nt = r.tile - r.mt * p.grid_n;
     }
-    r.m0 = mt * TC_ROWS;
-    r.n0 = r.nt * BN;
+    r.n0 = r.nt * CH;
     r.g0 = r.sp * p.gps;
     r.g1 = min(p.G, r.g0 + p.gps);
+    return r;
+}
+
+// The pixel that a thread's row stands for.
+struct Pixel {
+    int b, y, x;
+    bool in;  // else the pixel is the first or last one, and the row owns no output
+};
+
+template <int FOLD>
+__device__ __forceinline__ Pixel pixel_of(const TcRun& p, int mt, int row)
+{
+    // a folded row of pixels that does not end with the warp: 30 of its 32 rows own outputs, the first and last one
+    // are their neighbours' (no exchange between warps; 32 of 32 where 32 is a multiple of W)
+    const int lane = row & 31;
+    int q = FOLD == 1 ? mt * TC_ROWS + row : (mt * 4 + (row >> 5)) * p.lanes + lane - (p.lanes < 32 ? 1 : 0);
+    Pixel r;
+    r.in = unsigned(q) < unsigned(p.rows) && (FOLD == 1 || p.lanes == 32 || (lane > 0 && lane < 31));
+    q = min(max(q, 0), p.rows - 1);
+    r.b = int(fdiv(q, p.by_image));
+    const int t = q - r.b * p.image;
+    r.y = int(fdiv(t, p.by_row));
+    r.x = t - r.y * p.RW;
     return r;
 }
 
@@ -292,76 +327,59 @@ __device__ __forceinline__ int unit_groups(const TcRun& p, int u)
     return min(p.G, g0 + p.gps) - g0;
 }
 
-__device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ void epi_bar(int group) { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); }
 
-// Epilogue of 32 columns of one row: v (the int32 sums) at row m, columns n..n+31.
-// NEXT: the finished codes also (or only, when p.out is null) go into the byte planes of the next layer -- 32
-// channels of one pixel, 32 contiguous bytes per plane and thread.
-template <bool NEXT>
-__device__ __forceinline__ void tc_store(const TcRun& p, int (&v)[32], const int* colc, int m, int n, long long rowoff,
-                                         unsigned nextoff)
+// Epilogue of CC columns of one row, in steps: each step's condition is tested once for all columns (with the conditions
+// inside the loop over the columns the epilogue of a 1x1 layer took longer than its MMAs).
+
+// The residual of columns n.. at `o0`.
+template <int CC>
+__device__ __forceinline__ void load_residual(const TcRun& p, int (&r)[CC], int live, long long o0)
 {
-    if (m >= p.M) return;
-    const int live = min(32, p.N - n);
+    const int* q = p.residual + o0;
+#pragma unroll
+    for (int c = 0; c < CC; ++c, q += p.P) r[c] = (c < live && DS_O_OK(p, p.residual, q, 4)) ? *q : 0;
+}
+
+// v: the finished sums, residual included, at the row's outputs.  NEXT: the codes also (or only, when p.out is null) go
+// into the byte planes of the next layer -- CC channels of one pixel, CC contiguous bytes per plane and thread.
+template <bool NEXT, int CC>
+__device__ __forceinline__ void tc_store(const TcRun& p, int (&v)[CC], int n, int live, long long o0, unsigned nextoff)
+{
     int* oi = static_cast<int*>(p.out);
-    // Step by step over all 32 columns, each step's condition tested once: with the conditions inside the loop over
-    // the columns the epilogue of a 1x1 layer took longer than its MMAs.
-#pragma unroll
-    for (int c = 0; c < 32; c += 4) {
-        const int4 cc = *reinterpret_cast<const int4*>(colc + c);
-        v[c] += cc.x;
-        v[c + 1] += cc.y;
-        v[c + 2] += cc.z;
-        v[c + 3] += cc.w;
-    }
-    const long long o0 = rowoff + (long long)n * p.P;
-    if (p.residual) {
-        const int* ra = p.residual + o0;
-#pragma unroll
-        for (int h = 0; h < 32; h += 16) {
-            int r[16];
-#pragma unroll
-            for (int c = 0; c < 16; ++c) {
-                const int* q = ra + (long long)(h + c) * p.P;
-                r[c] = (h + c < live && DS_O_OK(p, p.residual, q, 4)) ? *q : 0;
-            }
-#pragma unroll
-            for (int c = 0; c < 16; ++c) v[h + c] = __float2int_rn(__int2float_rn(v[h + c]) + __int2float_rn(r[c]));
-        }
-    }
     if (p.relu) {
 #pragma unroll
-        for (int c = 0; c < 32; ++c) v[c] = max(v[c], 0);
+        for (int c = 0; c < CC; ++c) v[c] = max(v[c], 0);
     }
     if (p.requant) {
 #pragma unroll
-        for (int c = 0; c < 32; ++c) v[c] = min(max(v[c], p.rq_lo), p.rq_hi) * p.rq_mul + p.rq_add;
+        for (int c = 0; c < CC; ++c) v[c] = min(max(v[c], p.rq_lo), p.rq_hi) * p.rq_mul + p.rq_add;
     }
     if (p.round_f32) {
 #pragma unroll
-        for (int c = 0; c < 32; ++c) v[c] = __float2int_rn(__int2float_rn(v[c]));
+        for (int c = 0; c < CC; ++c) v[c] = __float2int_rn(__int2float_rn(v[c]));
     }
     if (p.out) {
         if (p.out_kind == DS_OUT_F32) {
 #pragma unroll
-            for (int c = 0; c < 32; ++c) v[c] = __float_as_int(__int2float_rn(v[c]) * p.inv_scale);
+            for (int c = 0; c < CC; ++c) v[c] = __float_as_int(__int2float_rn(v[c]) * p.inv_scale);
         }
         if (p.P == 1 && (p.N & 3) == 0) {
 #pragma unroll
-            for (int c = 0; c < 32; c += 4)
+            for (int c = 0; c < CC; c += 4)
                 if (c < live && DS_O_OK(p, oi, oi + o0 + c, 16))
                     *reinterpret_cast<int4*>(oi + o0 + c) = make_int4(v[c], v[c + 1], v[c + 2], v[c + 3]);
         } else {
             int* o = oi + o0;
 #pragma unroll
-            for (int c = 0; c < 32; ++c, o += p.P)
+            for (int c = 0; c < CC; ++c, o += p.P)
                 if (c < live && DS_O_OK(p, oi, o, 4)) *o = v[c];
         }
     }
     if (NEXT) {
         unsigned char* nx = p.next + (nextoff + unsigned(n));
 #pragma unroll
-        for (int h = 0; h < 32; h += 16) {
+        for (int h = 0; h < CC; h += 16) {
             if (h >= live) break;  // N is a multiple of 16 here
             unsigned lw[4], hw[4];
 #pragma unroll
@@ -376,6 +394,56 @@ __device__ __forceinline__ void tc_store(const TcRun& p, int (&v)[32], const int
             if (DS_N_OK(p, nx + h, 16)) *reinterpret_cast<uint4*>(nx + h) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
             if (DS_N_OK(p, nx + p.next_plane + h, 16))
                 *reinterpret_cast<uint4*>(nx + p.next_plane + h) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+        }
+    }
+}
+
+template <int CC>
+__device__ __forceinline__ void add_residual(int (&v)[CC], const int (&r)[CC])
+{
+#pragma unroll
+    for (int c = 0; c < CC; ++c) v[c] = __float2int_rn(__int2float_rn(v[c]) + __int2float_rn(r[c]));
+}
+
+// CC channels' sums of one row: `acc(col, v)` gives the raw sums of CC columns.  colc: the constants of the tile's
+// channels; for a folded window those of all three columns together, then minus those of the left and right one, which
+// stand in where the row's neighbour is not part of the image.
+template <int CH, int FOLD, int CC, class Acc>
+__device__ __forceinline__ void row_sums(int (&v)[CC], const int* colc, int c, bool left, bool right, Acc acc)
+{
+    acc(FOLD == 1 ? c : CH + c, v);
+    auto add = [&](const int (&w)[CC]) {
+#pragma unroll
+        for (int q = 0; q < CC; ++q) v[q] += w[q];
+    };
+    int w[CC];
+    auto consts = [&](int at) {
+#pragma unroll
+        for (int q = 0; q < CC; q += 4) {
+            const int4 cc = *reinterpret_cast<const int4*>(colc + at + q);
+            w[q] = cc.x;
+            w[q + 1] = cc.y;
+            w[q + 2] = cc.z;
+            w[q + 3] = cc.w;
+        }
+    };
+    consts(c);
+    add(w);
+    if (FOLD > 1) {
+        int t[CC];
+        acc(c, t);
+        consts(CH + c);
+#pragma unroll
+        for (int q = 0; q < CC; ++q) {
+            const int z = __shfl_up_sync(0xFFFFFFFFu, t[q], 1);
+            v[q] += left ? z : w[q];
+        }
+        acc(2 * CH + c, t);
+        consts(2 * CH + c);
+#pragma unroll
+        for (int q = 0; q < CC; ++q) {
+            const int z = __shfl_down_sync(0xFFFFFFFFu, t[q], 1);
+            v[q] += right ? z : w[q];
         }
     }
 }
@@ -404,7 +472,7 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
         bar_init(&s.done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 4 * T::WG + 4) {
+    if (warp == T::MMA_WARP) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(&s.tmem)), "n"(TC_TMEM_COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
@@ -428,16 +496,14 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
         // Unit u, `skip` groups in; units too short for that are passed over.
         auto enter = [&](int skip) {
             for (; u < p.units; u += gridDim.x) {
-                const Unit un = unit_of<BN>(p, u);
+                const Unit un = unit_of<T::CH>(p, u);
                 g = un.g0 + skip;
                 g1 = un.g1;
                 if (g < g1) {
                     kh = g / p.J;
                     j = g - kh * p.J;
-                    const int m = min(un.m0 + row, p.M - 1);
-                    const int b = m / p.P, pp = m - b * p.P;
-                    const int oh = pp / p.OW, ow = pp - oh * p.OW;
-                    roff = unsigned(b) * p.img_bytes + unsigned(oh) * p.row_step + unsigned(ow) * p.col_step;
+                    const Pixel px = pixel_of<T::FOLD>(p, un.mt, row);
+                    roff = unsigned(px.b) * p.img_bytes + unsigned(px.y) * p.row_step + unsigned(px.x) * p.col_step;
                     return;
                 }
                 skip = g - g1;
@@ -470,6 +536,10 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
             const uint4 l = nl, h = nh, t = nt;
             step();
             if (u < p.units) fetch();
+            constexpr int PER = T::SLOTS / T::WG;  // slots of this warpgroup, used in turn
+            const unsigned slot = wg + T::WG * (round % PER), use = round / PER;
+            const unsigned at = tmem_a + lane_base + slot * T::ASTRIDE;
+            ++round;
             unsigned v[64];
             planes_low(l.x, h.x, v, 0);
             planes_low(l.y, h.y, v, 1);
@@ -481,109 +551,148 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
             planes_high(h.w, v + 32, 3);
             // One hand-shake per 16 values (two, a slot per eight planes, cost a third of the rate at 128 columns),
             // and nothing but the stores between the slot's release and its hand-over.
-            constexpr int PER = T::SLOTS / T::WG;  // slots of this warpgroup, used in turn
-            const unsigned slot = wg + T::WG * (round % PER), use = round / PER;
             const bool ok = use == 0 || bar_wait(&s.empty[slot], (use - 1) & 1u, err, p.wait_ns);
-            ++round;
             if (!__all_sync(0xFFFFFFFFu, ok) || TC_HELD(p, 2)) break;  // the whole warp, or none of it
             tc_fence_after();
-            tmem_st32(tmem_a + lane_base + slot * T::ASTRIDE, v);
-            tmem_st32(tmem_a + lane_base + slot * T::ASTRIDE + 32, v + 32);
+            tmem_st32(at, v);
+            tmem_st32(at + 32, v + 32);
             if (WIDE) {
                 const unsigned w[16] = {t.x, t.y, t.z, t.w, t.x, t.y, t.z, t.w, t.x, t.y, t.z, t.w, t.x, t.y, t.z, t.w};
-                tmem_st16(tmem_a + lane_base + slot * T::ASTRIDE + 64, w);
+                tmem_st16(at + 64, w);
             }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             tc_fence_before();
             __syncwarp();
             if (lane == 0) bar_arrive(&s.full[slot]);
         }
-    } else if (warp < 4 * T::WG + 4) {
+    } else if (warp < T::MMA_WARP) {
         // ---- epilogue ----------------------------------------------------------------------------------
+        constexpr int CC = 16;  // channels at a time: their sums, up to two neighbours', constants and residuals in registers
         const int row = threadIdx.x & 127;
         const unsigned lane_base = unsigned(warp & 3) << 21;
-        auto next_offset = [&](int b, int pp) -> unsigned {
-            if (!NEXT) return 0;
-            const int oh = pp / p.OW;
-            return unsigned(b) * p.next_img + unsigned(oh) * p.next_row + unsigned(pp - oh * p.OW) * p.next_px;
-        };
-        unsigned acc = 0;
-        int par = 0;
+        const int eg = (warp - 4 * T::WG) >> 2;  // this epilogue warpgroup
+        unsigned acc = unsigned(eg);             // units of this CTA before this one
+        int par = 0, nt = -1;
         // A warp whose wait gives up walks on without the unit's sums: the named barriers below need all four.
-        for (int u = blockIdx.x; u < p.units; u += gridDim.x, ++acc, par ^= 1) {
-            const Unit un = unit_of<BN>(p, u);
-            // column constants of this tile; two copies, so a slow warp still reads the previous tile's
-            if (row < BN) {
-                const int n = un.n0 + row;
-                s.colc[par][row] = n < p.N ? __ldg(p.colc + n) + (p.bias ? __ldg(p.bias + n) : 0) : 0;
+        for (int u = blockIdx.x + eg * gridDim.x; u < p.units; u += T::EWG * gridDim.x, acc += T::EWG) {
+            const Unit un = unit_of<T::CH>(p, u);
+            if (un.nt != nt) {
+                // column constants of these channels; two copies, so a slow warp still reads the previous ones
+                nt = un.nt;
+                par ^= 1;
+                if (row < T::CH) {
+                    const int n = un.n0 + row;
+                    int c = 0, l = 0, r = 0;
+                    if (n < p.N) {
+                        c = __ldg(p.colc + n) + (p.bias ? __ldg(p.bias + n) : 0);
+                        if (T::FOLD > 1) {
+                            l = __ldg(p.colc + p.N + n);
+                            r = __ldg(p.colc + 2 * p.N + n);
+                        }
+                    }
+                    s.colc[eg][par][row] = c;
+                    if (T::FOLD > 1) {
+                        s.colc[eg][par][T::CH + row] = l;
+                        s.colc[eg][par][2 * T::CH + row] = r;
+                    }
+                }
+                epi_bar(eg);
             }
-            epi_bar();
+            const Pixel px = pixel_of<T::FOLD>(p, un.mt, row);
+            const int ox = T::FOLD > 1 ? px.x + p.pw1 : px.x;
+            const bool in = px.in && (T::FOLD == 1 || unsigned(ox) < unsigned(p.OW));
+            const bool left = px.x > 0, right = px.x + 1 < p.RW;
+            const long long rowoff = (long long)px.b * p.OC * p.P + px.y * p.OW + ox;
+            const unsigned nextoff = NEXT ? unsigned(px.b) * p.next_img + unsigned(px.y) * p.next_row + unsigned(ox) * p.next_px : 0u;
             const unsigned slot = acc % T::NACC;
+            int res[CC];
+            // the residual is fetched ahead: of the first columns while the sums are still being made
+            auto fetch = [&](int c) {
+                const int n = un.n0 + c;
+                if (p.residual && in && n < p.N) load_residual(p, res, p.N - n, rowoff + (long long)n * p.P);
+            };
+            auto finish = [&](int c, auto get) {
+                int v[CC];
+                row_sums<T::CH, T::FOLD>(v, s.colc[eg][par], c, left, right, get);
+                const int n = un.n0 + c;
+                if (p.residual) add_residual(v, res);
+                if (c + CC < T::CH) fetch(c + CC);
+                if (in && n < p.N) tc_store<NEXT>(p, v, n, p.N - n, rowoff + (long long)n * p.P, nextoff);
+            };
+            if (p.splits == 1) fetch(0);
             if (__all_sync(0xFFFFFFFFu, bar_wait(&s.accfull[slot], (acc / T::NACC) & 1u, err, p.wait_ns))) {
                 tc_fence_after();
-                const int m = un.m0 + row;
-                const int b = m / p.P, pp = m - b * p.P;
-                const long long rowoff = (long long)b * p.OC * p.P + pp;
-                const unsigned nextoff = next_offset(b, pp);
-#pragma unroll 1
-                for (int c = 0; c < BN; c += 32) {
-                    int v[32];
-                    tmem_ld32(tmem + lane_base + slot * T::ACC + c, v);
+                const unsigned base = tmem + lane_base + slot * T::ACC;
+                auto sums = [&](int c, int (&v)[CC]) {
+                    tmem_ld(base + c, v);
                     if (WIDE) {
-                        int w[32];
-                        tmem_ld32(tmem + lane_base + slot * T::ACC + BN + c, w);
+                        int w[CC];
+                        tmem_ld(base + BN + c, w);
 #pragma unroll
-                        for (int q = 0; q < 32; ++q) v[q] += int(unsigned(w[q]) << 8);
+                        for (int q = 0; q < CC; ++q) v[q] += int(unsigned(w[q]) << 8);
                     }
-                    if (c + 32 >= BN) {
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0 && !TC_HELD(p, 4)) bar_arrive(&s.accempty[slot]);
-                    }
-                    if (p.splits == 1) {
-                        tc_store<NEXT>(p, v, &s.colc[par][c], m, un.n0 + c, rowoff, nextoff);
-                    } else {
-                        int* dst = p.partials + (long long)(un.tile * p.splits + un.sp) * (BN * TC_ROWS) +
-                                   c * TC_ROWS + row;
+                };
+                auto release = [&]() {  // the accumulators have been read
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0 && !TC_HELD(p, 4)) bar_arrive(&s.accempty[slot]);
+                };
+                if (p.splits == 1) {
+#pragma unroll 1
+                    for (int c = 0; c < T::CH; c += CC)
+                        finish(c, [&](int col, int (&v)[CC]) {
+                            sums(col, v);
+                            if (col + CC == BN) release();
+                        });
+                } else {
+#pragma unroll 1
+                    for (int c = 0; c < BN; c += CC) {
+                        int v[CC];
+                        sums(c, v);
+                        if (c + CC == BN) release();
+                        int* dst = p.partials + (long long)(un.tile * p.splits + un.sp) * (BN * TC_ROWS) + c * TC_ROWS + row;
 #pragma unroll
-                        for (int q = 0; q < 32; ++q) __stcg(dst + q * TC_ROWS, v[q]);
+                        for (int q = 0; q < CC; ++q) __stcg(dst + q * TC_ROWS, v[q]);
                     }
                 }
             }
             if (p.splits > 1) {
                 // the split that arrives last adds all partial sums in order and applies the epilogue
                 __threadfence();
-                epi_bar();
-                if (row == 0) s.last_flag = atomicAdd(p.counters + un.tile, 1) == p.splits - 1;
-                epi_bar();
-                if (s.last_flag) {
+                epi_bar(eg);
+                if (row == 0) s.last_flag[eg] = atomicAdd(p.counters + un.tile, 1) == p.splits - 1;
+                epi_bar(eg);
+                if (s.last_flag[eg]) {
+                    constexpr int KU = BN == 96 ? 1 : T::FOLD > 1 ? 2 : 3;
                     __threadfence();
                     if (row == 0) p.counters[un.tile] = 0;  // for the next launch
-                    {
-                        const int m = un.m0 + row;
-                        const int b = m / p.P, pp = m - b * p.P;
-                        const long long rowoff = (long long)b * p.OC * p.P + pp;
-                        const unsigned nextoff = next_offset(b, pp);
+                    fetch(0);
 #pragma unroll 1
-                        for (int c = 0; c < BN; c += 32) {
-                            int v[32];
+                    for (int c = 0; c < T::CH; c += CC)
+                        finish(c, [&](int col, int (&v)[CC]) {
 #pragma unroll
-                            for (int q = 0; q < 32; ++q) v[q] = 0;
+                            for (int q = 0; q < CC; ++q) v[q] = 0;
 #pragma unroll 1
-                            for (int k = 0; k < p.splits; ++k) {
-                                const int* src = p.partials + (long long)(un.tile * p.splits + k) * (BN * TC_ROWS) +
-                                                 c * TC_ROWS + row;
+                            for (int k = 0; k < p.splits; k += KU) {  // KU loads of each column in flight
+                                int t[KU][CC];
 #pragma unroll
-                                for (int q = 0; q < 32; ++q) v[q] += __ldcg(src + q * TC_ROWS);
+                                for (int j = 0; j < KU; ++j) {
+                                    const int* src = p.partials + (long long)(un.tile * p.splits + k + j) * (BN * TC_ROWS) +
+                                                     col * TC_ROWS + row;
+#pragma unroll
+                                    for (int q = 0; q < CC; ++q) t[j][q] = k + j < p.splits ? __ldcg(src + q * TC_ROWS) : 0;
+                                }
+#pragma unroll
+                                for (int j = 0; j < KU; ++j)
+#pragma unroll
+                                    for (int q = 0; q < CC; ++q) v[q] += t[j][q];
                             }
-                            tc_store<NEXT>(p, v, &s.colc[par][c], m, un.n0 + c, rowoff, nextoff);
-                        }
-                    }
+                        });
                 }
-                epi_bar();  // last_flag is read by all before the next unit writes it
+                epi_bar(eg);  // last_flag is read by all before the next unit writes it
             }
         }
-    } else if (warp == 4 * T::WG + 4) {
+    } else if (warp == T::MMA_WARP) {
         // ---- MMA issue ---------------------------------------------------------------------------------
         // One elected lane walks the whole loop.  Its instructions are in one queue with the MMAs and, on its
         // scheduler, with the producers' stores to tensor memory: a wait costs 150 to 300 cycles even when what it
@@ -650,7 +759,7 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
             auto fetch = [&]() {
                 while (lleft == 0) {
                     if (lu >= p.units || TC_HELD(p, 1)) return;
-                    const Unit un = unit_of<BN>(p, lu);
+                    const Unit un = unit_of<T::CH>(p, lu);
                     src = p.wexp + ((long long)un.nt * p.G + un.g0) * T::STAGE;
                     lleft = un.g1 - un.g0;
                     lu += gridDim.x;
@@ -700,7 +809,7 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == 4 * T::WG + 4)
+    if (warp == T::MMA_WARP)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(TC_TMEM_COLS));
     if (threadIdx.x == 0 && s.err) *p.err_flag = 1;
 }
@@ -758,7 +867,7 @@ constexpr int TC_KEEP_WAIT = 1 << 22;  // rounds of at least 64 ns
 struct ExpandSmem {
     unsigned lut[6][33];
     int stale;
-    alignas(16) unsigned char codes[128 * 16];
+    alignas(16) unsigned char codes[192 * 16];
 };
 
 // Block (nt, g): the operand tile of group g, columns nt * BN.. -- [16 planes][BN][16 bytes].  A thread makes
@@ -766,30 +875,46 @@ struct ExpandSmem {
 // Blocks g = G.. compute the column constants -sum s 2^(15-r).
 __device__ __forceinline__ void expand_block(const TcExpand& p, int nt, int g, ExpandSmem& sm)
 {
-    const int n0 = nt * p.BN;
+    const int ch = p.BN / p.fold, n0 = nt * ch;
     const unsigned fmask = (1u << p.dec.fw) - 1u;
     if (g >= p.G) {
-        const int per = p.BN / TC_COLC_BLOCKS;  // 2, 4 or 8 columns: one per warp
+        // 1, 2, 4 or 8 channels, one per warp
+        const int per = ch / TC_COLC_BLOCKS;
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
         const int n = n0 + (g - p.G) * per + warp;
         if (warp >= per || n >= p.N) return;
         const int* src = p.packed + (long long)n * p.dec.row_len;
-        unsigned sum = 0;
+        unsigned sum = 0, first = 0, last = 0;  // folded: those of the window's first and last column apart
         bool far = false;
         for (int w = lane; w < p.dec.row_len; w += 32) {
             unsigned word = DS_W_OK(p, src + w, 4) ? unsigned(__ldg(src + w)) : 0u;
             const int k = w * p.dec.num;
+            int kw = p.fold > 1 ? k % p.KW : 1;
             for (int i = 0; i < p.dec.num && k + i < p.K; ++i, word >>= p.dec.fw) {
                 const int c = tc_code(p, word & fmask);
                 if (c < 32) {
                     if (p.wide) far |= (word & fmask & ((1u << p.dec.bits) - 1u)) >= 16u;
-                    const unsigned v = 1u << ((p.wide ? 23 : 15) - (c & 15));
-                    sum += (c & 16) ? v : 0u - v;
+                    const unsigned v = 1u << ((p.wide ? 23 : 15) - (c & 15)), s = (c & 16) ? v : 0u - v;
+                    sum += s;
+                    if (kw == 0) first += s;
+                    if (kw == 2) last += s;
                 }
+                if (p.fold > 1 && ++kw == p.KW) kw = 0;
             }
         }
 #pragma unroll
         for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+        if (p.fold > 1) {
+#pragma unroll
+            for (int o = 16; o; o >>= 1) {
+                first += __shfl_xor_sync(0xFFFFFFFFu, first, o);
+                last += __shfl_xor_sync(0xFFFFFFFFu, last, o);
+            }
+            if (lane == 0) {
+                p.colc[p.N + n] = -int(first);
+                p.colc[2 * p.N + n] = -int(last);
+            }
+        }
         if (p.wide && __any_sync(0xFFFFFFFFu, far) && lane == 0) {
             p.colc[p.N] = 1;
             if (p.range_flag) *p.range_flag = 1;
@@ -800,23 +925,25 @@ __device__ __forceinline__ void expand_block(const TcExpand& p, int nt, int g, E
     for (int i = threadIdx.x; i < 6 * 33; i += 256) (&sm.lut[0][0])[i] = g_tc_lut.w[i];
     // a thread keeps its place in the group (and with it the word and the bit position) and walks the columns
     const int kh = g / p.J, j = g - kh * p.J;
-    const int t = 16 * j + (threadIdx.x & 15);  // byte of the window row: (kw, c)
-    const int kw = t / p.Cp, c = t - kw * p.Cp;
-    const bool live = kw < p.KW && c < p.C;
-    const int k = (c * p.KH + kh) * p.KW + kw;
-    const int w = k / p.dec.num, at = (k - w * p.dec.num) * p.dec.fw;
+    const int t = 16 * j + (threadIdx.x & 15);  // byte of the window row: (kw, c), or c of a folded window
     const int nl0 = threadIdx.x >> 4;
-    const int* src = p.packed + (long long)(n0 + nl0) * p.dec.row_len + w;
+    for (int f = 0; f < p.fold; ++f) {
+        const int kw = p.fold > 1 ? f : t / p.Cp, c = p.fold > 1 ? t : t - kw * p.Cp;
+        const bool live = kw < p.KW && c < p.C;
+        const int k = (c * p.KH + kh) * p.KW + kw;
+        const int w = k / p.dec.num, at = (k - w * p.dec.num) * p.dec.fw;
+        const int* src = p.packed + (long long)(n0 + nl0) * p.dec.row_len + w;
 #pragma unroll 8
-    for (int nl = nl0; nl < p.BN; nl += 16, src += 16ll * p.dec.row_len) {
-        int code = 32;
-        if (live && n0 + nl < p.N && DS_W_OK(p, src, 4)) code = tc_code(p, (unsigned(__ldg(src)) >> at) & fmask);
-        sm.codes[nl * 16 + (threadIdx.x & 15)] = (unsigned char)code;
+        for (int nl = nl0; nl < ch; nl += 16, src += 16ll * p.dec.row_len) {
+            int code = 32;
+            if (live && n0 + nl < p.N && DS_W_OK(p, src, 4)) code = tc_code(p, (unsigned(__ldg(src)) >> at) & fmask);
+            sm.codes[(f * ch + nl) * 16 + (threadIdx.x & 15)] = (unsigned char)code;
+        }
     }
     __syncthreads();
     uint4* out = reinterpret_cast<uint4*>(p.wexp + ((long long)nt * p.G + g) * (p.BN * (p.wide ? TC_PLANES_WIDE : TC_PLANES) * TC_KG));
     for (int i = threadIdx.x; i < p.BN * (p.wide ? 6 : 4); i += 256) {
-        const int n = i & (p.BN - 1), q = i / p.BN;
+        const int q = i / p.BN, n = i - q * p.BN;
         const uint4 cw = *reinterpret_cast<const uint4*>(sm.codes + n * 16);
         const unsigned cws[4] = {cw.x, cw.y, cw.z, cw.w};
         unsigned o[4][4];  // [plane][word]
@@ -874,7 +1001,7 @@ __device__ __forceinline__ void keep_compare(const TcExpand& p, unsigned block)
         }
     }
     if (differs) {
-        p.colc[p.N] = 0;  // found again, if it holds, when the tiles are made
+        if (p.wide) p.colc[p.N] = 0;  // found again, if it holds, when the tiles are made
         p.state[0] = 1;
     }
     __threadfence();
@@ -1159,11 +1286,23 @@ int tc_launch_expand(const TcExpand& p, cudaStream_t st)
     return cudaGetLastError() == cudaSuccess ? DS_OK : DS_ERR_CUDA;
 }
 
+template <bool NEXT>
+static int launch_run(const TcRun& p, int BN, cudaStream_t st)
+{
+    switch (BN) {
+        case 192: return run_cfg<192, NEXT, false>(p, st);
+        case 128: return run_cfg<128, NEXT, false>(p, st);
+        case 96: return run_cfg<96, NEXT, false>(p, st);
+        case 64: return run_cfg<64, NEXT, false>(p, st);
+        case 48: return run_cfg<48, NEXT, false>(p, st);
+        default: return run_cfg<32, NEXT, false>(p, st);
+    }
+}
+
 int tc_launch_run(const TcRun& p, int BN, bool wide, cudaStream_t st)
 {
     if (wide) return run_cfg<64, false, true>(p, st);
-    if (p.next) return BN == 128 ? run_cfg<128, true, false>(p, st) : BN == 64 ? run_cfg<64, true, false>(p, st) : run_cfg<32, true, false>(p, st);
-    return BN == 128 ? run_cfg<128, false, false>(p, st) : BN == 64 ? run_cfg<64, false, false>(p, st) : run_cfg<32, false, false>(p, st);
+    return p.next ? launch_run<true>(p, BN, st) : launch_run<false>(p, BN, st);
 }
 
 }  // namespace ds

@@ -41,6 +41,19 @@ constexpr int TC_COLC_BLOCKS = 16;  // expansion blocks per column tile that com
 constexpr int TC_HEADER = 2048;
 constexpr int TC_MAX_SPLIT_TILES = (TC_HEADER - 16) / 4;
 
+// Division of n < 2^31 by a constant of the call: (n * mul >> 32) >> sh, mul = ceil(2^(31 + l) / d), l = ceil(log2 d).
+// Exact, since n (mul d - 2^(31 + l)) < 2^31 * 2^l.  mul = 0 stands for d = 1.
+struct FastDiv {
+    unsigned mul;
+    int sh;
+};
+
+// Folded windows.  A convolution whose columns move by one pixel (stride 1 along W) may multiply a pixel's channels by
+// the weights of all KW window columns at once: KW times as many columns, a KW-th of the items, and out[x] is the sum of
+// column block kw at pixel x + kw - (KW - 1) / 2, which the epilogue fetches from the neighbouring lanes.  An item costs
+// the producers 177 ALU instructions per scheduler whatever the columns are, so below 128 columns this is what counts.
+constexpr int TC_FOLD = 3;
+
 // Geometry and tiling of one call; a pure function of its arguments (weights expanded for a geometry
 // fit every later call of the same geometry).
 struct TcGeom {
@@ -52,7 +65,11 @@ struct TcGeom {
     int align;           // every load starts at a multiple of this: 16, 8 or 4
     long long plane;     // bytes of one byte plane
     int wide;            // 24-bit codes: three byte planes
-    int BN;              // tile: 128 rows, BN columns
+    int fold;            // window columns side by side in a tile: 1, or KW for a folded window
+    int BN;              // tile: 128 rows, BN columns = fold * channels
+    int RW;              // pixels along W that rows stand for: OW, or W for a folded window
+    int lanes;           // rows of a warp that own outputs: 32, or 30 where a warp's first and last only lend theirs
+    long long rows;      // B * OH * RW
     int grid_m, grid_n, splits, gps;  // gps: groups per split
     long long act_bytes;      // scratch of one call: header, partial sums, both planes
     long long planes_off;
@@ -69,6 +86,10 @@ struct TcRun {
     const int* residual;
     void* out;
     int M, N, P, OC, OW, G, J, align;
+    int rows, RW, lanes, pw1;  // as in TcGeom; pw - 1 of a folded window
+    int image;                 // OH * RW
+    FastDiv by_image, by_row;  // image, RW
+    FastDiv by_splits, by_tile;  // splits; grid_m (m_fast) or grid_n
     unsigned img_bytes, row_step, col_step, kh_step, j_step;  // byte offsets inside a plane
     int grid_m, grid_n, splits, gps, units, m_fast;
     // byte planes of the layer that reads this output (null: none); `next` is the pixel (0, 0, 0) of the l plane
@@ -119,7 +140,7 @@ struct TcExpand {
     unsigned char* wexp;
     int* colc;
     Decode dec;
-    int C, KH, KW, Cp, J, G, N, K, BN;
+    int C, KH, KW, Cp, J, G, N, K, BN, fold;
     int wide;            // 22 planes; colc[N] is set when a weight has a shift of 16..31
     int total;           // blocks of work: (G + TC_COLC_BLOCKS) per column tile
     // A kept buffer, looked after by blocks of the packing launch (tc_keep_*):

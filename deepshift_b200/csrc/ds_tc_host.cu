@@ -15,32 +15,66 @@ int g_hold = 0;
 
 long long round16(long long v) { return (v + 15) & ~15ll; }
 
+FastDiv fast_div(unsigned d)
+{
+    int l = 0;
+    while (l < 31 && (1u << l) < d) ++l;
+    if (l == 0) return {0u, 0};
+    return {unsigned(((1ull << (31 + l)) + d - 1) / d), l - 1};
+}
+
 // Bytes per pixel and plane, and the groups per window row that follow.  The (kw, c) run of one window row
 // is contiguous (KW * Cp bytes), so only its end is padded to 16; Cp a multiple of 4, 8 or 16 decides how
-// wide the loads are.  Fewest groups first, then the widest loads.
-void choose_pixel(TcGeom& g)
+// wide the loads are.  Fewest groups first, then the widest loads.  Of a folded window an item holds one pixel's channels.
+void choose_pixel(TcGeom& g, int fold)
 {
     int best_j = 1 << 30;
     for (int a = 16; a >= 4; a >>= 1) {
         const int cp = (g.C + a - 1) / a * a;
-        const int j = (g.KW * cp + 15) / 16;
+        const int j = ((fold > 1 ? 1 : g.KW) * cp + 15) / 16;
         if (j < best_j) {
             best_j = j;
             g.Cp = cp;
         }
     }
+    g.fold = fold;
     g.J = best_j;
     g.G = g.KH * g.J;
     g.align = 16;
     // offsets are sums of multiples of Cp * sw, of the row pitch Wp * Cp and of 16
     while (g.align > 4 && ((g.Cp * g.sw) % g.align || ((long long)g.Wp * g.Cp) % g.align)) g.align >>= 1;
+    g.RW = fold > 1 ? g.W : g.OW;
+    g.lanes = fold > 1 && 32 % g.W ? 30 : 32;
+    g.rows = (long long)g.B * g.OH * g.RW;
 }
 
-// Clock cycles of one (group, 128 rows) item: eight MMAs (eleven when wide).
+// Clock cycles of one (group, 128 rows) item: the MMAs at 192 and 128 columns (768 and 512), the producers below.
 double item_cycles(int bn, bool wide)
 {
     if (wide) return 1000;
-    return bn == 128 ? 700 : bn == 64 ? 520 : 480;
+    return bn == 192 ? 800 : bn == 128 ? 700 : bn == 64 ? 520 : 480;
+}
+
+const int kTiles[2][3] = {{128, 64, 32}, {192, 96, 48}};  // columns: plain, folded
+
+// Whether a tile of bn columns is one for this layer: not half of it empty.
+bool tile_fits(const TcGeom& g, int bn)
+{
+    return g.wide ? bn == 64 : bn == kTiles[g.fold > 1][2] || g.N > bn / g.fold / 2;
+}
+
+// Cycles that 128 pixels of a long run take with the best tile.
+double cycles_per_block(const TcGeom& g)
+{
+    double best = 1e30;
+    for (int bn : kTiles[g.fold > 1]) {
+        if (!tile_fits(g, bn)) continue;
+        const int ch = bn / g.fold;
+        const double item = bn == 128 ? 560 : bn == 192 ? 780 : item_cycles(bn, false);
+        const double c = double((g.N + ch - 1) / ch) * (g.G * item + (g.fold > 1 ? 1000 : 300)) * 32 / g.lanes;
+        if (c < best) best = c;
+    }
+    return best;
 }
 
 // Tile and split with the smallest estimated time: waves of units over the SMs, a unit being the longer of
@@ -48,11 +82,11 @@ double item_cycles(int bn, bool wide)
 void choose_tile(TcGeom& g)
 {
     double best = 1e30;
-    const int bns[3] = {128, 64, 32};
-    for (int bn : bns) {
-        if (g.wide ? bn != 64 : bn > 32 && g.N <= bn / 2) continue;
-        const long long gm = (g.M + TC_ROWS - 1ll) / TC_ROWS, gn = (g.N + bn - 1) / bn;
-        const double epi = TC_ROWS * (double)bn * 4 / 23;
+    for (int bn : kTiles[g.fold > 1]) {
+        if (!tile_fits(g, bn)) continue;
+        const int ch = bn / g.fold;
+        const long long gm = (g.rows + 4ll * g.lanes - 1) / (4 * g.lanes), gn = (g.N + ch - 1) / ch;
+        const double epi = TC_ROWS * (double)ch * 4 / 23;
         for (int sp = 1; sp <= 16; ++sp) {
             const int gps = (g.G + sp - 1) / sp;
             if (sp > 1 && (gps < 4 || (g.G + gps - 1) / gps != sp)) continue;
@@ -107,17 +141,29 @@ int tc_geometry(TcGeom& g, int B, int C, int H, int W, int OC, int KH, int KW, i
     if (pixels > limit || M > limit) return DS_ERR_UNSUPPORTED;
     g.Hp = int(hp); g.Wp = int(wp); g.OH = int(oh); g.OW = int(ow);
     g.M = int(M); g.K = int(K); g.N = OC; g.P = int(oh * ow);
-    choose_pixel(g);
+    choose_pixel(g, 1);
+    // A folded window's rows are the pixels of an image row, its outputs at most as many.  Folded where a long run is not
+    // slower, whatever the batch: a layer's weights then have three layouts at most.  Measured, us, plain -> folded:
+    // 64 channels 56 x 56, 256 images 447 -> 278, one 14.8 -> 10.8; 32 channels 16 x 16, 4096 images 314 -> 160; 16 channels
+    // 32 x 32 679 -> 313; 256 channels 14 x 14, 256 images 268 -> 258, 64 images 95 -> 74 (finer units), one 18.2 -> 14.8;
+    // 512 channels 7 x 7 263 -> 253, 96 -> 83, 22.9 -> 19.0.  128 channels 28 x 28: 257 -> 264, 78 -> 76, 14.9 -> 12.8; layers
+    // that one plain tile of 128 columns covers stay plain.
+    if (KW == TC_FOLD && g.sw == 1 && pw <= 1 && (OC <= 64 || OC > 128)) {
+        TcGeom f = g;
+        choose_pixel(f, TC_FOLD);
+        if (f.rows <= limit && pixels * f.Cp <= limit && OC <= 65535 * 16 && cycles_per_block(f) < 1.05 * cycles_per_block(g))
+            g = f;
+    }
+    choose_tile(g);
     if (pixels * g.Cp > limit) return DS_ERR_UNSUPPORTED;
     g.plane = round16(pixels * g.Cp + 16);  // the last group of a window row may read up to 15 bytes beyond it
-    choose_tile(g);
     const long long tiles = (long long)g.grid_m * g.grid_n;
     if (tiles * g.splits > limit || g.grid_n > 65535) return DS_ERR_UNSUPPORTED;
     if (g.splits > 1 && tiles > TC_MAX_SPLIT_TILES) return DS_ERR_UNSUPPORTED;
     g.planes_off = TC_HEADER + (g.splits > 1 ? tiles * g.splits * TC_ROWS * g.BN * 4 : 0);
     g.act_bytes = g.planes_off + (wide ? 3 : 2) * g.plane;
     g.colc_off = (long long)g.grid_n * g.G * g.BN * (wide ? TC_PLANES_WIDE : TC_PLANES) * TC_KG;
-    g.state_off = g.colc_off + round16(4ll * g.N + 4);  // the word behind: a shift of 16..31 exists (wide)
+    g.state_off = g.colc_off + round16(4ll * g.fold * g.N + 4);  // the word behind: a shift of 16..31 exists (wide)
     g.words_off = g.state_off + 16;
     const int num = 32 / (bits + 1);
     g.weight_bytes = g.words_off + round16(4ll * g.N * ((g.K + num - 1) / num));
@@ -225,7 +271,7 @@ extern "C" int ds_tc_columns(int B, int C, int H, int W, int OC, int KH, int KW,
     if (!fuse || tc_mode(*fuse, bits, base) == TC_NO ||
         tc_geometry(g, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, bits, fuse->in_kind == DS_IN_F32_LINEAR) != DS_OK)
         return 0;
-    return g.BN;
+    return g.BN;  // the folded widths are none of the plain ones
 }
 
 namespace ds {
@@ -246,6 +292,7 @@ TcExpand expand_params(const TcGeom& g, const int32_t* packed, int bits, void* w
     p.dec.base = 0;
     p.dec.row_len = (g.K + p.dec.num - 1) / p.dec.num;
     p.C = g.C; p.KH = g.KH; p.KW = g.KW; p.Cp = g.Cp; p.J = g.J; p.G = g.G; p.N = g.N; p.K = g.K; p.BN = g.BN;
+    p.fold = g.fold;
     p.wide = g.wide;
     p.nwords = (long long)g.N * p.dec.row_len;
     p.chk_w_bytes = p.nwords * 4;
@@ -416,6 +463,11 @@ int tc_conv2d(const void* x, const ds_planes_t* xp, const int32_t* packed, const
     p.residual = fuse->residual;
     p.out = out;
     p.M = g.M; p.N = g.N; p.P = g.P; p.OC = g.OC; p.OW = g.OW; p.G = g.G; p.J = g.J; p.align = g.align;
+    p.rows = int(g.rows); p.RW = g.RW; p.lanes = g.lanes; p.pw1 = pw - 1;
+    p.image = g.OH * g.RW;
+    p.by_image = fast_div(unsigned(p.image));
+    p.by_row = fast_div(unsigned(g.RW));
+    if (g.fold > 1) p.act += (long long)pw * g.Cp;  // rows are pixels, not windows
     p.kh_step = unsigned(Wp) * unsigned(g.Cp);
     p.img_bytes = rows ? 16u : unsigned(Hp) * p.kh_step;
     p.j_step = rows ? 16u * unsigned(g.M) : 16u;
@@ -443,6 +495,8 @@ int tc_conv2d(const void* x, const ds_planes_t* xp, const int32_t* packed, const
     // neighbouring CTAs share the smaller operand's tiles through L2: rows fastest when the weights are the
     // larger one
     p.m_fast = g.colc_off > 2 * g.plane;
+    p.by_splits = fast_div(unsigned(g.splits));
+    p.by_tile = fast_div(unsigned(p.m_fast ? g.grid_m : g.grid_n));
     p.counters = counters;
     p.partials = reinterpret_cast<int*>(a + TC_HEADER);
     p.out_kind = q.out_kind; p.relu = q.relu; p.requant = q.requant; p.round_f32 = q.round_f32;

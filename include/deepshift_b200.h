@@ -291,7 +291,8 @@ int ds_conv2d_prepare(const int32_t *packed, int B, int C, int H, int W, int OC,
  *                 layout has filled, ordered before this one: it is compared on the device with the packed words as
  *                 they are now and made again if they differ, so it never goes stale.  Calls that may overlap on the
  *                 GPU need buffers of their own.
- * ds_tc_columns   columns of the call's weight tiles (32, 64 or 128; 0: not served).  What ds_tc_expand writes, and a
+ * ds_tc_columns   columns of the call's weight tiles (32, 64 or 128; 48, 96 or 192 where the window's columns lie side
+ *                 by side, see csrc/ds_tc.cuh; 0: not served).  What ds_tc_expand writes, and a
  *                 kept buffer holds, depends on this number, C, OC, KH, KW, `bits` and on whether fuse->in_kind is
  *                 DS_IN_F32_LINEAR: calls that agree in these have one layout, whatever their batch and image size.
  */

@@ -63,6 +63,32 @@ def test_conv(oracle, cuda_device, shape):
     assert np.array_equal(got, oracle.conv2d(x, shift, sign, bias, s, p))
 
 
+# (B, C, H, W, OC, KH, stride, pad) of 3-wide windows that move by one pixel: rows of 1 to 70 pixels that end with a
+# warp's 32 lanes or do not, warps of which the first or last lane lends its sums only, outputs fewer than pixels, every
+# width of tile with all and with few of its channels live, K split over CTAs
+FOLDED = [(3, 16, 5, 1, 16, 3, 1, (1, 1)), (2, 32, 4, 3, 20, 3, 1, (1, 0)), (70, 16, 6, 8, 16, 3, 1, (1, 1)),
+          (5, 49, 9, 15, 33, 3, 1, (1, 1)), (3, 48, 7, 16, 32, 3, 2, (1, 1)), (4, 50, 11, 30, 9, 1, 1, (0, 1)),
+          (2, 64, 13, 31, 64, 3, 1, (1, 1)), (120, 16, 16, 16, 64, 3, 1, (1, 1)), (80, 16, 16, 16, 32, 3, 1, (1, 1)), (2, 33, 8, 33, 63, 2, 1, (0, 0)),
+          (1, 256, 9, 56, 50, 3, 1, (1, 1)), (1, 130, 6, 70, 17, 5, 1, (2, 1))]
+
+
+@pytest.mark.parametrize("shape", FOLDED)
+@pytest.mark.parametrize("residual", [False, True])
+def test_folded_windows(oracle, cuda_device, shape, residual):
+    from deepshift_b200 import _ffi, kernels
+    B, C, H, W, OC, KH, s, p = shape
+    rng = np.random.default_rng(sum(shape[:7]))
+    x = rng.integers(-16384, 16385, (B, C, H, W)).astype(np.int32)
+    shift, sign = weights(rng, (OC, C, KH, 3))
+    bias = rng.integers(-2000, 2000, OC).astype(np.int32)
+    want = oracle.conv2d(x, shift, sign, bias, (s, 1), p)
+    add = rng.integers(-2 ** 22, 2 ** 22, want.shape).astype(np.int32) if residual else None
+    geo = (B, C, H, W, OC, KH, 3, s, 1, p[0], p[1])
+    assert _ffi.lib().ds_tc_columns(*geo, 6, 0, kernels._fuse(0, act_bits=15)) in (48, 96, 192)
+    got = _run(cuda_device, x, shift, sign, bias, (s, 1), p, residual=add, relu=residual)
+    assert np.array_equal(got, np.maximum(want + add, 0) if residual else want)   # exact in fp32: below 2^24
+
+
 @pytest.mark.parametrize("mkn", [(1, 64, 10), (127, 100, 31), (128, 2047, 1001), (129, 16, 64), (300, 4096, 130),
                                  (1000, 33, 65), (640, 800, 500)])
 def test_linear_full_16_bit_range(oracle, cuda_device, mkn):
