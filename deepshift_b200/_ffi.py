@@ -64,6 +64,8 @@ _SIGNATURES = {
     "ds_tc_expand": [_VP] + [_I] * 13 + [ctypes.POINTER(Fuse), _VP, _LL, _VP],
     "ds_tc_conv2d": [_VP, _VP, _VP, _VP] + [_I] * 13 + [ctypes.POINTER(Fuse), _VP, _LL, _VP, _LL, _VP],
     "ds_tc_conv2d_packed": [_VP, _VP, _VP, _VP] + [_I] * 13 + [ctypes.POINTER(Fuse), _VP, _LL, _VP, _LL, _I, _VP],
+    "ds_tc_few_bytes": [_I] * 5 + [ctypes.POINTER(Fuse), _I, ctypes.POINTER(ctypes.c_longlong)],
+    "ds_tc_linear_few": [_VP, _VP, _VP, _VP] + [_I] * 5 + [ctypes.POINTER(Fuse), _VP, _LL, _VP],
     "ds_planes_pack": [_VP, _I, _I, _I, ctypes.POINTER(Planes), _VP],
     "ds_tc_conv2d_ex": [_VP, ctypes.POINTER(Planes), _VP, _VP, _VP, ctypes.POINTER(Planes)] + [_I] * 13 +
                        [ctypes.POINTER(Fuse), _VP, _LL, _VP, _LL, _VP],

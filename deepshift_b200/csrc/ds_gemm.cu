@@ -481,14 +481,14 @@ int launch_cfg(GemmParams p, cudaStream_t st)
     p.splits = 1;
     p.tiles_per_split = p.ntiles;
     const bool plain = p.out_kind == DS_OUT_I32 && !p.relu && !p.requant && !p.round_f32 && !p.residual;
-    if (AM == AM_LINEAR && plain && !p.gate && gx * gy < 148) {
+    if (AM == AM_LINEAR && plain && (!p.gate || p.out_zeroed) && gx * gy < 148) {
         // Few output tiles (small batch): split K across gridDim.z until two CTAs per SM have work;
         // the partial sums meet through integer atomics in the zeroed output.
         int splits = 1;
         while (splits < 16 && gx * gy * splits < 2 * 148 && p.ntiles / (splits * 2) >= 4) splits *= 2;
         p.tiles_per_split = (p.ntiles + splits - 1) / splits;
         p.splits = (p.ntiles + p.tiles_per_split - 1) / p.tiles_per_split;
-        if (p.splits > 1 && cudaMemsetAsync(p.out, 0, size_t(p.M) * size_t(p.N) * 4, st) != cudaSuccess) return DS_ERR_CUDA;
+        if (p.splits > 1 && !p.out_zeroed && cudaMemsetAsync(p.out, 0, size_t(p.M) * size_t(p.N) * 4, st) != cudaSuccess) return DS_ERR_CUDA;
     }
     kern<<<dim3((unsigned)gx, (unsigned)gy, (unsigned)p.splits), NT, smem, st>>>(p);
     note_launch();
@@ -850,10 +850,10 @@ int conv2d_run(const void* x, const int32_t* packed, const int32_t* bias, void* 
 long long check_shrink_x() { return g_check_shrink_x; }
 
 // The integer path behind a tensor-core launch: runs only if *gate == want.  A linear layer arrives as a
-// 1x1 convolution on 1x1 images; its arguments have passed the checks of the caller.
+// 1x1 convolution on 1x1 images; its arguments have passed the checks of the caller.  `zeroed`: see GemmParams.
 int launch_gated_int(const void* x, const int32_t* packed, const int32_t* bias, void* out, int B, int C, int H, int W,
                      int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits, int base, const ds_fuse_t* fuse,
-                     const int* gate, int want, cudaStream_t st)
+                     const int* gate, int want, bool zeroed, cudaStream_t st)
 {
     const int OH = (H + 2 * ph - KH) / sh + 1, OW = (W + 2 * pw - KW) / sw + 1;
     GemmParams p = {};
@@ -870,6 +870,7 @@ int launch_gated_int(const void* x, const int32_t* packed, const int32_t* bias, 
     if (rc) return rc;
     p.gate = gate;
     p.gate_want = want;
+    p.out_zeroed = zeroed;
     set_check_extents(p, (long long)B * C * H * W);
     if (H == 1 && W == 1 && KH == 1 && KW == 1 && ph == 0 && pw == 0) {
         const long long tiles128 = ((long long)(p.M + 127) / 128) * ((p.N + 127) / 128);

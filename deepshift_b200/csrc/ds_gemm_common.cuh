@@ -67,6 +67,7 @@ struct GemmParams {
     // the FP32-pipe launch wants 0, the integer-path launch behind it wants 1.  Null = always run.
     const int* gate;
     int gate_want;
+    int out_zeroed;  // gated: a kernel before has zeroed the output, which lets CTAs share K through atomics
     // Checked build (-DDS_BOUNDS_CHECK) only: byte extents of x, of the packed weights and of the output
     // (the residual has the output's element count), and where the first violation goes.
     long long chk_x_bytes, chk_w_bytes, chk_o_bytes;

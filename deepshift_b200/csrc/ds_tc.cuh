@@ -161,8 +161,9 @@ struct TcExpand {
 int setup_common(GemmParams& p, int bits, int base, const ds_fuse_t* fuse, bool& use_fp);
 int launch_gated_int(const void* x, const int32_t* packed, const int32_t* bias, void* out, int B, int C, int H, int W,
                      int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits, int base, const ds_fuse_t* fuse,
-                     const int* gate, int want, cudaStream_t st);
+                     const int* gate, int want, bool zeroed, cudaStream_t st);
 long long check_shrink_x();
+unsigned tc_wait_ns();  // limit of the tensor-core kernels' waits
 
 // `e` (may be null): a kept buffer of expanded weights to look after in the same launch.
 int tc_launch_pack(const TcPack& p, const TcExpand* e, bool wide, cudaStream_t st);

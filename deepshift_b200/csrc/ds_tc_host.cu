@@ -4,6 +4,7 @@
 namespace ds {
 
 int* bounds_status_ptr();
+unsigned tc_wait_ns();
 
 namespace {
 
@@ -244,6 +245,9 @@ bool worthwhile(const TcGeom& g, const ds_fuse_t& f)
 }
 
 }  // namespace
+
+unsigned tc_wait_ns() { return g_wait_ns; }
+
 }  // namespace ds
 
 using namespace ds;
@@ -509,7 +513,7 @@ int tc_conv2d(const void* x, const ds_planes_t* xp, const int32_t* packed, const
     p.chk_status = bounds_status_ptr();
     rc = tc_launch_run(p, g.BN, wide, st);
     if (rc || mode != TC_GATED) return rc;
-    return launch_gated_int(x, packed, bias, out, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, bits, base, fuse, flag, 1, st);
+    return launch_gated_int(x, packed, bias, out, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, bits, base, fuse, flag, 1, false, st);
 }
 
 }  // namespace

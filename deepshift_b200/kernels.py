@@ -224,6 +224,31 @@ def _tc_run(x, conc_weight, bias, out, geometry, fuse, keep_weights):
     return True
 
 
+@functools.lru_cache(maxsize=4096)
+def _few_bytes(M, K, N, bits, act_bits):
+    n = ctypes.c_longlong(0)
+    _ffi.check(_ffi.lib().ds_tc_few_bytes(M, K, N, bits, 0, _fuse(act_bits=act_bits), 0, ctypes.byref(n)), "tc_few_bytes")
+    return n.value
+
+
+def _few_run(x, conc_weight, bias, out, M, K, N, fuse):
+    """Runs a linear layer on int32 codes on the tensor cores with the weights expanded in the kernel (ds_tc_linear_few)
+    if it is a call for that; False otherwise.  Scratch as in ``_tc_run``."""
+    if conc_weight.base != 0:
+        return False
+    act_bytes = _few_bytes(M, K, N, conc_weight.bits, fuse.act_bits)
+    if act_bytes == 0:
+        return False
+    try:
+        act = torch.empty(act_bytes, dtype=torch.uint8, device=x.device)
+    except torch.OutOfMemoryError:
+        return False
+    _ffi.check(_ffi.lib().ds_tc_linear_few(x.data_ptr(), conc_weight.data.data_ptr(), bias.data_ptr() if bias is not None else None,
+                                           out.data_ptr(), M, K, N, conc_weight.bits, 0, fuse, act.data_ptr(), act_bytes,
+                                           _stream_ptr(x.device)), "tc_linear_few")
+    return True
+
+
 def tc_serves_fp32_conv(input_shape, weight_shape, stride, padding, conc_weight, act_integer_bits, act_fraction_bits):
     """Whether a shift convolution with fp32 input of these sizes runs on the tensor cores, which quantise
     every value once: no quantising pass is needed in front."""
@@ -275,6 +300,8 @@ def linear(input, shift, sign, bias=None, conc_weight=None, use_cuda=True, act_b
     f = _fuse(act_bits=ACT_BITS_AUTO if act_bits is None else act_bits,
               workspace=workspace(input.device) if M > 64 else None)
     with torch.cuda.device(input.device):
+        if M > 16 and _few_run(input, conc_weight, bias, out, M, K, N, f):
+            return out
         if M > 64 and _tc_run(input, conc_weight, bias, out, (M, K, 1, 1, N, 1, 1, 1, 1, 0, 0), f, False):
             return out
         rc = _ffi.lib().ds_linear_ex(input.data_ptr(), conc_weight.data.data_ptr(),

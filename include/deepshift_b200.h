@@ -296,6 +296,14 @@ int ds_conv2d_prepare(const int32_t *packed, int B, int C, int H, int W, int OC,
  *                 kept buffer holds, depends on this number, C, OC, KH, KW, `bits` and on whether fuse->in_kind is
  *                 DS_IN_F32_LINEAR: calls that agree in these have one layout, whatever their batch and image size.
  */
+/* Linear layers on the tensor cores without expanded weights, int32 codes (act_bits 1..15 or DS_ACT_BITS_AUTO), base == 0,
+ * nothing fused: the kernel decodes the packed words itself, which pays for batches too small for ds_tc_expand in every
+ * call.  ds_tc_few_bytes: size of `act` (scratch of one call, any contents, 16-byte aligned; 0: not served, or, unless
+ * any_size, not worth it).  Enqueues two kernels, three with the measured range, whose verdict is the first word of
+ * `act`; works under stream capture. */
+int ds_tc_few_bytes(int M, int K, int N, int bits, int base, const ds_fuse_t *fuse, int any_size, long long *act_bytes);
+int ds_tc_linear_few(const int32_t *x, const int32_t *packed, const int32_t *bias, int32_t *out, int M, int K, int N,
+                     int bits, int base, const ds_fuse_t *fuse, void *act, long long act_bytes, void *stream);
 int ds_tc_bytes(int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits, int base,
                 const ds_fuse_t *fuse, int any_size, long long *act_bytes, long long *weight_bytes);
 int ds_tc_columns(int B, int C, int H, int W, int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits, int base,

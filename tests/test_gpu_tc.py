@@ -351,3 +351,48 @@ def test_calls_that_expand_their_weights(oracle, cuda_device, kind, what):
                                           torch.cuda.current_stream(cuda_device).cuda_stream) == 0
     assert np.array_equal(out.cpu().numpy(), oracle.conv2d(codes, shift, sign, None, (1, 1), (k // 2, k // 2)))
     assert int(scratch[:4].view(torch.int32)) == int(what == "code" or (fp32 and what == "shift"))
+
+
+# (M, K, N, weight bits, zeros): rows at the edges of the 80- and 144-column tiles and of two of them, columns at those of
+# 128, every packed field width that has a whole kernel of its own, words and groups that K does not fill, K shared
+FEW = [(1, 16, 10, 5, True), (17, 300, 127, 5, True), (79, 1000, 128, 4, False), (80, 1024, 129, 3, False),
+       (143, 257, 300, 2, False), (144, 100, 31, 6, True), (200, 4096, 130, 5, False), (64, 47, 64, 6, False)]
+
+
+@pytest.mark.parametrize("case", FEW)
+@pytest.mark.parametrize("wide", [False, True])
+def test_linear_with_weights_expanded_in_the_kernel(oracle, cuda_device, case, wide):
+    """Codes over the whole 16-bit range; one beyond it sends the call to the integer path, found in the scratch's first word."""
+    from deepshift_b200 import _ffi, kernels, utils
+    M, K, N, wb, zeros = case
+    rng = np.random.default_rng(M + K + N)
+    x = rng.integers(-32768, 32768, (M, K)).astype(np.int32)
+    x.flat[::7] = -32768
+    x.flat[3::11] = 32767
+    if wide:
+        x[M - 1, K - 1] = -32769
+    shift = rng.integers(-(2 ** (wb - 1) - 1), 1, (N, K)).astype(np.int32)
+    shift[0, 0] = -(2 ** (wb - 1) - 1)   # the widest field of this case
+    sign = rng.choice([-1, 0, 1] if zeros else [-1, 1], (N, K)).astype(np.int32)
+    bias = rng.integers(-2000, 2000, N).astype(np.int32)
+    cw = utils.compress_bits(torch.from_numpy(shift).float(), torch.from_numpy(sign).float(), device=cuda_device)
+    f = kernels._fuse(act_bits=-1)
+    n = ctypes.c_longlong(0)
+    assert _ffi.lib().ds_tc_few_bytes(M, K, N, cw.bits, cw.base, f, 1, ctypes.byref(n)) == 0 and n.value > 0
+    xt, bt = torch.from_numpy(x).to(cuda_device), torch.from_numpy(bias).to(cuda_device)
+    act = torch.full((n.value + 64,), 0xA5, dtype=torch.uint8, device=cuda_device)
+    out = torch.full((M * N + 16,), 0x5EADBEE, dtype=torch.int32, device=cuda_device)
+    rc = _ffi.lib().ds_tc_linear_few(xt.data_ptr(), cw.data.data_ptr(), bt.data_ptr(), out.data_ptr(), M, K, N, cw.bits, cw.base,
+                                     f, act.data_ptr(), n.value, torch.cuda.current_stream(cuda_device).cuda_stream)
+    torch.cuda.synchronize(cuda_device)
+    assert rc == 0 and kernels.last_kernel_error() == 0
+    assert bool((act[n.value:] == 0xA5).all()) and bool((out[-16:] == 0x5EADBEE).all())
+    assert int(act[:4].view(torch.int32)) == int(wide)
+    assert np.array_equal(out[:-16].reshape(M, N).cpu().numpy(), oracle.linear(x, shift, sign, bias))
+
+
+def test_which_linear_calls_expand_their_weights_in_the_kernel(cuda_device):
+    from deepshift_b200 import kernels
+    assert kernels._few_bytes(64, 4096, 4096, 6, -1) > 0 and kernels._few_bytes(64, 4096, 4096, 6, 15) > 0
+    assert kernels._few_bytes(16, 4096, 4096, 6, -1) == 0 and kernels._few_bytes(8192, 4096, 4096, 6, -1) == 0
+    assert kernels._few_bytes(64, 4096, 4096, 6, 0) == 0 and kernels._few_bytes(64, 4096, 4096, 6, 16) == 0   # other promises
