@@ -40,6 +40,7 @@ struct FewParams {
     const int* bias;
     int* out;
     int* flag;           // whole call; the blocks' flags at flag + 4
+    int* report;         // as in TcRun
     unsigned char* planes;
     int M, K, N, row_len, G, wpg, kpg;
     int grid_m, grid_n, splits, gps, units, rpt;  // rpt: rows of x per tile, the last column is the row of zeros
@@ -152,7 +153,10 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) few_run_kernel(const FewParams
         int over = 0;
         for (int i = threadIdx.x; i < p.blocks; i += FEW_THREADS) over |= __ldg(p.flag + 4 + i);
         over = __syncthreads_or(over);
-        if (blockIdx.x == 0 && threadIdx.x == 0) *p.flag = over;  // for the integer path behind
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            *p.flag = over;  // for the integer path behind
+            if (p.report) *p.report = over;
+        }
         if (over) return;
     }
     volatile int* err = &s.err;
@@ -534,6 +538,8 @@ extern "C" int ds_tc_linear_few(const int32_t* x, const int32_t* packed, const i
     p.units = g.grid_m * g.grid_n * g.splits;
     p.blocks = g.blocks;
     p.gated = mode == 2;
+    std::unique_lock<std::mutex> lock;
+    if (p.gated && (p.report = workspace_gate_word(fuse)) != nullptr) lock = std::unique_lock<std::mutex>(gate_word_mutex());
     p.zero_out = g.splits > 1 || p.gated;  // the integer path behind may share K as well
     p.wait_ns = tc_wait_ns();
     p.err_flag = kernel_error_flag();

@@ -28,7 +28,7 @@
 //   AM_ROW + KW  convolution with a KW-wide window and a k-tile made of whole (ic,kh) rows:
 //                one table entry and one validity test per row, KW loads at constant
 //                offsets.  This is the cheap path used by 1x1, 3x3, 5x5 and 7x7 windows.
-#include "ds_gemm_common.cuh"
+#include "ds_tc.cuh"
 
 namespace ds {
 namespace {
@@ -677,14 +677,30 @@ __global__ void __launch_bounds__(256) range_kernel(const int* __restrict__ x, l
 // input without a promise, right shifts only and a workspace (whose last counter word is the flag).
 bool auto_range(const ds_fuse_t* fuse, int base)
 {
-    return fuse && fuse->act_bits == DS_ACT_BITS_AUTO && fuse->in_kind == DS_IN_I32 && base == 0 && fuse->workspace &&
-           fuse->workspace_bytes >= (long long)kWorkspaceCounters * 4;
+    return fuse && fuse->act_bits == DS_ACT_BITS_AUTO && fuse->in_kind == DS_IN_I32 && base == 0 && workspace_gate_word(fuse);
 }
+
+}  // namespace
+
+int* workspace_gate_word(const ds_fuse_t* fuse)
+{
+    return fuse->workspace && fuse->workspace_bytes >= (long long)kWorkspaceCounters * 4
+               ? static_cast<int*>(fuse->workspace) + kWorkspaceGateSlot
+               : nullptr;
+}
+
+std::mutex& gate_word_mutex()
+{
+    static std::mutex m;
+    return m;
+}
+
+namespace {
 
 // Zeroes the flag and measures the range of x on `st`; returns the flag's device address.
 int* launch_range(const void* x, long long n, const ds_fuse_t* fuse, cudaStream_t st)
 {
-    int* flag = static_cast<int*>(fuse->workspace) + kWorkspaceGateSlot;
+    int* flag = workspace_gate_word(fuse);
     if (cudaMemsetAsync(flag, 0, sizeof(int), st) != cudaSuccess) return nullptr;
     const long long want = (n / 4 + 255) / 256 + 1;
     range_kernel<<<unsigned(want > 148 * 16 ? 148 * 16 : want), 256, 0, st>>>(static_cast<const int*>(x), n, 1 << 15, flag);
@@ -726,6 +742,7 @@ extern "C" int ds_linear_ex(const void* x, const int32_t* packed, const int32_t*
     if (rc) return rc;
     if (auto_range(fuse, base) && M > 64) {
         // measure the range once, then launch both arithmetic paths gated on the result
+        const std::lock_guard<std::mutex> lock(gate_word_mutex());
         cudaStream_t st = static_cast<cudaStream_t>(stream);
         int* flag = launch_range(x, (long long)M * K, fuse, st);
         if (!flag) return DS_ERR_CUDA;
@@ -816,6 +833,7 @@ int conv2d_run(const void* x, const int32_t* packed, const int32_t* bias, void* 
     p.magic_kh = magic_of(KH);
     if (!prepare && auto_range(fuse, base)) {
         // measure the range once, then launch both arithmetic paths gated on the result
+        const std::lock_guard<std::mutex> lock(gate_word_mutex());
         cudaStream_t st = static_cast<cudaStream_t>(stream);
         int* flag = launch_range(x, (long long)B * C * H * W, fuse, st);
         if (!flag) return DS_ERR_CUDA;

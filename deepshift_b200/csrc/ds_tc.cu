@@ -264,7 +264,11 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
     using T = TcTile<BN, WIDE>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     TcSmem<BN, WIDE>& s = *reinterpret_cast<TcSmem<BN, WIDE>*>(smem_raw);
-    if (p.gate && *p.gate != p.gate_want) return;  // the other arithmetic path serves this input
+    if (p.gate) {
+        const int found = *p.gate;
+        if (p.report && blockIdx.x == 0 && threadIdx.x == 0) *p.report = found;
+        if (found != p.gate_want) return;  // the other arithmetic path serves this input
+    }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     volatile int* err = &s.err;
 

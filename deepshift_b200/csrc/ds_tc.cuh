@@ -26,6 +26,8 @@
 // so two more products with plane t go into the same sum (r >= 9: coefficients up to 128 as 64 + 64) and four
 // into a second accumulator of weight 2^8 (r <= 8: up to 256 as four times 64).
 #pragma once
+#include <mutex>
+
 #include "ds_gemm_common.cuh"
 
 namespace ds {
@@ -104,6 +106,7 @@ struct TcRun {
     float inv_scale;
     const int* gate;
     int gate_want;
+    int* report;         // receives *gate: the workspace's word, for who wants to know which path served; null = none
     unsigned wait_ns;    // limit of every wait
     int hold;            // checked build: see ds_tc_debug_waits
     int* err_flag;
@@ -163,6 +166,9 @@ int launch_gated_int(const void* x, const int32_t* packed, const int32_t* bias, 
                      int OC, int KH, int KW, int sh, int sw, int ph, int pw, int bits, int base, const ds_fuse_t* fuse,
                      const int* gate, int want, bool zeroed, cudaStream_t st);
 long long check_shrink_x();
+int* workspace_gate_word(const ds_fuse_t* fuse);  // null without a workspace
+// Held while the launches of a call with a measured range are enqueued: two threads on one stream share its workspace.
+std::mutex& gate_word_mutex();
 unsigned tc_wait_ns();  // limit of the tensor-core kernels' waits
 
 // `e` (may be null): a kept buffer of expanded weights to look after in the same launch.

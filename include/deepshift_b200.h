@@ -278,7 +278,8 @@ int ds_conv2d_prepare(const int32_t *packed, int B, int C, int H, int W, int OC,
  *   DS_IN_F32_LINEAR                  linear layers, codes of up to 24 bits (22 byte products instead of 16).
  * For the last two the packing pass looks at every code; when one does not fit, the tensor-core launch
  * returns at once and the integer-path launch enqueued behind it does the work.  The
- * range flag is the first word of `act`; fuse->workspace and fuse->prepared are not used.
+ * range flag is the first word of `act`; with DS_ACT_BITS_AUTO a copy of it goes into the last counter word of
+ * fuse->workspace, if there is one.  fuse->prepared is not used.
  *
  * ds_tc_bytes     sizes of `act` (scratch of one call, any contents, reusable in stream order) and `weights`;
  *                 both 0 when the call is not served, or, unless any_size, has too little work to be worth it.
