@@ -71,6 +71,8 @@ _SIGNATURES = {
                        [ctypes.POINTER(Fuse), _VP, _LL, _VP, _LL, _VP],
     "ds_compress": [_VP, _VP, _VP, _I, _I, _I, _I, _VP],
     "ds_pack_range_f32": [_VP, _VP, _LL, _VP, _VP],
+    "ds_pack_scan_f32": [_VP, _VP, _LL, _VP, _VP, _VP],
+    "ds_pack_codes": [_VP, _VP, _I, _I, _I, _I, _VP],
     "ds_pack_f32": [_VP, _VP, _VP, _I, _I, _I, _I, _VP],
     "ds_quantize_f32": [_VP, _VP, _LL, _I, _I, _I, _VP],
     "ds_maxpool2d_i32": [_VP, _VP, _I, _I, _I, _I, _I, _I, _I, _VP],

@@ -40,44 +40,113 @@ __global__ void compress_kernel(const int32_t* __restrict__ shiftp, const int32_
 // Right shift of one weight as compress_bits stores it: rint(-shift), 32 for a zero sign.
 __device__ __forceinline__ float pack_shift(float shift, float sign) { return sign == 0.f ? 32.f : rintf(-shift); }
 
+// Byte of a weight whose right shift lies in -64..63: the shift in seven bits, above it what the packed sign bit will be.
+__device__ __forceinline__ unsigned pack_byte(int shift, float sign)
+{
+    return (unsigned(shift) & 127u) | (sign == 0.f || sign >= 1.f ? 128u : 0u);  // int(sign) > 0, a zero sign counts as +1
+}
+
 // Largest right shift r[0], largest negated one r[1] (r starts at 0x80808080), r[2] = 1 when a value is no
 // integer of at most 24 bits (NaN, infinity), else 0 when one lies in 16..31 (or 80..95, ..).
-// HBM-bound: one read of both tensors; eight blocks per SM, so 32 registers (4096 x 4096: 33 us, 35 us with 34).
+// CODES: the weights' bytes as well, from which the words are made once the fields' width is known, instead of a second
+// read of the parameters.
+// HBM-bound: one read of both tensors; eight blocks per SM, so 32 registers.  One atomic per block and result: one per warp were
+// 28 000 on one address (4096 x 4096: 33 us without the bytes, 28 with them).
+template <bool CODES>
 __global__ void __launch_bounds__(256, 8) pack_range_kernel(const float* __restrict__ shift, const float* __restrict__ sign,
-                                                         long long n, int* r)
+                                                         long long n, int* r, unsigned char* __restrict__ codes)
 {
+    __shared__ int red[3];
+    if (threadIdx.x < 3) red[threadIdx.x] = INT_MIN;
+    __syncthreads();
     int hi = INT_MIN, nlo = INT_MIN;
     bool bad = false;
     int far = 0;  // bit 4: set without bit 5 in some shift
-    auto see = [&](float a, float g) {
+    auto see = [&](float a, float g) -> unsigned {
         const float v = pack_shift(a, g);
+        int i = 0;
         if (fabsf(v) <= 16777216.f) {
-            const int i = int(v);
+            i = int(v);
             hi = max(hi, i);
             nlo = max(nlo, -i);
             far |= i & ~(i >> 1);
         } else {
             bad = true;
         }
+        return CODES ? pack_byte(i, g) : 0u;
     };
     const long long t0 = blockIdx.x * 256ll + threadIdx.x, step = gridDim.x * 256ll;
     const long long n4 = ((reinterpret_cast<uintptr_t>(shift) | reinterpret_cast<uintptr_t>(sign)) & 15u) == 0 ? n / 4 : 0;
 #pragma unroll 2
     for (long long i = t0; i < n4; i += step) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(shift) + i), g = __ldg(reinterpret_cast<const float4*>(sign) + i);
-        see(a.x, g.x);
-        see(a.y, g.y);
-        see(a.z, g.z);
-        see(a.w, g.w);
+        const float4 a = __ldcs(reinterpret_cast<const float4*>(shift) + i), g = __ldcs(reinterpret_cast<const float4*>(sign) + i);
+        unsigned w = see(a.x, g.x);
+        w |= see(a.y, g.y) << 8;
+        w |= see(a.z, g.z) << 16;
+        w |= see(a.w, g.w) << 24;
+        if (CODES) reinterpret_cast<unsigned*>(codes)[i] = w;
     }
-    for (long long i = 4 * n4 + t0; i < n; i += step) see(__ldg(shift + i), __ldg(sign + i));
+    for (long long i = 4 * n4 + t0; i < n; i += step) {
+        const unsigned w = see(__ldg(shift + i), __ldg(sign + i));
+        if (CODES) codes[i] = (unsigned char)w;
+    }
     hi = __reduce_max_sync(0xFFFFFFFFu, hi);
     nlo = __reduce_max_sync(0xFFFFFFFFu, nlo);
     const bool any = __any_sync(0xFFFFFFFFu, bad), anyfar = __any_sync(0xFFFFFFFFu, (far & 16) != 0);
     if ((threadIdx.x & 31) == 0) {
-        atomicMax(r, hi);
-        atomicMax(r + 1, nlo);
-        if (any || anyfar) atomicMax(r + 2, any ? 1 : 0);
+        atomicMax(&red[0], hi);
+        atomicMax(&red[1], nlo);
+        if (any || anyfar) atomicMax(&red[2], any ? 1 : 0);
+    }
+    __syncthreads();
+    if (threadIdx.x < 3 && red[threadIdx.x] != INT_MIN) atomicMax(r + threadIdx.x, red[threadIdx.x]);
+}
+
+// Word of NUM weights from their bytes, `len` of them present.
+template <int NUM>
+__device__ __forceinline__ int pack_word(const unsigned (&c)[(NUM + 3) / 4], int len, int bits, int base)
+{
+    uint32_t value = 0;
+#pragma unroll
+    for (int j = 0; j < NUM; ++j) {
+        if (j >= len) break;
+        const unsigned b = c[j / 4] >> (8 * (j % 4));
+        const uint32_t field = uint32_t((int(b << 25) >> 25) - base);
+        value |= field << (j * (bits + 1)) | ((b >> 7) & 1u) << (j * (bits + 1) + bits);
+    }
+    return int32_t(value);
+}
+
+// The words from the weights' bytes; WORDS per thread: four of four weights where rows are whole groups of sixteen, else
+// one, VEC: read in whole 4-byte groups.  4096 x 4096, 7-bit fields: 17 MB read, mostly from L2 where the pass before has
+// left them, and as many written.
+template <int NUM, bool VEC, int WORDS>
+__global__ void __launch_bounds__(256) pack_codes_kernel(const unsigned char* __restrict__ codes, int32_t* __restrict__ packed,
+                                                         long long threads, int K, int bits, int base, int row_len)
+{
+    const long long i = blockIdx.x * 256ll + threadIdx.x;
+    if (i >= threads) return;
+    if constexpr (WORDS == 4) {
+        const uint4 q = __ldg(reinterpret_cast<const uint4*>(codes) + i);
+        const unsigned w[4][1] = {{q.x}, {q.y}, {q.z}, {q.w}};
+        reinterpret_cast<int4*>(packed)[i] = make_int4(pack_word<4>(w[0], 4, bits, base), pack_word<4>(w[1], 4, bits, base),
+                                                       pack_word<4>(w[2], 4, bits, base), pack_word<4>(w[3], 4, bits, base));
+    } else {
+        const long long oc = (i >> 31) == 0 ? unsigned(i) / unsigned(row_len) : i / row_len;
+        const int k0 = int(i - oc * row_len) * NUM;
+        const int len = min(NUM, K - k0);
+        const unsigned char* src = codes + oc * K + k0;
+        unsigned c[(NUM + 3) / 4];
+        if (VEC) {  // a row's last word may have fewer groups
+#pragma unroll
+            for (int j = 0; j < NUM / 4; ++j) c[j] = 4 * j < len ? __ldg(reinterpret_cast<const unsigned*>(src) + j) : 0u;
+        } else {
+#pragma unroll
+            for (int j = 0; j < (NUM + 3) / 4; ++j) c[j] = 0;
+#pragma unroll
+            for (int j = 0; j < NUM; ++j) c[j / 4] |= (j < len ? unsigned(__ldg(src + j)) : 0u) << (8 * (j % 4));
+        }
+        packed[i] = pack_word<NUM>(c, len, bits, base);
     }
 }
 
@@ -123,7 +192,7 @@ __global__ void __launch_bounds__(256) pack_f32_kernel(const float* __restrict__
     for (int j = 0; j < NUM; ++j) {
         if (j >= len) break;
         const uint32_t field = uint32_t(int(pack_shift(a[j], g[j])) - base);
-        const uint32_t pos = (g[j] == 0.f || g[j] >= 1.f) ? 1u : 0u;  // int(sign) > 0, a zero sign counts as +1
+        const uint32_t pos = pack_byte(0, g[j]) >> 7;
         value |= field << (j * (bits + 1)) | pos << (j * (bits + 1) + bits);
     }
     packed[i] = int32_t(value);
@@ -328,7 +397,55 @@ extern "C" int ds_pack_range_f32(const float* shift, const float* sign, long lon
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (cudaMemsetAsync(range, 0x80, 3 * sizeof(int), st) != cudaSuccess) return DS_ERR_CUDA;
     const long long want = (n / 4 + 255) / 256 + 1;
-    pack_range_kernel<<<unsigned(want > 148 * 8 ? 148 * 8 : want), 256, 0, st>>>(shift, sign, n, range);
+    pack_range_kernel<false><<<unsigned(want > 148 * 8 ? 148 * 8 : want), 256, 0, st>>>(shift, sign, n, range, nullptr);
+    note_launch();
+    return cudaGetLastError() == cudaSuccess ? DS_OK : DS_ERR_CUDA;
+}
+
+extern "C" int ds_pack_scan_f32(const float* shift, const float* sign, long long n, unsigned char* codes, int* range, void* stream)
+{
+    if (!shift || !sign || !codes || !range || n <= 0) return DS_ERR_BAD_ARG;
+    if ((reinterpret_cast<uintptr_t>(codes) | reinterpret_cast<uintptr_t>(range)) & 3u) return DS_ERR_ALIGN;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (cudaMemsetAsync(range, 0x80, 3 * sizeof(int), st) != cudaSuccess) return DS_ERR_CUDA;
+    const long long want = (n / 4 + 255) / 256 + 1;
+    pack_range_kernel<true><<<unsigned(want > 148 * 8 ? 148 * 8 : want), 256, 0, st>>>(shift, sign, n, range, codes);
+    note_launch();
+    return cudaGetLastError() == cudaSuccess ? DS_OK : DS_ERR_CUDA;
+}
+
+extern "C" int ds_pack_codes(const unsigned char* codes, int32_t* packed, int OC, int K, int bits, int base, void* stream)
+{
+    if (!codes || !packed || OC <= 0 || K <= 0) return DS_ERR_BAD_ARG;
+    if (bits < 1 || bits > 7) return DS_ERR_UNSUPPORTED;
+    const int num = 32 / (bits + 1);
+    const int row_len = (K + num - 1) / num;
+    const long long words = (long long)OC * row_len;
+    const long long blocks = (words + 255) / 256;
+    if (blocks > 2147483647ll) return DS_ERR_RANGE;
+    const bool vec = K % 4 == 0 && (reinterpret_cast<uintptr_t>(codes) & 3u) == 0;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const uintptr_t both = reinterpret_cast<uintptr_t>(codes) | reinterpret_cast<uintptr_t>(packed);
+    if (num == 4 && K % 16 == 0 && (both & 15u) == 0) {
+        pack_codes_kernel<4, true, 4><<<unsigned((words / 4 + 255) / 256), 256, 0, st>>>(codes, packed, words / 4, K, bits, base, row_len);
+        note_launch();
+        return cudaGetLastError() == cudaSuccess ? DS_OK : DS_ERR_CUDA;
+    }
+    auto go = [&](auto num_tag) {
+        constexpr int NUM = decltype(num_tag)::value;
+        if (NUM % 4 == 0 && vec)
+            pack_codes_kernel<NUM, NUM % 4 == 0, 1><<<unsigned(blocks), 256, 0, st>>>(codes, packed, words, K, bits, base, row_len);
+        else
+            pack_codes_kernel<NUM, false, 1><<<unsigned(blocks), 256, 0, st>>>(codes, packed, words, K, bits, base, row_len);
+    };
+    switch (num) {
+        case 4: go(std::integral_constant<int, 4>()); break;
+        case 5: go(std::integral_constant<int, 5>()); break;
+        case 6: go(std::integral_constant<int, 6>()); break;
+        case 8: go(std::integral_constant<int, 8>()); break;
+        case 10: go(std::integral_constant<int, 10>()); break;
+        default: go(std::integral_constant<int, 16>()); break;
+    }
     note_launch();
     return cudaGetLastError() == cudaSuccess ? DS_OK : DS_ERR_CUDA;
 }

@@ -364,20 +364,36 @@ def compress_sign_and_shift(shift, sign, comp_size, base, bits, row_length, num)
     return comp_weight
 
 
-def pack_range(shift, sign):
-    """(smallest, largest, one in 16..31?) of the right shifts of fp32 parameters as ``compress_bits`` stores them, or
-    None when they are not all finite integers of at most 24 bits.  Synchronises (the packing geometry depends on
-    it)."""
-    with torch.cuda.device(shift.device):
-        r = torch.empty(3, dtype=torch.int32, device=shift.device)
-        _ffi.check(_ffi.lib().ds_pack_range_f32(shift.data_ptr(), sign.data_ptr(), shift.numel(), r.data_ptr(),
-                                                _stream_ptr(shift.device)), "pack_range")
+def pack_scan(shift, sign):
+    """((smallest, largest, one in 16..31?), bytes) of the right shifts of fp32 parameters as ``compress_bits`` stores them,
+    or None when they are not all finite integers of at most 24 bits.  The bytes (``pack_codes``) are None when a shift does
+    not fit one.  Synchronises (the packing geometry depends on the range)."""
+    device = shift.device
+    with torch.cuda.device(device):
+        n = shift.numel()
+        r = torch.empty(3, dtype=torch.int32, device=device)
+        codes = torch.empty(n, dtype=torch.uint8, device=device)
+        _ffi.check(_ffi.lib().ds_pack_scan_f32(shift.data_ptr(), sign.data_ptr(), n, codes.data_ptr(), r.data_ptr(),
+                                               _stream_ptr(device)), "pack_scan")
     hi, nlo, bad = r.tolist()
-    return None if bad > 0 else (-nlo, hi, bad == 0)
+    if bad > 0:
+        return None
+    return (-nlo, hi, bad == 0), codes if hi <= 63 and nlo <= 64 else None
+
+
+def pack_codes(codes, OC, bits, base):
+    """Bytes of ``pack_scan`` -> packed int32 words."""
+    K = codes.numel() // OC
+    num = 32 // (bits + 1)
+    out = torch.empty([(K + num - 1) // num * OC], dtype=torch.int32, device=codes.device)
+    with torch.cuda.device(codes.device):
+        _ffi.check(_ffi.lib().ds_pack_codes(codes.data_ptr(), out.data_ptr(), OC, K, bits, base, _stream_ptr(codes.device)),
+                   "pack_codes")
+    return out
 
 
 def pack_f32(shift, sign, bits, base):
-    """fp32 (shift, sign) [OC, ...] -> packed int32 words, in one pass."""
+    """fp32 (shift, sign) [OC, ...] -> packed int32 words, in one pass over the parameters (shifts of any size)."""
     OC = shift.shape[0]
     K = shift.numel() // OC
     num = 32 // (bits + 1)

@@ -109,14 +109,16 @@ def compress_bits(shift, sign, device=None):
         # fp32 parameters on the GPU that runs the layer: two kernels instead of a chain of whole-tensor
         # torch passes (4096 x 4096: 415 -> 88 us)
         sh, sg = shift.detach().contiguous(), sign.detach().contiguous()
-        span = kernels.pack_range(sh, sg)
-        if span is not None:
+        scan = kernels.pack_scan(sh, sg)
+        if scan is not None:
+            span, codes = scan
             base = min(span[0], 0)
             bits = max(1, (span[1] - base).bit_length())
             if bits <= 7:
                 conc_weight.base, conc_weight.bits = base, bits
                 conc_weight.far_shifts = base == 0 and span[2]
-                conc_weight.data = kernels.pack_f32(sh, sg, bits, base)
+                conc_weight.data = (kernels.pack_codes(codes, sh.shape[0], bits, base) if codes is not None
+                                    else kernels.pack_f32(sh, sg, bits, base))
                 return conc_weight
     shift = shift.detach().clone()
     sign = sign.detach().clone()

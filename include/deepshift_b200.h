@@ -196,8 +196,13 @@ int ds_compress(const int32_t *shiftp, const int32_t *sign, int32_t *packed, int
  *                      value is not an integer of at most 24 bits, else 0 when a shift modulo 64 lies in
  *                      16..31, else negative (device int32[3]): what the caller chooses bits and base from.
  *   ds_pack_f32        the words.
+ *   ds_pack_scan_f32   the same as ds_pack_range_f32, and one byte per weight in `codes` (n bytes, 4-byte aligned): the
+ *                      right shift in seven bits, valid when all lie in -64..63, and the sign bit.
+ *   ds_pack_codes      the words from those bytes: the parameters are read once.
  */
 int ds_pack_range_f32(const float *shift, const float *sign, long long n, int *range, void *stream);
+int ds_pack_scan_f32(const float *shift, const float *sign, long long n, unsigned char *codes, int *range, void *stream);
+int ds_pack_codes(const unsigned char *codes, int32_t *packed, int OC, int K, int bits, int base, void *stream);
 int ds_pack_f32(const float *shift, const float *sign, int32_t *packed, int OC, int K, int bits, int base,
                 void *stream);
 
