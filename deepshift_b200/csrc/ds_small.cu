@@ -8,7 +8,7 @@
 //     packed words l, l+32, ... of each of its rows (one coalesced 128-byte request per row and
 //     step; 16- or 8-byte requests per lane when rows are whole groups of four or two words, and
 //     16- or 8-byte requests on x when a word's weights are), decodes each word's
-//     fields once through a small lookup table in shared memory, and applies every weight to the M
+//     fields once, and applies every weight to the M
 //     activations it meets (exact integer arithmetic: shift, then multiply by +-1 / +-2^k / 0);
 //   * when the columns alone do not fill the GPU, WPC warps of a CTA share a column group and split
 //     K between them as well;
@@ -23,19 +23,30 @@ namespace {
 constexpr int SM_WARPS = 8;
 constexpr int SM_THREADS = SM_WARPS * 32;
 
-template <int MR, int CN, int INK>
+// How a field is decoded.  From its bits where base == 0: the shift is a funnel shift by the field's low five bits (masked
+// below five), the multiplier -1, 0 or 1 a signed two-bit extract from a word made once per packed word.  With a table in
+// shared memory, the only way before, the reads and the queue they share were what the kernel waited for (M = 1, K = N = 4096:
+// 14.9 us); left shifts (base < 0) still take it.
+enum { DEC_TABLE = 0, DEC_BITS, DEC_BITS_MASKED };
+
+template <int MR, int CN, int INK, int DEC>
 __global__ void __launch_bounds__(SM_THREADS) small_linear_kernel(const GemmParams p, int wpc, int vecw)
 {
-    __shared__ int2 lut[256];                       // (right shift, multiplier) per field value
+    __shared__ int2 lut[DEC == DEC_TABLE ? 256 : 1];  // (right shift, multiplier) per field value
     __shared__ int part[SM_WARPS][MR * CN];         // partial sums of the warps that share a column group
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     if (p.gate && *p.gate != p.gate_want) return;
-    for (int f = t; f < (1 << p.dec.fw); f += SM_THREADS) {
-        int shv, mul;
-        decode_int(uint32_t(f), p.dec, true, shv, mul);
-        lut[f] = make_int2(shv, mul);
+    if (DEC == DEC_TABLE) {
+        for (int f = t; f < (1 << p.dec.fw); f += SM_THREADS) {
+            int shv, mul;
+            decode_int(uint32_t(f), p.dec, true, shv, mul);
+            lut[f] = make_int2(shv, mul);
+        }
+        __syncthreads();
     }
-    __syncthreads();
+    uint32_t lsb = 0;  // the lowest bit of every field
+    if (DEC != DEC_TABLE)
+        for (int j = 0; j < p.dec.num; ++j) lsb |= 1u << (j * p.dec.fw);
 
     const int groups_per_cta = SM_WARPS / wpc;
     const int group = blockIdx.x * groups_per_cta + warp / wpc;  // column group of this warp
@@ -56,6 +67,27 @@ __global__ void __launch_bounds__(SM_THREADS) small_linear_kernel(const GemmPara
     const bool pairx = !vecx && (num % 2 == 0) && (p.K % 2 == 0) && ((reinterpret_cast<uintptr_t>(p.x) & 7u) == 0);
     auto word_step = [&](int w, const uint32_t (&word)[CN]) {
         const int k0 = w * num;
+        uint32_t mulw[CN];  // per field: 1 when the weight is not zero, and above it 1 when it is negative
+#pragma unroll
+        for (int c = 0; c < CN; ++c) {
+            uint32_t live = lsb;
+            if (DEC == DEC_BITS && p.dec.bits > 5) live &= ~((word[c] >> 5) | (p.dec.bits > 6 ? word[c] >> 6 : 0u));
+            mulw[c] = live | ((live & ~(word[c] >> p.dec.bits)) << 1);
+        }
+        // field j of column c against the values of MR rows
+        auto weight = [&](int c, int j, const int (&xv)[MR], const int (&xs)[MR]) {
+            const uint32_t f = word[c] >> (j * fw);
+            if (DEC == DEC_TABLE) {
+                const int2 d = lut[f & fmask];
+#pragma unroll
+                for (int m = 0; m < MR; ++m) acc[m][c] += (xv[m] >> d.x) * d.y;
+            } else {
+                const uint32_t sh = DEC == DEC_BITS_MASKED ? f & (fmask >> 1) : f;
+                const int mul = int(mulw[c] << (30 - j * fw)) >> 30;
+#pragma unroll
+                for (int m = 0; m < MR; ++m) acc[m][c] += int(__funnelshift_r(uint32_t(xv[m]), uint32_t(xs[m]), sh)) * mul;
+            }
+        };
         if (vecx) {
             // four weights per word and rows of whole 16-byte groups: one 16-byte load per row
             int xv[MR][4];
@@ -72,12 +104,16 @@ __global__ void __launch_bounds__(SM_THREADS) small_linear_kernel(const GemmPara
             }
 #pragma unroll
             for (int j = 0; j < 4; ++j)
+{
+                int xj[MR], xs[MR];
 #pragma unroll
-                for (int c = 0; c < CN; ++c) {
-                    const int2 d = lut[(word[c] >> (j * fw)) & fmask];
-#pragma unroll
-                    for (int m = 0; m < MR; ++m) acc[m][c] += (xv[m][j] >> d.x) * d.y;
+                for (int m = 0; m < MR; ++m) {
+                    xj[m] = xv[m][j];
+                    xs[m] = xj[m] >> 31;
                 }
+#pragma unroll
+                for (int c = 0; c < CN; ++c) weight(c, j, xj, xs);
+            }
             return;
         }
         if (pairx) {
@@ -97,12 +133,16 @@ __global__ void __launch_bounds__(SM_THREADS) small_linear_kernel(const GemmPara
                 }
 #pragma unroll
                 for (int jj = 0; jj < 2; ++jj)
+{
+                    int xj[MR], xs[MR];
 #pragma unroll
-                    for (int c = 0; c < CN; ++c) {
-                        const int2 d = lut[(word[c] >> ((j + jj) * fw)) & fmask];
-#pragma unroll
-                        for (int m = 0; m < MR; ++m) acc[m][c] += (xv[m][jj] >> d.x) * d.y;
+                    for (int m = 0; m < MR; ++m) {
+                        xj[m] = xv[m][jj];
+                        xs[m] = xj[m] >> 31;
                     }
+#pragma unroll
+                    for (int c = 0; c < CN; ++c) weight(c, j + jj, xj, xs);
+                }
             }
             return;
         }
@@ -116,12 +156,11 @@ __global__ void __launch_bounds__(SM_THREADS) small_linear_kernel(const GemmPara
                 if (m0 + m < p.M && DS_X_OK(p, xi + (size_t)(m0 + m) * p.K + k, 4))
                     xv[m] = __float_as_int(operand_of<false, INK>(p, __ldg(xi + (size_t)(m0 + m) * p.K + k)));
             }
+            int xs[MR];
 #pragma unroll
-            for (int c = 0; c < CN; ++c) {
-                const int2 d = lut[(word[c] >> (j * fw)) & fmask];
+            for (int m = 0; m < MR; ++m) xs[m] = xv[m] >> 31;
 #pragma unroll
-                for (int m = 0; m < MR; ++m) acc[m][c] += (xv[m] >> d.x) * d.y;
-            }
+            for (int c = 0; c < CN; ++c) weight(c, j, xv, xs);
         }
     };
 
@@ -243,12 +282,18 @@ int launch_small(const GemmParams& p, cudaStream_t st)
     const uintptr_t pw = reinterpret_cast<uintptr_t>(p.packed);
     const int vecw = (p.dec.row_len % 4 == 0 && (pw & 15u) == 0) ? 4 : ((p.dec.row_len % 2 == 0 && (pw & 7u) == 0) ? 2 : 1);
     const dim3 grid((unsigned)gx, (unsigned)row_blocks);
-    if (p.in_kind == DS_IN_I32)
-        small_linear_kernel<MR, CN, INK_I32><<<grid, SM_THREADS, 0, st>>>(p, wpc, vecw);
-    else if (p.in_kind == DS_IN_I32_CLAMP)
-        small_linear_kernel<MR, CN, INK_I32_CLAMP><<<grid, SM_THREADS, 0, st>>>(p, wpc, vecw);
-    else
-        small_linear_kernel<MR, CN, INK_F32><<<grid, SM_THREADS, 0, st>>>(p, wpc, vecw);
+    auto go = [&](auto ink, auto dec) {
+        small_linear_kernel<MR, CN, decltype(ink)::value, decltype(dec)::value><<<grid, SM_THREADS, 0, st>>>(p, wpc, vecw);
+    };
+    auto kind = [&](auto dec) {
+        if (p.in_kind == DS_IN_I32) go(std::integral_constant<int, INK_I32>(), dec);
+        else if (p.in_kind == DS_IN_I32_CLAMP) go(std::integral_constant<int, INK_I32_CLAMP>(), dec);
+        else go(std::integral_constant<int, INK_F32>(), dec);
+    };
+    // M = 1, K = N = 4096: table 14.9 us, bits 11.8; 16 rows, in blocks of 8: 107, 98; but 4 rows 33, 37.
+    if (p.dec.base != 0 || MR == 2 || MR == 4) kind(std::integral_constant<int, DEC_TABLE>());
+    else if (p.dec.bits >= 5) kind(std::integral_constant<int, DEC_BITS>());
+    else kind(std::integral_constant<int, DEC_BITS_MASKED>());
     note_launch();
     return cudaGetLastError() == cudaSuccess ? DS_OK : DS_ERR_CUDA;
 }

@@ -232,7 +232,9 @@ __device__ __forceinline__ void add_partials(int* first, int splits)
                 for (int q = 0; q < 8; ++q)
                     t[j][q] = k + j < splits ? __ldcg(first + (long long)(k + j) * (BN * TC_ROWS) + (c + q) * TC_ROWS) : 0;
 #pragma unroll
-            for (int q = 0; q < 8; ++q) v[q] += t[0][q] + t[1][q] + t[2][q] + t[3][q];
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int q = 0; q < 8; ++q) v[q] += t[j][q];
         }
 #pragma unroll
         for (int q = 0; q < 8; ++q) __stcg(first + (c + q) * TC_ROWS, v[q]);
