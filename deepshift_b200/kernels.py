@@ -224,6 +224,9 @@ def _tc_run(x, conc_weight, bias, out, geometry, fuse, keep_weights):
     return True
 
 
+_FEW_MIN_WEIGHTS = 500_000   # below this ds_tc_few_bytes never takes a call
+
+
 @functools.lru_cache(maxsize=4096)
 def _few_bytes(M, K, N, bits, act_bits):
     n = ctypes.c_longlong(0)
@@ -300,7 +303,7 @@ def linear(input, shift, sign, bias=None, conc_weight=None, use_cuda=True, act_b
     f = _fuse(act_bits=ACT_BITS_AUTO if act_bits is None else act_bits,
               workspace=workspace(input.device) if M > 64 else None)
     with torch.cuda.device(input.device):
-        if M > 16 and _few_run(input, conc_weight, bias, out, M, K, N, f):
+        if M > 16 and N * K >= _FEW_MIN_WEIGHTS and _few_run(input, conc_weight, bias, out, M, K, N, f):
             return out
         if M > 64 and _tc_run(input, conc_weight, bias, out, (M, K, 1, 1, N, 1, 1, 1, 1, 0, 0), f, False):
             return out
@@ -364,17 +367,24 @@ def compress_sign_and_shift(shift, sign, comp_size, base, bits, row_length, num)
     return comp_weight
 
 
+_PACK_BYTES_FROM = 1 << 20   # weights from which one read of the parameters less pays for the bytes (2.5 us of host time)
+
+
 def pack_scan(shift, sign):
     """((smallest, largest, one in 16..31?), bytes) of the right shifts of fp32 parameters as ``compress_bits`` stores them,
-    or None when they are not all finite integers of at most 24 bits.  The bytes (``pack_codes``) are None when a shift does
-    not fit one.  Synchronises (the packing geometry depends on the range)."""
+    or None when they are not all finite integers of at most 24 bits.  The bytes (``pack_codes``) are None for small layers
+    and when a shift does not fit one.  Synchronises (the packing geometry depends on the range)."""
     device = shift.device
+    codes = None
     with torch.cuda.device(device):
         n = shift.numel()
         r = torch.empty(3, dtype=torch.int32, device=device)
-        codes = torch.empty(n, dtype=torch.uint8, device=device)
-        _ffi.check(_ffi.lib().ds_pack_scan_f32(shift.data_ptr(), sign.data_ptr(), n, codes.data_ptr(), r.data_ptr(),
-                                               _stream_ptr(device)), "pack_scan")
+        if n >= _PACK_BYTES_FROM:
+            codes = torch.empty(n, dtype=torch.uint8, device=device)
+            rc = _ffi.lib().ds_pack_scan_f32(shift.data_ptr(), sign.data_ptr(), n, codes.data_ptr(), r.data_ptr(), _stream_ptr(device))
+        else:
+            rc = _ffi.lib().ds_pack_range_f32(shift.data_ptr(), sign.data_ptr(), n, r.data_ptr(), _stream_ptr(device))
+        _ffi.check(rc, "pack_scan")
     hi, nlo, bad = r.tolist()
     if bad > 0:
         return None
