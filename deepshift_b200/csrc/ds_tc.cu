@@ -36,11 +36,11 @@ namespace {
 // phases away from it), and as many accumulator slots as the remaining columns hold: at least two, so
 // that the epilogue of a tile overlaps the next tile's MMAs.  Tiles of 192, 96 and 48 columns are 64, 32 and 16 channels of
 // a folded window.
-template <int BN, bool WIDE>
+template <int BN, bool WIDE, bool SHORT>
 struct TcTile {
     static constexpr int FOLD = BN % 3 == 0 ? TC_FOLD : 1;
     static constexpr int CH = BN / FOLD;             // channels
-    static constexpr int WG = WIDE || BN == 192 || BN == 48 ? 2 : 3;
+    static constexpr int WG = WIDE || SHORT || BN == 192 || BN == 48 ? 2 : 3;
     // Epilogue warpgroups, which take the tiles in turn: a folded tile of 16 channels may have three items only (4096
     // images, 32 x 32, with residual and codes: 498 -> 396 us; three and two warpgroups leave 80 registers, 819 us).
     static constexpr int EWG = BN == 48 ? 2 : 1;
@@ -50,7 +50,7 @@ struct TcTile {
     static constexpr int THREADS = (4 * WG + 4 * EWG + 2) * 32;  // + MMA warp + loader warp
     static constexpr int MMA_WARP = 4 * WG + 4 * EWG;
     // A slots, handed out round robin: item i fills slot i % SLOTS
-    static constexpr int SLOTS = (WIDE || BN >= 96 ? 1 : 2) * WG;
+    static constexpr int SLOTS = (WIDE || (BN >= 96 && !SHORT) ? 1 : 2) * WG;
     static constexpr int ACC_COLS = TC_TMEM_COLS - ASTRIDE * SLOTS;
     static constexpr int NACC = ACC_COLS / ACC < 4 ? ACC_COLS / ACC : 4;
     static constexpr int STAGE = BN * PLANES * TC_KG;
@@ -59,19 +59,19 @@ struct TcTile {
     static_assert(NACC >= 2 && NACC % EWG == 0 && STAGES > SLOTS, "slots");
 };
 
-template <int BN, bool WIDE>
+template <int BN, bool WIDE, bool SHORT>
 struct TcSmem {
-    alignas(128) unsigned char b[TcTile<BN, WIDE>::STAGES][TcTile<BN, WIDE>::STAGE];
-    alignas(8) unsigned long long bfull[TcTile<BN, WIDE>::STAGES];
-    unsigned long long full[TcTile<BN, WIDE>::SLOTS];   // both operands of the item in this slot are there
-    unsigned long long empty[TcTile<BN, WIDE>::SLOTS];  // its MMAs are done
+    alignas(128) unsigned char b[TcTile<BN, WIDE, SHORT>::STAGES][TcTile<BN, WIDE, SHORT>::STAGE];
+    alignas(8) unsigned long long bfull[TcTile<BN, WIDE, SHORT>::STAGES];
+    unsigned long long full[TcTile<BN, WIDE, SHORT>::SLOTS];   // both operands of the item in this slot are there
+    unsigned long long empty[TcTile<BN, WIDE, SHORT>::SLOTS];  // its MMAs are done
     unsigned long long accfull[6];
     unsigned long long accempty[6];
     unsigned long long done;
     unsigned tmem;
     int err;
     int last_flag[2];
-    alignas(16) int colc[TcTile<BN, WIDE>::EWG][2][BN];
+    alignas(16) int colc[TcTile<BN, WIDE, SHORT>::EWG][2][BN];
 };
 
 // Checked build: parts of the kernel that ds_tc_debug_waits keeps from doing their work, so that waits run out.
@@ -142,13 +142,12 @@ __device__ __forceinline__ void epi_bar(int group) { asm volatile("bar.sync %0, 
 // Epilogue of CC columns of one row, in steps: each step's condition is tested once for all columns (with the conditions
 // inside the loop over the columns the epilogue of a 1x1 layer took longer than its MMAs).
 
-// The residual of columns n.. at `o0`.
-template <int CC>
-__device__ __forceinline__ void load_residual(const TcRun& p, int (&r)[CC], int live, long long o0)
+// The residual of channels h..h+15 of those at `o0`, `live` of which exist.
+__device__ __forceinline__ void load_residual(const TcRun& p, int (&r)[16], int h, int live, long long o0)
 {
-    const int* q = p.residual + o0;
+    const int* q = p.residual + o0 + (long long)h * p.P;
 #pragma unroll
-    for (int c = 0; c < CC; ++c, q += p.P) r[c] = (c < live && DS_O_OK(p, p.residual, q, 4)) ? *q : 0;
+    for (int c = 0; c < 16; ++c, q += p.P) r[c] = (h + c < live && DS_O_OK(p, p.residual, q, 4)) ? *q : 0;
 }
 
 // v: the finished sums, residual included, at the row's outputs.  NEXT: the codes also (or only, when p.out is null) go
@@ -209,10 +208,10 @@ __device__ __forceinline__ void tc_store(const TcRun& p, int (&v)[CC], int n, in
 }
 
 template <int CC>
-__device__ __forceinline__ void add_residual(int (&v)[CC], const int (&r)[CC])
+__device__ __forceinline__ void add_residual(int (&v)[CC], const int (&r)[16], int h)
 {
 #pragma unroll
-    for (int c = 0; c < CC; ++c) v[c] = __float2int_rn(__int2float_rn(v[c]) + __int2float_rn(r[c]));
+    for (int c = 0; c < 16; ++c) v[h + c] = __float2int_rn(__int2float_rn(v[h + c]) + __int2float_rn(r[c]));
 }
 
 // Adds a row's partial sums of all splits into those of the first, 32 loads in flight.  A pass of its own: with the loads in
@@ -283,12 +282,12 @@ __device__ __forceinline__ void row_sums(int (&v)[CC], const int* colc, int c, b
     }
 }
 
-template <int BN, bool NEXT, bool WIDE>
-__global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(const TcRun p)
+template <int BN, bool NEXT, bool WIDE, bool SHORT>
+__global__ void __launch_bounds__(TcTile<BN, WIDE, SHORT>::THREADS, 1) tc_run_kernel(const TcRun p)
 {
-    using T = TcTile<BN, WIDE>;
+    using T = TcTile<BN, WIDE, SHORT>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    TcSmem<BN, WIDE>& s = *reinterpret_cast<TcSmem<BN, WIDE>*>(smem_raw);
+    TcSmem<BN, WIDE, SHORT>& s = *reinterpret_cast<TcSmem<BN, WIDE, SHORT>*>(smem_raw);
     if (p.gate) {
         const int found = *p.gate;
         if (p.report && blockIdx.x == 0 && threadIdx.x == 0) *p.report = found;
@@ -404,7 +403,10 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
         }
     } else if (warp < T::MMA_WARP) {
         // ---- epilogue ----------------------------------------------------------------------------------
-        constexpr int CC = 16;  // channels at a time: their sums, up to two neighbours', constants and residuals in registers
+        // Channels at a time.  16 of a folded window: their sums, a neighbour's, and residuals fetched ahead.  32 of a plain
+        // tile, with one wait for tensor memory and, at its end, for the residuals (16 at a time and fetched ahead: 36
+        // images of 5 channels, 82 x 82 -> 162 119 -> 147 us).
+        constexpr int CC = T::FOLD > 1 ? 16 : 32;
         const int row = threadIdx.x & 127;
         const unsigned lane_base = unsigned(warp & 3) << 21;
         const int eg = (warp - 4 * T::WG) >> 2;  // this epilogue warpgroup
@@ -442,18 +444,26 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
             const long long rowoff = (long long)px.b * p.OC * p.P + px.y * p.OW + ox;
             const unsigned nextoff = NEXT ? unsigned(px.b) * p.next_img + unsigned(px.y) * p.next_row + unsigned(ox) * p.next_px : 0u;
             const unsigned slot = acc % T::NACC;
-            int res[CC];
+            int res[16];
             // the residual is fetched ahead: of the first columns while the sums are still being made
             auto fetch = [&](int c) {
                 const int n = un.n0 + c;
-                if (p.residual && in && n < p.N) load_residual(p, res, p.N - n, rowoff + (long long)n * p.P);
+                if (T::FOLD > 1 && p.residual && in && n < p.N) load_residual(p, res, 0, p.N - n, rowoff + (long long)n * p.P);
             };
             auto finish = [&](int c, auto get) {
                 int v[CC];
                 row_sums<T::CH, T::FOLD>(v, s.colc[eg][par], c, left, right, get);
                 const int n = un.n0 + c;
-                if (p.residual) add_residual(v, res);
-                if (c + CC < T::CH) fetch(c + CC);
+                if (T::FOLD > 1) {
+                    if (p.residual) add_residual(v, res, 0);
+                    if (c + CC < T::CH) fetch(c + CC);
+                } else if (p.residual && in && n < p.N) {
+#pragma unroll
+                    for (int h = 0; h < CC; h += 16) {
+                        load_residual(p, res, h, p.N - n, rowoff + (long long)n * p.P);
+                        add_residual(v, res, h);
+                    }
+                }
                 if (in && n < p.N) tc_store<NEXT>(p, v, n, p.N - n, rowoff + (long long)n * p.P, nextoff);
             };
             if (p.splits == 1) fetch(0);
@@ -503,13 +513,20 @@ __global__ void __launch_bounds__(TcTile<BN, WIDE>::THREADS, 1) tc_run_kernel(co
                     __threadfence();
                     if (row == 0) p.counters[un.tile] = 0;  // for the next launch
                     int* all = p.partials + (long long)un.tile * p.splits * (BN * TC_ROWS) + row;
-                    add_partials<BN>(all, p.splits);
+                    if (T::FOLD > 1) add_partials<BN>(all, p.splits);
                     fetch(0);
 #pragma unroll 1
                     for (int c = 0; c < T::CH; c += CC)
                         finish(c, [&](int col, int (&v)[CC]) {
 #pragma unroll
                             for (int q = 0; q < CC; ++q) v[q] = __ldcg(all + (col + q) * TC_ROWS);
+                            if (T::FOLD == 1)
+#pragma unroll 1
+                                for (int k = 1; k < p.splits; ++k) {
+                                    const int* src = all + (long long)k * (BN * TC_ROWS) + col * TC_ROWS;
+#pragma unroll
+                                    for (int q = 0; q < CC; ++q) v[q] += __ldcg(src + q * TC_ROWS);
+                                }
                         });
                 }
                 epi_bar(eg);  // last_flag is read by all before the next unit writes it
@@ -966,15 +983,15 @@ __global__ void __launch_bounds__(256, 8) tc_pack_rows_kernel(const TcPack p, co
     if (over && p.flag) *p.flag = 1;
 }
 
-template <int BN, bool NEXT, bool WIDE>
+template <int BN, bool NEXT, bool WIDE, bool SHORT = false>
 int run_cfg(const TcRun& p0, cudaStream_t st)
 {
     TcRun p = p0;
     p.err_flag = kernel_error_flag();
     const int dev = device_slot();
     if (!p.err_flag || dev < 0) return DS_ERR_CUDA;
-    auto kern = tc_run_kernel<BN, NEXT, WIDE>;
-    const size_t smem = sizeof(TcSmem<BN, WIDE>);
+    auto kern = tc_run_kernel<BN, NEXT, WIDE, SHORT>;
+    const size_t smem = sizeof(TcSmem<BN, WIDE, SHORT>);
     static bool done[kMaxDevices];  // per instantiation and device
     static int sms[kMaxDevices];
     if (!done[dev]) {
@@ -988,7 +1005,7 @@ int run_cfg(const TcRun& p0, cudaStream_t st)
         done[dev] = true;
     }
     const int grid = p.units < sms[dev] ? p.units : sms[dev];
-    kern<<<grid, TcTile<BN, WIDE>::THREADS, smem, st>>>(p);
+    kern<<<grid, TcTile<BN, WIDE, SHORT>::THREADS, smem, st>>>(p);
     note_launch();
     return cudaGetLastError() == cudaSuccess ? DS_OK : DS_ERR_CUDA;
 }
@@ -1049,7 +1066,13 @@ static int launch_run(const TcRun& p, int BN, cudaStream_t st)
 {
     switch (BN) {
         case 192: return run_cfg<192, NEXT, false>(p, st);
-        case 128: return run_cfg<128, NEXT, false>(p, st);
+        case 128:
+            // Where K is shared or a tile has few items the epilogue sets the pace, and two producer warpgroups leave it more
+            // of the schedulers; in a long run three are faster.  Measured, us, three -> two: 7936 x 891 -> 377 (K shared)
+            // 102 -> 83, 51 images of 13 channels, 27 x 26, 7x7 -> 81 (K shared) 67 -> 50, 36 of 5, 82 x 82, 3x3 -> 162 (six
+            // items) 111 -> 102; but 8192 x 4096 -> 4096 1273 -> 1675 a call, 128 channels 28 x 28, 256 images 258 -> 295, 64
+            // images 79 -> 89.
+            return p.splits > 1 || p.G < 16 ? run_cfg<128, NEXT, false, true>(p, st) : run_cfg<128, NEXT, false>(p, st);
         case 96: return run_cfg<96, NEXT, false>(p, st);
         case 64: return run_cfg<64, NEXT, false>(p, st);
         case 48: return run_cfg<48, NEXT, false>(p, st);

@@ -159,6 +159,16 @@ __device__ __forceinline__ void tmem_st32(unsigned addr, const unsigned* v)
         : "memory");
 }
 
+__device__ __forceinline__ void tmem_ld(unsigned addr, int (&v)[32])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
+        "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n\ttcgen05.wait::ld.sync.aligned;"
+        : TC_W4(v, 0), TC_W4(v, 4), TC_W4(v, 8), TC_W4(v, 12), TC_W4(v, 16), TC_W4(v, 20), TC_W4(v, 24), TC_W4(v, 28)
+        : "r"(addr)
+        : "memory");
+}
+
 __device__ __forceinline__ void tmem_ld(unsigned addr, int (&v)[16])
 {
     asm volatile(
