@@ -23,7 +23,7 @@
 // 4096 x 4096: 1124 us = 122 T; 3x3 on 256 images, 64 channels 278 us = 106 T, 128 to 512 channels 253 to 257 us = 115 T).
 // Narrower tiles are bound by the producers, 177 ALU instructions per item and scheduler on a pipe that takes one every
 // other cycle (550 cycles per item of a plain tile of 64 columns, whose MMAs take 256): hence the folded windows.  Folded
-// tiles of 16 channels: 4096 images of 32 x 32, 313 us, 393 with residuals and codes; 2700 cycles for three items, of
+// tiles of 16 channels: 4096 images of 32 x 32, 309 us, 371 with residuals and codes; 2650 cycles for three items, of
 // which the MMAs take 576 and the ALU pipe 1440.
 #include "ds_tc_ptx.cuh"
 
