@@ -1,0 +1,23 @@
+"""Which 3-wide windows lie side by side in a tile (a "folded" window), as far as that needs no GPU."""
+import pytest
+
+
+def _columns(B, C, H, W, OC, pad, stride=1):
+    from deepshift_b200 import _ffi, kernels
+    f = kernels._fuse(_ffi.IN_F32_CONV, 0, 4, 12)
+    return _ffi.lib().ds_tc_columns(B, C, H, W, OC, 3, 3, stride, stride, pad, pad, 6, 0, f)
+
+
+@pytest.mark.parametrize("channels,width,folded", [
+    (256, 3, False), (256, 7, False), (256, 14, False), (512, 7, False), (512, 10, False), (512, 14, False),
+    (64, 3, False), (32, 3, False), (16, 3, False), (64, 56, True), (32, 16, True), (16, 32, True)])
+@pytest.mark.parametrize("batch", [1, 64, 4096])
+def test_windows_without_padding_count_the_pixels_that_own_no_output(channels, width, folded, batch):
+    """The rows of a folded window are the pixels of the image, W of them for W - 2 outputs."""
+    columns = _columns(batch, channels, width, width, channels, 0)
+    assert (columns % 3 == 0) == folded and columns > 0
+
+
+@pytest.mark.parametrize("channels,width", [(256, 14), (512, 7), (64, 56), (32, 16), (16, 32)])
+def test_padded_windows_stay_folded(channels, width):
+    assert _columns(64, channels, width, width, channels, 1) % 3 == 0
