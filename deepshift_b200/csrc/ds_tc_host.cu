@@ -243,8 +243,15 @@ bool worthwhile(const TcGeom& g, const ds_fuse_t& f)
         const double waves = tiles >= kSms ? double((tiles + kSms - 1) / kSms) : tiles * 4 >= kSms ? (double)tiles / kSms : 0.25;
         if (waves * g.K * (g.N > 64 ? 0.23 : 0.13) < 20) return false;
     }
-    const double padded = (double)g.grid_m * TC_ROWS * g.grid_n * g.BN * g.G * TC_KG;
-    return tiles <= 16 ? ops >= 6e6 : ops >= double(1 << 26) && ops * 5 >= padded;
+    auto padded = [](const TcGeom& t) { return (double)t.grid_m * TC_ROWS * t.grid_n * t.BN * t.G * TC_KG; };
+    double least = padded(g);
+    if (g.fold > 1) {  // chosen because it takes less time, often with more padding: never a reason to refuse
+        TcGeom h = g;
+        choose_pixel(h, 1);
+        choose_tile(h);
+        if (padded(h) < least) least = padded(h);
+    }
+    return tiles <= 16 ? ops >= 6e6 : ops >= double(1 << 26) && ops * 5 >= least;
 }
 
 }  // namespace

@@ -21,3 +21,12 @@ def test_windows_without_padding_count_the_pixels_that_own_no_output(channels, w
 @pytest.mark.parametrize("channels,width", [(256, 14), (512, 7), (64, 56), (32, 16), (16, 32)])
 def test_padded_windows_stay_folded(channels, width):
     assert _columns(64, channels, width, width, channels, 1) % 3 == 0
+
+
+@pytest.mark.parametrize("C,OC,W", [(5, 17, 56), (5, 21, 56), (5, 33, 56), (5, 43, 56), (5, 20, 32), (5, 40, 32), (6, 18, 56),
+                                    (6, 34, 56), (6, 17, 32), (6, 34, 32), (80, 4, 64), (114, 6, 12)])
+def test_padding_of_one_form_never_makes_a_layer_unserved(C, OC, W):
+    """Of one form's tiles less than a fifth of the product is live, of the other's more."""
+    from deepshift_b200 import _ffi, kernels, utils
+    f = kernels._fuse(_ffi.IN_F32_CONV, 0, 4, 12)
+    assert kernels.tc_bytes((256, C, W, W, OC, 3, 3, 1, 1, 1, 1), utils.ConcWeight(None, 0, 6), f)[0] > 0
