@@ -144,18 +144,22 @@ int tc_geometry(TcGeom& g, int B, int C, int H, int W, int OC, int KH, int KW, i
     g.M = int(M); g.K = int(K); g.N = OC; g.P = int(oh * ow);
     choose_pixel(g, 1);
     // A folded window's rows are the pixels of an image row, its outputs W + 2 pw - 2 of them, so the times of all rows are
-    // compared.  Folded where a long run is not slower, whatever the batch: a layer's weights then have three layouts at
-    // most.  Measured, us, plain -> folded, padding 1:
+    // compared.  Folded where a long run is not slower, with padding whatever the batch: a layer's weights then have three
+    // layouts at most.  Measured, us, plain -> folded, padding 1:
     // 64 channels 56 x 56, 256 images 447 -> 278, one 14.8 -> 10.8; 32 channels 16 x 16, 4096 images 314 -> 160; 16 channels
     // 32 x 32 679 -> 313; 256 channels 14 x 14, 256 images 268 -> 258, 64 images 95 -> 74 (finer units), one 18.2 -> 14.8;
     // 512 channels 7 x 7 263 -> 253, 96 -> 83, 22.9 -> 19.0.  128 channels 28 x 28: 257 -> 264, 78 -> 76, 14.9 -> 12.8; layers
     // that one plain tile of 128 columns covers stay plain.  Without padding, 64 images, a call: 512 channels 7 x 7 72 -> 133,
-    // 14 x 14 203 -> 233, 256 channels 14 x 14 60 -> 89, 28 x 28 258 -> 286 (all plain); 64 channels 56 x 56 152 -> 100.
+    // 14 x 14 203 -> 233, 256 channels 14 x 14 60 -> 89, 28 x 28 258 -> 286 (all plain); 64 channels 56 x 56 152 -> 100.  One
+    // wave of folded tiles, GPU time: 64 channels 3 x 3, 1024 images 14.3 -> 12.8, 256 channels 7 x 7, 64 images 33.1 -> 32.5,
+    // 512 channels 7 x 7, one 23.0 -> 22.0; two waves, 256 channels 10 x 10, 64 images 44 -> 57.
     if (KW == TC_FOLD && g.sw == 1 && pw <= 1 && (OC <= 64 || OC > 128)) {
         TcGeom f = g;
         choose_pixel(f, TC_FOLD);
-        if (f.rows <= limit && pixels * f.Cp <= limit && OC <= 65535 * 16 &&
-            cycles_per_block(f) * double(f.rows) < 1.05 * cycles_per_block(g) * double(g.rows))
+        // One wave: the longest unit counts, and a folded one has a third of the items.  pw = 1: both have the same rows.
+        const bool wave = (f.rows + 4ll * f.lanes - 1) / (4 * f.lanes) * ((OC + 63) / 64) <= kSms;
+        const double most = wave ? 1.05 : 1.05 * double(g.rows) / double(f.rows);
+        if (f.rows <= limit && pixels * f.Cp <= limit && OC <= 65535 * 16 && cycles_per_block(f) < most * cycles_per_block(g))
             g = f;
     }
     choose_tile(g);

@@ -8,12 +8,14 @@ def _columns(B, C, H, W, OC, pad, stride=1):
     return _ffi.lib().ds_tc_columns(B, C, H, W, OC, 3, 3, stride, stride, pad, pad, 6, 0, f)
 
 
-@pytest.mark.parametrize("channels,width,folded", [
-    (256, 3, False), (256, 7, False), (256, 14, False), (512, 7, False), (512, 10, False), (512, 14, False),
-    (64, 3, False), (32, 3, False), (16, 3, False), (64, 56, True), (32, 16, True), (16, 32, True)])
-@pytest.mark.parametrize("batch", [1, 64, 4096])
-def test_windows_without_padding_count_the_pixels_that_own_no_output(channels, width, folded, batch):
-    """The rows of a folded window are the pixels of the image, W of them for W - 2 outputs."""
+@pytest.mark.parametrize("batch,channels,width,folded", [
+    (64, 256, 10, False), (64, 256, 14, False), (64, 512, 7, False), (64, 512, 14, False), (64, 256, 28, False),
+    (40000, 64, 3, False), (40000, 32, 3, False), (40000, 16, 3, False), (4096, 256, 3, False), (4096, 512, 10, False),
+    (64, 64, 56, True), (4096, 32, 16, True), (4096, 16, 32, True),
+    (1024, 64, 3, True), (64, 256, 7, True), (1, 512, 7, True), (1, 256, 14, True), (2, 32, 3, True)])
+def test_windows_without_padding_count_the_pixels_that_own_no_output(batch, channels, width, folded):
+    """The rows of a folded window are the pixels of the image, W of them for W - 2 outputs: what counts in more than one
+    wave of tiles."""
     columns = _columns(batch, channels, width, width, channels, 0)
     assert (columns % 3 == 0) == folded and columns > 0
 
