@@ -1067,12 +1067,13 @@ static int launch_run(const TcRun& p, int BN, cudaStream_t st)
     switch (BN) {
         case 192: return run_cfg<192, NEXT, false>(p, st);
         case 128:
-            // Where K is shared or a tile has few items the epilogue sets the pace, and two producer warpgroups leave it more
-            // of the schedulers; in a long run three are faster.  Measured, us, three -> two: 7936 x 891 -> 377 (K shared)
-            // 102 -> 83, 51 images of 13 channels, 27 x 26, 7x7 -> 81 (K shared) 67 -> 50, 36 of 5, 82 x 82, 3x3 -> 162 (six
-            // items) 111 -> 102; but 8192 x 4096 -> 4096 1273 -> 1675 a call, 128 channels 28 x 28, 256 images 258 -> 295, 64
-            // images 79 -> 89.
-            return p.splits > 1 || p.G < 16 ? run_cfg<128, NEXT, false, true>(p, st) : run_cfg<128, NEXT, false>(p, st);
+            // Where K is shared, or several column tiles of few items each, the epilogue sets the pace, and two producer
+            // warpgroups leave it more of the schedulers; elsewhere three are faster.  Measured, us, three -> two.  K shared:
+            // 7936 x 891 -> 377 102 -> 85, 700 x 4096 -> 500 46 -> 36, 16 images of 256 channels, 14 x 14, 3x3 -> 128 37 -> 28,
+            // 1000 x 2048 -> 1000 34 -> 35.  1x1 on 36 images of 82 x 82: -> 162 channels, six items 109 -> 103, eight 127 -> 119,
+            // nine 126 -> 119, ten 132 -> 137; -> 256, eight 127 -> 118, nine 121 -> 128, ten 129 -> 147; -> 128 (one column
+            // tile), six 52 -> 54, nine 64 -> 70, ten 69 -> 80.  28 x 28, 256 images -> 128, fourteen 72 -> 88, 36 (3x3) 134 -> 152.
+            return p.splits > 1 || (p.grid_n > 1 && p.G <= 8) ? run_cfg<128, NEXT, false, true>(p, st) : run_cfg<128, NEXT, false>(p, st);
         case 96: return run_cfg<96, NEXT, false>(p, st);
         case 64: return run_cfg<64, NEXT, false>(p, st);
         case 48: return run_cfg<48, NEXT, false>(p, st);
