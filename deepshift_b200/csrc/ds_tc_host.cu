@@ -1,6 +1,8 @@
 // Tensor-core path: geometry, tile choice and the ds_tc_* entry points.  Kernels: ds_tc.cu.
 #include "ds_tc.cuh"
 
+#include <algorithm>
+
 namespace ds {
 
 int* bounds_status_ptr();
@@ -64,18 +66,31 @@ bool tile_fits(const TcGeom& g, int bn)
     return g.wide ? bn == 64 : bn == kTiles[g.fold > 1][2] || g.N > bn / g.fold / 2;
 }
 
-// Cycles that 128 rows of a long run take with the best tile.
+// Cycles of one tile in a long run: its items, and what of the epilogue they don't hide.  Fitted to 3x3 layers of 3 to 96
+// channels (1 to 18 items of a folded tile, 3 to 54 of a plain one) and 256 images of 14 x 14 and 7 x 7; within 10 %.
+double tile_cycles(int bn, double items)
+{
+    switch (bn) {
+        case 32: return 520 * items + 1500;
+        case 64: return 540 * items + 2100;
+        case 128: return 540 * items + 3000;
+        case 48: return 650 * items + 1400;
+        case 96: return std::max(390 * items + 3600, 600 * items + 1700);  // the epilogue's pace, the producers'
+        default: return std::max(600 * items + 4200, 780 * items + 2000);  // 192: the epilogue's, the MMAs'
+    }
+}
+
+// Cycles that 128 rows of a long run take with the best tile, and the packing of as many pixels beyond what each layer has.
 double cycles_per_block(const TcGeom& g)
 {
     double best = 1e30;
     for (int bn : kTiles[g.fold > 1]) {
         if (!tile_fits(g, bn)) continue;
         const int ch = bn / g.fold;
-        const double item = bn == 128 ? 560 : bn == 192 ? 780 : item_cycles(bn, false);
-        const double c = double((g.N + ch - 1) / ch) * (g.G * item + (g.fold > 1 ? 1000 : 300)) * 32 / g.lanes;
+        const double c = double((g.N + ch - 1) / ch) * tile_cycles(bn, g.G) * 32 / g.lanes;
         if (c < best) best = c;
     }
-    return best;
+    return best + 30.0 * g.Cp;
 }
 
 // Tile and split with the smallest estimated time: waves of units over the SMs, a unit being the longer of
@@ -143,24 +158,25 @@ int tc_geometry(TcGeom& g, int B, int C, int H, int W, int OC, int KH, int KW, i
     g.Hp = int(hp); g.Wp = int(wp); g.OH = int(oh); g.OW = int(ow);
     g.M = int(M); g.K = int(K); g.N = OC; g.P = int(oh * ow);
     choose_pixel(g, 1);
-    // A folded window's rows are the pixels of an image row, its outputs W + 2 pw - 2 of them, so the times of all rows are
-    // compared.  Folded where a long run is not slower, with padding whatever the batch: a layer's weights then have three
-    // layouts at most.  Measured, us, plain -> folded, padding 1:
+    // A folded window's rows are the pixels of an image row, its outputs W + 2 pw - 2 of them, so in a long run the times of
+    // all rows are compared; in one wave the longest unit counts, and a folded one has a third of the items.  A layer's
+    // weights have up to three layouts of either form, whatever the batches.  Measured, us, plain -> folded, padding 1:
     // 64 channels 56 x 56, 256 images 447 -> 278, one 14.8 -> 10.8; 32 channels 16 x 16, 4096 images 314 -> 160; 16 channels
     // 32 x 32 679 -> 313; 256 channels 14 x 14, 256 images 268 -> 258, 64 images 95 -> 74 (finer units), one 18.2 -> 14.8;
     // 512 channels 7 x 7 263 -> 253, 96 -> 83, 22.9 -> 19.0.  128 channels 28 x 28: 257 -> 264, 78 -> 76, 14.9 -> 12.8; layers
-    // that one plain tile of 128 columns covers stay plain.  Without padding, 64 images, a call: 512 channels 7 x 7 72 -> 133,
-    // 14 x 14 203 -> 233, 256 channels 14 x 14 60 -> 89, 28 x 28 258 -> 286 (all plain); 64 channels 56 x 56 152 -> 100.  One
-    // wave of folded tiles, GPU time: 64 channels 3 x 3, 1024 images 14.3 -> 12.8, 256 channels 7 x 7, 64 images 33.1 -> 32.5,
-    // 512 channels 7 x 7, one 23.0 -> 22.0; two waves, 256 channels 10 x 10, 64 images 44 -> 57.
+    // that one plain tile of 128 columns covers stay plain.  Few items, 64 images of 56 x 56, with the packing: 5 -> 20
+    // channels 32 -> 39, 8 -> 64 37 -> 51, 16 -> 144 111 -> 121, 17 -> 48 65 -> 62, 32 -> 160 161 -> 149, 96 -> 256 428 -> 444;
+    // 24 -> 144 140 -> 152, but 14 x 14, 256 images 51 -> 47.  One wave: 96 -> 256, 28 x 28, 16 images 59 -> 39, 24 -> 144, 14 x
+    // 14, eight 12.0 -> 10.4.  Without padding, 64 images: 512 channels 7 x 7 72 -> 133, 14 x 14 203 -> 233, 256 channels 14 x
+    // 14 60 -> 89, 28 x 28 258 -> 286, 64 channels 56 x 56 152 -> 100; one wave, 1024 images of 64 channels, 3 x 3 14.3 -> 12.8,
+    // 256 channels 7 x 7 33.1 -> 32.5; two, 256 channels 10 x 10 44 -> 57.
     if (KW == TC_FOLD && g.sw == 1 && pw <= 1 && (OC <= 64 || OC > 128)) {
         TcGeom f = g;
         choose_pixel(f, TC_FOLD);
-        // One wave: the longest unit counts, and a folded one has a third of the items.  pw = 1: both have the same rows.
         const bool wave = (f.rows + 4ll * f.lanes - 1) / (4 * f.lanes) * ((OC + 63) / 64) <= kSms;
-        const double most = wave ? 1.05 : 1.05 * double(g.rows) / double(f.rows);
-        if (f.rows <= limit && pixels * f.Cp <= limit && OC <= 65535 * 16 && cycles_per_block(f) < most * cycles_per_block(g))
-            g = f;
+        const bool faster = wave ? f.G < g.G
+                                 : cycles_per_block(f) * double(f.rows) < 1.05 * cycles_per_block(g) * double(g.rows);
+        if (f.rows <= limit && pixels * f.Cp <= limit && OC <= 65535 * 16 && faster) g = f;
     }
     choose_tile(g);
     if (pixels * g.Cp > limit) return DS_ERR_UNSUPPORTED;

@@ -32,3 +32,13 @@ def test_padding_of_one_form_never_makes_a_layer_unserved(C, OC, W):
     from deepshift_b200 import _ffi, kernels, utils
     f = kernels._fuse(_ffi.IN_F32_CONV, 0, 4, 12)
     assert kernels.tc_bytes((256, C, W, W, OC, 3, 3, 1, 1, 1, 1), utils.ConcWeight(None, 0, 6), f)[0] > 0
+
+
+@pytest.mark.parametrize("C,OC,W,batch,folded", [
+    (5, 17, 56, 64, False), (5, 64, 56, 64, False), (8, 32, 32, 256, False), (8, 48, 14, 256, False), (12, 144, 28, 64, False),
+    (16, 192, 56, 64, False), (3, 64, 224, 64, False), (96, 256, 56, 64, False), (8, 16, 32, 256, True), (17, 33, 56, 64, True),
+    (24, 32, 28, 64, True), (32, 160, 56, 64, True), (40, 144, 28, 64, True), (256, 256, 14, 64, True), (512, 512, 7, 256, True),
+    (512, 160, 7, 256, True), (24, 144, 14, 8, True), (96, 256, 28, 1, True), (48, 256, 32, 4, True), (3, 64, 14, 1, False)])
+def test_few_items_do_not_hide_the_epilogue_of_a_folded_tile(C, OC, W, batch, folded):
+    """Three items of 96 or 192 columns take less time than their epilogue: that counts in long runs."""
+    assert (_columns(batch, C, W, W, OC, 1) % 3 == 0) == folded
