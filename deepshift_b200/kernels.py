@@ -372,15 +372,20 @@ _PACK_BYTES_FROM = 1 << 20   # weights from which one read of the parameters les
 
 def pack_scan(shift, sign):
     """((smallest, largest, one in 16..31?), bytes) of the right shifts of fp32 parameters as ``compress_bits`` stores them,
-    or None when they are not all finite integers of at most 24 bits.  The bytes (``pack_codes``) are None for small layers
-    and when a shift does not fit one.  Synchronises (the packing geometry depends on the range)."""
+    or None when they are not all finite integers of at most 24 bits.  The bytes (``pack_codes``) are None for small layers,
+    when a shift does not fit one and when there is no memory for them.  Synchronises (the packing geometry depends on the
+    range)."""
     device = shift.device
     codes = None
     with torch.cuda.device(device):
         n = shift.numel()
         r = torch.empty(3, dtype=torch.int32, device=device)
         if n >= _PACK_BYTES_FROM:
-            codes = torch.empty(n, dtype=torch.uint8, device=device)
+            try:
+                codes = torch.empty(n, dtype=torch.uint8, device=device)
+            except torch.OutOfMemoryError:
+                pass
+        if codes is not None:
             rc = _ffi.lib().ds_pack_scan_f32(shift.data_ptr(), sign.data_ptr(), n, codes.data_ptr(), r.data_ptr(), _stream_ptr(device))
         else:
             rc = _ffi.lib().ds_pack_range_f32(shift.data_ptr(), sign.data_ptr(), n, r.data_ptr(), _stream_ptr(device))
@@ -388,7 +393,7 @@ def pack_scan(shift, sign):
     hi, nlo, bad = r.tolist()
     if bad > 0:
         return None
-    return (-nlo, hi, bad == 0), codes if hi <= 63 and nlo <= 64 else None
+    return (-nlo, hi, bad == 0), (codes if hi <= 63 and nlo <= 64 else None)
 
 
 def pack_codes(codes, OC, bits, base):
