@@ -26,7 +26,7 @@ constexpr int SM_THREADS = SM_WARPS * 32;
 // How a field is decoded.  From its bits where base == 0: the shift is a funnel shift by the field's low five bits (masked
 // below five), the multiplier -1, 0 or 1 a signed two-bit extract from a word made once per packed word.  With a table in
 // shared memory, the only way before, the reads and the queue they share were what the kernel waited for (M = 1, K = N = 4096:
-// 14.9 us); left shifts (base < 0) still take it.
+// 14.9 us); left shifts (base < 0) still take it, and where it is faster (decode_from_bits).
 enum { DEC_TABLE = 0, DEC_BITS, DEC_BITS_MASKED };
 
 template <int MR, int CN, int INK, int DEC>
@@ -103,8 +103,7 @@ __global__ void __launch_bounds__(SM_THREADS) small_linear_kernel(const GemmPara
                 if (m0 + m >= p.M) xv[m][0] = xv[m][1] = xv[m][2] = xv[m][3] = 0;
             }
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-{
+            for (int j = 0; j < 4; ++j) {
                 int xj[MR], xs[MR];
 #pragma unroll
                 for (int m = 0; m < MR; ++m) {
@@ -132,8 +131,7 @@ __global__ void __launch_bounds__(SM_THREADS) small_linear_kernel(const GemmPara
                     if (m0 + m >= p.M) xv[m][0] = xv[m][1] = 0;
                 }
 #pragma unroll
-                for (int jj = 0; jj < 2; ++jj)
-{
+                for (int jj = 0; jj < 2; ++jj) {
                     int xj[MR], xs[MR];
 #pragma unroll
                     for (int m = 0; m < MR; ++m) {
@@ -266,6 +264,33 @@ __global__ void __launch_bounds__(SM_THREADS) small_linear_kernel(const GemmPara
         }
 }
 
+// Which decoding is faster (base == 0 only).  Measured, us of GPU time, table -> bits, K x N.
+//   One row: the bits win once the table's reads queue up, for masked fields, which cost two more instructions, later; 2-bit
+//   fields never.  6 bits 4096 x 4096 14.8 -> 11.4, 2048 x 1024 4.9 -> 4.7, 1024 x 1024 4.5 -> 4.6; 5 bits 2048 x 2048 6.8 ->
+//   6.4, 300 x 4096 6.2 -> 6.6; 4 bits 2048 x 4096 11.6 -> 10.0, 4096 x 1024 6.0 -> 6.5, 1024 x 1024 3.8 -> 4.2; 3 bits 4096 x
+//   4096 21.0 -> 15.5, 2048 x 2048 7.7 -> 7.1, 1024 x 1024 6.5 -> 7.1; 2 bits 4096 x 4096 12.1 -> 13.4; 1 bit 23.8 -> 19.8, 2048
+//   x 2048 10.0 -> 10.6.  fp32 input, 6 bits: 4096 x 4096 16.8 -> 13.5, 3113 x 631 6.7 -> 7.3.
+//   Two and four rows: 4096 x 4096, four 33 -> 37.
+//   Blocks of eight rows: 6 bits where a lane has a whole 16-byte group of words, or rows allow none: 16 rows of 4096 x 4096
+//   107 -> 101, 8 of 4095 x 1000 36.2 -> 33.5, but 16 of 1024 x 1024 35.5 -> 38.2, 8 of 1024 x 4096 63 -> 70.  5 bits, 16 of 4096
+//   x 4096 117 -> 128; 4 bits 106 -> 98, odd K, 5 of 2047 x 2047 37.2 -> 39.7; 1 to 3 bits 8 of 2048 x 2048 53 -> 48 (3).  fp32
+//   input, 16 of 2048 x 2048 142 -> 148.
+template <int MR>
+bool decode_from_bits(const GemmParams& p, int wpc, int vecw)
+{
+    if (p.dec.base != 0 || MR == 2 || MR == 4) return false;
+    const int bits = p.dec.bits;
+    const bool f32 = p.in_kind != DS_IN_I32 && p.in_kind != DS_IN_I32_CLAMP;
+    if (MR == 1) {
+        const double weights = double(p.N) * p.K;
+        if (weights < (bits == 1 ? 8e6 : bits <= 4 || f32 ? 4e6 : bits == 5 ? 2e6 : 1.2e6)) return false;
+        return bits != 2 && (bits != 4 || (p.N >= p.K && !f32));
+    }
+    if (f32 || bits == 5) return false;
+    if (bits >= 6) return p.K % 4 != 0 || vecw != 4 || p.dec.row_len >= 128 * wpc;
+    return bits != 4 || p.K % 2 == 0;
+}
+
 template <int MR, int CN>
 int launch_small(const GemmParams& p, cudaStream_t st)
 {
@@ -290,8 +315,7 @@ int launch_small(const GemmParams& p, cudaStream_t st)
         else if (p.in_kind == DS_IN_I32_CLAMP) go(std::integral_constant<int, INK_I32_CLAMP>(), dec);
         else go(std::integral_constant<int, INK_F32>(), dec);
     };
-    // M = 1, K = N = 4096: table 14.9 us, bits 11.8; 16 rows, in blocks of 8: 107, 98; but 4 rows 33, 37.
-    if (p.dec.base != 0 || MR == 2 || MR == 4) kind(std::integral_constant<int, DEC_TABLE>());
+    if (!decode_from_bits<MR>(p, wpc, vecw)) kind(std::integral_constant<int, DEC_TABLE>());
     else if (p.dec.bits >= 5) kind(std::integral_constant<int, DEC_BITS>());
     else kind(std::integral_constant<int, DEC_BITS_MASKED>());
     note_launch();
