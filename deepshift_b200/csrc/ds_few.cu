@@ -24,6 +24,8 @@
 // MMAs (576 cycles per item).
 #include "ds_tc_ptx.cuh"
 
+#include <algorithm>
+
 namespace ds {
 
 int* bounds_status_ptr();
@@ -490,7 +492,9 @@ bool few_geometry(FewGeom& g, int M, int K, int N, int bits)
 // Whether this path beats the others.  Measured, us a call, range measured, other path (integer up to 64 rows, expanded
 // weights above) -> this one: 17 x 4096 -> 4096 133 -> 39, 64 x 4096 -> 4096 138 -> 42, 64 x 1024 -> 4096 46 -> 35, 64 x 1024 ->
 // 1024 20 -> 24, 64 x 2048 -> 1024 28 -> 35, 128 x 4096 -> 4096 175 -> 51, 256 x 1024 -> 1024 42 -> 28, 512 x 4096 -> 4096 203 -> 134,
-// 1024 x 4096 -> 4096 324 -> 284, 2000 x 4096 -> 4096 439 -> 473.  With a promise 64 x 4096 -> 4096 98 -> 38, 64 x 1024 -> 1024 18 -> 22.
+// 1024 x 4096 -> 4096 324 -> 284, 2000 x 4096 -> 4096 439 -> 473.  With a promise 64 x 4096 -> 4096 98 -> 38, 64 x 1024 -> 1024 18 -> 22;
+// above 64 rows the other path is then the FP32 pipe in one launch (ds_tc_host.cu, promised_linear): 80 x 1500 -> 400 23 -> 28,
+// 200 x 1216 -> 256 23 -> 28, 65 x 4096 -> 10 31 -> 29, 128 x 2048 -> 1000 31 -> 28, 128 x 4096 -> 1000 52 -> 29.
 // The 15 % keep calls at the crossing where they were.
 bool few_worthwhile(const FewGeom& g, int M, int K, int N, int mode)
 {
@@ -500,6 +504,10 @@ bool few_worthwhile(const FewGeom& g, int M, int K, int N, int mode)
     double there;
     if (M <= 64) there = 6 + 64 * weights / (mode == 2 ? 7.9e6 : 11.6e6);
     else there = 22 + 0.005 * K + 6.5e-6 * weights + (double)((M + 127) / 128 * 128) * weights / 100e6;
+    if (M > 64 && mode == 1) {
+        const double pipe = 8 + 0.09e-6 * ((M + 63) / 64 * 64) * (double)K * ((N + 127) / 128 * 128), depth = 1 + 0.0072 * K;
+        there = std::min(there, std::max({21.0, pipe, depth}));
+    }
     return (here > 26 ? here : 26) < 0.85 * there;
 }
 
