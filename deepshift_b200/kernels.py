@@ -224,7 +224,11 @@ def _tc_run(x, conc_weight, bias, out, geometry, fuse, keep_weights):
     return True
 
 
-_FEW_MIN_WEIGHTS = 500_000   # below this ds_tc_few_bytes never takes a call
+def _few_asked(M, weights):
+    """False for calls that ds_tc_few_bytes never takes, told apart before the question: up to 16 rows, and up to 64 with
+    fewer weights than the other path gets done in the 26 us that a call takes here at least, less its margin of 15 %.  Above 64
+    rows there is no such bound: 65 x 1728 -> 10 takes 36 us there, 29 here."""
+    return M > 64 or (M > 16 and weights > 3_000_000)
 
 
 @functools.lru_cache(maxsize=4096)
@@ -303,7 +307,7 @@ def linear(input, shift, sign, bias=None, conc_weight=None, use_cuda=True, act_b
     f = _fuse(act_bits=ACT_BITS_AUTO if act_bits is None else act_bits,
               workspace=workspace(input.device) if M > 64 else None)
     with torch.cuda.device(input.device):
-        if M > 16 and N * K >= _FEW_MIN_WEIGHTS and _few_run(input, conc_weight, bias, out, M, K, N, f):
+        if _few_asked(M, N * K) and _few_run(input, conc_weight, bias, out, M, K, N, f):
             return out
         if M > 64 and _tc_run(input, conc_weight, bias, out, (M, K, 1, 1, N, 1, 1, 1, 1, 0, 0), f, False):
             return out
