@@ -46,14 +46,17 @@ struct FewParams {
     int* flag;           // whole call; the blocks' flags at flag + 4
     int* report;         // as in TcRun
     unsigned char* planes;
-    int M, K, N, row_len, G, wpg, kpg;
+    int M, K, N, row_len, G, kpg;
     int grid_m, grid_n, splits, gps, units, rpt;  // rpt: rows of x per tile, the last column is the row of zeros
     int blocks;          // of few_pack
     int gated;           // the range is measured
     int zero_out;
     unsigned wait_ns;
     int* err_flag;
+    int hold;            // checked build: see ds_tc_debug_waits
     long long chk_x_bytes, chk_w_bytes, chk_o_bytes;
+    const unsigned char* chk_act;  // the whole scratch
+    long long chk_act_bytes;
     int* chk_status;
 };
 
@@ -116,7 +119,8 @@ __global__ void __launch_bounds__(256) few_pack_kernel(const FewParams p)
         }
         uint4* dst = reinterpret_cast<uint4*>(p.planes) + ((long long)tg * TC_PLANES * BN + r);
 #pragma unroll
-        for (int f = 0; f < TC_PLANES; ++f) dst[f * BN] = make_uint4(v[4 * f], v[4 * f + 1], v[4 * f + 2], v[4 * f + 3]);
+        for (int f = 0; f < TC_PLANES; ++f)
+            if (DS_A_OK(p, dst + f * BN, 16)) dst[f * BN] = make_uint4(v[4 * f], v[4 * f + 1], v[4 * f + 2], v[4 * f + 3]);
     }
     if (p.zero_out) {
         const long long n = (long long)p.M * p.N;
@@ -267,7 +271,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) few_run_kernel(const FewParams
                 transpose4(a[0].w, a[1].w, a[2].w, a[3].w, v[48 + q], v[52 + q], v[56 + q], v[60 + q]);
             }
             const bool ok = use == 0 || bar_wait(&s.empty[wg], (use - 1) & 1u, err, p.wait_ns);
-            if (!__all_sync(0xFFFFFFFFu, ok)) break;  // the whole warp, or none of it
+            if (!__all_sync(0xFFFFFFFFu, ok) || TC_HELD(p, 2)) break;  // the whole warp, or none of it
             tc_fence_after();
             tmem_st32(at, v);
             tmem_st32(at + 32, v + 32);
@@ -306,7 +310,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) few_run_kernel(const FewParams
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) bar_arrive(&s.accempty[slot]);
+            if (lane == 0 && !TC_HELD(p, 4)) bar_arrive(&s.accempty[slot]);
         }
     } else if (warp == 4 * FEW_WG + 4) {
         // ---- MMA issue: one lane, one wait and one commit per item, asked ahead (ds_tc.cu) -------------------
@@ -357,13 +361,14 @@ __global__ void __launch_bounds__(FEW_THREADS, 1) few_run_kernel(const FewParams
             unsigned lst = 0, issued = 0;
             auto fetch = [&]() {
                 while (lleft == 0) {
-                    if (lu >= p.units) return;
+                    if (lu >= p.units || TC_HELD(p, 1)) return;
                     const FewUnit un = few_unit(p, lu);
                     src = p.planes + ((long long)un.mt * p.G + un.g0) * T::STAGE;
                     lleft = un.g1 - un.g0;
                     lu += gridDim.x;
                 }
-                bulk_load(s32(&s.b[lst][0]), src, T::STAGE, &s.bfull[lst]);
+                if (DS_A_OK(p, src, T::STAGE)) bulk_load(s32(&s.b[lst][0]), src, T::STAGE, &s.bfull[lst]);
+                else bar_arrive(&s.bfull[lst]);
                 src += T::STAGE;
                 --lleft;
                 ++issued;
@@ -543,7 +548,7 @@ extern "C" int ds_tc_linear_few(const int32_t* x, const int32_t* packed, const i
     p.x = x; p.packed = packed; p.bias = bias; p.out = out;
     p.flag = static_cast<int*>(act);
     p.planes = static_cast<unsigned char*>(act) + FEW_HEADER;
-    p.M = M; p.K = K; p.N = N; p.row_len = g.row_len; p.G = g.G; p.wpg = g.wpg; p.kpg = g.kpg;
+    p.M = M; p.K = K; p.N = N; p.row_len = g.row_len; p.G = g.G; p.kpg = g.kpg;
     p.grid_m = g.grid_m; p.grid_n = g.grid_n; p.splits = g.splits; p.gps = g.gps; p.rpt = g.rpt;
     p.units = g.grid_m * g.grid_n * g.splits;
     p.blocks = g.blocks;
@@ -552,8 +557,11 @@ extern "C" int ds_tc_linear_few(const int32_t* x, const int32_t* packed, const i
     if (p.gated && (p.report = workspace_gate_word(fuse)) != nullptr) lock = std::unique_lock<std::mutex>(gate_word_mutex());
     p.zero_out = g.splits > 1 || p.gated;  // the integer path behind may share K as well
     p.wait_ns = tc_wait_ns();
+    p.hold = tc_hold();
     p.err_flag = kernel_error_flag();
     if (!p.err_flag) return DS_ERR_CUDA;
+    p.chk_act = static_cast<const unsigned char*>(act);
+    p.chk_act_bytes = g.act_bytes;
     p.chk_x_bytes = (long long)M * K * 4 - check_shrink_x();
     p.chk_w_bytes = (long long)N * g.row_len * 4;
     p.chk_o_bytes = (long long)M * N * 4;

@@ -74,13 +74,6 @@ struct TcSmem {
     alignas(16) int colc[TcTile<BN, WIDE, SHORT>::EWG][2][BN];
 };
 
-// Checked build: parts of the kernel that ds_tc_debug_waits keeps from doing their work, so that waits run out.
-#ifdef DS_BOUNDS_CHECK
-#define TC_HELD(p, bit) (((p).hold & (bit)) != 0)
-#else
-#define TC_HELD(p, bit) false
-#endif
-
 __device__ __forceinline__ unsigned fdiv(unsigned n, FastDiv d) { return d.mul ? __umulhi(n, d.mul) >> d.sh : n; }
 
 struct Unit {

@@ -170,6 +170,7 @@ int* workspace_gate_word(const ds_fuse_t* fuse);  // null without a workspace
 // Held while the launches of a call with a measured range are enqueued: two threads on one stream share its workspace.
 std::mutex& gate_word_mutex();
 unsigned tc_wait_ns();  // limit of the tensor-core kernels' waits
+int tc_hold();          // checked build: see ds_tc_debug_waits
 
 // `e` (may be null): a kept buffer of expanded weights to look after in the same launch.
 int tc_launch_pack(const TcPack& p, const TcExpand* e, bool wide, cudaStream_t st);

@@ -277,6 +277,7 @@ bool worthwhile(const TcGeom& g, const ds_fuse_t& f)
 }  // namespace
 
 unsigned tc_wait_ns() { return g_wait_ns; }
+int tc_hold() { return g_hold; }
 
 }  // namespace ds
 

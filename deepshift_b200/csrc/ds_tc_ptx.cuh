@@ -15,6 +15,13 @@ constexpr int TC_WAIT_ROUNDS = 1 << 22;    // rounds of one wait, each up to TC_
 constexpr unsigned TC_WAIT_NS = 1000000;   // suspend hint of one round
 constexpr unsigned long long TC_DRAIN_NS = 2000000000ull;  // limit on what a CTA has in flight when it ends
 
+// Checked build: parts of the kernels that ds_tc_debug_waits keeps from doing their work, so that waits run out.
+#ifdef DS_BOUNDS_CHECK
+#define TC_HELD(p, bit) (((p).hold & (bit)) != 0)
+#else
+#define TC_HELD(p, bit) false
+#endif
+
 __device__ __forceinline__ unsigned s32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void bar_init(unsigned long long* b, int count)

@@ -453,7 +453,7 @@ int ds_last_kernel_error(int *flag);
  *                           says whether this library was built with the checks.
  *   ds_bounds_debug_shrink_x  checked build only: declares x `bytes` shorter than it is, so that the
  *                           checks can be seen to fire without anything leaving a real buffer.
- *   ds_tc_debug_waits       checked build only: limit of every wait of the tensor-core kernel, in nanoseconds
+ *   ds_tc_debug_waits       checked build only: limit of every wait of the tensor-core kernels, in nanoseconds
  *                           (at most the normal two seconds; 0 restores them), and what holds still so that
  *                           waits run out: 1 the weight tiles, 2 the activations, 4 the release of finished
  *                           accumulators.  The kernel ends with the flag of ds_last_kernel_error set.
