@@ -82,6 +82,7 @@ _SIGNATURES = {
     "ds_pipe_peak": [_I, _I, ctypes.POINTER(ctypes.c_double), _VP],
     "ds_last_kernel_error": [ctypes.POINTER(ctypes.c_int)],
     "ds_bounds_status": [ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)],
+    "ds_gate_debug_hold": [_VP, _LL, _I],
     "ds_bounds_debug_shrink_x": [_LL],
     "ds_tc_debug_waits": [_LL, _I],
     "ds_unopt_linear_f32": [_VP, _VP, _VP, _VP, _I, _I, _I, _VP],

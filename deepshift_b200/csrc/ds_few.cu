@@ -553,8 +553,8 @@ extern "C" int ds_tc_linear_few(const int32_t* x, const int32_t* packed, const i
     p.units = g.grid_m * g.grid_n * g.splits;
     p.blocks = g.blocks;
     p.gated = mode == 2;
-    std::unique_lock<std::mutex> lock;
-    if (p.gated && (p.report = workspace_gate_word(fuse)) != nullptr) lock = std::unique_lock<std::mutex>(gate_word_mutex());
+    std::optional<GateLock> lock;
+    if (p.gated && (p.report = workspace_gate_word(fuse)) != nullptr) lock.emplace(p.report);
     p.zero_out = g.splits > 1 || p.gated;  // the integer path behind may share K as well
     p.wait_ns = tc_wait_ns();
     p.hold = tc_hold();

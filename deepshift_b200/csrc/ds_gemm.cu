@@ -30,6 +30,9 @@
 //                offsets.  This is the cheap path used by 1x1, 3x3, 5x5 and 7x7 windows.
 #include "ds_tc.cuh"
 
+#include <condition_variable>
+#include <mutex>
+
 namespace ds {
 namespace {
 
@@ -689,10 +692,34 @@ int* workspace_gate_word(const ds_fuse_t* fuse)
                : nullptr;
 }
 
-std::mutex& gate_word_mutex()
+namespace {
+std::mutex g_gates;
+std::condition_variable g_gate_left;
+GateLock* g_gate_holders;  // one per workspace at most; the nodes are the locks themselves
+std::optional<GateLock> g_debug_gate;
+}  // namespace
+
+GateLock::GateLock(const int* word) : word_(word)
 {
-    static std::mutex m;
-    return m;
+    std::unique_lock<std::mutex> l(g_gates);
+    g_gate_left.wait(l, [&] {
+        for (const GateLock* p = g_gate_holders; p; p = p->next_)
+            if (p->word_ == word_) return false;
+        return true;
+    });
+    next_ = g_gate_holders;
+    g_gate_holders = this;
+}
+
+GateLock::~GateLock()
+{
+    {
+        const std::lock_guard<std::mutex> l(g_gates);
+        GateLock** p = &g_gate_holders;
+        while (*p != this) p = &(*p)->next_;
+        *p = next_;
+    }
+    g_gate_left.notify_all();
 }
 
 namespace {
@@ -742,7 +769,7 @@ extern "C" int ds_linear_ex(const void* x, const int32_t* packed, const int32_t*
     if (rc) return rc;
     if (auto_range(fuse, base) && M > 64) {
         // measure the range once, then launch both arithmetic paths gated on the result
-        const std::lock_guard<std::mutex> lock(gate_word_mutex());
+        const GateLock lock(workspace_gate_word(fuse));
         cudaStream_t st = static_cast<cudaStream_t>(stream);
         int* flag = launch_range(x, (long long)M * K, fuse, st);
         if (!flag) return DS_ERR_CUDA;
@@ -833,7 +860,7 @@ int conv2d_run(const void* x, const int32_t* packed, const int32_t* bias, void* 
     p.magic_kh = magic_of(KH);
     if (!prepare && auto_range(fuse, base)) {
         // measure the range once, then launch both arithmetic paths gated on the result
-        const std::lock_guard<std::mutex> lock(gate_word_mutex());
+        const GateLock lock(workspace_gate_word(fuse));
         cudaStream_t st = static_cast<cudaStream_t>(stream);
         int* flag = launch_range(x, (long long)B * C * H * W, fuse, st);
         if (!flag) return DS_ERR_CUDA;
@@ -989,6 +1016,28 @@ extern "C" int ds_conv2d_noalloc(const void* x, const int32_t* packed, const int
     f.workspace = counters;
     f.workspace_bytes = (long long)kNoAllocMaxTiles * (long long)sizeof(int);
     return ds_conv2d_ex(x, packed, bias, out, B, C, H, W, OC, KH, KW, sh, sw, ph, pw, bits, base, &f, stream);
+}
+
+// Checked build only: takes (hold != 0) or gives back the lock of a workspace, as a call does while it enqueues the launches
+// of a measured range, so that a test can watch who waits.  DS_ERR_UNSUPPORTED in a normal build.
+extern "C" int ds_gate_debug_hold(void* workspace, long long workspace_bytes, int hold)
+{
+#ifdef DS_BOUNDS_CHECK
+    ds::g_debug_gate.reset();
+    if (!hold) return DS_OK;
+    ds_fuse_t f = {};
+    f.workspace = workspace;
+    f.workspace_bytes = workspace_bytes;
+    const int* word = ds::workspace_gate_word(&f);
+    if (!word) return DS_ERR_BAD_ARG;
+    ds::g_debug_gate.emplace(word);
+    return DS_OK;
+#else
+    (void)workspace;
+    (void)workspace_bytes;
+    (void)hold;
+    return DS_ERR_UNSUPPORTED;
+#endif
 }
 
 // Checked build only: declares the activations `bytes` shorter than they are for the calls that

@@ -26,7 +26,7 @@
 // so two more products with plane t go into the same sum (r >= 9: coefficients up to 128 as 64 + 64) and four
 // into a second accumulator of weight 2^8 (r <= 8: up to 256 as four times 64).
 #pragma once
-#include <mutex>
+#include <optional>
 
 #include "ds_gemm_common.cuh"
 
@@ -167,8 +167,19 @@ int launch_gated_int(const void* x, const int32_t* packed, const int32_t* bias, 
                      const int* gate, int want, bool zeroed, cudaStream_t st);
 long long check_shrink_x();
 int* workspace_gate_word(const ds_fuse_t* fuse);  // null without a workspace
-// Held while the launches of a call with a measured range are enqueued: two threads on one stream share its workspace.
-std::mutex& gate_word_mutex();
+// Held while the launches of a call with a measured range are enqueued: two threads on one stream share its workspace.  Calls
+// with other workspaces (streams, devices) don't wait for one another.  Allocates nothing: the lock is its own list node.
+class GateLock {
+public:
+    explicit GateLock(const int* word);  // the workspace's gate word
+    ~GateLock();
+    GateLock(const GateLock&) = delete;
+    GateLock& operator=(const GateLock&) = delete;
+
+private:
+    const int* word_;
+    GateLock* next_;
+};
 unsigned tc_wait_ns();  // limit of the tensor-core kernels' waits
 int tc_hold();          // checked build: see ds_tc_debug_waits
 

@@ -452,7 +452,7 @@ int tc_conv2d(const void* x, const ds_planes_t* xp, const int32_t* packed, const
     int* flag = static_cast<int*>(act);
 
     const bool rows = !xp && H == 1 && W == 1 && g.Hp == 1 && g.Wp == 1;  // a matrix: its planes lie group by group
-    std::unique_lock<std::mutex> lock;
+    std::optional<GateLock> lock;
     TcRun p = {};
     int Hp = g.Hp, Wp = g.Wp, step_h = g.sh, step_w = g.sw;
     if (xp) {
@@ -483,7 +483,7 @@ int tc_conv2d(const void* x, const ds_planes_t* xp, const int32_t* packed, const
         if (mode == TC_GATED) {
             p.gate = pk.flag = flag;
             if (!wide) p.report = workspace_gate_word(fuse);  // what DS_ACT_BITS_AUTO promises
-            if (p.report) lock = std::unique_lock<std::mutex>(gate_word_mutex());
+            if (p.report) lock.emplace(p.report);
         }
         if (pk.flag && cudaMemsetAsync(flag, 0, sizeof(int), st) != cudaSuccess) return DS_ERR_CUDA;
         const bool kept = tiles == TILES_FRESH || tiles == TILES_KEPT;

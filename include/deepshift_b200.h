@@ -457,10 +457,13 @@ int ds_last_kernel_error(int *flag);
  *                           (at most the normal two seconds; 0 restores them), and what holds still so that
  *                           waits run out: 1 the weight tiles, 2 the activations, 4 the release of finished
  *                           accumulators.  The kernel ends with the flag of ds_last_kernel_error set.
+ *   ds_gate_debug_hold      checked build only: takes or gives back the lock of a workspace that a call with a measured range
+ *                           holds while it enqueues its launches.
  */
 int ds_bounds_status(int *status, int *checked);
 int ds_bounds_debug_shrink_x(long long bytes);
 int ds_tc_debug_waits(long long limit_ns, int hold);
+int ds_gate_debug_hold(void *workspace, long long workspace_bytes, int hold);
 
 /*
  * Timing build.  The library compiled with -DDS_WS_TIMING (flavour "timing":
