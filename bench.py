@@ -390,14 +390,17 @@ def run_ours(args, rank, world, local):
                 peaks = json.load(fh)
             hbm_peak, hbm_src = float(peaks["hbm_gbs"]), "of measured"
             bf16_peak, bf16_src = float(peaks["bf16_tflops"]), "of measured"
-        peak_s8 = 2 * bf16_peak * 1e12 / 32
+        mhz = clocks.get("sm_max_mhz") or 1965.0
+        peak_s8 = torch.cuda.get_device_properties(dev).multi_processor_count * 8192 * mhz * 1e6 / 16
         roofline = {
             # sixteen u8 x s8 products with int32 accumulation per shift-accumulate (csrc/ds_tc.cuh): the rate of
-            # the 8-bit tensor-core MMA bounds it, twice the bf16 rate
+            # the 8-bit tensor-core MMA bounds it
             "bound": "int8_tensor", "kernel": "3x3 convolutions (%d launches/step)" % dom_n,
             "achieved": achieved / 1e12, "peak": peak_s8 / 1e12, "unit": "Tshift-op/s (1 shift-op = 16 8-bit MACs)",
             "frac": achieved / peak_s8,
-            "peak_note": "2 x the bf16 GEMM rate (%.0f TFLOP/s, %s) / 32" % (bf16_peak, bf16_src),
+            "peak_note": "8192 8-bit MACs per SM and clock (tcgen05 kind::i8) / 16, at %.0f MHz, the maximum; twice the "
+                         "bf16 GEMM rate (%.0f TFLOP/s, %s: under the power limit) / 32 is %.1f"
+                         % (mhz, bf16_peak, bf16_src, 2 * bf16_peak / 32),
             "fma_issue_peak": peak_fma / 1e12, "fma_issue_frac": achieved / peak_fma,
             "int32_alu_peak": peak_alu / 1e12, "int32_alu_frac": achieved / peak_alu,
             "int32_alu_note": "the FFMA.RM and INT32 shift+add issue probes (ds_pipe_peak modes 2 and 0): what the "

@@ -53,11 +53,13 @@ struct FewParams {
     int zero_out;
     unsigned wait_ns;
     int* err_flag;
-    int hold;            // checked build: see ds_tc_debug_waits
     long long chk_x_bytes, chk_w_bytes, chk_o_bytes;
+    int* chk_status;
+#ifdef DS_BOUNDS_CHECK
     const unsigned char* chk_act;  // the whole scratch
     long long chk_act_bytes;
-    int* chk_status;
+    int hold;                      // see ds_tc_debug_waits
+#endif
 };
 
 template <int BN>
@@ -477,7 +479,10 @@ bool few_geometry(FewGeom& g, int M, int K, int N, int bits)
     g.act_bytes = FEW_HEADER + bytes;
     const long long want = ((long long)g.grid_m * g.G * g.BN + 255) / 256;
     g.blocks = int(want > FEW_FLAGS ? FEW_FLAGS : want);
-    // K is shared until the units fill the SMs evenly; an item is 16 weights of 128 columns
+    // K is shared until the units fill the SMs evenly; an item is 16 weights of 128 columns.  The cycles are what a short unit's
+    // items cost beyond its 1500: an item of a long one takes 700 (80 columns) and 880 (144), start and end of the launch 12000
+    // in all.  The choice is what they are for: on 14 shapes (17 to 512 rows, 1024 to 8192 x 512 to 11008) it is within 2 % of
+    // the best of all splits; and with the 10 us of few_worthwhile, the calls that take this path.
     const double item = g.BN == 144 ? 600 : 420;
     g.run_us = 1e30;
     for (int sp = 1; sp <= 64; ++sp) {
@@ -557,15 +562,17 @@ extern "C" int ds_tc_linear_few(const int32_t* x, const int32_t* packed, const i
     if (p.gated && (p.report = workspace_gate_word(fuse)) != nullptr) lock.emplace(p.report);
     p.zero_out = g.splits > 1 || p.gated;  // the integer path behind may share K as well
     p.wait_ns = tc_wait_ns();
-    p.hold = tc_hold();
     p.err_flag = kernel_error_flag();
     if (!p.err_flag) return DS_ERR_CUDA;
-    p.chk_act = static_cast<const unsigned char*>(act);
-    p.chk_act_bytes = g.act_bytes;
     p.chk_x_bytes = (long long)M * K * 4 - check_shrink_x();
     p.chk_w_bytes = (long long)N * g.row_len * 4;
     p.chk_o_bytes = (long long)M * N * 4;
     p.chk_status = bounds_status_ptr();
+#ifdef DS_BOUNDS_CHECK
+    p.chk_act = static_cast<const unsigned char*>(act);
+    p.chk_act_bytes = g.act_bytes;
+    p.hold = tc_hold();
+#endif
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int rc = g.BN == 144 ? few_launch<144>(p, bits + 1, st) : few_launch<80>(p, bits + 1, st);
     if (rc || !p.gated) return rc;

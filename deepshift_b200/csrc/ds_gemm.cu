@@ -696,30 +696,35 @@ namespace {
 std::mutex g_gates;
 std::condition_variable g_gate_left;
 GateLock* g_gate_holders;  // one per workspace at most; the nodes are the locks themselves
+int g_gate_waiters;
 std::optional<GateLock> g_debug_gate;
 }  // namespace
 
 GateLock::GateLock(const int* word) : word_(word)
 {
     std::unique_lock<std::mutex> l(g_gates);
-    g_gate_left.wait(l, [&] {
+    auto held = [&] {
         for (const GateLock* p = g_gate_holders; p; p = p->next_)
-            if (p->word_ == word_) return false;
-        return true;
-    });
+            if (p->word_ == word_) return true;
+        return false;
+    };
+    if (held()) {
+        ++g_gate_waiters;
+        do g_gate_left.wait(l);
+        while (held());
+        --g_gate_waiters;
+    }
     next_ = g_gate_holders;
     g_gate_holders = this;
 }
 
 GateLock::~GateLock()
 {
-    {
-        const std::lock_guard<std::mutex> l(g_gates);
-        GateLock** p = &g_gate_holders;
-        while (*p != this) p = &(*p)->next_;
-        *p = next_;
-    }
-    g_gate_left.notify_all();
+    const std::lock_guard<std::mutex> l(g_gates);
+    GateLock** p = &g_gate_holders;
+    while (*p != this) p = &(*p)->next_;
+    *p = next_;
+    if (g_gate_waiters) g_gate_left.notify_all();
 }
 
 namespace {

@@ -15,7 +15,8 @@
 //                   next         one thread issues the MMAs: 128 x BN x 32 bytes, A from TMEM, B from shared memory.
 //                   last         one thread fetches weight tiles with cp.async.bulk into a ring.
 //                 TMEM: a ring of BN-column accumulator slots, so that the epilogue of a tile overlaps the next tile's
-//                 MMAs, and two A slots per producer warpgroup (sixteen planes x 16 bytes x 128 rows each).
+//                 MMAs, and one A slot per producer warpgroup (sixteen planes x 16 bytes x 128 rows), two up to 64 columns and
+//                 in the two-warpgroup form of 128.
 //
 // What bounds it: the s8 MMA rate, 16 byte-products per shift-accumulate (8192 per SM and clock: 144 T
 // shift-op/s at 1.9 GHz).  A takes N / 2 cycles per MMA from tensor memory, whatever N; from shared memory 40 + N / 8

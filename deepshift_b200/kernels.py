@@ -307,7 +307,7 @@ def linear(input, shift, sign, bias=None, conc_weight=None, use_cuda=True, act_b
     f = _fuse(act_bits=ACT_BITS_AUTO if act_bits is None else act_bits,
               workspace=workspace(input.device) if M > 64 else None)
     with torch.cuda.device(input.device):
-        if _few_asked(M, N * K) and _few_run(input, conc_weight, bias, out, M, K, N, f):
+        if M > 16 and _few_asked(M, N * K) and _few_run(input, conc_weight, bias, out, M, K, N, f):
             return out
         if M > 64 and _tc_run(input, conc_weight, bias, out, (M, K, 1, 1, N, 1, 1, 1, 1, 0, 0), f, False):
             return out
