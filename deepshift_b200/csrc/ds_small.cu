@@ -273,8 +273,8 @@ __global__ void __launch_bounds__(SM_THREADS) small_linear_kernel(const GemmPara
 //   Two and four rows: 4096 x 4096, four 33 -> 37.
 //   Blocks of eight rows: 6 bits where a lane has a whole 16-byte group of words, or rows allow none: 16 rows of 4096 x 4096
 //   107 -> 101, 8 of 4095 x 1000 36.2 -> 33.5, but 16 of 1024 x 1024 35.5 -> 38.2, 8 of 1024 x 4096 63 -> 70.  5 bits, 16 of 4096
-//   x 4096 117 -> 128; 4 bits 106 -> 98, odd K, 5 of 2047 x 2047 37.2 -> 39.7; 1 to 3 bits 8 of 2048 x 2048 53 -> 48 (3).  fp32
-//   input, 16 of 2048 x 2048 142 -> 148.
+//   x 4096 117 -> 128; 4 bits 106 -> 98, odd K, 5 of 2047 x 2047 37.2 -> 39.7; 2 bits 8 of 4096 x 4096 84 -> 80, odd K, 5 of
+//   3247 x 2240 37.7 -> 39.0; 3 bits 8 of 2048 x 2048 53 -> 48.  fp32 input, 16 of 2048 x 2048 142 -> 148.
 template <int MR>
 bool decode_from_bits(const GemmParams& p, int wpc, int vecw)
 {
@@ -288,7 +288,7 @@ bool decode_from_bits(const GemmParams& p, int wpc, int vecw)
     }
     if (f32 || bits == 5) return false;
     if (bits >= 6) return p.K % 4 != 0 || vecw != 4 || p.dec.row_len >= 128 * wpc;
-    return bits != 4 || p.K % 2 == 0;
+    return (bits != 4 && bits != 2) || p.K % 2 == 0;
 }
 
 template <int MR, int CN>
