@@ -658,12 +658,39 @@ struct ExpandSmem {
     alignas(16) unsigned char codes[192 * 16];
 };
 
+// A lane's share of -sum s 2^(15-r) over the weights of channel n.
+template <bool FOLD>
+__device__ __forceinline__ void column_sums(const TcExpand& p, int n, int lane, unsigned& sum, unsigned& first, unsigned& last,
+                                            bool& far)
+{
+    const unsigned fmask = (1u << p.dec.fw) - 1u;
+    const int* src = p.packed + (long long)n * p.dec.row_len;
+    for (int w = lane; w < p.dec.row_len; w += 32) {
+        unsigned word = DS_W_OK(p, src + w, 4) ? unsigned(__ldg(src + w)) : 0u;
+        const int k = w * p.dec.num;
+        int kw = FOLD ? k % p.KW : 1;
+        for (int i = 0; i < p.dec.num && k + i < p.K; ++i, word >>= p.dec.fw) {
+            const int c = tc_code(p, word & fmask);
+            if (c < 32) {
+                if (p.wide) far |= (word & fmask & ((1u << p.dec.bits) - 1u)) >= 16u;
+                const unsigned v = 1u << ((p.wide ? 23 : 15) - (c & 15)), s = (c & 16) ? v : 0u - v;
+                sum += s;
+                if (FOLD && kw == 0) first += s;
+                if (FOLD && kw == 2) last += s;
+            }
+            if (FOLD && ++kw == p.KW) kw = 0;
+        }
+    }
+}
+
 // Block (nt, g): the operand tile of group g, columns nt * BN.. -- [16 planes][BN][16 bytes].  A thread makes
 // four planes of one column: 16 table words (four planes each, sign applied), transposed 4 x 4 bytes.
 // Blocks g = G.. compute the column constants -sum s 2^(15-r).
-__device__ __forceinline__ void expand_block(const TcExpand& p, int nt, int g, ExpandSmem& sm)
+// FOLD apart: as branches it cost the plain form a fifth (4096 x 4096 weights 92 -> 111 us).
+template <bool FOLD>
+__device__ __forceinline__ void expand_form(const TcExpand& p, int nt, int g, ExpandSmem& sm)
 {
-    const int ch = p.BN / p.fold, n0 = nt * ch;
+    const int ch = FOLD ? p.BN / TC_FOLD : p.BN, n0 = nt * ch;
     const unsigned fmask = (1u << p.dec.fw) - 1u;
     if (g >= p.G) {
         // 1, 2, 4 or 8 channels, one per warp
@@ -671,28 +698,12 @@ __device__ __forceinline__ void expand_block(const TcExpand& p, int nt, int g, E
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
         const int n = n0 + (g - p.G) * per + warp;
         if (warp >= per || n >= p.N) return;
-        const int* src = p.packed + (long long)n * p.dec.row_len;
         unsigned sum = 0, first = 0, last = 0;  // folded: those of the window's first and last column apart
         bool far = false;
-        for (int w = lane; w < p.dec.row_len; w += 32) {
-            unsigned word = DS_W_OK(p, src + w, 4) ? unsigned(__ldg(src + w)) : 0u;
-            const int k = w * p.dec.num;
-            int kw = p.fold > 1 ? k % p.KW : 1;
-            for (int i = 0; i < p.dec.num && k + i < p.K; ++i, word >>= p.dec.fw) {
-                const int c = tc_code(p, word & fmask);
-                if (c < 32) {
-                    if (p.wide) far |= (word & fmask & ((1u << p.dec.bits) - 1u)) >= 16u;
-                    const unsigned v = 1u << ((p.wide ? 23 : 15) - (c & 15)), s = (c & 16) ? v : 0u - v;
-                    sum += s;
-                    if (kw == 0) first += s;
-                    if (kw == 2) last += s;
-                }
-                if (p.fold > 1 && ++kw == p.KW) kw = 0;
-            }
-        }
+        column_sums<FOLD>(p, n, lane, sum, first, last, far);
 #pragma unroll
         for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
-        if (p.fold > 1) {
+        if (FOLD) {
 #pragma unroll
             for (int o = 16; o; o >>= 1) {
                 first += __shfl_xor_sync(0xFFFFFFFFu, first, o);
@@ -715,8 +726,9 @@ __device__ __forceinline__ void expand_block(const TcExpand& p, int nt, int g, E
     const int kh = g / p.J, j = g - kh * p.J;
     const int t = 16 * j + (threadIdx.x & 15);  // byte of the window row: (kw, c), or c of a folded window
     const int nl0 = threadIdx.x >> 4;
-    for (int f = 0; f < p.fold; ++f) {
-        const int kw = p.fold > 1 ? f : t / p.Cp, c = p.fold > 1 ? t : t - kw * p.Cp;
+#pragma unroll
+    for (int f = 0; f < (FOLD ? TC_FOLD : 1); ++f) {
+        const int kw = FOLD ? f : t / p.Cp, c = FOLD ? t : t - kw * p.Cp;
         const bool live = kw < p.KW && c < p.C;
         const int k = (c * p.KH + kh) * p.KW + kw;
         const int w = k / p.dec.num, at = (k - w * p.dec.num) * p.dec.fw;
@@ -731,7 +743,7 @@ __device__ __forceinline__ void expand_block(const TcExpand& p, int nt, int g, E
     __syncthreads();
     uint4* out = reinterpret_cast<uint4*>(p.wexp + ((long long)nt * p.G + g) * (p.BN * (p.wide ? TC_PLANES_WIDE : TC_PLANES) * TC_KG));
     for (int i = threadIdx.x; i < p.BN * (p.wide ? 6 : 4); i += 256) {
-        const int q = i / p.BN, n = i - q * p.BN;
+        const int q = i / p.BN, n = FOLD ? i - q * p.BN : i & (p.BN - 1);
         const uint4 cw = *reinterpret_cast<const uint4*>(sm.codes + n * 16);
         const unsigned cws[4] = {cw.x, cw.y, cw.z, cw.w};
         unsigned o[4][4];  // [plane][word]
@@ -748,10 +760,17 @@ __device__ __forceinline__ void expand_block(const TcExpand& p, int nt, int g, E
     }
 }
 
+__device__ __forceinline__ void expand_block(const TcExpand& p, int nt, int g, ExpandSmem& sm)
+{
+    if (p.fold > 1) expand_form<true>(p, nt, g, sm);
+    else expand_form<false>(p, nt, g, sm);
+}
+
+template <bool FOLD>
 __global__ void __launch_bounds__(256) tc_expand_kernel(const TcExpand p)
 {
     __shared__ ExpandSmem sm;
-    expand_block(p, blockIdx.y, blockIdx.x, sm);
+    expand_form<FOLD>(p, blockIdx.y, blockIdx.x, sm);
 }
 
 // Kept buffers.  The tiles stay with the packed words they were made from, and the packing launch of every call looks
@@ -1050,7 +1069,9 @@ int tc_launch_pack(const TcPack& p, const TcExpand* e0, bool wide, cudaStream_t 
 int tc_launch_expand(const TcExpand& p, cudaStream_t st)
 {
     if (p.wide && cudaMemsetAsync(p.colc + p.N, 0, sizeof(int), st) != cudaSuccess) return DS_ERR_CUDA;
-    tc_expand_kernel<<<dim3(unsigned(p.G + TC_COLC_BLOCKS), unsigned(p.total / (p.G + TC_COLC_BLOCKS))), 256, 0, st>>>(p);
+    const dim3 grid(unsigned(p.G + TC_COLC_BLOCKS), unsigned(p.total / (p.G + TC_COLC_BLOCKS)));
+    if (p.fold > 1) tc_expand_kernel<true><<<grid, 256, 0, st>>>(p);
+    else tc_expand_kernel<false><<<grid, 256, 0, st>>>(p);
     note_launch();
     return cudaGetLastError() == cudaSuccess ? DS_OK : DS_ERR_CUDA;
 }
